@@ -168,6 +168,16 @@ rsh_config tuned_config(const rsh_config& base, const rsh_scene* sc) {
     return c;
 }
 
+// per-ray job words and packet stack entries hold an object-node index of level >= 1 in 20 bits; cluster
+// triangles are staged in shared memory (at most 32)
+rsh_status check_batched_scene(const rsh_scene* sc) {
+    if ((sc->h.levels > 1 && sc->h.level_size[1] > (1u << 20)) || sc->h.cluster > 32) {
+        set_error("batched traversal needs at most 1,048,576 level-1 object nodes and clusters of <= 32");
+        return RSH_ERR_INVALID;
+    }
+    return RSH_OK;
+}
+
 rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t count, BatchPlan& pl) {
     if (!ctx || (!segs && count)) return RSH_ERR_INVALID;
     if (count > 1024) {
@@ -263,12 +273,7 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         p.hits = reinterpret_cast<unsigned long long*>(g.hits);
         const rsh_config tc = tuned_config(ctx->cfg, sc);
         RSH_TRY(make_hash_params(sc, tc, 0, p.hp));
-        // per-ray job words and packet stack entries hold an object-node index of level >= 1 in 20 bits;
-        // cluster triangles are staged in shared memory (at most 32)
-        if ((sc->h.levels > 1 && sc->h.level_size[1] > (1u << 20)) || sc->h.cluster > 32) {
-            set_error("batched traversal needs at most 1,048,576 level-1 object nodes and clusters of <= 32");
-            return RSH_ERR_INVALID;
-        }
+        RSH_TRY(check_batched_scene(sc));
         FusedSeg& f = pl.h_fsegs[s];
         std::memset(&f, 0, sizeof(f));
         f.spheres = sc->h.spheres;
@@ -443,7 +448,6 @@ rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
     fa.sorted_ids = static_cast<uint32_t*>(pl.padded);
     fa.segs = static_cast<FusedSeg*>(pl.fsegs);
     fa.nseg = pl.nseg;
-    fa.unit_seg = nullptr;
     fa.units_max = pl.max_padded / pl.unit_rays;
     fa.d_units = totals + 1;
     fa.work = static_cast<uint32_t*>(pl.work);
@@ -469,6 +473,39 @@ struct GraphExec {
 }  // namespace
 
 namespace rsh {
+// The rays of one batch against one scene, each alone from the root of the scene's box tree
+// (k_fused_rays): in the order sorted_ids[0 .. *d_count) (device count; null: n), or in their own order
+// (sorted_ids null). cand_pairs (optional) counts the (ray, cluster) pairs whose triangles were tested.
+rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* sorted_ids, uint32_t n,
+                       const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
+                       unsigned long long* cand_pairs, cudaStream_t s) {
+    if (n == 0 || sc->tri_count == 0) return RSH_OK;
+    void* work;
+    RSH_TRY(ensure(ctx, "b_work", 64, &work));
+    RSH_CUDA(cudaMemsetAsync(work, 0, 16, s));
+    FusedArgs fa{};
+    fa.sorted_ids = sorted_ids;
+    fa.ordered_n = n;
+    fa.d_rays = d_count;
+    fa.one.wtris = sc->h.wtris;
+    fa.one.wnodes = sc->h.wnodes;
+    fa.one.wnroot = sc->h.wnroot;
+    fa.one.levels = sc->h.levels;
+    fa.one.any_hit = any_hit ? 1u : 0u;
+    fa.one.rays = rays;
+    fa.one.flags = flags;
+    fa.one.hits = hits;
+    fa.work = static_cast<uint32_t*>(work);
+    fa.blocks_per_sm = ctx->cfg.fused_blocks;
+    fa.share_tail = (ctx->cfg.flags & RSH_FLAG_SEQUENTIAL_RAYS) ? 0u : 1u;
+    fa.node_tests = ctx->d_stats;
+    fa.tri_tests = ctx->d_stats + 1;
+    fa.cand_pairs = cand_pairs;
+    fa.err = ctx->d_err;
+    RSH_CUDA(launch_rays_one(fa, s));
+    return RSH_OK;
+}
+
 // One segment whose rays are already in a coherent order (the frame's primary rays, generated tile by
 // tile), traced by the rays-only kernel in that order: no hash, compression, sort or ray hierarchy.
 // Scenes whose rays use packets below the root go through batch_trace.
@@ -476,37 +513,12 @@ rsh_status batch_trace_ordered(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaS
     if (!ctx || !seg.scene) return RSH_ERR_INVALID;
     const rsh_config tc = tuned_config(ctx->cfg, seg.scene);
     if (seg.n == 0 || tc.ray_level < seg.scene->h.levels) return batch_trace(ctx, &seg, 1, s, false);
-    BatchPlan pl;
-    RSH_TRY(batch_prepare(ctx, &seg, 1, pl));
-    pl.h_fsegs[0].unit_begin = 0;
-    char* tables = nullptr;
-    cudaEvent_t fence = nullptr;
-    RSH_TRY(stage_tables(ctx, pl, &tables, &fence));
-    RSH_CUDA(cudaMemcpyAsync(pl.fsegs, tables + sizeof(PrepSeg) * pl.nseg, sizeof(FusedSeg), cudaMemcpyHostToDevice,
-                             s));
-    RSH_CUDA(cudaEventRecord(fence, s));
+    RSH_TRY(check_batched_scene(seg.scene));
     if (seg.any_hit) RSH_CUDA(cudaMemsetAsync(seg.flags, 0, 4ull * seg.n, s));
     else RSH_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long*>(seg.hits), RSH_HIT_NONE, seg.n, s));
-    RSH_CUDA(cudaMemsetAsync(pl.work, 0, 16, s));
-    FusedArgs fa{};
-    fa.packet = pl.P;
-    fa.rays = seg.rays;
-    fa.sorted_ids = nullptr;
-    fa.ordered_n = seg.n;
-    fa.segs = static_cast<FusedSeg*>(pl.fsegs);
-    fa.nseg = 1;
-    fa.unit_seg = nullptr;
-    fa.units_max = (seg.n + pl.unit_rays - 1) / pl.unit_rays;
-    fa.d_units = nullptr;
-    fa.work = static_cast<uint32_t*>(pl.work);
-    fa.rays_only = 1;
-    fa.blocks_per_sm = ctx->cfg.fused_blocks;
-    fa.share_tail = (ctx->cfg.flags & RSH_FLAG_SEQUENTIAL_RAYS) ? 0u : 1u;
-    fa.node_tests = ctx->d_stats;
-    fa.tri_tests = ctx->d_stats + 1;
-    fa.err = ctx->d_err;
     ctx->last_stream = s;
-    RSH_CUDA(launch_fused(fa, s));
+    RSH_TRY(trace_alone(ctx, seg.scene, seg.rays, nullptr, seg.n, nullptr, seg.any_hit != 0, seg.flags,
+                        reinterpret_cast<unsigned long long*>(seg.hits), nullptr, s));
     ctx->batch_counts_host.assign(1, seg.n);
     return RSH_OK;
 }

@@ -64,7 +64,7 @@ struct rsh_ctx {
     uint64_t allocated = 0;
     std::map<std::string, rsh::DevBuf> bufs;
     uint32_t* d_err = nullptr;
-    unsigned long long* d_stats = nullptr;   // [0] node tests [1] tri tests [2] candidates [3..] spare
+    unsigned long long* d_stats = nullptr;   // [0] node tests [1] tri tests [STAT_CAND] (ray, cluster) pairs
     uint32_t* h_pinned = nullptr;            // small pinned readback area
     rsh_light lights[8]{};
     uint32_t light_count = 0;
@@ -117,6 +117,14 @@ rsh_status batch_key_layout(rsh_ctx* ctx, const rsh_batch_segment* segments, uin
 // One segment of rays already in a coherent order, traced in that order (rays-only kernel); adds to the
 // test counters.
 rsh_status batch_trace_ordered(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t stream);
+
+// ctx->d_stats word of a frame's (ray, cluster) pairs: past the words a frame zeroes again after its primary
+// rays (the pairs cover them, the test counts do not)
+constexpr uint32_t STAT_CAND = 8;
+// The rays of one batch against one scene, each alone from the root of its box tree (batch.cu).
+rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* sorted_ids, uint32_t n,
+                       const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
+                       unsigned long long* cand_pairs, cudaStream_t s);
 
 // One secondary batch through compress -> sort -> decompress -> build -> traverse -> intersect.
 // keys: per slot (RSH_KEY_NONE = no ray); rays indexed by slot. Output flags/hits indexed by slot

@@ -582,7 +582,11 @@ __global__ void __launch_bounds__(FW * 32, RSH_FUSED_MIN_BLOCKS) k_fused(FusedAr
 // finished takes the next ray of the warp's current unit straight from global memory (its id from the
 // sorted order, the ray itself from the segment's array), fetching the next unit when the current one runs
 // out. So lanes are refilled continuously and no lane waits for the slowest ray of a unit; a lane writes its
-// ray's result (shadow flag or hit record) itself when the ray ends. The launch's last units go out as
+// ray's result (shadow flag or hit record) itself when the ray ends. The stack's top entry lives in a register:
+// most node steps hit one child, which is then the next step without a store to and a load from local memory
+// in between (frames 2.8-3.9% faster: the architecture frame 3.79 ms against 3.90, the soup frame 3.34 against
+// 3.47; loading a plane of eight children with one 32-byte load instead of two 16-byte ones took 4.17 ms at this
+// register limit and 3.96 ms without spills at 6 CTAs per SM). The launch's last units go out as
 // pieces of RSH_RAYS_UNIT / RSH_TAIL_SPLIT rays. Single long rays (up to 20x the median ray's tests) still
 // hold an SM after the others have finished; the SHARE instance (the default) lets a drained warp's idle
 // lanes take their subtrees (described at its loop's top), at the price of about 4% on every step, which
@@ -660,28 +664,40 @@ RSH_DEV void slab4(float4 px, float4 py, float4 pz, float ix, float iy, float iz
 #define RSH_TAIL_SPLIT 2
 #endif
 
-template <int U, bool SHARE>
-__global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(FusedArgs a) {
+// Which segments a launch of the rays-only kernel traces, known at compile time where it can be:
+//   SEGS  the batch's segment table, closest- and any-hit segments mixed;
+//   ANY1 / CLOSEST1  one segment of one kind, read from the kernel's own arguments: the scene, the output and
+//     the kind are launch constants, not per-lane state (6 registers fewer), and no table is uploaded.
+enum RaysOf { SEGS = 0, ANY1 = 1, CLOSEST1 = 2 };
+
+template <int U, bool SHARE, int OF>
+__global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(const __grid_constant__ FusedArgs a) {
+    constexpr bool ONE = OF != SEGS;
     // SHARE: a drained warp's rays shared among its idle lanes; the records of the rays being shared, one per
     // lane: the owner's best hit key (closest hit), occluded (any hit), helpers still on a subtree of it
     __shared__ unsigned long long sh_best[SHARE ? FW : 1][32];
     __shared__ uint32_t sh_occ[SHARE ? FW : 1][32], sh_pend[SHARE ? FW : 1][32];
     const uint32_t lane = lane_id();
-    const uint32_t units = dev_count(a.d_units, a.units_max);
+    const uint32_t nrays = ONE ? dev_count(a.d_rays, a.ordered_n) : 0u;
+    const uint32_t units = ONE ? (nrays + U - 1u) / U : dev_count(a.d_units, a.units_max);
     const uint32_t tail = min(units, (uint32_t)RSH_TAIL_PER_WARP * gridDim.x * FW);
     const uint32_t head = units - tail, tickets = head + RSH_TAIL_SPLIT * tail;
     uint32_t ntests = 0, ttests = 0;  // the lane's counts, flushed to the launch's counters before 2^31
+    uint32_t ncand = 0;               // ONE: clusters whose triangles the lane tested
     // the warp's current unit: sorted rays [nk, nend) of segment cs
     uint32_t nk = 0, nend = 0, cs = 0;
     bool drained = false;
     // the lane's ray
-    bool has = false, any = false;
+    bool has = false, any_v = false;
     uint32_t seg = 0, slot = 0;
-    const float4* __restrict__ nodes = nullptr;
-    const float4* __restrict__ tris = nullptr;
+    const float4* nodes_v = nullptr;
+    const float4* tris_v = nullptr;
+    // the stack: its top entry in registers (a step's first child is the next step, with no trip through local
+    // memory), the entries below it in local memory
+    uint32_t top = 0u;
     int sp = 0;
     uint32_t stk[J_STACK];
-    float stt[J_STACK];  // closest hit: each entry's entry distance, from its parent's test
+    float stt[OF == ANY1 ? 1 : J_STACK];  // closest hit: each entry's entry distance, from its parent's test
     float ox = 0.f, oy = 0.f, oz = 0.f, tmin = 0.f, tcur = 0.f;
     float ix = 0.f, iy = 0.f, iz = 0.f, oix = 0.f, oiy = 0.f, oiz = 0.f;
     uint32_t oct = 0;  // the direction's octant: bit a set when component a is negative
@@ -690,22 +706,45 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
     bool sharing = false;  // warp-uniform (SHARE): the warp shares its last rays
     bool done = false;     // sharing: the lane's subtree is done, its result not yet merged
     uint32_t own = lane;   // sharing: the lane whose ray this lane works on
+    auto any_of = [&]() -> bool { return OF == ANY1 ? true : OF == CLOSEST1 ? false : any_v; };
+    auto seg_of = [&](uint32_t i) -> const FusedSeg& { return ONE ? a.one : a.segs[i]; };
     // the ray is done: its result, written by its own lane (while sharing: merged at the loop's top)
     auto finish = [&]() {
+        has = false;
         if (SHARE && sharing) {
             done = true;
-            has = false;
             return;
         }
-        const FusedSeg& sg = a.segs[seg];
-        if (any) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
+        const FusedSeg& sg = seg_of(seg);
+        if (any_of()) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
         else sg.hits[slot] = best;
-        has = false;
         // one ray adds fewer than 2^28 node tests (8 per slot) and 2^24 triangle tests
         if ((ntests | ttests) >> 31) {
             if (a.node_tests) atomicAdd(a.node_tests, (unsigned long long)ntests);
             if (a.tri_tests) atomicAdd(a.tri_tests, (unsigned long long)ttests);
-            ntests = ttests = 0;
+            if (ONE && a.cand_pairs) atomicAdd(a.cand_pairs, (unsigned long long)ncand);
+            ntests = ttests = ncand = 0;
+        }
+    };
+    // the next entry of the lane's stack into `top`; closest hit: entries that the ray enters beyond its
+    // current best are dropped unread (their subtrees cannot hold a nearer hit: a child's box lies inside its
+    // parent's, so no child is entered before its parent). Finishes the ray when nothing is left.
+    auto pop = [&]() {
+        if (any_of()) {
+            if (sp == 0) finish();
+            else top = stk[--sp];
+        } else {
+            for (;;) {
+                if (sp == 0) {
+                    finish();
+                    break;
+                }
+                --sp;
+                if (!(stt[sp] > tcur)) {
+                    top = stk[sp];
+                    break;
+                }
+            }
         }
     };
     for (;;) {
@@ -731,27 +770,38 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                 }
                 nk = u * U + lo;
                 nend = u * U + hi;
-                cs = find_segment(a.segs, a.nseg, u);
+                if (!ONE) cs = find_segment(a.segs, a.nseg, u);
             }
             const uint32_t k = nk + __popc(need & lanemask_lt());
             if (!has && k < nend) {
-                // no sorted order: the rays' own order, padded past ordered_n
-                const uint32_t id = a.sorted_ids ? __ldg(a.sorted_ids + k) : (k < a.ordered_n ? k : INVALID_ID);
+                // ONE: the first nrays sorted slots, or the rays in their own order; SEGS: the padded layout, whose
+                // padding slots hold INVALID_ID
+                uint32_t id = INVALID_ID;
+                if (ONE) {
+                    if (k < nrays) id = a.sorted_ids ? __ldg(a.sorted_ids + k) : k;
+                    if (id >= a.ordered_n) id = INVALID_ID;
+                } else {
+                    id = __ldg(a.sorted_ids + k);
+                }
                 if (id != INVALID_ID) {
-                    const FusedSeg& sg = a.segs[cs];
+                    const FusedSeg& sg = seg_of(cs);
+                    if (!ONE) id -= sg.slot_base;
                     float4 o, d;
-                    load_ray(sg.rays, id - sg.slot_base, o, d);
+                    load_ray(sg.rays, id, o, d);
                     if (d.w > o.w) {
+                        const bool sany = OF == ANY1 ? true : OF == CLOSEST1 ? false : sg.any_hit != 0u;
                         if (sg.levels == 0u) {
                             // a scene without triangles has no tree: the ray misses
-                            if (sg.any_hit) sg.flags[id - sg.slot_base] = 0u;
-                            else sg.hits[id - sg.slot_base] = RSH_HIT_NONE;
+                            if (sany) sg.flags[id] = 0u;
+                            else sg.hits[id] = RSH_HIT_NONE;
                         } else {
-                            seg = cs;
-                            slot = id - sg.slot_base;
-                            any = sg.any_hit != 0u;
-                            nodes = sg.wnodes;
-                            tris = sg.wtris;
+                            slot = id;
+                            if (!ONE) {
+                                seg = cs;
+                                any_v = sany;
+                                nodes_v = sg.wnodes;
+                                tris_v = sg.wtris;
+                            }
                             ox = o.x;
                             oy = o.y;
                             oz = o.z;
@@ -766,9 +816,8 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                             w = wt_setup(o, d);
                             best = RSH_HIT_NONE;
                             oct = (ix < 0.f ? 1u : 0u) | (iy < 0.f ? 2u : 0u) | (iz < 0.f ? 4u : 0u);
-                            stk[0] = sg.wnroot;
-                            stt[0] = -INFINITY;
-                            sp = 1;
+                            top = sg.wnroot;
+                            sp = 0;
                             has = true;
                         }
                     }
@@ -785,6 +834,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
         // happens here, between steps: the steps themselves are the sequential ones.
         if (SHARE && drained && (sharing || __popc(__ballot_sync(0xffffffffu, has)) <= RSH_SHARE_BUSY)) {
             const uint32_t wp = threadIdx.x >> 5;
+            const bool any = any_of();
             if (!sharing) {
                 sh_best[wp][lane] = has ? best : RSH_HIT_NONE;
                 sh_occ[wp][lane] = 0u;
@@ -796,7 +846,6 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
             if (has) {
                 if (any) {
                     if (sh_occ[wp][own]) {
-                        sp = 0;
                         done = true;
                         has = false;
                     }
@@ -808,7 +857,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                 // the owner, with no helper left: the ray's merged result
                 if (any) best = (best == 0ull || sh_occ[wp][lane]) ? 0ull : best;
                 else best = min(best, sh_best[wp][lane]);
-                const FusedSeg& sg = a.segs[seg];
+                const FusedSeg& sg = seg_of(seg);
                 if (any) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
                 else sg.hits[slot] = best;
                 done = false;
@@ -824,29 +873,25 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
             }
             __syncwarp();
             const uint32_t idle = __ballot_sync(0xffffffffu, !has && !done);
-            const uint32_t donors = __ballot_sync(0xffffffffu, has && sp >= 2);
+            const uint32_t donors = __ballot_sync(0xffffffffu, has && sp >= 1);
             if (idle && donors) {
                 const uint32_t r = __popc(idle & lanemask_lt());
                 const bool recv = !has && !done && r < (uint32_t)__popc(donors);
                 const uint32_t src = recv ? __fns(donors, 0u, (int)r + 1) : lane;
-                const bool give = has && sp >= 2 && (uint32_t)__popc(donors & lanemask_lt()) < (uint32_t)__popc(idle);
-                uint32_t ge = 0u;
-                float gt = 0.0f;
-                if (give) {
-                    --sp;
-                    ge = stk[sp];
-                    gt = stt[sp];
-                }
+                const bool give = has && sp >= 1 && (uint32_t)__popc(donors & lanemask_lt()) < (uint32_t)__popc(idle);
+                uint32_t ge = 0u;  // the donor's second entry; it goes on with its top
+                if (give) ge = stk[--sp];
                 ge = __shfl_sync(0xffffffffu, ge, src);
-                gt = __shfl_sync(0xffffffffu, gt, src);
                 const uint32_t go = __shfl_sync(0xffffffffu, own, src);
-                any = __shfl_sync(0xffffffffu, any, src);
-                seg = __shfl_sync(0xffffffffu, seg, src);
+                if (!ONE) {
+                    any_v = __shfl_sync(0xffffffffu, any_v, src);
+                    seg = __shfl_sync(0xffffffffu, seg, src);
+                    nodes_v = reinterpret_cast<const float4*>(
+                        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(nodes_v), src));
+                    tris_v = reinterpret_cast<const float4*>(
+                        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(tris_v), src));
+                }
                 slot = __shfl_sync(0xffffffffu, slot, src);
-                nodes = reinterpret_cast<const float4*>(
-                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(nodes), src));
-                tris = reinterpret_cast<const float4*>(
-                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(tris), src));
                 tmin = __shfl_sync(0xffffffffu, tmin, src);
                 tcur = __shfl_sync(0xffffffffu, tcur, src);
                 ix = __shfl_sync(0xffffffffu, ix, src);
@@ -869,9 +914,8 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                 w.tmax = __shfl_sync(0xffffffffu, w.tmax, src);
                 if (recv) {
                     own = go;
-                    stk[0] = ge;
-                    stt[0] = gt;
-                    sp = 1;
+                    top = ge;
+                    sp = 0;
                     best = RSH_HIT_NONE;
                     has = true;
                     atomicAdd(&sh_pend[wp][own], 1u);
@@ -879,27 +923,24 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
             }
             __syncwarp();
         }
-        // closest hit: entries that the ray enters beyond its current best are dropped unread (their
-        // subtrees cannot hold a nearer hit: a child's box lies inside its parent's, so no child is entered
-        // before its parent)
-        if (has && !any) {
-            while (sp > 0 && stt[sp - 1] > tcur) --sp;
-            if (sp == 0) finish();
-        }
         // one kind of step per iteration, the kind more lanes want
         bool do_nodes;
         {
-            const bool node = has && (stk[sp - 1] >> 31) != 0u;
+            const bool node = has && (top >> 31) != 0u;
             const uint32_t nn = __popc(__ballot_sync(0xffffffffu, node));
             const uint32_t nc = __popc(__ballot_sync(0xffffffffu, has && !node));
             do_nodes = nn >= nc;
         }
-        if (has && ((stk[sp - 1] >> 31) != 0u) == do_nodes) {
-            const uint32_t e = stk[--sp];
+        if (has && ((top >> 31) != 0u) == do_nodes) {
+            const bool any = any_of();
+            const uint32_t e = top;
             if (!(e >> 31)) {
                 // a cluster: its triangles t0 .. t0 + count - 1 (its box was tested with the parent's
                 // children; a closest-hit ray re-checks only its entry distance, above)
+                const float4* __restrict__ tris = ONE ? a.one.wtris : tris_v;
                 const uint32_t t0 = e & 0x7FFFFFu, t1 = t0 + ((e >> 23) & 63u) + 1u;
+                if (ONE) ++ncand;
+                bool occluded = false;
                 for (uint32_t tt = t0; tt < t1; ++tt) {
                     const float4 v0 = __ldg(tris + 3ull * tt), v1 = __ldg(tris + 3ull * tt + 1),
                                  v2 = __ldg(tris + 3ull * tt + 2);
@@ -907,8 +948,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                     ++ttests;
                     if (wt_hit(w, v0, v1, v2, th)) {
                         if (any) {
-                            best = 0ull;  // occluded
-                            sp = 0;
+                            occluded = true;
                             break;
                         }
                         const unsigned long long key = hit_key(th, __float_as_uint(v0.w));
@@ -918,18 +958,27 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                         }
                     }
                 }
+                if (any && occluded) {
+                    best = 0ull;
+                    sp = 0;
+                    finish();
+                } else {
+                    pop();
+                }
             } else {
                 // a node record: the children's near planes and far planes, axis by axis, then their entries
+                const float4* __restrict__ nodes = ONE ? a.one.wnodes : nodes_v;
                 const uint32_t cnt = ((e >> 28) & 7u) + 1u;
                 const float4* rec = nodes + REC_F4 * (size_t)(e & 0x0FFFFFFFu);
                 ntests += cnt;
                 if (sp + cnt > J_STACK) {
                     raise_device_error(a.err, RSH_DEVERR_OVERFLOW);
+                    pop();
                 } else {
                     const uint32_t nxo = (oct & 1u) << 1, nyo = 4u | (oct & 2u), nzo = 8u | ((oct >> 1) & 2u);
                     float tn[8];
                     uint32_t hm = 0;
-#pragma unroll
+                    #pragma unroll
                     for (uint32_t h = 0; h < 2; ++h) {
                         float n4[4], f4[4];
                         slab4(__ldg(rec + nxo + h), __ldg(rec + nyo + h), __ldg(rec + nzo + h), ix, iy, iz, oix,
@@ -943,23 +992,23 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                         }
                     }
                     const uint32_t* ent = reinterpret_cast<const uint32_t*>(rec + 12);
-                    if (any) {
-                        // any hit: every child whose box the ray crosses is pushed in child order (the last
-                        // pops first)
-#pragma unroll
-                        for (uint32_t h = 0; h < 2; ++h) {
-                            if ((hm >> (4 * h)) & 15u) {
-                                const uint4 ee = __ldg(reinterpret_cast<const uint4*>(ent) + h);
-                                const uint32_t ce[4] = {ee.x, ee.y, ee.z, ee.w};
-#pragma unroll
-                                for (uint32_t k = 0; k < 4; ++k)
-                                    if ((hm >> (4 * h + k)) & 1u) stk[sp++] = ce[k];
-                            }
+                    if (hm == 0u) {
+                        pop();
+                    } else if (any) {
+                        // any hit: the last child whose box the ray crosses is next, the others are pushed in
+                        // child order (the last pops first)
+                        const uint32_t last = 31u - (uint32_t)__clz(hm);
+                        top = __ldg(ent + last);  // an L1 hit: the record was just read
+                        hm &= ~(1u << last);
+                        while (hm) {
+                            const uint32_t c = __ffs(hm) - 1u;
+                            hm &= hm - 1u;
+                            stk[sp++] = __ldg(ent + c);
                         }
                     } else {
-                        // closest hit: the hits pushed farthest first, so that the nearest pops first (among
-                        // equal entry distances the lower child)
-                        while (hm) {
+                        // closest hit: the hits in order farthest first, the nearest is next (among equal entry
+                        // distances the lower child)
+                        for (;;) {
                             uint32_t bc = 0;
                             float bt = -INFINITY;
 #pragma unroll
@@ -969,50 +1018,56 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(Fus
                                     bc = c;
                                 }
                             hm &= ~(1u << bc);
-                            stk[sp] = __ldg(ent + bc);  // an L1 hit: the record was just read
+                            const uint32_t ce = __ldg(ent + bc);
+                            if (hm == 0u) {
+                                top = ce;
+                                break;
+                            }
+                            stk[sp] = ce;
                             stt[sp++] = bt;
                         }
                     }
                 }
             }
-            if (sp == 0) finish();
         }
     }
-    unsigned long long nt = ntests, tt = ttests;
+    unsigned long long nt = ntests, tt = ttests, nc = ncand;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         nt += __shfl_xor_sync(0xffffffffu, nt, d);
         tt += __shfl_xor_sync(0xffffffffu, tt, d);
+        if (ONE) nc += __shfl_xor_sync(0xffffffffu, nc, d);
     }
     if (lane == 0) {
         if (a.node_tests) atomicAdd(a.node_tests, nt);
         if (a.tri_tests) atomicAdd(a.tri_tests, tt);
+        if (ONE && a.cand_pairs) atomicAdd(a.cand_pairs, nc);
     }
 }
 
-template <int U, bool SHARE>
+template <int U, bool SHARE, int OF>
 static cudaError_t launch_fused_rays_s(const FusedArgs& a, cudaStream_t s) {
     int dev = 0, sms = 152, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_rays<U, SHARE>, FW * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_rays<U, SHARE, OF>, FW * 32, 0);
     if (per_sm < 1) per_sm = 1;
     if (a.blocks_per_sm && (int)a.blocks_per_sm < per_sm) per_sm = (int)a.blocks_per_sm;
     uint32_t grid = (uint32_t)(sms * per_sm);
     const uint32_t need = (a.units_max + FW - 1) / FW;
     if (need < grid) grid = need > 0 ? need : 1;
-    k_fused_rays<U, SHARE><<<grid, FW * 32, 0, s>>>(a);
+    k_fused_rays<U, SHARE, OF><<<grid, FW * 32, 0, s>>>(a);
     note_launch();
     return cudaGetLastError();
 }
-template <int U>
+template <int U, int OF>
 static cudaError_t launch_fused_rays_u(const FusedArgs& a, cudaStream_t s) {
-    return a.share_tail ? launch_fused_rays_s<U, true>(a, s) : launch_fused_rays_s<U, false>(a, s);
+    return a.share_tail ? launch_fused_rays_s<U, true, OF>(a, s) : launch_fused_rays_s<U, false, OF>(a, s);
 }
 
 template <int P>
 static cudaError_t launch_fused_p(const FusedArgs& a, cudaStream_t s) {
-    if (a.rays_only) return launch_fused_rays_u<RSH_RAYS_UNIT>(a, s);  // units of RSH_RAYS_UNIT rays
+    if (a.rays_only) return launch_fused_rays_u<RSH_RAYS_UNIT, SEGS>(a, s);  // units of RSH_RAYS_UNIT rays
     const size_t smem = sizeof(FusedSmem<P>) * FW;
     cudaError_t e = cudaFuncSetAttribute(k_fused<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1028,6 +1083,13 @@ static cudaError_t launch_fused_p(const FusedArgs& a, cudaStream_t s) {
     k_fused<P><<<grid, FW * 32, smem, s>>>(a);
     note_launch();
     return cudaGetLastError();
+}
+
+cudaError_t launch_rays_one(FusedArgs a, cudaStream_t s) {
+    if (a.ordered_n == 0) return cudaSuccess;
+    a.units_max = (a.ordered_n + RSH_RAYS_UNIT - 1) / RSH_RAYS_UNIT;
+    return a.one.any_hit ? launch_fused_rays_u<RSH_RAYS_UNIT, ANY1>(a, s)
+                         : launch_fused_rays_u<RSH_RAYS_UNIT, CLOSEST1>(a, s);
 }
 
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t s) {

@@ -230,11 +230,9 @@ struct FusedArgs {
     uint32_t node_off[4];
     uint32_t packet;
     const rsh_ray* rays;
-    const uint32_t* sorted_ids;    // null (rays-only kernel): rays in their own order, ordered_n of them
-    uint32_t ordered_n;
+    const uint32_t* sorted_ids;    // launch_rays_one: may be null (the rays in their own order)
     const FusedSeg* segs;          // device
     uint32_t nseg;
-    const uint32_t* unit_seg;      // device: work unit -> segment (size = units)
     uint32_t units_max;
     const uint32_t* d_units;       // device count of units
     uint32_t* work;
@@ -244,8 +242,16 @@ struct FusedArgs {
     unsigned long long* node_tests;
     unsigned long long* tri_tests;
     uint32_t* err;
+    // launch_rays_one: the one segment (slot_base 0), its ray slots, the device count of sorted_ids entries (null:
+    // ordered_n) and, if wanted, the count of (ray, cluster) pairs whose triangles were tested
+    FusedSeg one;
+    uint32_t ordered_n;
+    const uint32_t* d_rays;
+    unsigned long long* cand_pairs;
 };
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t s);
+// The rays of one segment alone from the root (no packets, no segment table).
+cudaError_t launch_rays_one(FusedArgs a, cudaStream_t s);
 // rays per work unit of the rays-only kernel (a multiple of 64, at most 256: job words hold 8 bits)
 #ifndef RSH_RAYS_UNIT
 #define RSH_RAYS_UNIT 64
