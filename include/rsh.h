@@ -138,15 +138,18 @@ typedef struct rsh_config {
     uint32_t cluster_size;     /* most triangles per object-hierarchy leaf: 1..64 (default 6; batched form <= 32) */
     float epsilon;             /* ray offset (default 0.01; RayTracer.cu:34) */
     uint64_t hbm_budget;       /* bytes the context may allocate (0: 90% of free memory) */
-    uint64_t candidate_capacity; /* plain-path traversal candidates per pass (0: automatic) */
+    uint64_t candidate_capacity; /* plain-path packet candidates per pass (0: automatic; packets only) */
     uint32_t flags;            /* RSH_FLAG_* */
     float reflect_jitter;      /* 0: mirror reflections; >0: cosine-lobe perturbation weight */
     uint32_t seed;             /* seed of the reflection perturbation */
     uint32_t ray_level;        /* batched form: object-tree level at and below which rays leave their packet
                                   and descend one by one (0: packets down to the clusters; at or above the tree depth:
                                   from the root, no packet phase, no ray hierarchy; default 15) */
-    uint32_t plain_ray_level;  /* plain per-frame path: object-tree level at and below which the traversal
-                                  emits per-ray candidates (0: packet candidates only; default 4) */
+    uint32_t plain_ray_level;  /* plain per-frame path. 0: packets of the ray hierarchy down to the triangle
+                                  clusters, as candidates. 1..15 (default 4): rays alone, from the root of the
+                                  scene's box tree, no ray hierarchy and no candidate buffer; a packet walk
+                                  above single rays is slower than this at every level between, so the values
+                                  1..15 trace alike */
     uint32_t fused_blocks;     /* batched form: CTAs of the persistent traversal launch per SM (0: as many
                                   as fit, the default; fewer share each SM's L1 among fewer rays) */
 } rsh_config;
@@ -179,7 +182,8 @@ typedef struct rsh_frame_stats {
     uint64_t shadow_rays;        /* traced after trimming, all bounces */
     uint64_t reflection_rays;    /* traced after trimming, all bounces */
     uint64_t chunks;             /* compressed runs, all secondary batches */
-    uint64_t candidates;         /* (packet, cluster) pairs emitted by traversal */
+    uint64_t candidates;         /* plain path: (packet, cluster) pairs emitted by the packet traversal, or the
+                                    (ray, cluster) pairs whose triangles a ray alone tested */
     uint64_t node_tests;         /* node tests executed (packet-node x sphere; a single ray x node box);
                                     rsh_render_frame: secondary rays only */
     uint64_t tri_tests;          /* ray x triangle tests executed (rsh_render_frame: secondary rays only) */

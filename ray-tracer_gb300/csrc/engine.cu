@@ -142,9 +142,6 @@ static rsh_status traverse_and_intersect(rsh_ctx* ctx, const rsh_scene* sc, cons
     ta.capacity = cap;
     ta.cand_count = cc;
     ta.work = w;
-    ta.ray_level = ctx->cfg.plain_ray_level;
-    ta.rays = rays;
-    ta.sorted_ids = sorted_ids;
     ta.node_tests = ctx->d_stats + 0;
     ta.err = ctx->d_err;
     IsectArgs ia{};
@@ -164,7 +161,6 @@ static rsh_status traverse_and_intersect(rsh_ctx* ctx, const rsh_scene* sc, cons
     ia.flags = flags;
     ia.hits = hits;
     ia.tri_tests = ctx->d_stats + 1;
-    ia.per_ray = ctx->cfg.plain_ray_level > 0 ? 1u : 0u;
     // Passes over a window of work units [start, start + window). Without overflow the first pass covers
     // every unit. After an overflow the window restarts at the first unfinished unit; if a pass made no
     // progress the window shrinks (units of one pass race for the buffer), down to a single unit, which
@@ -206,12 +202,28 @@ static rsh_status traverse_and_intersect(rsh_ctx* ctx, const rsh_scene* sc, cons
     return RSH_OK;
 }
 
+// Rays that leave their packets (plain_ray_level >= 1) go down the scene's box tree one by one, testing
+// triangles as they meet them, so hits end or shorten a ray's walk at once: no ray hierarchy, no candidates.
+// (A packet walk above the switch level with every cluster along a ray written out as a candidate and
+// tested afterwards took 218 + 26 ms of the architecture frame's 232 ms, and at no switch level was a packet
+// walk above single rays faster than single rays from the root: 12.6-60 ms against 3.9 a frame.)
+static rsh_status trace_rays_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* sorted_ids,
+                                   uint32_t n, const uint32_t* d_count, bool any_hit, uint32_t* flags,
+                                   unsigned long long* hits, cudaStream_t s) {
+    const int th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
+    const rsh_status st = trace_alone(ctx, sc, rays, sorted_ids, n, d_count, any_hit, flags, hits,
+                                      ctx->d_stats + STAT_CAND, s);
+    stage_end(ctx, th, s);
+    return st;
+}
+
 rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* keys,
                        uint32_t n_slots, uint32_t key_bits, bool any_hit, uint32_t* flags,
                        unsigned long long* hits, uint32_t* counts_out, cudaStream_t s) {
     if (n_slots == 0) return RSH_OK;
     const uint32_t P = ctx->cfg.packet_size;
-    void *trimmed, *ckeys, *cbases, *counts, *skeys, *svals, *sorted_keys, *sorted_ids, *nodes, *scr;
+    const bool packets = ctx->cfg.plain_ray_level == 0;
+    void *trimmed, *ckeys, *cbases, *counts, *skeys, *svals, *sorted_keys, *sorted_ids, *nodes = nullptr, *scr;
     RSH_TRY(ensure(ctx, "trimmed", 4ull * n_slots, &trimmed));
     RSH_TRY(ensure(ctx, "ckeys", 4ull * n_slots + 4, &ckeys));
     RSH_TRY(ensure(ctx, "cbases", 4ull * n_slots + 4, &cbases));
@@ -220,9 +232,11 @@ rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, c
     RSH_TRY(ensure(ctx, "svals", 4ull * n_slots, &svals));
     RSH_TRY(ensure(ctx, "sorted_keys", 4ull * n_slots, &sorted_keys));
     RSH_TRY(ensure(ctx, "sorted_ids", 4ull * n_slots, &sorted_ids));
-    uint32_t off[4];
-    const uint32_t cap_nodes = hierarchy_capacity(n_slots, P, off);
-    RSH_TRY(ensure(ctx, "nodes", sizeof(rsh_node) * (size_t)cap_nodes, &nodes));
+    if (packets) {
+        uint32_t off[4];
+        const uint32_t cap_nodes = hierarchy_capacity(n_slots, P, off);
+        RSH_TRY(ensure(ctx, "nodes", sizeof(rsh_node) * (size_t)cap_nodes, &nodes));
+    }
     size_t scr_bytes = compress_scratch_bytes(n_slots);
     scr_bytes = std::max(scr_bytes, sort_scratch_bytes(n_slots, key_bits));
     scr_bytes = std::max(scr_bytes, decompress_scratch_bytes(n_slots));
@@ -232,36 +246,32 @@ rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, c
     RSH_CUDA(launch_compress(keys, n_slots, static_cast<uint32_t*>(trimmed), static_cast<uint32_t*>(ckeys),
                              static_cast<uint32_t*>(cbases), cnt, scr, ctx->d_err, s));
     stage_end(ctx, th, s);
-    if (ctx->cfg.flags & RSH_FLAG_RAH) {
-        // ablation: no sort, packets of consecutive trimmed rays (the reference's RAH path)
-        th = stage_begin(ctx, RSH_STAGE_BUILD, s);
-        RSH_CUDA(launch_build_rsh(rays, static_cast<uint32_t*>(trimmed), n_slots, cnt, P,
-                                  static_cast<rsh_node*>(nodes), s));
+    // ablation (RSH_FLAG_RAH): no sort, the trimmed rays in slot order (the reference's RAH path)
+    uint32_t* order = static_cast<uint32_t*>(trimmed);
+    if (!(ctx->cfg.flags & RSH_FLAG_RAH)) {
+        order = static_cast<uint32_t*>(sorted_ids);
+        th = stage_begin(ctx, RSH_STAGE_SORT, s);
+        RSH_CUDA(launch_sort_pairs(static_cast<uint32_t*>(ckeys), nullptr, static_cast<uint32_t*>(skeys),
+                                   static_cast<uint32_t*>(svals), n_slots, cnt + 1, key_bits, scr, ctx->d_err, s));
         stage_end(ctx, th, s);
-        return traverse_and_intersect(ctx, sc, static_cast<rsh_node*>(nodes), rays,
-                                      static_cast<uint32_t*>(trimmed), n_slots, cnt, any_hit, flags, hits, s);
+        th = stage_begin(ctx, RSH_STAGE_DECOMPRESS, s);
+        RSH_CUDA(launch_decompress(static_cast<uint32_t*>(skeys), static_cast<uint32_t*>(svals),
+                                   static_cast<uint32_t*>(cbases), static_cast<uint32_t*>(trimmed), cnt,
+                                   n_slots, static_cast<uint32_t*>(sorted_keys), order, scr, ctx->d_err, s));
+        stage_end(ctx, th, s);
     }
-    th = stage_begin(ctx, RSH_STAGE_SORT, s);
-    RSH_CUDA(launch_sort_pairs(static_cast<uint32_t*>(ckeys), nullptr, static_cast<uint32_t*>(skeys),
-                               static_cast<uint32_t*>(svals), n_slots, cnt + 1, key_bits, scr, ctx->d_err, s));
-    stage_end(ctx, th, s);
-    th = stage_begin(ctx, RSH_STAGE_DECOMPRESS, s);
-    RSH_CUDA(launch_decompress(static_cast<uint32_t*>(skeys), static_cast<uint32_t*>(svals),
-                               static_cast<uint32_t*>(cbases), static_cast<uint32_t*>(trimmed), cnt,
-                               n_slots, static_cast<uint32_t*>(sorted_keys),
-                               static_cast<uint32_t*>(sorted_ids), scr, ctx->d_err, s));
-    stage_end(ctx, th, s);
+    if (!packets) return trace_rays_alone(ctx, sc, rays, order, n_slots, cnt, any_hit, flags, hits, s);
     th = stage_begin(ctx, RSH_STAGE_BUILD, s);
-    RSH_CUDA(launch_build_rsh(rays, static_cast<uint32_t*>(sorted_ids), n_slots, cnt, P,
-                              static_cast<rsh_node*>(nodes), s));
+    RSH_CUDA(launch_build_rsh(rays, order, n_slots, cnt, P, static_cast<rsh_node*>(nodes), s));
     stage_end(ctx, th, s);
-    return traverse_and_intersect(ctx, sc, static_cast<rsh_node*>(nodes), rays,
-                                  static_cast<uint32_t*>(sorted_ids), n_slots, cnt, any_hit, flags, hits, s);
+    return traverse_and_intersect(ctx, sc, static_cast<rsh_node*>(nodes), rays, order, n_slots, cnt, any_hit, flags,
+                                  hits, s);
 }
 
 rsh_status trace_ordered(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t n,
                          bool any_hit, uint32_t* flags, unsigned long long* hits, cudaStream_t s) {
     if (n == 0) return RSH_OK;
+    if (ctx->cfg.plain_ray_level > 0) return trace_rays_alone(ctx, sc, rays, nullptr, n, nullptr, any_hit, flags, hits, s);
     const uint32_t P = ctx->cfg.packet_size;
     uint32_t off[4];
     const uint32_t cap_nodes = hierarchy_capacity(n, P, off);
@@ -1107,7 +1117,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     ctx->tev_used = 0;
     ctx->tmarks.clear();
     std::memset(&ctx->stats, 0, sizeof(ctx->stats));
-    RSH_CUDA(cudaMemsetAsync(ctx->d_stats, 0, 64, s));
+    RSH_CUDA(cudaMemsetAsync(ctx->d_stats, 0, 8 * (STAT_CAND + 1), s));
     const uint32_t LS = L * S;  // light samples per pixel
     uint32_t lbits = 0;
     while ((1u << lbits) < LS) ++lbits;
@@ -1275,7 +1285,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     RSH_CUDA(cudaEventRecord(ctx->ev[3], s));
     // counters (async; read by rsh_frame_stats_get)
     RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 16, fc, 8ull * 2 * (depth + 1), cudaMemcpyDeviceToHost, s));
-    RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 256, ctx->d_stats, 64, cudaMemcpyDeviceToHost, s));
+    RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 256, ctx->d_stats, 8 * (STAT_CAND + 1), cudaMemcpyDeviceToHost, s));
     ctx->stats.primary_rays = (uint64_t)W * H;
     return RSH_OK;
 }
@@ -1303,10 +1313,11 @@ rsh_status rsh_frame_stats_get(rsh_ctx* ctx, rsh_frame_stats* out) {
         st.chunks += fc[4 * b + 1] + fc[4 * b + 3];
         st.reflection_rays += fc[4 * b + 2];
     }
-    unsigned long long d[8];
-    std::memcpy(d, ctx->h_pinned + 256, 64);
+    unsigned long long d[STAT_CAND + 1];
+    std::memcpy(d, ctx->h_pinned + 256, sizeof(d));
     st.node_tests = d[0];
     st.tri_tests = d[1];
+    st.candidates += d[STAT_CAND];
     cudaEventElapsedTime(&st.secondary_ms, ctx->ev[1], ctx->ev[2]);
     cudaEventElapsedTime(&st.frame_ms, ctx->ev[0], ctx->ev[3]);
     for (float& v : st.stage_ms) v = 0.0f;
