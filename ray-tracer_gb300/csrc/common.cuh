@@ -111,6 +111,68 @@ RSH_DEV uint32_t lanemask_lt() {
     return m;
 }
 
+RSH_DEV void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Decoupled look-back over tiles that each contribute two counts (a, b < 2^24), packed a | b << 24; one status
+// word per tile holds a state, an epoch (words of an earlier launch over the same array do not count, so the
+// array is cleared once per 2^14 launches, not per launch) and the packed counts. Called by one whole warp of
+// the tile's block, with the tile's own sum; returns the sum over the tiles before it. Tiles are taken by
+// ticket, so every earlier tile is running or done. A wait that gives up raises RSH_DEVERR_TIMEOUT, publishes
+// LB_DEAD, which every later tile passes on, and returns LB_FAILED: the caller then writes nothing.
+constexpr unsigned long long LB_COUNTS = (1ull << 48) - 1ull;
+constexpr unsigned long long LB_FAILED = ~0ull;
+constexpr uint32_t LB_SUM = 1u, LB_PREFIX = 2u, LB_DEAD = 3u;
+constexpr uint32_t LB_EPOCHS = 1u << 14;
+RSH_DEV unsigned long long look_back2(unsigned long long* status, uint32_t tile, unsigned long long sum,
+                                      uint32_t epoch, uint32_t* err) {
+    const uint32_t lane = lane_id();
+    auto word = [&](uint32_t state, unsigned long long v) {
+        return ((unsigned long long)state << 62) | ((unsigned long long)epoch << 48) | v;
+    };
+    if (tile == 0u) {
+        if (lane == 0) st_relaxed_u64(status, word(LB_PREFIX, sum));
+        return 0ull;
+    }
+    if (lane == 0) st_relaxed_u64(status + tile, word(LB_SUM, sum));
+    unsigned long long excl = 0ull;
+    int64_t j = (int64_t)tile - 1;  // newest tile not yet added
+    uint32_t spins = 0;
+    bool dead = false;
+    for (;;) {
+        const int64_t q = j - (int64_t)lane;
+        const unsigned long long v = q >= 0 ? ld_relaxed_u64(status + q) : word(LB_PREFIX, 0ull);
+        const bool ready = ((uint32_t)(v >> 48) & (LB_EPOCHS - 1u)) == epoch && (v >> 62) != 0ull;
+        const uint32_t state = (uint32_t)(v >> 62);
+        const uint32_t waiting = __ballot_sync(0xffffffffu, !ready);
+        const uint32_t stops = __ballot_sync(0xffffffffu, ready && state != LB_SUM);
+        // the lanes to add: up to the first prefix, or up to the first tile still to wait for
+        const uint32_t first_stop = stops ? (uint32_t)__ffs(stops) - 1u : 32u;
+        const uint32_t first_wait = waiting ? (uint32_t)__ffs(waiting) - 1u : 32u;
+        const bool found = first_stop < first_wait;
+        const uint32_t upto = found ? first_stop + 1u : min(first_wait, 32u);
+        unsigned long long add = lane < upto ? v & LB_COUNTS : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+        excl += add;
+        if (found) {
+            dead = __shfl_sync(0xffffffffu, state, (int)first_stop) == LB_DEAD;
+            break;
+        }
+        j -= (int64_t)upto;
+        if (waiting) {
+            if (++spins > RSH_SPIN_LIMIT) {
+                if (lane == 0) raise_device_error(err, RSH_DEVERR_TIMEOUT);
+                dead = true;
+                break;
+            }
+            if (spins > 16u) __nanosleep(32);
+        }
+    }
+    if (lane == 0) st_relaxed_u64(status + tile, dead ? word(LB_DEAD, 0ull) : word(LB_PREFIX, (excl + sum) & LB_COUNTS));
+    return dead ? LB_FAILED : excl;
+}
+
 // device count helper: n = *d_count when given (clamped to n_max), else n_max
 RSH_DEV uint32_t dev_count(const uint32_t* d_count, uint32_t n_max) {
     if (!d_count) return n_max;

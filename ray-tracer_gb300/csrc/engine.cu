@@ -628,8 +628,7 @@ rsh_status rsh_scene_upload(rsh_ctx* ctx, const rsh_scene_desc* d, rsh_scene** o
         rsh_scene_destroy(ctx, sc);
         return cuda_status(e, "rsh_scene_upload scratch");
     }
-    e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, lo, hi, sc->h, scr, scr_bytes,
-                               ctx->d_err, s);
+    e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, lo, hi, sc->h, scr, ctx->d_err, s);
     cudaFree(scr);
     if (e != cudaSuccess) {
         rsh_scene_destroy(ctx, sc);
@@ -656,14 +655,8 @@ rsh_status rsh_scene_destroy(rsh_ctx* ctx, rsh_scene* sc) {
     if (sc->pos_rest) cudaFree(sc->pos_rest);
     if (sc->nrm_rest) cudaFree(sc->nrm_rest);
     if (sc->materials) cudaFree(sc->materials);
-    if (sc->h.spheres) cudaFree(sc->h.spheres);
-    if (sc->h.kids) cudaFree(sc->h.kids);
-    if (sc->h.tris) cudaFree(sc->h.tris);
-    if (sc->h.order) cudaFree(sc->h.order);
-    if (sc->h.boxes) cudaFree(sc->h.boxes);
-    if (sc->h.wboxes) cudaFree(sc->h.wboxes);
-    if (sc->h.wtris) cudaFree(sc->h.wtris);
-    if (sc->h.wnodes) cudaFree(sc->h.wnodes);
+    if (sc->build_scratch) cudaFree(sc->build_scratch);
+    free_object_hierarchy(sc->h);
     if (ctx && ctx->allocated >= sc->bytes) ctx->allocated -= sc->bytes;
     delete sc;
     return RSH_OK;
@@ -691,17 +684,17 @@ rsh_status rsh_build_object_hierarchy(rsh_ctx* ctx, rsh_scene* sc, rsh_stream_t 
             sc->hi[a] = hb[3 + a];
         }
     }
-    RSH_CUDA(cudaStreamSynchronize(s));
-    for (void* p : {(void*)sc->h.spheres, (void*)sc->h.kids, (void*)sc->h.tris, (void*)sc->h.order,
-                    (void*)sc->h.boxes, (void*)sc->h.wboxes, (void*)sc->h.wtris, (void*)sc->h.wnodes})
-        if (p) cudaFree(p);
-    sc->h = ObjHierarchy();
-    void* scr = nullptr;
-    const size_t scr_bytes = objh_scratch_bytes(T ? T : 1);
-    RSH_CUDA(cudaMalloc(&scr, scr_bytes));
+    // the tree is rebuilt in place: nothing may still be reading it, on any stream
+    RSH_CUDA(cudaDeviceSynchronize());
+    // a scene whose objects move (it has a rest pose) keeps the build's scratch for its next pose; it goes with
+    // the scene
+    const bool keep = sc->pos_rest != nullptr;
+    void* scr = sc->build_scratch;
+    if (!scr) RSH_CUDA(cudaMalloc(&scr, objh_scratch_bytes(T)));
+    if (keep) sc->build_scratch = scr;
     const cudaError_t e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, sc->lo, sc->hi, sc->h, scr,
-                                                 scr_bytes, ctx->d_err, s);
-    cudaFree(scr);
+                                                 ctx->d_err, s);
+    if (!keep) cudaFree(scr);
     if (e != cudaSuccess) return cuda_status(e, "rsh_build_object_hierarchy");
     return RSH_OK;
 }

@@ -45,6 +45,7 @@ struct rsh_scene {
     uint32_t object_count = 1;
     float4* pos_rest = nullptr;  // rest pose for rsh_scene_set_transforms (kept from the first call on)
     float4* nrm_rest = nullptr;
+    void* build_scratch = nullptr;  // of a scene with a rest pose: the hierarchy build's scratch
     rsh_material* materials = nullptr;
     uint32_t material_count = 0;
     rsh::ObjHierarchy h;

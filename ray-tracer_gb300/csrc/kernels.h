@@ -139,6 +139,7 @@ struct ObjHierarchy {
     // the same tree as traversal records (14 float4 per node: child boxes plane by plane, child entries)
     float4* wnodes = nullptr;
     uint32_t wnode_count = 0;
+    uint32_t wnode_cap = 0;        // records allocated
     uint32_t wnroot = 0;           // the root's entry in record form
 };
 // A traversal record of the box tree: REC_F4 float4 (the eight children's box planes lo x, hi x, lo y, hi y,
@@ -146,12 +147,17 @@ struct ObjHierarchy {
 // << 28 | record index, a cluster's its first triangle | (triangles - 1) << 23.
 constexpr uint32_t REC_F4 = 14;
 constexpr uint32_t REC_NODE = 0x80000000u;
-// Builds the single-ray box tree from h.tris (Morton order) and h.cluster; boxes widened by `pad`.
-cudaError_t build_box_tree(ObjHierarchy& h, float pad, cudaStream_t s);
+// Builds the single-ray box tree from h.tris (Morton order) and h.cluster; boxes widened by `pad`. The scratch
+// is the caller's (box_tree_scratch_bytes). Synchronises the stream.
+size_t box_tree_scratch_bytes(uint32_t tri_count);
+cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* err, cudaStream_t s);
+// Builds (or, for the same triangle count, rebuilds in place) the object hierarchy and the box tree; scratch of
+// objh_scratch_bytes. Synchronises the stream.
 cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t tri_count, uint32_t cluster,
                                    const float lo[3], const float hi[3], ObjHierarchy& h,
-                                   void* scratch, size_t scratch_bytes, uint32_t* err, cudaStream_t s);
+                                   void* scratch, uint32_t* err, cudaStream_t s);
 size_t objh_scratch_bytes(uint32_t tri_count);
+void free_object_hierarchy(ObjHierarchy& h);
 
 // ---- traversal (traverse.cu)
 struct TravArgs {
