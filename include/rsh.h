@@ -161,8 +161,9 @@ typedef struct rsh_config {
  * 1680-1696); shadow slots per pixel = lights x 16. Each sample is traced exactly (the reference tests the
  * samples only against the centre ray's candidate triangles). */
 #define RSH_FLAG_SOFT_SHADOWS 8u
-/* Batched form: sort the hashed slots directly instead of their runs of equal keys (no compression or
- * decompression), for incoherent batches whose keys hardly repeat; rsh_autotune_scenes tries both. */
+/* Batched form, packets below the root: sort the hashed slots directly instead of their runs of equal keys (no
+ * compression or decompression), for incoherent batches whose keys hardly repeat; rsh_autotune_scenes tries
+ * both. Rays alone from the root (the default switch level) are never cut into runs. */
 #define RSH_FLAG_NO_COMPRESS 16u
 /* Batched form: every ray is traced by one lane from its first step to its last. By default, once a warp
  * of the rays-only kernel has no ray left to take and at most 16 of its lanes still trace one, its idle
@@ -181,7 +182,8 @@ typedef struct rsh_frame_stats {
     uint64_t primary_rays;
     uint64_t shadow_rays;        /* traced after trimming, all bounces */
     uint64_t reflection_rays;    /* traced after trimming, all bounces */
-    uint64_t chunks;             /* compressed runs, all secondary batches */
+    uint64_t chunks;             /* compressed runs, all secondary batches (rays that are not cut into runs:
+                                    one each) */
     uint64_t candidates;         /* plain path: (packet, cluster) pairs emitted by the packet traversal, or the
                                     (ray, cluster) pairs whose triangles a ray alone tested */
     uint64_t node_tests;         /* node tests executed (packet-node x sphere; a single ray x node box);
@@ -316,8 +318,10 @@ rsh_status rsh_camera_look_at(const float eye[3], const float target[3], const f
 /* ---------------------------------------------------------------- the per-frame path */
 
 /* Renders one frame headless: primary rays, then `depth` bounces of shadow + reflection batches, each
- * through hash -> compress -> sort -> decompress -> build -> traverse -> intersect, then shading into
- * `rgba_out` (device, width*height uint32 RGBA8). Replaces display() stages 2-4 (main.cpp:1077-1303)
+ * traced, then shading into `rgba_out` (device, width*height uint32 RGBA8). Rays alone from the root (both
+ * forms' default) are traced in the order of the pixels, in which they are as coherent as sorted ones; packets
+ * (ray_level below the object tree's depth, plain_ray_level 0) go through hash -> compress -> sort ->
+ * decompress -> build -> traverse -> intersect. Replaces display() stages 2-4 (main.cpp:1077-1303)
  * with the GL rasteriser replaced by a primary ray cast. rgba_out may be NULL (no shading). */
 rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* scene, uint32_t width, uint32_t height,
                             uint32_t depth, uint32_t* rgba_out, rsh_stream_t stream);
@@ -474,7 +478,8 @@ rsh_status rsh_resolve_hits(const rsh_scene* scene, const rsh_ray* rays, const u
                             const uint32_t* pixel_of_ray, uint32_t n, float* surface_pos,
                             float* surface_nrm, rsh_stream_t stream);
 
-/* Ray-by-ray trace through the whole pipeline (hash .. intersect) of an arbitrary ray set:
+/* Ray-by-ray trace of an arbitrary ray set (plain_ray_level 0: packets, hash .. intersect; else rays alone, as
+ * rsh_batch_trace traces them):
  * closest-hit records (any_hit == 0) or shadow flags (any_hit != 0), indexed like `rays`.
  * Rays with tmax <= tmin are skipped. Output buffers are filled by the call. */
 rsh_status rsh_trace_rays(rsh_ctx* ctx, const rsh_scene* scene, const rsh_ray* rays, uint32_t n,
@@ -492,10 +497,11 @@ typedef struct rsh_batch_segment {
     uint32_t* flags;    /* shadow output (any_hit != 0) */
 } rsh_batch_segment;
 
-/* Traces many ray batches of uneven size over several resident scenes: one hash, one compress, one
- * sort and one decompress over all segments (the segment index is the key's tag), one hierarchy
- * build, then ONE persistent fused traversal + intersection launch. Without host synchronisation,
- * so the whole call can be captured in a CUDA graph (rsh_batch_graph_*). */
+/* Traces many ray batches of uneven size over several resident scenes in ONE persistent fused traversal +
+ * intersection launch. Up to two million rays are traced in their own order; more are hashed and sorted first
+ * (the segment index is the key's tag). With packets below the root (ray_level below a scene's tree depth): one
+ * hash, one compress, one sort and one decompress over all segments, one hierarchy build, then the launch.
+ * Without host synchronisation, so the whole call can be captured in a CUDA graph (rsh_batch_graph_*). */
 rsh_status rsh_batch_trace(rsh_ctx* ctx, const rsh_batch_segment* segments, uint32_t count,
                            rsh_stream_t stream);
 /* Captures rsh_batch_trace for a fixed segment list into a CUDA graph; replays with _launch. */

@@ -2,10 +2,16 @@
 //
 // The reference has no batched path: every batch is a host loop of wrappers with a blocking count
 // readback after each stage (main.cpp:951-1054, RayTracer.cu:2316-2832). Here, for S segments:
+// Rays alone (switch level at or above every segment's tree depth, the default):
+//   up to SORT_RAYS rays, they are traced as they come, in ONE launch that also writes the misses of empty
+//   slots; above that they are hashed (k_batch_prep), sorted by key -- the slots themselves, the last pass
+//   leaving each segment's trimmed ids -- and k_batch_units gives each segment its range and its work units.
+//   No run compression: the traversal reads ids, and runs of incoherent rays hardly repeat.
+// Packets below the root (k_fused):
 //   k_batch_prep     one pass over all rays: key = segment << shift | hash (per-segment scene box),
 //                    pre-fill each segment's output, count each segment's rays (shared-memory counters,
-//                    one global atomic per segment per block); it gathers the rays into one array only for
-//                    the packet kernel when the segments do not already lie back to back;
+//                    one global atomic per segment per block); it gathers the rays into one array when the
+//                    segments do not already lie back to back;
 //   k_batch_bounds   from those counts (one block): each segment's range of the sorted order (the
 //                    segment tag is the top key digit, so the sorted order is segment-major: a segmented
 //                    sort for free) and of the padded layout, padded so that no level-1 ray node straddles
@@ -15,9 +21,8 @@
 //   compress / sort / decompress over all keys at once; decompress writes each ray straight to its
 //                    padded position (RSH_FLAG_NO_COMPRESS: the slots are sorted as they are and
 //                    k_batch_scatter writes them to the padded layout);
-//   build            ray-space hierarchy over the padded order (packet kernel only);
-//   fused            ONE persistent traversal + intersection launch over every segment's work units
-//                    (the rays-only kernel reads each segment's rays in place).
+//   build            ray-space hierarchy over the padded order;
+//   fused            ONE persistent traversal + intersection launch over every segment's work units.
 // Nothing reads a count back to the host, so the whole sequence is captured in a CUDA graph.
 #include <algorithm>
 #include <chrono>
@@ -117,6 +122,54 @@ __global__ void k_batch_bounds(const uint32_t* __restrict__ seg_cnt, uint32_t ns
             padded[q] = INVALID_ID;
 }
 
+// Rays alone: each segment's ids, their number and its first work unit, in schedule order; one block, a thread
+// per segment. sorted != nullptr: the segments' trimmed ids lie one after the other there, in segment order,
+// seg_cnt[s] of them for segment s; else each segment has its own list and count (FusedSeg).
+__global__ void __launch_bounds__(1024)
+k_batch_units(FusedSeg* __restrict__ fsegs, uint32_t nseg, const uint32_t* __restrict__ sorted,
+              const uint32_t* __restrict__ seg_cnt, const uint32_t* __restrict__ sched, uint32_t unit_rays,
+              uint32_t* __restrict__ totals) {
+    __shared__ uint32_t s_begin[1024], s_warp[32];
+    const uint32_t k = threadIdx.x, lane = lane_id(), warp = k >> 5;
+    auto exclusive = [&](uint32_t v) {  // over the block
+        uint32_t x = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= (uint32_t)d) x += y;
+        }
+        __syncthreads();  // s_warp may still be read
+        if (lane == 31) s_warp[warp] = x;
+        __syncthreads();
+        uint32_t w = s_warp[lane];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, w, d);
+            if (lane >= (uint32_t)d) w += y;
+        }
+        return x - v + (warp ? __shfl_sync(0xffffffffu, w, (int)warp - 1) : 0u);
+    };
+    const bool in = k < nseg;
+    uint32_t n = 0;
+    if (sorted) {
+        s_begin[k] = exclusive(in ? seg_cnt[k] : 0u);
+        __syncthreads();
+        if (in) {
+            const uint32_t s = sched[k];
+            n = seg_cnt[s];
+            fsegs[k].ids = sorted + s_begin[s];
+        }
+    } else if (in) {
+        n = dev_count(fsegs[k].count, fsegs[k].n);
+    }
+    const uint32_t units = (n + unit_rays - 1u) / unit_rays, ub = exclusive(units);
+    if (in) {
+        fsegs[k].n = n;
+        fsegs[k].unit_begin = ub;
+        if (k == nseg - 1u) totals[1] = ub + units;
+    }
+}
+
 // Without run compression: the sorted slots go straight to the padded layout (valid keys sort before
 // every empty slot, whose key has the bit above the key's width set); also the stats words (rays,
 // "chunks" = rays) from the per-segment counts.
@@ -149,6 +202,10 @@ namespace {
 struct BatchPlan {
     uint32_t nseg = 0, total = 0, tag_shift = 0, key_bits = 0, P = 8, unit_rays = 64, max_padded = 0, hash_drop = 0;
     uint32_t rays_only = 1;  // cleared by any segment whose rays use packets below the root
+    bool sorted = true;      // hashed and sorted before the traversal
+    bool listed = false;     // rays alone: ray generation listed each segment's ids
+    uint32_t empty_bit = 0;  // slots sorted as they are: one more key bit sorted, that of the empty slots
+    uint32_t units_max = 0;  // rays alone: work units if every slot held a ray
     bool contiguous = false; // the segments' rays lie back to back in one array: no gather
     bool gather = false;     // copy every segment's rays into one array (packet kernel, not contiguous)
     void *rays_all, *keys, *trimmed, *ckeys, *cbases, *counts, *skeys, *svals, *sorted_keys, *sorted_ids, *scr;
@@ -157,6 +214,11 @@ struct BatchPlan {
     std::vector<FusedSeg> h_fsegs;  // in schedule order
     std::vector<uint32_t> h_sched;  // schedule position -> segment index
 };
+
+// Rays at or below this count are traced in their own order. Sorting incoherent rays makes their traversal 11-13%
+// shorter (their nodes are in the L1 more often), whatever their number; the hash and the sort cost 0.10 ms for
+// 1.3 M rays in 8 segments (traversal 0.526 against 0.587 ms), 0.6 ms for 13.8 M in 64 (4.95 against 5.77 ms).
+constexpr uint32_t SORT_RAYS = 2000000;
 
 // The context's configuration with a scene's own tuning (rsh_scene_set_tuning) applied.
 rsh_config tuned_config(const rsh_config& base, const rsh_scene* sc) {
@@ -178,7 +240,10 @@ rsh_status check_batched_scene(const rsh_scene* sc) {
     return RSH_OK;
 }
 
-rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t count, BatchPlan& pl) {
+// lists: every segment's ids and their device counts, from ray generation (rays alone only). plain: the plain
+// path's rays alone, whatever the scenes' tuning and switch levels.
+rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t count, BatchPlan& pl,
+                         const SegList* lists = nullptr, bool plain = false) {
     if (!ctx || (!segs && count)) return RSH_ERR_INVALID;
     if (count > 1024) {
         set_error("at most 1024 batch segments");
@@ -200,7 +265,7 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
     // the tag sits above the widest.
     uint32_t hash_bits = 0;
     for (uint32_t s = 0; s < count; ++s) {
-        const rsh_config c = tuned_config(ctx->cfg, segs[s].scene);
+        const rsh_config c = plain ? ctx->cfg : tuned_config(ctx->cfg, segs[s].scene);
         hash_bits = std::max(hash_bits, 3 * c.grid_bits + 2 * c.dir_log2);
     }
     pl.hash_drop = (hash_bits + tag_bits > 31) ? hash_bits + tag_bits - 31 : 0u;
@@ -208,20 +273,26 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         set_error("too many batch segments for a 31-bit key");
         return RSH_ERR_INVALID;
     }
+    pl.P = ctx->cfg.packet_size;
+    for (uint32_t s = 0; s < count && !plain; ++s)
+        if (tuned_config(ctx->cfg, segs[s].scene).ray_level < segs[s].scene->h.levels) pl.rays_only = 0;
+    pl.listed = lists != nullptr;
+    if (pl.listed && !pl.rays_only) return RSH_ERR_INVALID;
+    pl.sorted = !pl.listed && (!pl.rays_only || (pl.total > SORT_RAYS && !(plain && (ctx->cfg.flags & RSH_FLAG_RAH))));
+    const bool packets = !pl.rays_only;
     {
+        // slots sorted as they are: an empty slot's key has every bit set, so it goes last by the tag alone
+        // unless the tag's last value is a segment's (then one more bit is sorted)
+        const bool slots = pl.rays_only || (ctx->cfg.flags & RSH_FLAG_NO_COMPRESS);
+        pl.empty_bit = slots && count == (1u << tag_bits) ? 1u : 0u;
         // a last 8-bit digit pass for 1 or 2 leftover key bits would read and write every pair once more
-        // for almost no order: those lowest hash bits are dropped instead (a frame's two segments over a
-        // 24-bit hash sort in 3 passes, not 4)
-        const uint32_t empty_bit = (ctx->cfg.flags & RSH_FLAG_NO_COMPRESS) ? 1u : 0u;  // sorts one more bit
-        const uint32_t kb = hash_bits + tag_bits - pl.hash_drop + empty_bit, tail = kb % 8u;
+        // for almost no order: those lowest hash bits are dropped instead
+        const uint32_t kb = hash_bits + tag_bits - pl.hash_drop + pl.empty_bit, tail = kb % 8u;
         if (kb > 8u && tail != 0u && tail <= 2u && hash_bits - pl.hash_drop > tail) pl.hash_drop += tail;
     }
     pl.tag_shift = hash_bits - pl.hash_drop;
     pl.key_bits = pl.tag_shift + tag_bits;
-    pl.P = ctx->cfg.packet_size;
-    for (uint32_t s = 0; s < count; ++s)
-        if (tuned_config(ctx->cfg, segs[s].scene).ray_level < segs[s].scene->h.levels) pl.rays_only = 0;
-    // work units: 8 packets for the packet kernel, RSH_RAYS_UNIT sorted rays for the rays-only kernel
+    // work units: 8 packets for the packet kernel, RSH_RAYS_UNIT rays for the rays-only kernel
     pl.unit_rays = pl.rays_only ? (uint32_t)RSH_RAYS_UNIT : 8 * pl.P;
     pl.max_padded = pl.total + count * pl.unit_rays;
     const uint32_t n = pl.total ? pl.total : 1;
@@ -230,35 +301,37 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         if (segs[s].n && segs[s].rays != segs[0].rays + at) pl.contiguous = false;
     // one ray array for the ray hierarchy and the packet kernel: the segments' own when they lie back to
     // back, else a gathered copy; the rays-only kernel reads every segment's rays in place
-    pl.gather = !pl.contiguous && !pl.rays_only;
+    pl.gather = !pl.contiguous && packets;
     if (pl.contiguous) pl.rays_all = const_cast<rsh_ray*>(segs[0].rays);
     else if (pl.gather) RSH_TRY(ensure(ctx, "b_rays", sizeof(rsh_ray) * (size_t)n, &pl.rays_all));
     else pl.rays_all = nullptr;
-    RSH_TRY(ensure(ctx, "b_keys", 4ull * n, &pl.keys));
-    RSH_TRY(ensure(ctx, "trimmed", 4ull * n, &pl.trimmed));
-    RSH_TRY(ensure(ctx, "ckeys", 4ull * n + 4, &pl.ckeys));
-    RSH_TRY(ensure(ctx, "cbases", 4ull * n + 4, &pl.cbases));
     RSH_TRY(ensure(ctx, "b_counts", 64, &pl.counts));
-    RSH_TRY(ensure(ctx, "skeys", 4ull * n, &pl.skeys));
-    RSH_TRY(ensure(ctx, "svals", 4ull * n, &pl.svals));
-    RSH_TRY(ensure(ctx, "sorted_keys", 4ull * n, &pl.sorted_keys));
-    RSH_TRY(ensure(ctx, "sorted_ids", 4ull * n, &pl.sorted_ids));
-    size_t scr = std::max(compress_scratch_bytes(n), sort_scratch_bytes(n, pl.key_bits + 1u));
-    scr = std::max(scr, decompress_scratch_bytes(n));
-    RSH_TRY(ensure(ctx, "scratch", scr, &pl.scr));
-    RSH_TRY(ensure(ctx, "b_padded", 4ull * pl.max_padded, &pl.padded));
-    uint32_t off[4];
-    const uint32_t capn = hierarchy_capacity(pl.max_padded, pl.P, off);
-    RSH_TRY(ensure(ctx, "b_nodes", sizeof(rsh_node) * (size_t)capn, &pl.nodes));
-    RSH_TRY(ensure(ctx, "b_prep", sizeof(PrepSeg) * (count ? count : 1), &pl.prep));
-    RSH_TRY(ensure(ctx, "b_fsegs", sizeof(FusedSeg) * (count ? count : 1), &pl.fsegs));
-    RSH_TRY(ensure(ctx, "b_seg_begin", 4ull * (count + 1), &pl.seg_begin));
-    RSH_TRY(ensure(ctx, "b_seg_cnt", 4ull * (count + 1), &pl.seg_cnt));
-    RSH_TRY(ensure(ctx, "b_pstart", 4ull * (count + 1), &pl.pstart));
     RSH_TRY(ensure(ctx, "b_totals", 64, &pl.totals));
     RSH_TRY(ensure(ctx, "b_work", 64, &pl.work));
+    RSH_TRY(ensure(ctx, "b_prep", sizeof(PrepSeg) * (count ? count : 1), &pl.prep));
+    RSH_TRY(ensure(ctx, "b_fsegs", sizeof(FusedSeg) * (count ? count : 1), &pl.fsegs));
     RSH_TRY(ensure(ctx, "b_sched", 4ull * (count + 1), &pl.sched));
-    RSH_TRY(ensure(ctx, "b_seg_delta", 4ull * (count + 1), &pl.seg_delta));
+    RSH_TRY(ensure(ctx, "b_seg_cnt", 4ull * (count + 1), &pl.seg_cnt));
+    if (pl.sorted) {
+        RSH_TRY(ensure(ctx, "b_keys", 4ull * n, &pl.keys));
+        RSH_TRY(ensure(ctx, "skeys", 4ull * n, &pl.skeys));
+        RSH_TRY(ensure(ctx, "svals", 4ull * n, &pl.svals));
+        size_t scr = sort_scratch_bytes(n, pl.key_bits + pl.empty_bit);
+        if (packets) scr = std::max(scr, std::max(compress_scratch_bytes(n), decompress_scratch_bytes(n)));
+        RSH_TRY(ensure(ctx, "scratch", scr, &pl.scr));
+    }
+    if (packets) {
+        RSH_TRY(ensure(ctx, "trimmed", 4ull * n, &pl.trimmed));
+        RSH_TRY(ensure(ctx, "ckeys", 4ull * n + 4, &pl.ckeys));
+        RSH_TRY(ensure(ctx, "cbases", 4ull * n + 4, &pl.cbases));
+        RSH_TRY(ensure(ctx, "b_padded", 4ull * pl.max_padded, &pl.padded));
+        uint32_t off[4];
+        const uint32_t capn = hierarchy_capacity(pl.max_padded, pl.P, off);
+        RSH_TRY(ensure(ctx, "b_nodes", sizeof(rsh_node) * (size_t)capn, &pl.nodes));
+        RSH_TRY(ensure(ctx, "b_seg_begin", 4ull * (count + 1), &pl.seg_begin));
+        RSH_TRY(ensure(ctx, "b_pstart", 4ull * (count + 1), &pl.pstart));
+        RSH_TRY(ensure(ctx, "b_seg_delta", 4ull * (count + 1), &pl.seg_delta));
+    }
     pl.h_prep.resize(count);
     pl.h_fsegs.resize(count);
     uint32_t start = 0;
@@ -271,9 +344,9 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         p.any_hit = g.any_hit ? 1u : 0u;
         p.flags = g.flags;
         p.hits = reinterpret_cast<unsigned long long*>(g.hits);
-        const rsh_config tc = tuned_config(ctx->cfg, sc);
+        const rsh_config tc = plain ? ctx->cfg : tuned_config(ctx->cfg, sc);
         RSH_TRY(make_hash_params(sc, tc, 0, p.hp));
-        RSH_TRY(check_batched_scene(sc));
+        if (!plain) RSH_TRY(check_batched_scene(sc));
         FusedSeg& f = pl.h_fsegs[s];
         std::memset(&f, 0, sizeof(f));
         f.spheres = sc->h.spheres;
@@ -296,7 +369,14 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         f.rays = g.rays;
         f.flags = g.flags;
         f.hits = reinterpret_cast<unsigned long long*>(g.hits);
-        f.slot_base = start;
+        f.slots = g.n;
+        f.n = g.n;
+        if (pl.listed) {
+            f.ids = lists[s].ids;
+            f.count = lists[s].count;
+        } else if (pl.sorted) {
+            f.slot_base = start;  // a sorted id counts over all segments
+        }
         start += g.n;
     }
     // schedule: closest-hit segments first (incoherent, long rays), then by size, descending
@@ -307,7 +387,13 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         return segs[a].n > segs[b].n;
     });
     std::vector<FusedSeg> by_seg(pl.h_fsegs);
-    for (uint32_t k = 0; k < count; ++k) pl.h_fsegs[k] = by_seg[pl.h_sched[k]];
+    uint32_t units = 0;
+    for (uint32_t k = 0; k < count; ++k) {
+        pl.h_fsegs[k] = by_seg[pl.h_sched[k]];
+        pl.h_fsegs[k].unit_begin = units;  // final where the segments' own order is traced
+        units += (pl.h_fsegs[k].n + pl.unit_rays - 1) / pl.unit_rays;
+    }
+    pl.units_max = units;
     return RSH_OK;
 }
 
@@ -360,21 +446,99 @@ rsh_status stage_tables(rsh_ctx* ctx, const BatchPlan& pl, char** out, cudaEvent
     return RSH_OK;
 }
 
-// pre_staged != nullptr: tables already in pinned memory owned by the caller (a captured graph, which must
-// not allocate while capturing); otherwise a fenced ring slot of the context.
-// reset_stats: zero the node / triangle test counters first (a frame keeps counting over its batches).
-rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_staged = nullptr,
-                         bool reset_stats = true, bool prekeyed = false) {
-    if (pl.nseg == 0) return RSH_OK;
-    char* tables = pre_staged;
-    cudaEvent_t fence = nullptr;
-    if (!tables) RSH_TRY(stage_tables(ctx, pl, &tables, &fence));
+rsh_status copy_tables(BatchPlan& pl, char* tables, cudaEvent_t fence, cudaStream_t s) {
     RSH_CUDA(cudaMemcpyAsync(pl.prep, tables, sizeof(PrepSeg) * pl.nseg, cudaMemcpyHostToDevice, s));
     RSH_CUDA(cudaMemcpyAsync(pl.fsegs, tables + sizeof(PrepSeg) * pl.nseg, sizeof(FusedSeg) * pl.nseg,
                              cudaMemcpyHostToDevice, s));
     RSH_CUDA(cudaMemcpyAsync(pl.sched, tables + (sizeof(PrepSeg) + sizeof(FusedSeg)) * pl.nseg, 4ull * pl.nseg,
                              cudaMemcpyHostToDevice, s));
     if (fence) RSH_CUDA(cudaEventRecord(fence, s));
+    return RSH_OK;
+}
+
+// What every launch of the rays-only kernel shares.
+FusedArgs alone_args(rsh_ctx* ctx, void* work) {
+    FusedArgs fa{};
+    fa.work = static_cast<uint32_t*>(work);
+    fa.blocks_per_sm = ctx->cfg.fused_blocks;
+    fa.share_tail = (ctx->cfg.flags & RSH_FLAG_SEQUENTIAL_RAYS) ? 0u : 1u;
+    fa.node_tests = ctx->d_stats;
+    fa.tri_tests = ctx->d_stats + 1;
+    fa.err = ctx->d_err;
+    return fa;
+}
+
+// Rays alone: in their own order, by their segments' lists, or hashed and sorted first.
+rsh_status enqueue_alone(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_staged, bool reset_stats) {
+    if (reset_stats) RSH_CUDA(cudaMemsetAsync(ctx->d_stats, 0, 64, s));
+    uint32_t* cnt = static_cast<uint32_t*>(pl.counts);
+    RSH_CUDA(cudaMemsetAsync(cnt, 0, 8, s));  // the rays traced, counted by the traversal
+    if (pl.total == 0) return RSH_OK;
+    const bool one = pl.nseg == 1;  // traced from the launch's arguments
+    if (!one || pl.sorted) {
+        char* tables = pre_staged;
+        cudaEvent_t fence = nullptr;
+        if (!tables) RSH_TRY(stage_tables(ctx, pl, &tables, &fence));
+        RSH_TRY(copy_tables(pl, tables, fence, s));
+    }
+    int th = -1;
+    if (pl.sorted) {
+        th = stage_begin(ctx, RSH_STAGE_RAYGEN, s);  // hash + per-segment counts + prefilled results
+        RSH_CUDA(cudaMemsetAsync(pl.seg_cnt, 0, 4ull * pl.nseg, s));
+        k_batch_prep<<<(pl.total + 255) / 256, 256, 0, s>>>(
+            static_cast<PrepSeg*>(pl.prep), pl.nseg, pl.total, pl.tag_shift, pl.hash_drop, nullptr, false,
+            static_cast<uint32_t*>(pl.keys), static_cast<uint32_t*>(pl.seg_cnt));
+        note_launch();
+        RSH_CUDA(cudaGetLastError());
+        stage_end(ctx, th, s);
+        th = stage_begin(ctx, RSH_STAGE_SORT, s);
+        RSH_CUDA(launch_sort_pairs(static_cast<uint32_t*>(pl.keys), nullptr, static_cast<uint32_t*>(pl.skeys),
+                                   static_cast<uint32_t*>(pl.svals), pl.total, nullptr, pl.key_bits + pl.empty_bit,
+                                   pl.scr, ctx->d_err, s));
+        stage_end(ctx, th, s);
+    }
+    RSH_CUDA(cudaMemsetAsync(pl.work, 0, 16, s));
+    FusedArgs fa = alone_args(ctx, pl.work);
+    fa.valid = cnt;
+    th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);  // traversal and intersection in one kernel
+    if (one) {
+        fa.one = pl.h_fsegs[0];
+        if (pl.sorted) {
+            fa.one.ids = static_cast<uint32_t*>(pl.svals);
+            fa.one.count = static_cast<uint32_t*>(pl.seg_cnt);
+        }
+        RSH_CUDA(launch_rays_one(fa, s));
+    } else {
+        uint32_t* totals = static_cast<uint32_t*>(pl.totals);
+        fa.segs = static_cast<FusedSeg*>(pl.fsegs);
+        fa.nseg = pl.nseg;
+        fa.units_max = pl.units_max;
+        if (pl.sorted || pl.listed) {
+            k_batch_units<<<1, 1024, 0, s>>>(static_cast<FusedSeg*>(pl.fsegs), pl.nseg,
+                                             pl.sorted ? static_cast<uint32_t*>(pl.svals) : nullptr,
+                                             static_cast<uint32_t*>(pl.seg_cnt), static_cast<uint32_t*>(pl.sched),
+                                             pl.unit_rays, totals);
+            note_launch();
+            RSH_CUDA(cudaGetLastError());
+            fa.d_units = totals + 1;
+        }
+        RSH_CUDA(launch_rays_segs(fa, s));
+    }
+    stage_end(ctx, th, s);
+    return RSH_OK;
+}
+
+// pre_staged != nullptr: tables already in pinned memory owned by the caller (a captured graph, which must
+// not allocate while capturing); otherwise a fenced ring slot of the context.
+// reset_stats: zero the node / triangle test counters first (a frame keeps counting over its batches).
+rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_staged = nullptr,
+                         bool reset_stats = true, bool prekeyed = false) {
+    if (pl.nseg == 0) return RSH_OK;
+    if (pl.rays_only) return enqueue_alone(ctx, pl, s, pre_staged, reset_stats);
+    char* tables = pre_staged;
+    cudaEvent_t fence = nullptr;
+    if (!tables) RSH_TRY(stage_tables(ctx, pl, &tables, &fence));
+    RSH_TRY(copy_tables(pl, tables, fence, s));
     if (reset_stats) RSH_CUDA(cudaMemsetAsync(ctx->d_stats, 0, 64, s));
     if (pl.total == 0) return RSH_OK;
     uint32_t* cnt = static_cast<uint32_t*>(pl.counts);
@@ -402,8 +566,8 @@ rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
         // scatter the sorted slots to the padded layout
         th = stage_begin(ctx, RSH_STAGE_SORT, s);
         RSH_CUDA(launch_sort_pairs(static_cast<uint32_t*>(pl.keys), nullptr, static_cast<uint32_t*>(pl.skeys),
-                                   static_cast<uint32_t*>(pl.svals), pl.total, nullptr, pl.key_bits + 1u, pl.scr,
-                                   ctx->d_err, s));
+                                   static_cast<uint32_t*>(pl.svals), pl.total, nullptr, pl.key_bits + pl.empty_bit,
+                                   pl.scr, ctx->d_err, s));
         stage_end(ctx, th, s);
         th = stage_begin(ctx, RSH_STAGE_DECOMPRESS, s);
         k_batch_scatter<<<(pl.total + 255) / 256, 256, 0, s>>>(
@@ -433,12 +597,10 @@ rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
                                nullptr, nullptr, pl.scr, ctx->d_err, s, &po));
     stage_end(ctx, th, s);
     }
-    if (!pl.rays_only) {  // rays that leave their packets at the root never read the ray hierarchy
-        th = stage_begin(ctx, RSH_STAGE_BUILD, s);
-        RSH_CUDA(launch_build_rsh(static_cast<rsh_ray*>(pl.rays_all), static_cast<uint32_t*>(pl.padded),
-                                  pl.max_padded, totals, pl.P, static_cast<rsh_node*>(pl.nodes), s));
-        stage_end(ctx, th, s);
-    }
+    th = stage_begin(ctx, RSH_STAGE_BUILD, s);
+    RSH_CUDA(launch_build_rsh(static_cast<rsh_ray*>(pl.rays_all), static_cast<uint32_t*>(pl.padded), pl.max_padded,
+                              totals, pl.P, static_cast<rsh_node*>(pl.nodes), s));
+    stage_end(ctx, th, s);
     RSH_CUDA(cudaMemsetAsync(pl.work, 0, 16, s));
     FusedArgs fa{};
     fa.nodes = static_cast<rsh_node*>(pl.nodes);
@@ -451,9 +613,7 @@ rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
     fa.units_max = pl.max_padded / pl.unit_rays;
     fa.d_units = totals + 1;
     fa.work = static_cast<uint32_t*>(pl.work);
-    fa.rays_only = pl.rays_only;
     fa.blocks_per_sm = ctx->cfg.fused_blocks;
-    fa.share_tail = (ctx->cfg.flags & RSH_FLAG_SEQUENTIAL_RAYS) ? 0u : 1u;
     fa.node_tests = ctx->d_stats;
     fa.tri_tests = ctx->d_stats + 1;
     fa.err = ctx->d_err;
@@ -473,20 +633,10 @@ struct GraphExec {
 }  // namespace
 
 namespace rsh {
-// The rays of one batch against one scene, each alone from the root of the scene's box tree
-// (k_fused_rays): in the order sorted_ids[0 .. *d_count) (device count; null: n), or in their own order
-// (sorted_ids null). cand_pairs (optional) counts the (ray, cluster) pairs whose triangles were tested.
-rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* sorted_ids, uint32_t n,
+rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
-                       unsigned long long* cand_pairs, cudaStream_t s) {
-    if (n == 0 || sc->tri_count == 0) return RSH_OK;
-    void* work;
-    RSH_TRY(ensure(ctx, "b_work", 64, &work));
-    RSH_CUDA(cudaMemsetAsync(work, 0, 16, s));
-    FusedArgs fa{};
-    fa.sorted_ids = sorted_ids;
-    fa.ordered_n = n;
-    fa.d_rays = d_count;
+                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s) {
+    FusedArgs fa = alone_args(ctx, ticket);
     fa.one.wtris = sc->h.wtris;
     fa.one.wnodes = sc->h.wnodes;
     fa.one.wnroot = sc->h.wnroot;
@@ -495,32 +645,37 @@ rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, c
     fa.one.rays = rays;
     fa.one.flags = flags;
     fa.one.hits = hits;
-    fa.work = static_cast<uint32_t*>(work);
-    fa.blocks_per_sm = ctx->cfg.fused_blocks;
-    fa.share_tail = (ctx->cfg.flags & RSH_FLAG_SEQUENTIAL_RAYS) ? 0u : 1u;
-    fa.node_tests = ctx->d_stats;
-    fa.tri_tests = ctx->d_stats + 1;
+    fa.one.ids = ids;
+    fa.one.n = fa.one.slots = slots;
+    fa.one.count = d_count;
     fa.cand_pairs = cand_pairs;
-    fa.err = ctx->d_err;
     RSH_CUDA(launch_rays_one(fa, s));
     return RSH_OK;
 }
 
-// One segment whose rays are already in a coherent order (the frame's primary rays, generated tile by
-// tile), traced by the rays-only kernel in that order: no hash, compression, sort or ray hierarchy.
-// Scenes whose rays use packets below the root go through batch_trace.
-rsh_status batch_trace_ordered(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t s) {
-    if (!ctx || !seg.scene) return RSH_ERR_INVALID;
-    const rsh_config tc = tuned_config(ctx->cfg, seg.scene);
-    if (seg.n == 0 || tc.ray_level < seg.scene->h.levels) return batch_trace(ctx, &seg, 1, s, false);
-    RSH_TRY(check_batched_scene(seg.scene));
-    if (seg.any_hit) RSH_CUDA(cudaMemsetAsync(seg.flags, 0, 4ull * seg.n, s));
-    else RSH_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long*>(seg.hits), RSH_HIT_NONE, seg.n, s));
+rsh_status check_alone(rsh_ctx* ctx, const rsh_scene* sc) {
+    (void)ctx;
+    return check_batched_scene(sc);
+}
+
+bool batch_alone(const rsh_ctx* ctx, const rsh_scene* sc) {
+    return tuned_config(ctx->cfg, sc).ray_level >= sc->h.levels;
+}
+
+rsh_status batch_trace_listed(rsh_ctx* ctx, const rsh_batch_segment* segments, const SegList* lists, uint32_t count,
+                              cudaStream_t s) {
+    ctx->tev_used = 0;  // stage timers (RSH_FLAG_STAGE_TIMERS) cover this call only
+    ctx->tmarks.clear();
+    BatchPlan pl;
+    RSH_TRY(batch_prepare(ctx, segments, count, pl, lists));
     ctx->last_stream = s;
-    RSH_TRY(trace_alone(ctx, seg.scene, seg.rays, nullptr, seg.n, nullptr, seg.any_hit != 0, seg.flags,
-                        reinterpret_cast<unsigned long long*>(seg.hits), nullptr, s));
-    ctx->batch_counts_host.assign(1, seg.n);
-    return RSH_OK;
+    return batch_enqueue(ctx, pl, s);
+}
+
+rsh_status trace_plain(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t s) {
+    BatchPlan pl;
+    RSH_TRY(batch_prepare(ctx, &seg, 1, pl, nullptr, true));
+    return batch_enqueue(ctx, pl, s, nullptr, false);  // the test counters run on
 }
 
 // rsh_batch_trace without resetting the stage timers (a fused frame keeps its own).
@@ -528,7 +683,7 @@ rsh_status batch_key_layout(rsh_ctx* ctx, const rsh_batch_segment* segments, uin
     if (count > 2) return RSH_ERR_INVALID;
     BatchPlan pl;
     RSH_TRY(batch_prepare(ctx, segments, count, pl));
-    if (pl.gather || (count && !pl.contiguous)) {
+    if (pl.rays_only || pl.gather || (count && !pl.contiguous)) {
         set_error("keys from ray generation need the segments' rays back to back in one array");
         return RSH_ERR_INVALID;
     }

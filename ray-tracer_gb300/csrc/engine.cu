@@ -202,28 +202,12 @@ static rsh_status traverse_and_intersect(rsh_ctx* ctx, const rsh_scene* sc, cons
     return RSH_OK;
 }
 
-// Rays that leave their packets (plain_ray_level >= 1) go down the scene's box tree one by one, testing
-// triangles as they meet them, so hits end or shorten a ray's walk at once: no ray hierarchy, no candidates.
-// (A packet walk above the switch level with every cluster along a ray written out as a candidate and
-// tested afterwards took 218 + 26 ms of the architecture frame's 232 ms, and at no switch level was a packet
-// walk above single rays faster than single rays from the root: 12.6-60 ms against 3.9 a frame.)
-static rsh_status trace_rays_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* sorted_ids,
-                                   uint32_t n, const uint32_t* d_count, bool any_hit, uint32_t* flags,
-                                   unsigned long long* hits, cudaStream_t s) {
-    const int th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
-    const rsh_status st = trace_alone(ctx, sc, rays, sorted_ids, n, d_count, any_hit, flags, hits,
-                                      ctx->d_stats + STAT_CAND, s);
-    stage_end(ctx, th, s);
-    return st;
-}
-
 rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* keys,
                        uint32_t n_slots, uint32_t key_bits, bool any_hit, uint32_t* flags,
                        unsigned long long* hits, uint32_t* counts_out, cudaStream_t s) {
     if (n_slots == 0) return RSH_OK;
     const uint32_t P = ctx->cfg.packet_size;
-    const bool packets = ctx->cfg.plain_ray_level == 0;
-    void *trimmed, *ckeys, *cbases, *counts, *skeys, *svals, *sorted_keys, *sorted_ids, *nodes = nullptr, *scr;
+    void *trimmed, *ckeys, *cbases, *counts, *skeys, *svals, *sorted_keys, *sorted_ids, *nodes, *scr;
     RSH_TRY(ensure(ctx, "trimmed", 4ull * n_slots, &trimmed));
     RSH_TRY(ensure(ctx, "ckeys", 4ull * n_slots + 4, &ckeys));
     RSH_TRY(ensure(ctx, "cbases", 4ull * n_slots + 4, &cbases));
@@ -232,11 +216,9 @@ rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, c
     RSH_TRY(ensure(ctx, "svals", 4ull * n_slots, &svals));
     RSH_TRY(ensure(ctx, "sorted_keys", 4ull * n_slots, &sorted_keys));
     RSH_TRY(ensure(ctx, "sorted_ids", 4ull * n_slots, &sorted_ids));
-    if (packets) {
-        uint32_t off[4];
-        const uint32_t cap_nodes = hierarchy_capacity(n_slots, P, off);
-        RSH_TRY(ensure(ctx, "nodes", sizeof(rsh_node) * (size_t)cap_nodes, &nodes));
-    }
+    uint32_t off[4];
+    const uint32_t cap_nodes = hierarchy_capacity(n_slots, P, off);
+    RSH_TRY(ensure(ctx, "nodes", sizeof(rsh_node) * (size_t)cap_nodes, &nodes));
     size_t scr_bytes = compress_scratch_bytes(n_slots);
     scr_bytes = std::max(scr_bytes, sort_scratch_bytes(n_slots, key_bits));
     scr_bytes = std::max(scr_bytes, decompress_scratch_bytes(n_slots));
@@ -260,7 +242,6 @@ rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, c
                                    n_slots, static_cast<uint32_t*>(sorted_keys), order, scr, ctx->d_err, s));
         stage_end(ctx, th, s);
     }
-    if (!packets) return trace_rays_alone(ctx, sc, rays, order, n_slots, cnt, any_hit, flags, hits, s);
     th = stage_begin(ctx, RSH_STAGE_BUILD, s);
     RSH_CUDA(launch_build_rsh(rays, order, n_slots, cnt, P, static_cast<rsh_node*>(nodes), s));
     stage_end(ctx, th, s);
@@ -271,7 +252,6 @@ rsh_status trace_keyed(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, c
 rsh_status trace_ordered(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t n,
                          bool any_hit, uint32_t* flags, unsigned long long* hits, cudaStream_t s) {
     if (n == 0) return RSH_OK;
-    if (ctx->cfg.plain_ray_level > 0) return trace_rays_alone(ctx, sc, rays, nullptr, n, nullptr, any_hit, flags, hits, s);
     const uint32_t P = ctx->cfg.packet_size;
     uint32_t off[4];
     const uint32_t cap_nodes = hierarchy_capacity(n, P, off);
@@ -1080,6 +1060,8 @@ rsh_status rsh_trace_rays(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays
     if (n == 0) return RSH_OK;
     HashP hp;
     RSH_TRY(make_hash_params(sc, ctx->cfg, 0, hp));
+    if (ctx->cfg.plain_ray_level > 0)
+        return trace_plain(ctx, rsh_batch_segment{sc, rays, n, any_hit, hits, flags}, stream);
     void* keys;
     RSH_TRY(ensure(ctx, "keys", 4ull * n, &keys));
     if (any_hit) RSH_CUDA(cudaMemsetAsync(flags, 0, 4ull * n, stream));
@@ -1101,6 +1083,14 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     const uint32_t L = ctx->light_count;
     const uint32_t npix = W * H;
     const bool fused = (ctx->cfg.flags & RSH_FLAG_FUSED) != 0;
+    // Rays alone (no packets): ray generation lists the slots that hold a ray and the rays are traced in that
+    // order, the pixels'. Hashing and sorting them first did not shorten the traversal of any frame measured
+    // (architecture 2.35 ms in pixel order, 2.36 sorted; object soup 1.92 / 1.95; Cornell 0.091 / 0.094: rays of
+    // neighbouring pixels are as coherent as sorted ones, also after a cosine-lobe bounce) and cost 0.45, 0.41
+    // and 0.10 ms with their compression and expansion.
+    const bool alone = fused ? batch_alone(ctx, sc) : ctx->cfg.plain_ray_level > 0;
+    if (fused && alone) RSH_TRY(check_alone(ctx, sc));
+    ctx->falone = alone;
     ctx->fw = W;
     ctx->fh = H;
     ctx->fdepth = depth;
@@ -1130,7 +1120,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     RSH_TRY(ensure_buf(ctx, ctx->surf0_nrm, 16ull * npix));
     void *accum, *keys;
     RSH_TRY(ensure(ctx, "accum", 16ull * npix, &accum));
-    RSH_TRY(ensure(ctx, "keys", 4ull * npix * (LS ? LS : 1), &keys));
+    RSH_TRY(ensure(ctx, "keys", 4ull * npix * ((LS ? LS : 1) + 1), &keys));  // keys, or the lists of both ray kinds
     for (uint32_t b = 0; b < depth; ++b) {
         BounceBufs& bb = ctx->bounce[b];
         // shadow slots, then the reflection slots right behind them: the batched form traces both
@@ -1142,19 +1132,26 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
         RSH_TRY(ensure_buf(ctx, bb.surf_nrm, 16ull * npix));
     }
     void* cnt_acc;
-    RSH_TRY(ensure(ctx, "frame_counts", 8ull * 2 * (depth + 1), &cnt_acc));
+    // per bounce (rays, chunks) of the shadow and of the reflection batch, then a work ticket per launch of rays
+    // alone (the primary rays' and two a bounce)
+    const size_t fc_bytes = 16ull * (depth + 1);
+    RSH_TRY(ensure(ctx, "frame_counts", fc_bytes + 4ull * (2 * depth + 1), &cnt_acc));
     uint32_t* fc = static_cast<uint32_t*>(cnt_acc);
-    RSH_CUDA(cudaMemsetAsync(fc, 0, 8ull * 2 * (depth + 1), s));
+    uint32_t* tickets = fc + 4 * (depth + 1);
+    unsigned long long* pairs = fused ? nullptr : ctx->d_stats + STAT_CAND;
+    RSH_CUDA(cudaMemsetAsync(fc, 0, fc_bytes + 4ull * (2 * depth + 1), s));
     RSH_CUDA(cudaEventRecord(ctx->ev[0], s));
     int th = stage_begin(ctx, RSH_STAGE_PRIMARY, s);
     rsh_ray* prays = static_cast<rsh_ray*>(ctx->prim_rays.ptr);
     unsigned long long* phits = static_cast<unsigned long long*>(ctx->prim_hits.ptr);
     uint32_t* ppix = static_cast<uint32_t*>(ctx->prim_pix.ptr);
     RSH_CUDA(launch_raygen_primary(to_camp(ctx->cam), W, H, prays, ppix, s));
-    if (fused) {
+    if (alone) {
+        RSH_TRY(trace_alone(ctx, sc, prays, np, nullptr, nullptr, false, nullptr, phits, tickets, pairs, s));
+    } else if (fused) {
         rsh_batch_segment seg{sc, prays, np, 0, reinterpret_cast<uint64_t*>(phits), nullptr};
         ctx->timers_paused = true;  // the primary window times the whole primary pass
-        const rsh_status pst = batch_trace_ordered(ctx, seg, s);  // tile order is already coherent
+        const rsh_status pst = batch_trace(ctx, &seg, 1, s, false);
         ctx->timers_paused = false;
         RSH_TRY(pst);
     } else {
@@ -1194,7 +1191,26 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
         uint32_t* sflags = static_cast<uint32_t*>(bb.shadow_flags.ptr);
         rsh_ray* rrays = srays + (size_t)npix * LS;
         unsigned long long* rhits = static_cast<unsigned long long*>(bb.refl_hits.ptr);
-        if (fused) {
+        if (alone) {
+            RayOut so, ro;
+            so.ids = static_cast<uint32_t*>(keys);
+            so.count = fc + 4 * b;
+            so.flags = sflags;
+            ro.ids = so.ids + (size_t)npix * LS;
+            ro.count = fc + 4 * b + 2;
+            ro.hits = rhits;
+            th = stage_begin(ctx, RSH_STAGE_RAYGEN, s);
+            RSH_CUDA(launch_raygen_shadow(spos, snrm, W, H, lp, ctx->cfg.epsilon, hp_s, srays, nullptr, s, so));
+            RSH_CUDA(launch_raygen_reflect(spos, snrm, incident, ctx->cam.eye, W, H, ctx->cfg.epsilon,
+                                           ctx->cfg.reflect_jitter, ctx->cfg.seed, b, hp_r, rrays, nullptr, s, ro));
+            stage_end(ctx, th, s);
+            th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
+            RSH_TRY(trace_alone(ctx, sc, rrays, npix, ro.ids, ro.count, false, nullptr, rhits, tickets + 1 + 2 * b,
+                                pairs, s));
+            RSH_TRY(trace_alone(ctx, sc, srays, npix * LS, so.ids, so.count, true, sflags, nullptr,
+                                tickets + 2 + 2 * b, pairs, s));
+            stage_end(ctx, th, s);
+        } else if (fused) {
             // both batches of the bounce in one batched call: 2 segments, one persistent launch; ray
             // generation writes the batch's keys, segment counts and prefilled results itself
             rsh_batch_segment segs[2] = {
@@ -1202,7 +1218,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
                 {sc, rrays, npix, 0, reinterpret_cast<uint64_t*>(rhits), nullptr}};
             BatchKeyLayout kl;
             RSH_TRY(batch_key_layout(ctx, segs, 2, kl));
-            BatchKeyOut bs, br;
+            RayOut bs, br;
             bs.keys = kl.keys + kl.start[0];
             bs.tag = 0u;
             bs.drop = kl.hash_drop;
@@ -1277,7 +1293,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     }
     RSH_CUDA(cudaEventRecord(ctx->ev[3], s));
     // counters (async; read by rsh_frame_stats_get)
-    RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 16, fc, 8ull * 2 * (depth + 1), cudaMemcpyDeviceToHost, s));
+    RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 16, fc, fc_bytes, cudaMemcpyDeviceToHost, s));
     RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 256, ctx->d_stats, 8 * (STAT_CAND + 1), cudaMemcpyDeviceToHost, s));
     ctx->stats.primary_rays = (uint64_t)W * H;
     return RSH_OK;
@@ -1303,7 +1319,8 @@ rsh_status rsh_frame_stats_get(rsh_ctx* ctx, rsh_frame_stats* out) {
     const uint32_t* fc = ctx->h_pinned + 16;
     for (uint32_t b = 0; b < ctx->fdepth; ++b) {
         st.shadow_rays += fc[4 * b];
-        st.chunks += fc[4 * b + 1] + fc[4 * b + 3];
+        // rays alone are not cut into runs: a run each
+        st.chunks += ctx->falone ? fc[4 * b] + fc[4 * b + 2] : fc[4 * b + 1] + fc[4 * b + 3];
         st.reflection_rays += fc[4 * b + 2];
     }
     unsigned long long d[STAT_CAND + 1];

@@ -72,6 +72,7 @@ struct rsh_ctx {
     rsh_camera cam{};
     bool cam_set = false;
     // frame state
+    bool falone = false;  // the frame's rays were traced alone
     uint32_t fw = 0, fh = 0, fdepth = 0, flights = 0;  // flights: shadow slots per pixel (lights x samples)
     std::vector<BounceBufs> bounce;
     rsh::DevBuf prim_rays, prim_hits, prim_pix, surf0_pos, surf0_nrm;
@@ -115,17 +116,30 @@ struct BatchKeyLayout {
     HashP hp[2]{};
 };
 rsh_status batch_key_layout(rsh_ctx* ctx, const rsh_batch_segment* segments, uint32_t count, BatchKeyLayout& out);
-// One segment of rays already in a coherent order, traced in that order (rays-only kernel); adds to the
-// test counters.
-rsh_status batch_trace_ordered(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t stream);
+// Whether a scene's rays in the batched form go alone from the root (no packets), and whether the batched form
+// takes the scene at all.
+bool batch_alone(const rsh_ctx* ctx, const rsh_scene* sc);
+rsh_status check_alone(rsh_ctx* ctx, const rsh_scene* sc);
+// A batched call whose segments' rays ray generation has listed (trimmed ids and their device counts) and whose
+// results it has prefilled: no hash, no sort. Every segment's rays must go alone.
+struct SegList {
+    const uint32_t* ids;
+    const uint32_t* count;  // null: every slot, ids unused
+};
+rsh_status batch_trace_listed(rsh_ctx* ctx, const rsh_batch_segment* segments, const SegList* lists, uint32_t count,
+                              cudaStream_t stream);
+// The plain path's rays alone (rsh_trace_rays at plain_ray_level >= 1).
+rsh_status trace_plain(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t stream);
 
 // ctx->d_stats word of a frame's (ray, cluster) pairs: past the words a frame zeroes again after its primary
 // rays (the pairs cover them, the test counts do not)
 constexpr uint32_t STAT_CAND = 8;
-// The rays of one batch against one scene, each alone from the root of its box tree (batch.cu).
-rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, const uint32_t* sorted_ids, uint32_t n,
+// The rays of one segment alone from the root of the scene's box tree (batch.cu), in one launch: the slots
+// ids[0 .. *d_count), whose results are prefilled, or (ids null) every slot, the results of empty ones written
+// too. ticket: a zeroed device word.
+rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
-                       unsigned long long* cand_pairs, cudaStream_t s);
+                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s);
 
 // One secondary batch through compress -> sort -> decompress -> build -> traverse -> intersect.
 // keys: per slot (RSH_KEY_NONE = no ray); rays indexed by slot. Output flags/hits indexed by slot

@@ -677,14 +677,18 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
     // lane: the owner's best hit key (closest hit), occluded (any hit), helpers still on a subtree of it
     __shared__ unsigned long long sh_best[SHARE ? FW : 1][32];
     __shared__ uint32_t sh_occ[SHARE ? FW : 1][32], sh_pend[SHARE ? FW : 1][32];
+    __shared__ uint32_t s_rays, s_ended;  // a.valid: the block's rays, its warps that have ended
     const uint32_t lane = lane_id();
-    const uint32_t nrays = ONE ? dev_count(a.d_rays, a.ordered_n) : 0u;
-    const uint32_t units = ONE ? (nrays + U - 1u) / U : dev_count(a.d_units, a.units_max);
+    if (a.valid) {
+        if (threadIdx.x == 0) s_rays = s_ended = 0u;
+        __syncthreads();
+    }
+    const uint32_t units = ONE ? (dev_count(a.one.count, a.one.n) + U - 1u) / U : dev_count(a.d_units, a.units_max);
     const uint32_t tail = min(units, (uint32_t)RSH_TAIL_PER_WARP * gridDim.x * FW);
     const uint32_t head = units - tail, tickets = head + RSH_TAIL_SPLIT * tail;
     uint32_t ntests = 0, ttests = 0;  // the lane's counts, flushed to the launch's counters before 2^31
     uint32_t ncand = 0;               // ONE: clusters whose triangles the lane tested
-    // the warp's current unit: sorted rays [nk, nend) of segment cs
+    // the warp's current unit: rays [nk, nend) of segment cs, in its order
     uint32_t nk = 0, nend = 0, cs = 0;
     bool drained = false;
     // the lane's ray
@@ -768,60 +772,66 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                     lo = (h % RSH_TAIL_SPLIT) * (U / RSH_TAIL_SPLIT);
                     hi = lo + U / RSH_TAIL_SPLIT;
                 }
-                nk = u * U + lo;
-                nend = u * U + hi;
-                if (!ONE) cs = find_segment(a.segs, a.nseg, u);
+                if (ONE) {
+                    nk = u * U + lo;
+                    nend = min(u * U + hi, dev_count(a.one.count, a.one.n));
+                } else {
+                    cs = find_segment(a.segs, a.nseg, u);
+                    const FusedSeg& sg = a.segs[cs];
+                    nk = (u - sg.unit_begin) * U;
+                    nend = min(nk + hi, sg.n);
+                    nk += lo;
+                }
+                if (nk >= nend) continue;  // a piece past the segment's last ray
             }
             const uint32_t k = nk + __popc(need & lanemask_lt());
+            bool ray = false;
             if (!has && k < nend) {
-                // ONE: the first nrays sorted slots, or the rays in their own order; SEGS: the padded layout, whose
-                // padding slots hold INVALID_ID
-                uint32_t id = INVALID_ID;
-                if (ONE) {
-                    if (k < nrays) id = a.sorted_ids ? __ldg(a.sorted_ids + k) : k;
-                    if (id >= a.ordered_n) id = INVALID_ID;
-                } else {
-                    id = __ldg(a.sorted_ids + k);
-                }
-                if (id != INVALID_ID) {
-                    const FusedSeg& sg = seg_of(cs);
-                    if (!ONE) id -= sg.slot_base;
+                const FusedSeg& sg = seg_of(cs);
+                uint32_t id = sg.ids ? __ldg(sg.ids + k) : k;
+                if (!ONE) id -= sg.slot_base;
+                if (id < sg.slots) {
                     float4 o, d;
                     load_ray(sg.rays, id, o, d);
-                    if (d.w > o.w) {
-                        const bool sany = OF == ANY1 ? true : OF == CLOSEST1 ? false : sg.any_hit != 0u;
-                        if (sg.levels == 0u) {
-                            // a scene without triangles has no tree: the ray misses
+                    const bool sany = OF == ANY1 ? true : OF == CLOSEST1 ? false : sg.any_hit != 0u;
+                    ray = d.w > o.w;
+                    if (!ray || sg.levels == 0u) {
+                        // no ray, or a scene without triangles (no tree): a miss
+                        if (ray || !sg.ids) {
                             if (sany) sg.flags[id] = 0u;
                             else sg.hits[id] = RSH_HIT_NONE;
-                        } else {
-                            slot = id;
-                            if (!ONE) {
-                                seg = cs;
-                                any_v = sany;
-                                nodes_v = sg.wnodes;
-                                tris_v = sg.wtris;
-                            }
-                            ox = o.x;
-                            oy = o.y;
-                            oz = o.z;
-                            tmin = o.w;
-                            tcur = d.w;
-                            ix = safe_rcp(d.x);
-                            iy = safe_rcp(d.y);
-                            iz = safe_rcp(d.z);
-                            oix = ox * ix;
-                            oiy = oy * iy;
-                            oiz = oz * iz;
-                            w = wt_setup(o, d);
-                            best = RSH_HIT_NONE;
-                            oct = (ix < 0.f ? 1u : 0u) | (iy < 0.f ? 2u : 0u) | (iz < 0.f ? 4u : 0u);
-                            top = sg.wnroot;
-                            sp = 0;
-                            has = true;
                         }
+                    } else {
+                        slot = id;
+                        if (!ONE) {
+                            seg = cs;
+                            any_v = sany;
+                            nodes_v = sg.wnodes;
+                            tris_v = sg.wtris;
+                        }
+                        ox = o.x;
+                        oy = o.y;
+                        oz = o.z;
+                        tmin = o.w;
+                        tcur = d.w;
+                        ix = safe_rcp(d.x);
+                        iy = safe_rcp(d.y);
+                        iz = safe_rcp(d.z);
+                        oix = ox * ix;
+                        oiy = oy * iy;
+                        oiz = oz * iz;
+                        w = wt_setup(o, d);
+                        best = RSH_HIT_NONE;
+                        oct = (ix < 0.f ? 1u : 0u) | (iy < 0.f ? 2u : 0u) | (iz < 0.f ? 4u : 0u);
+                        top = sg.wnroot;
+                        sp = 0;
+                        has = true;
                     }
                 }
+            }
+            if (a.valid) {  // counted in shared memory: a per-lane count would cost a register all along
+                const uint32_t c = __popc(__ballot_sync(0xffffffffu, ray));
+                if (lane == 0 && c) atomicAdd(&s_rays, c);
             }
             nk = min(nend, nk + __popc(need));
         }
@@ -1031,6 +1041,17 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
             }
         }
     }
+    if (a.valid && lane == 0) {
+        __threadfence_block();
+        if (atomicAdd(&s_ended, 1u) == FW - 1u) {  // the block's last warp
+            __threadfence_block();
+            const uint32_t c = *(volatile uint32_t*)&s_rays;
+            if (c) {
+                atomicAdd(a.valid, c);
+                atomicAdd(a.valid + 1, c);
+            }
+        }
+    }
     unsigned long long nt = ntests, tt = ttests, nc = ncand;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -1054,7 +1075,8 @@ static cudaError_t launch_fused_rays_s(const FusedArgs& a, cudaStream_t s) {
     if (per_sm < 1) per_sm = 1;
     if (a.blocks_per_sm && (int)a.blocks_per_sm < per_sm) per_sm = (int)a.blocks_per_sm;
     uint32_t grid = (uint32_t)(sms * per_sm);
-    const uint32_t need = (a.units_max + FW - 1) / FW;
+    const uint32_t most = OF == SEGS ? a.units_max : (a.one.n + U - 1) / U;
+    const uint32_t need = (most + FW - 1) / FW;
     if (need < grid) grid = need > 0 ? need : 1;
     k_fused_rays<U, SHARE, OF><<<grid, FW * 32, 0, s>>>(a);
     note_launch();
@@ -1067,7 +1089,6 @@ static cudaError_t launch_fused_rays_u(const FusedArgs& a, cudaStream_t s) {
 
 template <int P>
 static cudaError_t launch_fused_p(const FusedArgs& a, cudaStream_t s) {
-    if (a.rays_only) return launch_fused_rays_u<RSH_RAYS_UNIT, SEGS>(a, s);  // units of RSH_RAYS_UNIT rays
     const size_t smem = sizeof(FusedSmem<P>) * FW;
     cudaError_t e = cudaFuncSetAttribute(k_fused<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1085,9 +1106,12 @@ static cudaError_t launch_fused_p(const FusedArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_rays_one(FusedArgs a, cudaStream_t s) {
-    if (a.ordered_n == 0) return cudaSuccess;
-    a.units_max = (a.ordered_n + RSH_RAYS_UNIT - 1) / RSH_RAYS_UNIT;
+cudaError_t launch_rays_segs(const FusedArgs& a, cudaStream_t s) {
+    return launch_fused_rays_u<RSH_RAYS_UNIT, SEGS>(a, s);
+}
+
+cudaError_t launch_rays_one(const FusedArgs& a, cudaStream_t s) {
+    if (a.one.n == 0) return cudaSuccess;
     return a.one.any_hit ? launch_fused_rays_u<RSH_RAYS_UNIT, ANY1>(a, s)
                          : launch_fused_rays_u<RSH_RAYS_UNIT, CLOSEST1>(a, s);
 }

@@ -48,27 +48,29 @@ struct CameraP {
 // ---- raygen + hash (raygen.cu)
 cudaError_t launch_raygen_primary(const CameraP& cam, uint32_t w, uint32_t h, rsh_ray* rays,
                                   uint32_t* pixel_of_ray, cudaStream_t s);
-// Keys of a batched call written by ray generation itself (the batched form of a frame): key = tag |
-// (ray hash >> drop) or RSH_KEY_NONE, the segment's ray count (one atomic per block into *count), and the
-// segment's results prefilled (flags 0 for an any-hit segment, hits RSH_HIT_NONE otherwise), so the batch
-// need not read the rays back to hash them.
-struct BatchKeyOut {
-    uint32_t* keys = nullptr;      // the batch's key array at the segment's first slot; null: not used
+// What ray generation writes for a traversal beside the rays, with the segment's results prefilled (flags 0 for
+// an any-hit segment, hits RSH_HIT_NONE otherwise) and its ray count added to *count (one atomic per block):
+//   ids   the slots that hold a ray, appended block by block: a trimmed list for rays traced alone, in the order
+//         of the pixels, with no key, compression or sort;
+//   keys  the keys of a batched call whose rays use packets: tag | (ray hash >> drop) or RSH_KEY_NONE.
+struct RayOut {
+    uint32_t* ids = nullptr;
+    uint32_t* keys = nullptr;      // the batch's key array at the segment's first slot
     uint32_t tag = 0;
     uint32_t drop = 0;
     HashP hp{};                    // the segment scene's hash (tag 0)
-    uint32_t* count = nullptr;
+    uint32_t* count = nullptr;     // null: the caller keys or counts the rays itself
     uint32_t* flags = nullptr;
     unsigned long long* hits = nullptr;
 };
 cudaError_t launch_raygen_shadow(const float4* spos, const float4* snrm, uint32_t w, uint32_t h,
                                  const LightsP& lights, float eps, const HashP& hp, rsh_ray* rays,
-                                 uint32_t* keys, cudaStream_t s, const BatchKeyOut& bk = BatchKeyOut());
+                                 uint32_t* keys, cudaStream_t s, const RayOut& out = RayOut());
 cudaError_t launch_raygen_reflect(const float4* spos, const float4* snrm, const rsh_ray* prev,
                                   const float eye[3], uint32_t w, uint32_t h, float eps,
                                   float jitter, uint32_t seed, uint32_t bounce, const HashP& hp,
                                   rsh_ray* rays, uint32_t* keys, cudaStream_t s,
-                                  const BatchKeyOut& bk = BatchKeyOut());
+                                  const RayOut& out = RayOut());
 cudaError_t launch_raygen_refract(const float4* spos, const float4* snrm, const rsh_ray* prev, const float eye[3],
                                   uint32_t w, uint32_t h, float eps, float eta, const HashP& hp, rsh_ray* rays,
                                   uint32_t* keys, cudaStream_t s);
@@ -217,42 +219,44 @@ struct FusedSeg {
     uint32_t levels;
     uint32_t lvl_off[16];
     uint32_t lvl_size[16];
-    uint32_t ray_begin, ray_end;   // sorted ray range of this segment
-    uint32_t unit_begin;           // first work unit (level-1 node) of this segment
+    uint32_t unit_begin;           // first work unit of this segment
     uint32_t any_hit;
     uint32_t ray_level;            // object-tree level at and below which rays descend individually
     const rsh_ray* rays;           // the segment's own rays (slot - slot_base); read in place by the rays-only kernel
     uint32_t* flags;               // indexed by slot - slot_base
     unsigned long long* hits;
-    uint32_t slot_base;
+    uint32_t slot_base;            // subtracted from an id: ids of a sorted batch count over all segments
+    // the rays-only kernel: the segment's ray slots in the order they are traced, n of them (null: every slot
+    // 0 .. n - 1, and the kernel also writes the result of a slot without a ray)
+    const uint32_t* ids;
+    uint32_t n;
+    uint32_t slots;                // the segment's ray slots: an id outside them is skipped
+    const uint32_t* count;         // device count of ids (null: n); at most n
 };
 struct FusedArgs {
     const rsh_node* nodes;
     uint32_t node_off[4];
     uint32_t packet;
     const rsh_ray* rays;
-    const uint32_t* sorted_ids;    // launch_rays_one: may be null (the rays in their own order)
-    const FusedSeg* segs;          // device
+    const uint32_t* sorted_ids;    // packet kernel
+    const FusedSeg* segs;          // device; rays-only: count already folded into n
     uint32_t nseg;
     uint32_t units_max;
     const uint32_t* d_units;       // device count of units
     uint32_t* work;
-    uint32_t rays_only;            // every segment's switch level >= its tree depth: no packet phase
     uint32_t blocks_per_sm;        // CTAs per SM of the launch (0: as many as fit)
     uint32_t share_tail;           // rays-only kernel: a drained warp shares its last rays among its lanes
     unsigned long long* node_tests;
     unsigned long long* tri_tests;
     uint32_t* err;
-    // launch_rays_one: the one segment (slot_base 0), its ray slots, the device count of sorted_ids entries (null:
-    // ordered_n) and, if wanted, the count of (ray, cluster) pairs whose triangles were tested
-    FusedSeg one;
-    uint32_t ordered_n;
-    const uint32_t* d_rays;
-    unsigned long long* cand_pairs;
+    FusedSeg one;                      // launch_rays_one: the one segment (slot_base 0)
+    uint32_t* valid;                   // rays-only: the rays traced are added to valid[0] and valid[1] (null: not)
+    unsigned long long* cand_pairs;    // launch_rays_one: counts (ray, cluster) pairs tested (null: not counted)
 };
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t s);
-// The rays of one segment alone from the root (no packets, no segment table).
-cudaError_t launch_rays_one(FusedArgs a, cudaStream_t s);
+// Rays alone from the root: the segments of the table / one segment, from the arguments.
+cudaError_t launch_rays_segs(const FusedArgs& a, cudaStream_t s);
+cudaError_t launch_rays_one(const FusedArgs& a, cudaStream_t s);
 // rays per work unit of the rays-only kernel (a multiple of 64, at most 256: job words hold 8 bits)
 #ifndef RSH_RAYS_UNIT
 #define RSH_RAYS_UNIT 64

@@ -73,111 +73,120 @@ RSH_DEV v3 soft_sample_pos(v3 lp, v3 d, uint32_t k) {
               (lp.z + (a0.z * ca) * 0.125f) + (a1.z * cb) * 0.125f};
 }
 
-// The batch keys of a block's slots (BatchKeyOut): each slot's key and prefilled result, and the block's
-// count of rays in one atomic. Every thread of the block calls it (it synchronises the block).
-RSH_DEV void batch_key_out(const BatchKeyOut& bk, uint32_t slot, bool in_range, bool valid, float4 o, float4 d) {
-    __shared__ uint32_t s_cnt;
-    if (threadIdx.x == 0) s_cnt = 0u;
+// A block's share of a segment's ray count and, in list mode, of its id list: reserves `rays` entries with one
+// atomic and returns the first to every thread. Every thread of the block calls it.
+RSH_DEV uint32_t reserve_rays(uint32_t* count, uint32_t rays) {
+    __shared__ uint32_t s_base;
+    if (threadIdx.x == 0) s_base = rays ? atomicAdd(count, rays) : 0u;
     __syncthreads();
-    if (in_range) {
-        bk.keys[slot] = valid ? bk.tag | (ray_hash(o.x, o.y, o.z, d.x, d.y, d.z, bk.hp, 0u) >> bk.drop)
-                              : RSH_KEY_NONE;
-        if (bk.flags) bk.flags[slot] = 0u;
-        else bk.hits[slot] = RSH_HIT_NONE;
-    }
-    const uint32_t b = __ballot_sync(0xffffffffu, in_range && valid);
-    if (lane_id() == 0 && b) atomicAdd(&s_cnt, (uint32_t)__popc(b));
-    __syncthreads();
-    if (threadIdx.x == 0 && s_cnt) atomicAdd(bk.count, s_cnt);
+    return s_base;
 }
 
 // One thread per pixel: the pixel's surface point and normal are read and the normal normalised once,
 // then its V = L x S slots are written (slot = x + W (v + V y), RayTracer.cu:700-702 with S samples per
-// light), each with the same arithmetic as a thread per slot would use. The block's rays are counted once
-// (BatchKeyOut). The light positions are copied to shared memory first: indexing the parameter bank with
-// the light number is a constant load with a register index, which the SM issues through its narrow
-// address-divergence pipe, and three of those per slot made that pipe the kernel's bound. 12 blocks per SM
-// (at most 40 registers, no spills) keep enough warps in flight to cover the surface reads.
-__global__ void __launch_bounds__(128, 12) k_raygen_shadow(const float4* __restrict__ spos,
-                                                           const float4* __restrict__ snrm, uint32_t w, uint32_t h,
-                                                           LightsP lights, float eps, HashP hp, rsh_ray* rays,
-                                                           uint32_t* keys, BatchKeyOut bk) {
-    __shared__ uint32_t s_cnt;
+// light), each with the same arithmetic as a thread per slot would use. The block's rays are counted once and
+// listed warp by warp, a light's 32 pixels together (RayOut). The light positions are copied to shared memory
+// first: indexing the parameter bank with the light number is a constant load with a register index, which the
+// SM issues through its narrow address-divergence pipe, and three of those per slot made that pipe the kernel's
+// bound. 12 blocks per SM (at most 40 registers, no spills) keep enough warps in flight to cover the surface
+// reads.
+constexpr uint32_t RS_THREADS = 128;
+__global__ void __launch_bounds__(RS_THREADS, 12)
+k_raygen_shadow(const float4* __restrict__ spos, const float4* __restrict__ snrm, uint32_t w, uint32_t h,
+                LightsP lights, float eps, HashP hp, rsh_ray* rays, uint32_t* keys, RayOut out) {
     __shared__ float s_lp[8 * 3];
+    __shared__ uint32_t s_bal[RS_THREADS / 32][8 * 16];  // per warp and light sample: the lanes with a ray
+    __shared__ uint32_t s_cnt[RS_THREADS / 32];
     const uint32_t L = lights.count, S = lights.samples ? lights.samples : 1u, V = L * S;
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x, lane = lane_id(), warp = threadIdx.x >> 5;
     const bool in_range = pix < w * h;
     const bool a32 = (reinterpret_cast<uintptr_t>(rays) & 31u) == 0u;
-    uint32_t nvalid = 0;
-    if (threadIdx.x == 0) s_cnt = 0u;
+    uint32_t nvalid = 0;  // the warp's rays
     if (threadIdx.x < 3u * L) s_lp[threadIdx.x] = (&lights.pos[0][0])[threadIdx.x];
     __syncthreads();
-    if (in_range) {
-        const uint32_t y = pix / w, x = pix - y * w;
-        const float4 p4 = __ldg(spos + pix);
-        const bool surface = p4.w != 0.0f;
-        const v3 p = mk3(p4);
-        const v3 nn = surface ? norm3(mk3(__ldg(snrm + pix))) : v3{0.f, 0.f, 0.f};
-        for (uint32_t v = 0; v < V; ++v) {
-            const uint32_t slot = x + w * (v + V * y);
-            const uint32_t l = S == 1u ? v : v / S, sm = S == 1u ? 0u : v % S;
-            bool valid = false;
-            float4 ro = make_float4(0.f, 0.f, 0.f, 0.f), rd = make_float4(0.f, 0.f, 0.f, -1.f);
-            uint32_t key = RSH_KEY_NONE;
-            if (surface) {
-                const v3 lp = mk3(s_lp[3u * l], s_lp[3u * l + 1u], s_lp[3u * l + 2u]);
-                const v3 vl = p - lp;
-                const float len = len3(vl);
-                const v3 d = v3{vl.x / len, vl.y / len, vl.z / len};
-                const float diffuse = dot3(d, -nn);
-                const float tmax = len - 2.0f * eps;
-                if (diffuse > 0.0f && tmax > eps) {
-                    v3 src = lp, dir = d;
-                    float tm = tmax;
-                    bool ok = true;
-                    if (S > 1) {  // a sample of the 4x4 grid: its own origin, direction and interval
-                        src = soft_sample_pos(lp, d, sm);
-                        const v3 vs = p - src;
-                        const float ls = len3(vs);
-                        dir = v3{vs.x / ls, vs.y / ls, vs.z / ls};
-                        tm = ls - 2.0f * eps;
-                        ok = tm > eps;
-                    }
-                    if (ok) {
-                        const v3 o = src + dir * eps;
-                        ro = make_float4(o.x, o.y, o.z, eps);
-                        rd = make_float4(dir.x, dir.y, dir.z, tm);
-                        key = keys ? ray_hash(o.x, o.y, o.z, dir.x, dir.y, dir.z, hp, v) : 0u;
-                        valid = true;
-                    }
+    const uint32_t y = pix / w, x = pix - y * w;
+    const float4 p4 = in_range ? __ldg(spos + pix) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool surface = p4.w != 0.0f;
+    const v3 p = mk3(p4);
+    const v3 nn = surface ? norm3(mk3(__ldg(snrm + pix))) : v3{0.f, 0.f, 0.f};
+    for (uint32_t v = 0; v < V; ++v) {
+        const uint32_t slot = x + w * (v + V * y);
+        const uint32_t l = S == 1u ? v : v / S, sm = S == 1u ? 0u : v % S;
+        bool valid = false;
+        float4 ro = make_float4(0.f, 0.f, 0.f, 0.f), rd = make_float4(0.f, 0.f, 0.f, -1.f);
+        uint32_t key = RSH_KEY_NONE;
+        if (surface) {
+            const v3 lp = mk3(s_lp[3u * l], s_lp[3u * l + 1u], s_lp[3u * l + 2u]);
+            const v3 vl = p - lp;
+            const float len = len3(vl);
+            const v3 d = v3{vl.x / len, vl.y / len, vl.z / len};
+            const float diffuse = dot3(d, -nn);
+            const float tmax = len - 2.0f * eps;
+            if (diffuse > 0.0f && tmax > eps) {
+                v3 src = lp, dir = d;
+                float tm = tmax;
+                bool ok = true;
+                if (S > 1) {  // a sample of the 4x4 grid: its own origin, direction and interval
+                    src = soft_sample_pos(lp, d, sm);
+                    const v3 vs = p - src;
+                    const float ls = len3(vs);
+                    dir = v3{vs.x / ls, vs.y / ls, vs.z / ls};
+                    tm = ls - 2.0f * eps;
+                    ok = tm > eps;
+                }
+                if (ok) {
+                    const v3 o = src + dir * eps;
+                    ro = make_float4(o.x, o.y, o.z, eps);
+                    rd = make_float4(dir.x, dir.y, dir.z, tm);
+                    key = keys ? ray_hash(o.x, o.y, o.z, dir.x, dir.y, dir.z, hp, v) : 0u;
+                    valid = true;
                 }
             }
+        }
+        if (in_range) {
             // an empty slot holds an explicit no-ray (tmax < tmin) for consumers without keys
             store_ray32(rays, slot, ro, rd, a32);
             if (keys) keys[slot] = key;
-            if (bk.keys) {
-                bk.keys[slot] = valid ? bk.tag | (ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, bk.hp, 0u) >> bk.drop)
-                                      : RSH_KEY_NONE;
-                if (bk.flags) bk.flags[slot] = 0u;
-                else bk.hits[slot] = RSH_HIT_NONE;
+            if (out.count) {
+                if (out.keys)
+                    out.keys[slot] = valid ? out.tag | (ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, out.hp, 0u) >> out.drop)
+                                           : RSH_KEY_NONE;
+                if (out.flags) out.flags[slot] = 0u;
+                else out.hits[slot] = RSH_HIT_NONE;
             }
-            nvalid += valid ? 1u : 0u;
+        }
+        if (out.count) {
+            const uint32_t b = __ballot_sync(0xffffffffu, valid);
+            nvalid += __popc(b);
+            if (out.ids && lane == 0) s_bal[warp][v] = b;
         }
     }
-    if (bk.keys) {
-        const uint32_t c = __reduce_add_sync(0xffffffffu, nvalid);
-        if (lane_id() == 0 && c) atomicAdd(&s_cnt, c);
+    if (out.count) {
+        if (lane == 0) s_cnt[warp] = nvalid;
         __syncthreads();
-        if (threadIdx.x == 0 && s_cnt) atomicAdd(bk.count, s_cnt);
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < RS_THREADS / 32; ++q) {
+            if (q < warp) before += s_cnt[q];
+            all += s_cnt[q];
+        }
+        uint32_t at = reserve_rays(out.count, all) + before;
+        if (out.ids)
+            for (uint32_t v = 0; v < V; ++v) {
+                const uint32_t b = s_bal[warp][v];
+                if ((b >> lane) & 1u) out.ids[at + __popc(b & lanemask_lt())] = x + w * (v + V * y);
+                at += __popc(b);
+            }
     }
 }
 
 cudaError_t launch_raygen_shadow(const float4* spos, const float4* snrm, uint32_t w, uint32_t h,
                                  const LightsP& lights, float eps, const HashP& hp, rsh_ray* rays,
-                                 uint32_t* keys, cudaStream_t s, const BatchKeyOut& bk) {
+                                 uint32_t* keys, cudaStream_t s, const RayOut& out) {
     const uint32_t n = w * h;
     if (n == 0 || lights.count == 0) return cudaSuccess;
-    k_raygen_shadow<<<(n + 127u) / 128u, 128, 0, s>>>(spos, snrm, w, h, lights, eps, hp, rays, keys, bk);
+    k_raygen_shadow<<<(n + RS_THREADS - 1u) / RS_THREADS, RS_THREADS, 0, s>>>(spos, snrm, w, h, lights, eps, hp, rays,
+                                                                              keys, out);
     note_launch();
     return cudaGetLastError();
 }
@@ -208,7 +217,8 @@ RSH_DEV v3 sphere_sample(uint32_t seed, uint32_t slot, uint32_t bounce) {
 __global__ void k_raygen_reflect(const float4* __restrict__ spos, const float4* __restrict__ snrm,
                                  const rsh_ray* __restrict__ prev, v3 eye, uint32_t n, float eps,
                                  float jitter, uint32_t seed, uint32_t bounce, HashP hp,
-                                 rsh_ray* rays, uint32_t* keys, BatchKeyOut bk) {
+                                 rsh_ray* rays, uint32_t* keys, RayOut out) {
+    __shared__ uint32_t s_cnt[8];
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in_range = slot < n;
     const bool a32 = (reinterpret_cast<uintptr_t>(rays) & 31u) == 0u;
@@ -250,17 +260,36 @@ __global__ void k_raygen_reflect(const float4* __restrict__ spos, const float4* 
         if (!valid) store_ray32(rays, slot, ro, rd, a32);
         if (keys) keys[slot] = key;
     }
-    if (bk.keys) batch_key_out(bk, slot, in_range, valid, ro, rd);
+    if (out.count) {
+        if (in_range) {
+            if (out.keys)
+                out.keys[slot] = valid ? out.tag | (ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, out.hp, 0u) >> out.drop)
+                                       : RSH_KEY_NONE;
+            if (out.flags) out.flags[slot] = 0u;
+            else out.hits[slot] = RSH_HIT_NONE;
+        }
+        const uint32_t warp = threadIdx.x >> 5, b = __ballot_sync(0xffffffffu, valid);
+        if (lane_id() == 0) s_cnt[warp] = __popc(b);
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q) {  // 256 threads
+            if (q < warp) before += s_cnt[q];
+            all += s_cnt[q];
+        }
+        const uint32_t at = reserve_rays(out.count, all) + before;
+        if (out.ids && valid) out.ids[at + __popc(b & lanemask_lt())] = slot;
+    }
 }
 
 cudaError_t launch_raygen_reflect(const float4* spos, const float4* snrm, const rsh_ray* prev,
                                   const float eye[3], uint32_t w, uint32_t h, float eps,
                                   float jitter, uint32_t seed, uint32_t bounce, const HashP& hp,
-                                  rsh_ray* rays, uint32_t* keys, cudaStream_t s, const BatchKeyOut& bk) {
+                                  rsh_ray* rays, uint32_t* keys, cudaStream_t s, const RayOut& out) {
     const uint32_t n = w * h;
     if (n == 0) return cudaSuccess;
     k_raygen_reflect<<<(n + 255u) / 256u, 256, 0, s>>>(spos, snrm, prev, v3{eye[0], eye[1], eye[2]}, n,
-                                                     eps, jitter, seed, bounce, hp, rays, keys, bk);
+                                                     eps, jitter, seed, bounce, hp, rays, keys, out);
     note_launch();
     return cudaGetLastError();
 }

@@ -164,8 +164,27 @@ constexpr size_t kDepth = 2;
 rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
     cudaStream_t st = s->stream;
     std::vector<rsh_batch_segment> segs;
+    std::vector<SegList> lists;
     segs.reserve(rec.act.size() * 2);
     rec.seg_at.clear();
+    // Rays alone (no scene of the step uses packets below the root): ray generation lists each segment's rays,
+    // counts them and prefills their results, so the batch neither reads the rays back to hash them nor sorts
+    // them (k_batch_prep alone was 0.9 of the 13.9 ms of kernels of a burst of 16 requests).
+    bool alone = true;
+    uint64_t ids_total = 0;
+    for (Req* q : rec.act) {
+        alone = alone && batch_alone(s->ctx, s->scenes[q->r.scene_index]);
+        if (q->stage > 0) ids_total += (uint64_t)q->r.width * q->r.height * (q->r.light_count + 1u);
+    }
+    void *ids_buf = nullptr, *cnt_buf = nullptr;
+    RSH_TRY(ensure(s->ctx, "step_counts", 4ull * 2 * (rec.act.size() + 1), &cnt_buf));
+    uint32_t* counts = static_cast<uint32_t*>(cnt_buf);  // per segment
+    uint32_t* ids = nullptr;
+    if (alone) {
+        RSH_TRY(ensure(s->ctx, "step_ids", 4ull * (ids_total + 1), &ids_buf));
+        ids = static_cast<uint32_t*>(ids_buf);
+        RSH_CUDA(cudaMemsetAsync(counts, 0, 4ull * 2 * rec.act.size(), st));
+    }
     for (Req* q : rec.act) {
         const rsh_request& r = q->r;
         const rsh_scene* sc = s->scenes[r.scene_index];
@@ -183,9 +202,19 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
             const uint32_t np = ((W + 7) / 8) * ((H + 7) / 8) * 64;
             segs.push_back(rsh_batch_segment{sc, q->prim_rays, np, 0, reinterpret_cast<uint64_t*>(q->prim_hits),
                                              nullptr});
+            lists.push_back(SegList{nullptr, nullptr});
         } else {
             const uint32_t b = q->stage - 1;
-            // the batched call keys every segment itself: the ray generators write no keys
+            RayOut so, ro;
+            if (alone) {
+                so.ids = ids;
+                so.count = counts + segs.size();
+                so.flags = q->flags + (size_t)b * npix * L;
+                ro.ids = ids + (size_t)npix * L;
+                ro.count = counts + segs.size() + 1;
+                ro.hits = q->hits + (size_t)b * npix;
+                ids += (size_t)npix * (L + 1u);
+            }
             HashP hp_r;
             RSH_TRY(make_hash_params(sc, s->ctx->cfg, 0, hp_r));
             LightsP lp{};
@@ -193,17 +222,21 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
             lp.samples = 1;
             for (uint32_t l = 0; l < L; ++l)
                 for (int i = 0; i < 3; ++i) lp.pos[l][i] = r.lights[l].position[i];
-            RSH_CUDA(launch_raygen_shadow(q->spos, q->snrm, W, H, lp, s->ctx->cfg.epsilon, hp_r, q->srays, nullptr, st));
+            RSH_CUDA(launch_raygen_shadow(q->spos, q->snrm, W, H, lp, s->ctx->cfg.epsilon, hp_r, q->srays, nullptr,
+                                          st, so));
             const rsh_ray* prev = (b == 0) ? nullptr : q->rrays[(b - 1) & 1];
             rsh_ray* cur = q->rrays[b & 1];
             RSH_CUDA(launch_raygen_reflect(q->spos, q->snrm, prev, r.camera.eye, W, H, s->ctx->cfg.epsilon,
-                                           s->ctx->cfg.reflect_jitter, s->ctx->cfg.seed, b, hp_r, cur, nullptr, st));
+                                           s->ctx->cfg.reflect_jitter, s->ctx->cfg.seed, b, hp_r, cur, nullptr, st, ro));
             segs.push_back(rsh_batch_segment{sc, q->srays, npix * L, 1, nullptr, q->flags + (size_t)b * npix * L});
             segs.push_back(rsh_batch_segment{sc, cur, npix, 0,
                                              reinterpret_cast<uint64_t*>(q->hits + (size_t)b * npix), nullptr});
+            lists.push_back(SegList{so.ids, so.count});
+            lists.push_back(SegList{ro.ids, ro.count});
         }
     }
-    RSH_TRY(rsh_batch_trace(s->ctx, segs.data(), (uint32_t)segs.size(), st));
+    if (alone) RSH_TRY(batch_trace_listed(s->ctx, segs.data(), lists.data(), (uint32_t)segs.size(), st));
+    else RSH_TRY(rsh_batch_trace(s->ctx, segs.data(), (uint32_t)segs.size(), st));
     if (rec.cap < segs.size() + 1) {
         if (rec.pinned) cudaFreeHost(rec.pinned);
         rec.pinned = nullptr;
@@ -211,8 +244,8 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
         RSH_CUDA(cudaMallocHost(&rec.pinned, 4 * rec.cap));
     }
     // rays traced per segment (after trimming): read when the step retires
-    RSH_CUDA(cudaMemcpyAsync(rec.pinned, s->ctx->bufs["b_seg_cnt"].ptr, 4 * segs.size(), cudaMemcpyDeviceToHost,
-                             st));
+    RSH_CUDA(cudaMemcpyAsync(rec.pinned, alone ? counts : s->ctx->bufs["b_seg_cnt"].ptr, 4 * segs.size(),
+                             cudaMemcpyDeviceToHost, st));
     // advance: resolve hits into the next surface
     for (Req* q : rec.act) {
         const rsh_request& r = q->r;
