@@ -494,7 +494,7 @@ rsh_status enqueue_alone(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
         th = stage_begin(ctx, RSH_STAGE_SORT, s);
         RSH_CUDA(launch_sort_pairs(static_cast<uint32_t*>(pl.keys), nullptr, static_cast<uint32_t*>(pl.skeys),
                                    static_cast<uint32_t*>(pl.svals), pl.total, nullptr, pl.key_bits + pl.empty_bit,
-                                   pl.scr, ctx->d_err, s));
+                                   pl.scr, ctx->d_err, s, false));
         stage_end(ctx, th, s);
     }
     RSH_CUDA(cudaMemsetAsync(pl.work, 0, 16, s));

@@ -6,13 +6,18 @@
 //
 //  1. one histogram kernel reads the keys once and builds all passes' 256-bin digit histograms; its last
 //     CTA turns them into per-pass exclusive digit offsets;
-//  2. one kernel per 8-bit digit pass: each CTA takes a 3840-key tile by atomic ticket, ranks its keys
-//     stably (warp peer masks: every third item by match_any, the others from 8 ballots, 9 in a partial
-//     tile; per-warp digit counters), publishes its per-digit counts,
-//     resolves the per-digit exclusive prefix over earlier tiles by decoupled look-back (bounded spin),
-//     then scatters through shared memory so that global writes are runs of one digit. A status word
-//     holds flag and count together and nothing else is read through it, so it is published and read
-//     with relaxed (not release / acquire) accesses: no memory barrier per tile.
+//  2. one kernel per 8-bit digit pass: each CTA takes a tile by atomic ticket, ranks its keys stably (the lanes
+//     of a row of 32 keys find the others of their digit through a lane mask in shared memory, per warp and
+//     digit beside the count so far), publishes its per-digit counts, scatters keys and values into shared
+//     memory in digit order, resolves the per-digit exclusive prefix over earlier tiles by decoupled look-back
+//     (bounded spin), and writes runs of one digit. A status word holds flag and count together and nothing else
+//     is read through it, so it is published and read with relaxed (not release / acquire) accesses: no memory
+//     barrier per tile. The passes are chained (programmatic dependent launch): a pass's CTAs are placed as the
+//     ones before it leave.
+// What bounds a pass: at 16 M random pairs 102 us (2.5 TB/s of its 16 B a pair), with the shared-memory pipe at
+// 70%: a row of 32 keys costs about 44 of its cycles (random banks: ranking, counters, scatter). Eight ballots a
+// key instead of the lane mask were bound by issue slots (139 us a pass at 24 warps an SM; alternating the two
+// row by row 103 us). 16 M random 31-bit pairs: 625 us before, now 428; 20,000: 54 -> 36.
 #include <algorithm>
 
 #include "common.cuh"
@@ -21,37 +26,34 @@
 namespace rsh {
 
 namespace {
-constexpr int SR_THREADS = 256;
-constexpr int SR_WARPS = SR_THREADS / 32;
-constexpr int SR_ITEMS = 15;
-constexpr int SR_TILE = SR_THREADS * SR_ITEMS;  // 3840
 constexpr uint32_t FLAG_AGG = 1u << 30;
 constexpr uint32_t FLAG_PRE = 2u << 30;
 constexpr uint32_t VAL_MASK = (1u << 30) - 1u;
-
-#ifndef RSH_SORT_MATCH_EVERY
-#define RSH_SORT_MATCH_EVERY 3
-#endif
-#ifndef RSH_SORT_FULL8
-#define RSH_SORT_FULL8 1
-#endif
-
+// Tile shapes (threads, keys a thread, CTAs per SM): large tiles for long runs of one digit in the output and few
+// tiles to look back over; small ones where large ones would leave SMs without a tile (512 x 14 against 256 x 8:
+// 16 M random 31-bit pairs 440 / 590 us, 1 M 69 / 85, 320,000 64 / 56, 20,000 57 / 45).
+constexpr int L_T = 512, L_I = 14, L_MB = 2, S_T = 256, S_I = 8, S_MB = 6;
+constexpr uint32_t SMALL_PAIRS = 1u << 19;
+constexpr uint32_t L_TILE = L_T * L_I, S_TILE = S_T * S_I;
+inline bool small_tiles(uint32_t n_max) { return n_max <= SMALL_PAIRS; }
+inline uint32_t tile_of(uint32_t n_max) { return small_tiles(n_max) ? S_TILE : L_TILE; }
 inline uint32_t num_passes(uint32_t key_bits) { return key_bits == 0 ? 1u : (key_bits + 7u) / 8u; }
 }  // namespace
 
 // --- histograms of every pass in one read; also clears the look-back status rows of the tiles that
-// the passes will use (ceil(n / SR_TILE) rows of 256 words per pass, pass stride `stride` words)
+// the passes will use (ceil(n / tile) rows of 256 words per pass, pass stride `stride` words)
 __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
-                            const uint32_t* __restrict__ d_count, uint32_t passes,
+                            const uint32_t* __restrict__ d_count, uint32_t passes, uint32_t tile_keys,
                             uint32_t* __restrict__ hist, uint32_t* __restrict__ status, size_t stride,
                             uint32_t* __restrict__ done) {
     __shared__ uint32_t sh[4][256];
     __shared__ uint32_t s_last;
+    asm volatile("griddepcontrol.launch_dependents;");
     for (uint32_t i = threadIdx.x; i < 4u * 256u; i += blockDim.x) (&sh[0][0])[i] = 0u;
     __syncthreads();
     const uint32_t n = dev_count(d_count, n_max);
     {
-        const size_t words = (size_t)((n + SR_TILE - 1) / SR_TILE) * 256u;  // multiple of 4
+        const size_t words = (size_t)((n + tile_keys - 1) / tile_keys) * 256u;  // multiple of 4
         const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
         for (uint32_t p = 0; p < passes; ++p) {
             uint4* row = reinterpret_cast<uint4*>(status + p * stride);
@@ -144,205 +146,252 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
     }
 }
 
-__global__ void __launch_bounds__(SR_THREADS, 3)
+// One digit pass. T threads, I keys a thread; MB CTAs per SM.
+template <int T, int I>
+struct SweepSmem {
+    uint32_t keys[T * I];
+    uint32_t vals[T * I];
+    // per warp and digit, while ranking: (count so far, lanes of the row at hand) in one 64-bit word; then, in
+    // the counts' place, the tile-local position of each warp's run
+    uint2 rk[T / 32][256];
+    uint32_t gbase[256];             // global position of the tile's first key of a digit, less its local one
+    uint32_t scan[8];
+    uint32_t tile, next;
+};
+
+template <int T, int I, int MB>
+__global__ void __launch_bounds__(T, MB)
 k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
            uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n_max,
            const uint32_t* __restrict__ d_count, uint32_t shift, const uint32_t* __restrict__ hist,
            uint32_t* __restrict__ status, uint32_t* __restrict__ ticket, uint32_t* err, uint32_t spin_limit) {
-    __shared__ uint32_t s_wc[SR_WARPS][256];    // per-warp digit counts -> exclusive warp offsets
-    __shared__ uint32_t s_keys[SR_TILE];
-    __shared__ uint32_t s_vals[SR_TILE];
-    __shared__ uint32_t s_start[256];            // tile-local digit start
-    __shared__ uint32_t s_gbase[256];            // global position of the tile's first key of a digit
-    __shared__ uint32_t s_scan[SR_WARPS];
-    __shared__ uint32_t s_tile;
-
+    constexpr uint32_t TILE = T * I, W = T / 32;
+    static_assert(T >= 256, "a thread per digit");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SweepSmem<T, I>& S = *reinterpret_cast<SweepSmem<T, I>*>(smem_raw);
+    // the next pass may take this one's place CTA by CTA; this one reads what the kernel before it wrote only
+    // once that is complete (a no-op in a launch that is not chained)
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t n = dev_count(d_count, n_max);
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-    const uint32_t num_tiles = (n + SR_TILE - 1) / SR_TILE;
-  for (;;) {  // tiles by ticket until none is left (the grid is capped at the resident CTAs)
-    if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+    const uint32_t num_tiles = (n + TILE - 1) / TILE;
+    uint2* rk = S.rk[warp];
+    uint32_t key[I];
+    auto load_keys = [&](uint32_t t) {
+        if (t >= num_tiles) return;
+        const uint32_t b = t * TILE + warp * (I * 32u) + lane;
+        const bool whole = t * TILE + TILE <= n;
+#pragma unroll
+        for (int j = 0; j < I; ++j) key[j] = whole || b + j * 32u < n ? __ldg(keys_in + b + j * 32u) : 0xFFFFFFFFu;
+    };
+    if (tid == 0) S.tile = atomicAdd(ticket, 1u);
     __syncthreads();
-    const uint32_t tile = s_tile;
-    if (tile >= num_tiles) return;
-    for (uint32_t i = tid; i < SR_WARPS * 256u; i += SR_THREADS) (&s_wc[0][0])[i] = 0u;
-    __syncthreads();
-    const uint32_t base = tile * SR_TILE;
-    const uint32_t wbase = base + warp * (SR_ITEMS * 32u);
-
-    uint32_t key[SR_ITEMS], val[SR_ITEMS], rank[SR_ITEMS];
-#pragma unroll
-    for (int j = 0; j < SR_ITEMS; ++j) {
-        const uint32_t idx = wbase + j * 32u + lane;
-        if (idx < n) {
-            key[j] = __ldg(keys_in + idx);
-            val[j] = vals_in ? __ldg(vals_in + idx) : idx;
-        } else {
-            key[j] = 0xFFFFFFFFu;
-            val[j] = 0u;
-        }
-    }
-    const bool full = base + SR_TILE <= n;  // the whole tile holds valid items
-    // stable in-warp ranking: items in (j, lane) order = index order
-#pragma unroll
-    for (int j = 0; j < SR_ITEMS; ++j) {
-        const uint32_t idx = wbase + j * 32u + lane;
-        const bool valid = idx < n;
-        const uint32_t d = valid ? ((key[j] >> shift) & 255u) : 256u;
-        uint32_t peers;  // lanes holding the same digit (or also invalid)
-        if (RSH_SORT_MATCH_EVERY && (j % RSH_SORT_MATCH_EVERY) == RSH_SORT_MATCH_EVERY - 1) {
-            // some items by match_any (the MIO pipe), the others by ballots (the ALU pipe): the two
-            // pipes share the ranking instead of one of them bounding it
-            peers = __match_any_sync(0xffffffffu, d);
-        } else {
-            peers = 0xffffffffu;
-            if (RSH_SORT_FULL8 && full) {  // a full tile has no invalid items: 8 digit bits decide
-#pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    const bool bit = (d >> b) & 1u;
-                    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-                    peers &= bit ? bal : ~bal;
-                }
-            } else {
-#pragma unroll
-                for (int b = 0; b < 9; ++b) {
-                    const bool bit = (d >> b) & 1u;
-                    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-                    peers &= bit ? bal : ~bal;
-                }
-            }
-        }
-        const uint32_t before = __popc(peers & lanemask_lt());
-        uint32_t cnt = 0u;
-        if (valid) cnt = s_wc[warp][d];
-        __syncwarp();
-        if (valid && before == 0u) s_wc[warp][d] = cnt + __popc(peers);
-        __syncwarp();
-        rank[j] = cnt + before;
-    }
-    __syncthreads();
-    // per digit (thread = digit): warp-exclusive offsets and the tile count
-    const uint32_t dg = tid;  // SR_THREADS == 256
-    uint32_t tcount = 0u;
-#pragma unroll
-    for (int w = 0; w < SR_WARPS; ++w) {
-        const uint32_t c = s_wc[w][dg];
-        s_wc[w][dg] = tcount;
-        tcount += c;
-    }
-    // publish the tile's count for this digit early so successors can proceed
-    uint32_t* st = status + (size_t)tile * 256u + dg;
-    if (tile == 0) st_relaxed_u32(st, FLAG_PRE | tcount);
-    else st_relaxed_u32(st, FLAG_AGG | tcount);
-    // exclusive scan over digits of tcount -> s_start
-    {
-        uint32_t x = tcount;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= (uint32_t)d) x += y;
-        }
-        if (lane == 31) s_scan[warp] = x;
-        __syncthreads();
-        if (tid == 0) {
-            uint32_t r = 0;
-            for (int w = 0; w < SR_WARPS; ++w) {
-                const uint32_t t = s_scan[w];
-                s_scan[w] = r;
-                r += t;
-            }
+    uint32_t tile = S.tile;
+    load_keys(tile);
+    // tiles by ticket until none is left (the grid is capped at the resident CTAs); the next tile's keys are
+    // loaded while this one waits for its prefix and is written out
+    while (tile < num_tiles) {
+        if (tid == 0) S.next = atomicAdd(ticket, 1u);
+        {
+            uint4* z = reinterpret_cast<uint4*>(&S.rk[0][0]);
+            for (uint32_t i = tid; i < W * 128u; i += T) z[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         __syncthreads();
-        const uint32_t start = s_scan[warp] + x - tcount;
-        s_start[dg] = start;
+        const uint32_t base = tile * TILE, wbase = base + warp * (I * 32u);
+        const bool full = base + TILE <= n;  // the whole tile holds valid items
+        // stable in-warp ranking: items in (j, lane) order = index order. The lanes of a digit find each other
+        // through a lane mask in shared memory
+        uint32_t rank[(I + 1) / 2];  // two 16-bit ranks a word
 #pragma unroll
-        for (int w = 0; w < SR_WARPS; ++w) s_wc[w][dg] += start;  // tile-local position of each warp's run
-    }
-    // global digit offset of this pass (exclusive, from the histogram kernel)
-    const uint32_t gex = __ldg(hist + dg);
-    // decoupled look-back for this digit, LB predecessors per step: their status words are loaded
-    // together (flag and count share one word, so relaxed loads suffice) and folded newest first up to
-    // the first one holding an inclusive prefix; a not-yet-published word restarts the step there
-    uint32_t excl = 0u;
-    if (tile > 0) {
-#ifndef RSH_SORT_LB
-#define RSH_SORT_LB 8
-#endif
-        constexpr int LB = RSH_SORT_LB;
-        int64_t j = (int64_t)tile - 1;
-        uint32_t spins = 0;
-        while (j >= 0) {
-            uint32_t sv[LB];
-#pragma unroll
-            for (int q = 0; q < LB; ++q)
-                sv[q] = (j - q >= 0) ? ld_relaxed_u32(status + (size_t)(j - q) * 256u + dg) : FLAG_PRE;
-            int used = 0;
-            bool done = false, stall = false;
-#pragma unroll
-            for (int q = 0; q < LB; ++q) {
-                if (done || stall) continue;
-                const uint32_t f = sv[q] & ~VAL_MASK;
-                if (f == 0u) {
-                    stall = true;
-                    continue;
-                }
-                excl += sv[q] & VAL_MASK;
-                ++used;
-                if (f == FLAG_PRE) done = true;
-            }
-            if (done) break;
-            j -= used;
-            if (stall) {
-                if (++spins > spin_limit) {
-                    raise_device_error(err, RSH_DEVERR_TIMEOUT);
-                    break;
-                }
-                if (spins > 16) __nanosleep(32);
-            }
-        }
-        st_relaxed_u32(st, FLAG_PRE | (excl + tcount));
-    }
-    s_gbase[dg] = gex + excl - s_start[dg];
-    __syncthreads();
-    // scatter into shared memory in tile-sorted order
-#pragma unroll
-    for (int j = 0; j < SR_ITEMS; ++j) {
-        const uint32_t idx = wbase + j * 32u + lane;
-        if (idx < n) {
+        for (int j = 0; j < I; ++j) {
+            const bool valid = full || wbase + j * 32u + lane < n;
             const uint32_t d = (key[j] >> shift) & 255u;
-            const uint32_t pos = s_wc[warp][d] + rank[j];
-            s_keys[pos] = key[j];
-            s_vals[pos] = val[j];
+            if (valid) atomicOr(&rk[d].y, 1u << lane);
+            __syncwarp();
+            const uint2 e = rk[d];
+            const uint32_t before = e.y & lanemask_lt();
+            __syncwarp();
+            if (valid && before == 0u) rk[d] = make_uint2(e.x + __popc(e.y), 0u);
+            __syncwarp();
+            const uint32_t r = e.x + __popc(before);
+            if (j & 1) rank[j / 2] |= r << 16;
+            else rank[j / 2] = r;
         }
-    }
-    __syncthreads();
-    const uint32_t tn = (n - base) < (uint32_t)SR_TILE ? (n - base) : (uint32_t)SR_TILE;
-    for (uint32_t i = tid; i < tn; i += SR_THREADS) {
-        const uint32_t k = s_keys[i];
-        const uint32_t d = (k >> shift) & 255u;
-        const uint32_t g = s_gbase[d] + i;
-        if (g < n) {  // only false after a look-back timeout (error word raised)
-            keys_out[g] = k;
-            vals_out[g] = s_vals[i];
+        __syncthreads();
+        // per digit (thread = digit): warp-exclusive offsets and the tile count, published early so that
+        // successors can proceed
+        uint32_t tcount = 0u, start = 0u;
+        uint32_t* st = status + (size_t)tile * 256u + tid;
+        uint32_t x = 0u;
+        if (tid < 256u) {
+#pragma unroll
+            for (uint32_t w = 0; w < W; ++w) {
+                const uint32_t c = S.rk[w][tid].x;
+                S.rk[w][tid].x = tcount;
+                tcount += c;
+            }
+            st_relaxed_u32(st, (tile == 0 ? FLAG_PRE : FLAG_AGG) | tcount);
+            x = tcount;  // exclusive scan over the digits
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= (uint32_t)d) x += y;
+            }
+            if (lane == 31) S.scan[warp] = x;
         }
+        __syncthreads();
+        if (tid < 256u) {
+            start = x - tcount;
+            for (uint32_t w = 0; w < warp; ++w) start += S.scan[w];
+#pragma unroll
+            for (uint32_t w = 0; w < W; ++w) S.rk[w][tid].x += start;
+        }
+        __syncthreads();
+        // scatter into shared memory in tile-sorted order (before the look-back, whose predecessors gain time)
+        {
+            uint32_t val[I];
+#pragma unroll
+            for (int j = 0; j < I; ++j) {
+                const uint32_t idx = wbase + j * 32u + lane;
+                val[j] = idx;
+                if (vals_in && (full || idx < n)) val[j] = __ldg(vals_in + idx);
+            }
+#pragma unroll
+            for (int j = 0; j < I; ++j) {
+                if (full || wbase + j * 32u + lane < n) {
+                    const uint32_t pos = rk[(key[j] >> shift) & 255u].x + ((rank[j / 2] >> (16 * (j & 1))) & 0xFFFFu);
+                    S.keys[pos] = key[j];
+                    S.vals[pos] = val[j];
+                }
+            }
+        }
+        const uint32_t next = S.next;
+        load_keys(next);
+        if (tid < 256u) {
+            // global digit offset of this pass (exclusive, from the histogram kernel)
+            const uint32_t gex = __ldg(hist + tid);
+            // decoupled look-back for this digit, LB predecessors per step: their status words are loaded
+            // together (flag and count share one word, so relaxed loads suffice) and folded newest first up to
+            // the first one holding an inclusive prefix; a not-yet-published word restarts the step there
+            uint32_t excl = 0u;
+            if (tile > 0) {
+                constexpr int LB = 8;
+                int64_t j = (int64_t)tile - 1;
+                uint32_t spins = 0;
+                while (j >= 0) {
+                    uint32_t sv[LB];
+#pragma unroll
+                    for (int q = 0; q < LB; ++q)
+                        sv[q] = (j - q >= 0) ? ld_relaxed_u32(status + (size_t)(j - q) * 256u + tid) : FLAG_PRE;
+                    int used = 0;
+                    bool done = false, stall = false;
+#pragma unroll
+                    for (int q = 0; q < LB; ++q) {
+                        if (done || stall) continue;
+                        const uint32_t f = sv[q] & ~VAL_MASK;
+                        if (f == 0u) {
+                            stall = true;
+                            continue;
+                        }
+                        excl += sv[q] & VAL_MASK;
+                        ++used;
+                        if (f == FLAG_PRE) done = true;
+                    }
+                    if (done) break;
+                    j -= used;
+                    if (stall) {
+                        if (++spins > spin_limit) {
+                            raise_device_error(err, RSH_DEVERR_TIMEOUT);
+                            break;
+                        }
+                        if (spins > 16) __nanosleep(32);
+                    }
+                }
+                st_relaxed_u32(st, FLAG_PRE | (excl + tcount));
+            }
+            S.gbase[tid] = gex + excl - start;
+        }
+        __syncthreads();
+        const uint32_t tn = full ? TILE : n - base;
+#pragma unroll 4
+        for (uint32_t i = tid; i < tn; i += T) {
+            const uint32_t k = S.keys[i];
+            const uint32_t g = S.gbase[(k >> shift) & 255u] + i;
+            if (g < n) {  // only false after a look-back timeout (error word raised)
+                if (keys_out) keys_out[g] = k;
+                vals_out[g] = S.vals[i];
+            }
+        }
+        __syncthreads();  // shared state is reused by the next tile
+        tile = next;
     }
-    __syncthreads();  // shared state is reused by the next tile
-  }
 }
+
+namespace {
+
+// A kernel that may start while the one before it in the stream still runs; it waits itself
+// (griddepcontrol.wait) before it touches what that one wrote.
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem,
+                           cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+template <int T, int I, int MB>
+cudaError_t sweep(uint32_t n_max, uint32_t sms, uint32_t grid_max, bool chained, const uint32_t* ki, const uint32_t* vi,
+                  uint32_t* ko, uint32_t* vo, const uint32_t* d_count, uint32_t shift, const uint32_t* hist,
+                  uint32_t* status, uint32_t* ticket, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
+    const auto kernel = k_onesweep<T, I, MB>;
+    constexpr size_t smem = sizeof(SweepSmem<T, I>), SM_BYTES = 228 * 1024, MOST = 227 * 1024;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST);
+    if (e != cudaSuccess) return e;
+    // at most the CTAs resident at once: tiles beyond the device count cost nothing, and every ticket below a
+    // CTA's tile is held by a running CTA (forward progress of the look-back)
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, T, smem);
+    if (per_sm < 1) per_sm = 1;
+    const uint32_t tiles = (n_max + T * I - 1) / (T * I);
+    const uint32_t grid = std::min(std::min(tiles, sms * (uint32_t)per_sm), grid_max);
+    // A chained launch's CTAs are placed while the pass before it still runs, on whichever SMs have room: with
+    // room for more CTAs than an SM's share, some SMs get several and others none. Asking for the shared memory
+    // of an SM's share leaves room for no more
+    const uint32_t share = (grid + sms - 1) / sms;
+    // (1 M random pairs: 61 us, 71 unchained, 75 chained without this; 16 M: 428 / 440).
+    const size_t padded = share < (uint32_t)per_sm
+                              ? std::max(smem, std::min(MOST, SM_BYTES / share - 1024) & ~size_t(127)) : smem;
+    e = launch_chained(chained, kernel, grid, T, padded, s, ki, vi, ko, vo, n_max, d_count, shift, hist, status, ticket,
+                       err, spin_limit);
+    note_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+}  // namespace
 
 size_t sort_scratch_bytes(uint32_t n_max, uint32_t key_bits) {
     const size_t passes = num_passes(key_bits);
-    const size_t tiles = (n_max + SR_TILE - 1) / SR_TILE + 1;
+    const size_t tiles = (n_max + tile_of(n_max) - 1) / tile_of(n_max) + 1;
     const size_t words = 4 * 256 + 16 + passes * tiles * 256;
     return words * 4 + 2 * (size_t)n_max * 4 + 1024;
 }
 
 cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                               uint32_t* vals_out, uint32_t n_max, const uint32_t* d_count,
-                              uint32_t key_bits, void* scratch, uint32_t* err, cudaStream_t s) {
+                              uint32_t key_bits, void* scratch, uint32_t* err, cudaStream_t s, bool keys_wanted) {
     if (n_max == 0) return cudaSuccess;
     const uint32_t passes = num_passes(key_bits);
-    const size_t tiles = (n_max + SR_TILE - 1) / SR_TILE + 1;
+    const uint32_t tile = tile_of(n_max);
+    const size_t tiles = (n_max + tile - 1) / tile + 1;
     uint32_t* w = static_cast<uint32_t*>(scratch);
     uint32_t* hist = w;                       // passes * 256 (room for 4)
     uint32_t* tickets = w + 4 * 256;          // 16: one per pass, [8] = histogram CTAs done
@@ -352,31 +401,28 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
     uint32_t* alt_vals = alt_keys + n_max;
     cudaError_t e = cudaMemsetAsync(w, 0, (4 * 256 + 16) * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    k_sort_hist<<<152 * 2, 256, 0, s>>>(keys_in, n_max, d_count, passes, hist, status, tiles * 256, tickets + 8);
-    // at most the CTAs resident at once: tiles beyond the device count cost nothing, and every ticket
-    // below a CTA's tile is held by a running CTA (forward progress of the look-back)
-    int dev = 0, sms = 152, per_sm = 1;
+    int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_onesweep, SR_THREADS, 0);
-    if (per_sm < 1) per_sm = 1;
-    const uint32_t resident = (uint32_t)(sms * per_sm);
+    // four CTAs per SM count 16 M keys in half the time of two; fewer when there is not a run of 16 keys for each
+    // thread
+    const uint32_t hgrid = std::min<uint32_t>((uint32_t)sms * 4u, (n_max + 4095u) / 4096u);
+    k_sort_hist<<<hgrid, 256, 0, s>>>(keys_in, n_max, d_count, passes, tile, hist, status, tiles * 256, tickets + 8);
     note_launch();
     // ping-pong so that the last pass lands in the output
     const uint32_t* ki = keys_in;
     const uint32_t* vi = vals_in;
     for (uint32_t p = 0; p < passes; ++p) {
-        const bool last = (p + 1 == passes);
         // choose destinations: passes alternate between out and alt, ending in out
         const bool to_out = ((passes - 1 - p) % 2u) == 0u;
         uint32_t* ko = to_out ? keys_out : alt_keys;
         uint32_t* vo = to_out ? vals_out : alt_vals;
-        (void)last;
-        const uint32_t grid = std::min<uint32_t>((uint32_t)(tiles - 1 > 0 ? tiles - 1 : 1), resident);
-        k_onesweep<<<grid, SR_THREADS, 0, s>>>(ki, vi, ko, vo, n_max, d_count, 8u * p, hist + 256u * p,
-                                               status + p * tiles * 256, tickets + p, err, RSH_SPIN_LIMIT);
-        note_launch();
-        e = cudaGetLastError();
+        if (p + 1 == passes && !keys_wanted) ko = nullptr;
+        e = small_tiles(n_max)
+                ? sweep<S_T, S_I, S_MB>(n_max, (uint32_t)sms, ~0u, true, ki, vi, ko, vo, d_count, 8u * p, hist + 256u * p,
+                                        status + p * tiles * 256, tickets + p, err, RSH_SPIN_LIMIT, s)
+                : sweep<L_T, L_I, L_MB>(n_max, (uint32_t)sms, ~0u, true, ki, vi, ko, vo, d_count, 8u * p, hist + 256u * p,
+                                        status + p * tiles * 256, tickets + p, err, RSH_SPIN_LIMIT, s);
         if (e != cudaSuccess) return e;
         ki = ko;
         vi = vo;
@@ -389,11 +435,11 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
 // publishes. The wait must give up after `spin_limit` polls and raise RSH_DEVERR_TIMEOUT in *err
 // instead of hanging; every write stays in bounds. Buffers (2 tiles of keys in/out, status, tickets)
 // come from the caller's scratch of sort_selftest_scratch_bytes().
-size_t sort_selftest_scratch_bytes() { return (size_t)(4 * 2 * SR_TILE + 2 * 256 + 256 + 8) * 4 + 1024; }
+size_t sort_selftest_scratch_bytes() { return (size_t)(4 * 2 * S_TILE + 2 * 256 + 256 + 8) * 4 + 1024; }
 
 cudaError_t sort_selftest_timeout(void* scratch, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
     uint32_t* w = static_cast<uint32_t*>(scratch);
-    const uint32_t n = 2 * SR_TILE;
+    const uint32_t n = 2 * S_TILE;
     uint32_t* keys_in = w;
     uint32_t* vals_in = keys_in + n;
     uint32_t* keys_out = vals_in + n;
@@ -405,10 +451,9 @@ cudaError_t sort_selftest_timeout(void* scratch, uint32_t* err, uint32_t spin_li
     if (e != cudaSuccess) return e;
     const uint32_t one = 1u;  // tile 0's ticket is already gone: the one CTA gets tile 1
     if ((e = cudaMemcpyAsync(ticket, &one, 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-    k_onesweep<<<1, SR_THREADS, 0, s>>>(keys_in, vals_in, keys_out, vals_out, n, nullptr, 0u, hist, status, ticket, err,
-                                        spin_limit);
-    note_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = sweep<S_T, S_I, S_MB>(n, 1u, 1u, false, keys_in, vals_in, keys_out, vals_out, nullptr, 0u, hist, status, ticket,
+                              err, spin_limit, s);
+    if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(s);
 }
 
