@@ -122,14 +122,15 @@ __global__ void k_batch_bounds(const uint32_t* __restrict__ seg_cnt, uint32_t ns
             padded[q] = INVALID_ID;
 }
 
-// Rays alone: each segment's ids, their number and its first work unit, in schedule order; one block, a thread
-// per segment. sorted != nullptr: the segments' trimmed ids lie one after the other there, in segment order,
+// Rays alone: each segment's ids, their number and its first work unit among those of its kind, in schedule order
+// (the nclosest closest-hit segments come first; totals[1] their units, totals[2] the any-hit ones'); one block, a
+// thread per segment. sorted != nullptr: the segments' trimmed ids lie one after the other there, in segment order,
 // seg_cnt[s] of them for segment s; else each segment has its own list and count (FusedSeg).
 __global__ void __launch_bounds__(1024)
-k_batch_units(FusedSeg* __restrict__ fsegs, uint32_t nseg, const uint32_t* __restrict__ sorted,
+k_batch_units(FusedSeg* __restrict__ fsegs, uint32_t nseg, uint32_t nclosest, const uint32_t* __restrict__ sorted,
               const uint32_t* __restrict__ seg_cnt, const uint32_t* __restrict__ sched, uint32_t unit_rays,
               uint32_t* __restrict__ totals) {
-    __shared__ uint32_t s_begin[1024], s_warp[32];
+    __shared__ uint32_t s_begin[1024], s_warp[32], s_closest;
     const uint32_t k = threadIdx.x, lane = lane_id(), warp = k >> 5;
     auto exclusive = [&](uint32_t v) {  // over the block
         uint32_t x = v;
@@ -163,10 +164,16 @@ k_batch_units(FusedSeg* __restrict__ fsegs, uint32_t nseg, const uint32_t* __res
         n = dev_count(fsegs[k].count, fsegs[k].n);
     }
     const uint32_t units = (n + unit_rays - 1u) / unit_rays, ub = exclusive(units);
+    if (k == 0u && nclosest == 0u) s_closest = 0u;
+    if (k + 1u == nclosest) s_closest = ub + units;
+    __syncthreads();
     if (in) {
         fsegs[k].n = n;
-        fsegs[k].unit_begin = ub;
-        if (k == nseg - 1u) totals[1] = ub + units;
+        fsegs[k].unit_begin = k < nclosest ? ub : ub - s_closest;
+        if (k == nseg - 1u) {
+            totals[1] = s_closest;
+            totals[2] = ub + units - s_closest;
+        }
     }
 }
 
@@ -205,7 +212,8 @@ struct BatchPlan {
     bool sorted = true;      // hashed and sorted before the traversal
     bool listed = false;     // rays alone: ray generation listed each segment's ids
     uint32_t empty_bit = 0;  // slots sorted as they are: one more key bit sorted, that of the empty slots
-    uint32_t units_max = 0;  // rays alone: work units if every slot held a ray
+    uint32_t units_max[2] = {0, 0};  // rays alone: work units if every slot held a ray, closest- and any-hit
+    uint32_t nclosest = 0;           // closest-hit segments (first in the schedule)
     bool contiguous = false; // the segments' rays lie back to back in one array: no gather
     bool gather = false;     // copy every segment's rays into one array (packet kernel, not contiguous)
     void *rays_all, *keys, *trimmed, *ckeys, *cbases, *counts, *skeys, *svals, *sorted_keys, *sorted_ids, *scr;
@@ -387,13 +395,14 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         return segs[a].n > segs[b].n;
     });
     std::vector<FusedSeg> by_seg(pl.h_fsegs);
-    uint32_t units = 0;
     for (uint32_t k = 0; k < count; ++k) {
-        pl.h_fsegs[k] = by_seg[pl.h_sched[k]];
-        pl.h_fsegs[k].unit_begin = units;  // final where the segments' own order is traced
-        units += (pl.h_fsegs[k].n + pl.unit_rays - 1) / pl.unit_rays;
+        FusedSeg& f = pl.h_fsegs[k];
+        f = by_seg[pl.h_sched[k]];
+        uint32_t& units = pl.units_max[f.any_hit];
+        f.unit_begin = units;  // final where the segments' own order is traced
+        units += (f.n + pl.unit_rays - 1) / pl.unit_rays;
+        if (!f.any_hit) ++pl.nclosest;
     }
-    pl.units_max = units;
     return RSH_OK;
 }
 
@@ -500,6 +509,7 @@ rsh_status enqueue_alone(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
     RSH_CUDA(cudaMemsetAsync(pl.work, 0, 16, s));
     FusedArgs fa = alone_args(ctx, pl.work);
     fa.valid = cnt;
+    fa.pixel_order = pl.listed;
     th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);  // traversal and intersection in one kernel
     if (one) {
         fa.one = pl.h_fsegs[0];
@@ -510,19 +520,26 @@ rsh_status enqueue_alone(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
         RSH_CUDA(launch_rays_one(fa, s));
     } else {
         uint32_t* totals = static_cast<uint32_t*>(pl.totals);
-        fa.segs = static_cast<FusedSeg*>(pl.fsegs);
-        fa.nseg = pl.nseg;
-        fa.units_max = pl.units_max;
-        if (pl.sorted || pl.listed) {
-            k_batch_units<<<1, 1024, 0, s>>>(static_cast<FusedSeg*>(pl.fsegs), pl.nseg,
+        const bool counted = pl.sorted || pl.listed;
+        if (counted) {
+            k_batch_units<<<1, 1024, 0, s>>>(static_cast<FusedSeg*>(pl.fsegs), pl.nseg, pl.nclosest,
                                              pl.sorted ? static_cast<uint32_t*>(pl.svals) : nullptr,
                                              static_cast<uint32_t*>(pl.seg_cnt), static_cast<uint32_t*>(pl.sched),
                                              pl.unit_rays, totals);
             note_launch();
             RSH_CUDA(cudaGetLastError());
-            fa.d_units = totals + 1;
         }
-        RSH_CUDA(launch_rays_segs(fa, s));
+        // the closest-hit segments, then beside them the any-hit ones
+        const bool both = pl.units_max[0] && pl.units_max[1];
+        for (uint32_t any = 0; any < 2; ++any) {
+            fa.segs = static_cast<FusedSeg*>(pl.fsegs) + (any ? pl.nclosest : 0u);
+            fa.nseg = any ? pl.nseg - pl.nclosest : pl.nclosest;
+            fa.units_max = pl.units_max[any];
+            fa.d_units = counted ? totals + 1 + any : nullptr;
+            fa.work = static_cast<uint32_t*>(pl.work) + any;
+            fa.pair = both ? 1u + any : 0u;
+            RSH_CUDA(launch_rays_segs(fa, any != 0, s));
+        }
     }
     stage_end(ctx, th, s);
     return RSH_OK;
@@ -635,8 +652,10 @@ struct GraphExec {
 namespace rsh {
 rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
-                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s) {
+                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair) {
     FusedArgs fa = alone_args(ctx, ticket);
+    fa.pair = pair;
+    fa.pixel_order = true;
     fa.one.wtris = sc->h.wtris;
     fa.one.wnodes = sc->h.wnodes;
     fa.one.wnroot = sc->h.wnroot;

@@ -1205,10 +1205,12 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
                                            ctx->cfg.reflect_jitter, ctx->cfg.seed, b, hp_r, rrays, nullptr, s, ro));
             stage_end(ctx, th, s);
             th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
+            // side by side: the shadow rays' warps start as the reflection rays' end (Cornell frame 200 -> 171 us,
+            // architecture frame 3.37 -> 3.27 ms)
             RSH_TRY(trace_alone(ctx, sc, rrays, npix, ro.ids, ro.count, false, nullptr, rhits, tickets + 1 + 2 * b,
-                                pairs, s));
+                                pairs, s, 1));
             RSH_TRY(trace_alone(ctx, sc, srays, npix * LS, so.ids, so.count, true, sflags, nullptr,
-                                tickets + 2 + 2 * b, pairs, s));
+                                tickets + 2 + 2 * b, pairs, s, 2));
             stage_end(ctx, th, s);
         } else if (fused) {
             // both batches of the bounce in one batched call: 2 segments, one persistent launch; ray

@@ -1,7 +1,7 @@
 // Fused persistent traversal + intersection (the batched form's single launch). Two kernels:
 //   k_fused_rays (switch level at or above every segment's tree depth, the default): each lane traces one
-//     ray at a time from the root, refilled from the warp's current unit of 64 sorted rays; no packet
-//     phase and no ray hierarchy; the launch's last units go out as half units, and (instance SHARE) a
+//     ray at a time from the root, refilled from the warp's current unit of 64 rays; no packet
+//     phase and no ray hierarchy; the launch's last units go out in pieces, and (instance SHARE) a
 //     drained warp's last rays are shared among its idle lanes;
 //   k_fused (a lower switch level): packets of the ray hierarchy walk the upper object tree, rays leave
 //     them at the switch level, as described next.
@@ -586,8 +586,8 @@ __global__ void __launch_bounds__(FW * 32, RSH_FUSED_MIN_BLOCKS) k_fused(FusedAr
 // most node steps hit one child, which is then the next step without a store to and a load from local memory
 // in between (frames 2.8-3.9% faster: the architecture frame 3.79 ms against 3.90, the soup frame 3.34 against
 // 3.47; loading a plane of eight children with one 32-byte load instead of two 16-byte ones took 4.17 ms at this
-// register limit and 3.96 ms without spills at 6 CTAs per SM). The launch's last units go out as
-// pieces of RSH_RAYS_UNIT / RSH_TAIL_SPLIT rays. Single long rays (up to 20x the median ray's tests) still
+// register limit and 3.96 ms without spills at 6 CTAs per SM). The launch's last units go out in pieces
+// (tail_split). Single long rays (up to 20x the median ray's tests) still
 // hold an SM after the others have finished; the SHARE instance (the default) lets a drained warp's idle
 // lanes take their subtrees (described at its loop's top), at the price of about 4% on every step, which
 // the instance without it (RSH_FLAG_SEQUENTIAL_RAYS) does not pay.
@@ -660,39 +660,53 @@ RSH_DEV void slab4(float4 px, float4 py, float4 pz, float ix, float iy, float iz
 #ifndef RSH_TAIL_PER_WARP
 #define RSH_TAIL_PER_WARP 16
 #endif
-#ifndef RSH_TAIL_SPLIT
-#define RSH_TAIL_SPLIT 2
-#endif
 
-// Which segments a launch of the rays-only kernel traces, known at compile time where it can be:
-//   SEGS  the batch's segment table, closest- and any-hit segments mixed;
-//   ANY1 / CLOSEST1  one segment of one kind, read from the kernel's own arguments: the scene, the output and
-//     the kind are launch constants, not per-lane state (6 registers fewer), and no table is uploaded.
-enum RaysOf { SEGS = 0, ANY1 = 1, CLOSEST1 = 2 };
+// log2 of the pieces that a launch's last units are cut into, for `units` of RSH_RAYS_UNIT rays over `warps` warps:
+// halves by default; smaller ones, down to 4 rays, while there are fewer than one for every second warp (the launch
+// then takes as long as its slowest warp, and idle lanes take subtrees: 20,001 rays 55 -> 45 us, 1000 rays 48 ->
+// 33); quarters of rays in no particular order where a warp gets between 32 and 96 of them (200,000 rays: 107 us
+// instead of 120; halves are 1.5 a warp). Rays in pixel order lose by quarters (Cornell frame 176 -> 180 us), and
+// with more rays they cost more tickets than they balance (architecture frame 3.42 ms, halves 3.27).
+constexpr uint32_t SPLIT_MOST = 4;
+__host__ __device__ __forceinline__ uint32_t tail_split(uint32_t units, uint32_t warps, bool pixel_order) {
+    if (!pixel_order && (uint64_t)units * 2u >= warps && units < warps + warps / 2u) return 2u;
+    uint32_t split = 1;
+    while (split < SPLIT_MOST && ((uint64_t)units << (split + 1u)) < warps) ++split;
+    return split;
+}
+
+// What a launch of the rays-only kernel traces: closest-hit or any-hit segments, never both (the kind is a launch
+// constant: no per-lane flag, no any-hit code in a closest-hit step, no entry distances for any-hit rays), of the
+// batch's segment table (SEGS) or one segment from the kernel's own arguments (the scene and the output are launch
+// constants too, 5 registers fewer, and no table is uploaded). A batch of both kinds is a pair of launches.
+enum RaysOf { SEGS_CLOSEST = 0, SEGS_ANY = 1, ONE_CLOSEST = 2, ONE_ANY = 3 };
 
 template <int U, bool SHARE, int OF>
 __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(const __grid_constant__ FusedArgs a) {
-    constexpr bool ONE = OF != SEGS;
+    constexpr bool ONE = OF == ONE_CLOSEST || OF == ONE_ANY, any = OF == SEGS_ANY || OF == ONE_ANY;
     // SHARE: a drained warp's rays shared among its idle lanes; the records of the rays being shared, one per
     // lane: the owner's best hit key (closest hit), occluded (any hit), helpers still on a subtree of it
     __shared__ unsigned long long sh_best[SHARE ? FW : 1][32];
     __shared__ uint32_t sh_occ[SHARE ? FW : 1][32], sh_pend[SHARE ? FW : 1][32];
     __shared__ uint32_t s_rays, s_ended;  // a.valid: the block's rays, its warps that have ended
     const uint32_t lane = lane_id();
+    asm volatile("griddepcontrol.launch_dependents;");
     if (a.valid) {
         if (threadIdx.x == 0) s_rays = s_ended = 0u;
         __syncthreads();
     }
     const uint32_t units = ONE ? (dev_count(a.one.count, a.one.n) + U - 1u) / U : dev_count(a.d_units, a.units_max);
-    const uint32_t tail = min(units, (uint32_t)RSH_TAIL_PER_WARP * gridDim.x * FW);
-    const uint32_t head = units - tail, tickets = head + RSH_TAIL_SPLIT * tail;
+    // the last units go out in pieces of U >> split rays
+    const uint32_t tail = min(units, (uint32_t)RSH_TAIL_PER_WARP * gridDim.x * FW), 
+                   split = tail_split(units, a.warps, a.pixel_order);
+    const uint32_t head = units - tail, tickets = head + (tail << split);
     uint32_t ntests = 0, ttests = 0;  // the lane's counts, flushed to the launch's counters before 2^31
     uint32_t ncand = 0;               // ONE: clusters whose triangles the lane tested
     // the warp's current unit: rays [nk, nend) of segment cs, in its order
     uint32_t nk = 0, nend = 0, cs = 0;
     bool drained = false;
     // the lane's ray
-    bool has = false, any_v = false;
+    bool has = false;
     uint32_t seg = 0, slot = 0;
     const float4* nodes_v = nullptr;
     const float4* tris_v = nullptr;
@@ -701,7 +715,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
     uint32_t top = 0u;
     int sp = 0;
     uint32_t stk[J_STACK];
-    float stt[OF == ANY1 ? 1 : J_STACK];  // closest hit: each entry's entry distance, from its parent's test
+    float stt[any ? 1 : J_STACK];  // closest hit: each entry's entry distance, from its parent's test
     float ox = 0.f, oy = 0.f, oz = 0.f, tmin = 0.f, tcur = 0.f;
     float ix = 0.f, iy = 0.f, iz = 0.f, oix = 0.f, oiy = 0.f, oiz = 0.f;
     uint32_t oct = 0;  // the direction's octant: bit a set when component a is negative
@@ -710,7 +724,6 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
     bool sharing = false;  // warp-uniform (SHARE): the warp shares its last rays
     bool done = false;     // sharing: the lane's subtree is done, its result not yet merged
     uint32_t own = lane;   // sharing: the lane whose ray this lane works on
-    auto any_of = [&]() -> bool { return OF == ANY1 ? true : OF == CLOSEST1 ? false : any_v; };
     auto seg_of = [&](uint32_t i) -> const FusedSeg& { return ONE ? a.one : a.segs[i]; };
     // the ray is done: its result, written by its own lane (while sharing: merged at the loop's top)
     auto finish = [&]() {
@@ -720,7 +733,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
             return;
         }
         const FusedSeg& sg = seg_of(seg);
-        if (any_of()) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
+        if (any) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
         else sg.hits[slot] = best;
         // one ray adds fewer than 2^28 node tests (8 per slot) and 2^24 triangle tests
         if ((ntests | ttests) >> 31) {
@@ -734,7 +747,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
     // current best are dropped unread (their subtrees cannot hold a nearer hit: a child's box lies inside its
     // parent's, so no child is entered before its parent). Finishes the ray when nothing is left.
     auto pop = [&]() {
-        if (any_of()) {
+        if (any) {
             if (sp == 0) finish();
             else top = stk[--sp];
         } else {
@@ -768,9 +781,9 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                 uint32_t u = t, lo = 0, hi = U;
                 if (t >= head) {
                     const uint32_t h = t - head;
-                    u = head + h / RSH_TAIL_SPLIT;
-                    lo = (h % RSH_TAIL_SPLIT) * (U / RSH_TAIL_SPLIT);
-                    hi = lo + U / RSH_TAIL_SPLIT;
+                    u = head + (h >> split);
+                    lo = (h & ((1u << split) - 1u)) * (U >> split);
+                    hi = lo + (U >> split);
                 }
                 if (ONE) {
                     nk = u * U + lo;
@@ -793,19 +806,17 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                 if (id < sg.slots) {
                     float4 o, d;
                     load_ray(sg.rays, id, o, d);
-                    const bool sany = OF == ANY1 ? true : OF == CLOSEST1 ? false : sg.any_hit != 0u;
                     ray = d.w > o.w;
                     if (!ray || sg.levels == 0u) {
                         // no ray, or a scene without triangles (no tree): a miss
                         if (ray || !sg.ids) {
-                            if (sany) sg.flags[id] = 0u;
+                            if (any) sg.flags[id] = 0u;
                             else sg.hits[id] = RSH_HIT_NONE;
                         }
                     } else {
                         slot = id;
                         if (!ONE) {
                             seg = cs;
-                            any_v = sany;
                             nodes_v = sg.wnodes;
                             tris_v = sg.wtris;
                         }
@@ -844,7 +855,6 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
         // happens here, between steps: the steps themselves are the sequential ones.
         if (SHARE && drained && (sharing || __popc(__ballot_sync(0xffffffffu, has)) <= RSH_SHARE_BUSY)) {
             const uint32_t wp = threadIdx.x >> 5;
-            const bool any = any_of();
             if (!sharing) {
                 sh_best[wp][lane] = has ? best : RSH_HIT_NONE;
                 sh_occ[wp][lane] = 0u;
@@ -894,7 +904,6 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                 ge = __shfl_sync(0xffffffffu, ge, src);
                 const uint32_t go = __shfl_sync(0xffffffffu, own, src);
                 if (!ONE) {
-                    any_v = __shfl_sync(0xffffffffu, any_v, src);
                     seg = __shfl_sync(0xffffffffu, seg, src);
                     nodes_v = reinterpret_cast<const float4*>(
                         __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(nodes_v), src));
@@ -942,7 +951,6 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
             do_nodes = nn >= nc;
         }
         if (has && ((top >> 31) != 0u) == do_nodes) {
-            const bool any = any_of();
             const uint32_t e = top;
             if (!(e >> 31)) {
                 // a cluster: its triangles t0 .. t0 + count - 1 (its box was tested with the parent's
@@ -979,29 +987,38 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                 // a node record: the children's near planes and far planes, axis by axis, then their entries
                 const float4* __restrict__ nodes = ONE ? a.one.wnodes : nodes_v;
                 const uint32_t cnt = ((e >> 28) & 7u) + 1u;
-                const float4* rec = nodes + REC_F4 * (size_t)(e & 0x0FFFFFFFu);
                 ntests += cnt;
                 if (sp + cnt > J_STACK) {
                     raise_device_error(a.err, RSH_DEVERR_OVERFLOW);
                     pop();
                 } else {
-                    const uint32_t nxo = (oct & 1u) << 1, nyo = 4u | (oct & 2u), nzo = 8u | ((oct >> 1) & 2u);
+                    // byte offsets from the tree's first record fit in 32 bits (fewer than 2^23 records of 224
+                    // bytes): a load adds them to one base, with no 64-bit arithmetic per plane
+                    const uint32_t off = (e & 0x0FFFFFFFu) * (16u * REC_F4);
+                    const uint32_t nx = off + ((oct & 1u) << 5), ny = off + 64u + ((oct & 2u) << 4),
+                                   nz = off + 128u + ((oct & 4u) << 3);
+                    const uint32_t fx = nx + 32u - ((oct & 1u) << 6), fy = ny + 32u - ((oct & 2u) << 5),
+                                   fz = nz + 32u - ((oct & 4u) << 4);
+                    auto at = [&](uint32_t o) {
+                        return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + o));
+                    };
                     float tn[8];
                     uint32_t hm = 0;
-                    #pragma unroll
+#pragma unroll
                     for (uint32_t h = 0; h < 2; ++h) {
                         float n4[4], f4[4];
-                        slab4(__ldg(rec + nxo + h), __ldg(rec + nyo + h), __ldg(rec + nzo + h), ix, iy, iz, oix,
-                              oiy, oiz, tmin, n4, true);
-                        slab4(__ldg(rec + (nxo ^ 2u) + h), __ldg(rec + (nyo ^ 2u) + h), __ldg(rec + (nzo ^ 2u) + h),
-                              ix, iy, iz, oix, oiy, oiz, tcur, f4, false);
+                        slab4(at(nx + 16u * h), at(ny + 16u * h), at(nz + 16u * h), ix, iy, iz, oix, oiy, oiz, tmin, n4,
+                              true);
+                        slab4(at(fx + 16u * h), at(fy + 16u * h), at(fz + 16u * h), ix, iy, iz, oix, oiy, oiz, tcur, f4,
+                              false);
 #pragma unroll
                         for (uint32_t k = 0; k < 4; ++k) {
                             tn[4 * h + k] = n4[k];
                             hm |= (n4[k] <= f4[k] ? 1u : 0u) << (4 * h + k);
                         }
                     }
-                    const uint32_t* ent = reinterpret_cast<const uint32_t*>(rec + 12);
+                    const uint32_t* ent =
+                        reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(nodes) + off) + 48;
                     if (hm == 0u) {
                         pop();
                     } else if (any) {
@@ -1064,10 +1081,12 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
         if (a.tri_tests) atomicAdd(a.tri_tests, tt);
         if (ONE && a.cand_pairs) atomicAdd(a.cand_pairs, nc);
     }
+    // chained behind an independent launch: done only when that one is, so what follows this one follows both
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <int U, bool SHARE, int OF>
-static cudaError_t launch_fused_rays_s(const FusedArgs& a, cudaStream_t s) {
+static cudaError_t launch_fused_rays_s(FusedArgs a, cudaStream_t s) {
     int dev = 0, sms = 152, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1075,12 +1094,15 @@ static cudaError_t launch_fused_rays_s(const FusedArgs& a, cudaStream_t s) {
     if (per_sm < 1) per_sm = 1;
     if (a.blocks_per_sm && (int)a.blocks_per_sm < per_sm) per_sm = (int)a.blocks_per_sm;
     uint32_t grid = (uint32_t)(sms * per_sm);
-    const uint32_t most = OF == SEGS ? a.units_max : (a.one.n + U - 1) / U;
-    const uint32_t need = (most + FW - 1) / FW;
-    if (need < grid) grid = need > 0 ? need : 1;
-    k_fused_rays<U, SHARE, OF><<<grid, FW * 32, 0, s>>>(a);
+    const uint32_t most = OF == SEGS_CLOSEST || OF == SEGS_ANY ? a.units_max : (a.one.n + U - 1) / U;
+    // two launches that run side by side have half of the warps each
+    a.warps = grid * FW / (a.pair ? 2u : 1u);
+    // a piece a warp: with more warps some SMs' would take them all
+    const uint64_t need = (((uint64_t)most << tail_split(most, a.warps, a.pixel_order)) + FW - 1) / FW;
+    if (need < grid) grid = need > 0 ? (uint32_t)need : 1;
+    const cudaError_t e = launch_chained(a.pair == 2u, k_fused_rays<U, SHARE, OF>, grid, FW * 32, 0, s, a);
     note_launch();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 template <int U, int OF>
 static cudaError_t launch_fused_rays_u(const FusedArgs& a, cudaStream_t s) {
@@ -1106,14 +1128,16 @@ static cudaError_t launch_fused_p(const FusedArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_rays_segs(const FusedArgs& a, cudaStream_t s) {
-    return launch_fused_rays_u<RSH_RAYS_UNIT, SEGS>(a, s);
+cudaError_t launch_rays_segs(const FusedArgs& a, bool any_hit, cudaStream_t s) {
+    if (a.units_max == 0) return cudaSuccess;
+    return any_hit ? launch_fused_rays_u<RSH_RAYS_UNIT, SEGS_ANY>(a, s)
+                   : launch_fused_rays_u<RSH_RAYS_UNIT, SEGS_CLOSEST>(a, s);
 }
 
 cudaError_t launch_rays_one(const FusedArgs& a, cudaStream_t s) {
     if (a.one.n == 0) return cudaSuccess;
-    return a.one.any_hit ? launch_fused_rays_u<RSH_RAYS_UNIT, ANY1>(a, s)
-                         : launch_fused_rays_u<RSH_RAYS_UNIT, CLOSEST1>(a, s);
+    return a.one.any_hit ? launch_fused_rays_u<RSH_RAYS_UNIT, ONE_ANY>(a, s)
+                         : launch_fused_rays_u<RSH_RAYS_UNIT, ONE_CLOSEST>(a, s);
 }
 
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t s) {

@@ -17,6 +17,24 @@ namespace rsh {
 // Counts this library's kernel launches (rsh_kernel_launches).
 void note_launch(unsigned n = 1);
 
+// A kernel that may start while the one before it in the stream still runs; it waits itself
+// (griddepcontrol.wait) before it touches what that one wrote.
+template <class... P, class... A>
+inline cudaError_t launch_chained(bool chained, void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem,
+                           cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 struct HashP {
     float lo[3];
     float scale[3];
@@ -250,13 +268,17 @@ struct FusedArgs {
     unsigned long long* node_tests;
     unsigned long long* tri_tests;
     uint32_t* err;
+    uint32_t warps;                    // set by the launch: warps that the GPU holds
+    bool pixel_order;                  // rays of neighbouring pixels lie together
+    uint32_t pair;                     // rays-only: 1, 2: the first / second of two launches that neither read
+                                       // nor write what the other writes; the second may start while the first runs
     FusedSeg one;                      // launch_rays_one: the one segment (slot_base 0)
     uint32_t* valid;                   // rays-only: the rays traced are added to valid[0] and valid[1] (null: not)
     unsigned long long* cand_pairs;    // launch_rays_one: counts (ray, cluster) pairs tested (null: not counted)
 };
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t s);
-// Rays alone from the root: the segments of the table / one segment, from the arguments.
-cudaError_t launch_rays_segs(const FusedArgs& a, cudaStream_t s);
+// Rays alone from the root: the segments of the table, all of one kind / one segment, from the arguments.
+cudaError_t launch_rays_segs(const FusedArgs& a, bool any_hit, cudaStream_t s);
 cudaError_t launch_rays_one(const FusedArgs& a, cudaStream_t s);
 // rays per work unit of the rays-only kernel (a multiple of 64, at most 256: job words hold 8 bits)
 #ifndef RSH_RAYS_UNIT

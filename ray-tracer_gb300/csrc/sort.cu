@@ -330,24 +330,6 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
 
 namespace {
 
-// A kernel that may start while the one before it in the stream still runs; it waits itself
-// (griddepcontrol.wait) before it touches what that one wrote.
-template <class... P, class... A>
-cudaError_t launch_chained(bool chained, void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem,
-                           cudaStream_t s, A... args) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &at;
-    c.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&c, kernel, P(args)...);
-}
-
 template <int T, int I, int MB>
 cudaError_t sweep(uint32_t n_max, uint32_t sms, uint32_t grid_max, bool chained, const uint32_t* ki, const uint32_t* vi,
                   uint32_t* ko, uint32_t* vo, const uint32_t* d_count, uint32_t shift, const uint32_t* hist,
