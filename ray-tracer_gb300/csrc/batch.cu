@@ -652,10 +652,11 @@ struct GraphExec {
 namespace rsh {
 rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
-                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair) {
+                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair, bool count_tests) {
     FusedArgs fa = alone_args(ctx, ticket);
     fa.pair = pair;
     fa.pixel_order = true;
+    if (!count_tests) fa.node_tests = fa.tri_tests = nullptr;
     fa.one.wtris = sc->h.wtris;
     fa.one.wnodes = sc->h.wnodes;
     fa.one.wnroot = sc->h.wnroot;

@@ -1147,7 +1147,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     uint32_t* ppix = static_cast<uint32_t*>(ctx->prim_pix.ptr);
     RSH_CUDA(launch_raygen_primary(to_camp(ctx->cam), W, H, prays, ppix, s));
     if (alone) {
-        RSH_TRY(trace_alone(ctx, sc, prays, np, nullptr, nullptr, false, nullptr, phits, tickets, pairs, s));
+        RSH_TRY(trace_alone(ctx, sc, prays, np, nullptr, nullptr, false, nullptr, phits, tickets, pairs, s, 0, false));
     } else if (fused) {
         rsh_batch_segment seg{sc, prays, np, 0, reinterpret_cast<uint64_t*>(phits), nullptr};
         ctx->timers_paused = true;  // the primary window times the whole primary pass
@@ -1161,10 +1161,13 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
         ctx->timers_paused = false;
         RSH_TRY(pst);
     }
-    RSH_CUDA(launch_resolve(sc->pos, sc->nrm, sc->mat, prays, phits, ppix, np,
-                            static_cast<float4*>(ctx->surf0_pos.ptr), static_cast<float4*>(ctx->surf0_nrm.ptr), s));
+    if (!alone) {
+        RSH_CUDA(launch_resolve(sc->pos, sc->nrm, sc->mat, prays, phits, ppix, np,
+                                static_cast<float4*>(ctx->surf0_pos.ptr), static_cast<float4*>(ctx->surf0_nrm.ptr),
+                                s));
+        RSH_CUDA(cudaMemsetAsync(ctx->d_stats, 0, 64, s));  // the frame's test counters cover secondary rays
+    }
     stage_end(ctx, th, s);
-    RSH_CUDA(cudaMemsetAsync(ctx->d_stats, 0, 64, s));  // the frame's test counters cover secondary rays
     RSH_CUDA(cudaEventRecord(ctx->ev[1], s));  // secondary window starts
 
     const float4* spos = static_cast<const float4*>(ctx->surf0_pos.ptr);
@@ -1185,34 +1188,75 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     sa.samples = S;
     for (uint32_t l = 0; l < L; ++l) sa.light[l] = ctx->lights[l];
     for (int i = 0; i < 3; ++i) sa.eye[i] = ctx->cam.eye[i];
-    for (uint32_t b = 0; b < depth; ++b) {
+    if (alone) {
+        // step b resolves the hits of the primary rays (b = 0) or of bounce b - 1, writes bounce b's rays and
+        // shades the surface before; the last step, b = depth, shades both remaining surfaces into the image
+        BounceArgs ba{};
+        ba.w = W;
+        ba.h = H;
+        ba.pos = sc->pos;
+        ba.nrm = sc->nrm;
+        ba.mat = sc->mat;
+        ba.lights = lp;
+        ba.eps = ctx->cfg.epsilon;
+        ba.jitter = ctx->cfg.reflect_jitter;
+        ba.seed = ctx->cfg.seed;
+        for (int i = 0; i < 3; ++i) ba.eye[i] = ctx->cam.eye[i];
+        ba.sids = static_cast<uint32_t*>(keys);
+        ba.rids = ba.sids + (size_t)npix * LS;
+        ba.rgba = rgba_out;
+        ba.sh = sa;
+        const rsh_ray* before = nullptr;  // the rays that met the surface to shade (bounce b - 2's)
+        for (uint32_t b = 0; b <= depth; ++b) {
+            ba.tiles_x = b == 0 ? tx : 0u;
+            ba.tiles_y = b == 0 ? ty : 0u;
+            ba.rays = b == 0 ? prays : incident;
+            ba.hits = b == 0 ? phits : static_cast<unsigned long long*>(ctx->bounce[b - 1].refl_hits.ptr);
+            ba.spos = static_cast<float4*>(b == 0 ? ctx->surf0_pos.ptr : ctx->bounce[b - 1].surf_pos.ptr);
+            ba.snrm = static_cast<float4*>(b == 0 ? ctx->surf0_nrm.ptr : ctx->bounce[b - 1].surf_nrm.ptr);
+            if (b > 0) {
+                ba.sh.spos = spos;
+                ba.sh.snrm = snrm;
+                ba.sh.shadow = static_cast<uint32_t*>(ctx->bounce[b - 1].shadow_flags.ptr);
+                ba.sh.bounce = b - 1;
+                ba.sh.incident = before;
+                before = incident;
+            }
+            const bool gen = b < depth;
+            if (gen) {
+                BounceBufs& bb = ctx->bounce[b];
+                ba.srays = static_cast<rsh_ray*>(bb.shadow_rays.ptr);
+                ba.rrays = ba.srays + (size_t)npix * LS;
+                ba.sflags = static_cast<uint32_t*>(bb.shadow_flags.ptr);
+                ba.rhits = static_cast<unsigned long long*>(bb.refl_hits.ptr);
+                ba.scount = fc + 4 * b;
+                ba.rcount = fc + 4 * b + 2;
+                ba.bounce = b;
+            }
+            th = stage_begin(ctx, gen ? RSH_STAGE_RAYGEN : RSH_STAGE_SHADE, s);
+            RSH_CUDA(launch_bounce(ba, rgba_out && b > 0, gen, rgba_out && !gen, s));
+            stage_end(ctx, th, s);
+            if (!gen) break;
+            th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
+            // side by side: the shadow rays' warps start as the reflection rays' end (Cornell frame 200 -> 171 us,
+            // architecture frame 3.37 -> 3.27 ms)
+            RSH_TRY(trace_alone(ctx, sc, ba.rrays, npix, ba.rids, ba.rcount, false, nullptr, ba.rhits,
+                                tickets + 1 + 2 * b, pairs, s, 1));
+            RSH_TRY(trace_alone(ctx, sc, ba.srays, npix * LS, ba.sids, ba.scount, true, ba.sflags, nullptr,
+                                tickets + 2 + 2 * b, pairs, s, 2));
+            stage_end(ctx, th, s);
+            spos = ba.spos;
+            snrm = ba.snrm;
+            incident = ba.rrays;
+        }
+    }
+    for (uint32_t b = 0; b < depth && !alone; ++b) {
         BounceBufs& bb = ctx->bounce[b];
         rsh_ray* srays = static_cast<rsh_ray*>(bb.shadow_rays.ptr);
         uint32_t* sflags = static_cast<uint32_t*>(bb.shadow_flags.ptr);
         rsh_ray* rrays = srays + (size_t)npix * LS;
         unsigned long long* rhits = static_cast<unsigned long long*>(bb.refl_hits.ptr);
-        if (alone) {
-            RayOut so, ro;
-            so.ids = static_cast<uint32_t*>(keys);
-            so.count = fc + 4 * b;
-            so.flags = sflags;
-            ro.ids = so.ids + (size_t)npix * LS;
-            ro.count = fc + 4 * b + 2;
-            ro.hits = rhits;
-            th = stage_begin(ctx, RSH_STAGE_RAYGEN, s);
-            RSH_CUDA(launch_raygen_shadow(spos, snrm, W, H, lp, ctx->cfg.epsilon, hp_s, srays, nullptr, s, so));
-            RSH_CUDA(launch_raygen_reflect(spos, snrm, incident, ctx->cam.eye, W, H, ctx->cfg.epsilon,
-                                           ctx->cfg.reflect_jitter, ctx->cfg.seed, b, hp_r, rrays, nullptr, s, ro));
-            stage_end(ctx, th, s);
-            th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
-            // side by side: the shadow rays' warps start as the reflection rays' end (Cornell frame 200 -> 171 us,
-            // architecture frame 3.37 -> 3.27 ms)
-            RSH_TRY(trace_alone(ctx, sc, rrays, npix, ro.ids, ro.count, false, nullptr, rhits, tickets + 1 + 2 * b,
-                                pairs, s, 1));
-            RSH_TRY(trace_alone(ctx, sc, srays, npix * LS, so.ids, so.count, true, sflags, nullptr,
-                                tickets + 2 + 2 * b, pairs, s, 2));
-            stage_end(ctx, th, s);
-        } else if (fused) {
+        if (fused) {
             // both batches of the bounce in one batched call: 2 segments, one persistent launch; ray
             // generation writes the batch's keys, segment counts and prefilled results itself
             rsh_batch_segment segs[2] = {
@@ -1282,7 +1326,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
         incident = rrays;
     }
     RSH_CUDA(cudaEventRecord(ctx->ev[2], s));  // secondary window ends
-    if (rgba_out) {
+    if (rgba_out && !alone) {
         th = stage_begin(ctx, RSH_STAGE_SHADE, s);
         sa.spos = spos;
         sa.snrm = snrm;

@@ -140,7 +140,8 @@ constexpr uint32_t STAT_CAND = 8;
 // the second may start while the first still runs (FusedArgs::pair).
 rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
-                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair = 0);
+                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair = 0,
+                       bool count_tests = true);
 
 // One secondary batch through compress -> sort -> decompress -> build -> traverse -> intersect.
 // keys: per slot (RSH_KEY_NONE = no ray); rays indexed by slot. Output flags/hits indexed by slot

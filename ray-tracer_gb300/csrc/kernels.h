@@ -308,6 +308,31 @@ struct ShadeArgs {
 cudaError_t launch_shade(const ShadeArgs& a, cudaStream_t s);
 cudaError_t launch_pack_rgba(const float4* accum, uint32_t n, uint32_t* rgba, cudaStream_t s);
 
+// ---- a frame's work between two traversals (bounce.cu)
+struct BounceArgs {
+    uint32_t w, h;
+    const float4 *pos, *nrm;          // the scene's triangles, normals and material ids (original order)
+    const uint32_t* mat;
+    const rsh_ray* rays;              // the traced rays whose hits are the next surface: the primary rays (tile
+    const unsigned long long* hits;   // order: tiles_x x tiles_y tiles) or reflection rays by pixel (tiles_x 0)
+    uint32_t tiles_x, tiles_y;
+    float4 *spos, *snrm;              // that surface (written)
+    // its rays (ray generation)
+    LightsP lights;
+    float eps, jitter;
+    uint32_t seed, bounce;
+    float eye[3];
+    rsh_ray *srays, *rrays;
+    uint32_t *sflags, *sids, *scount, *rids, *rcount;
+    unsigned long long* rhits;
+    // shading of the surface before it (ShadeArgs: its surface, flags, bounce and incident rays), the image
+    ShadeArgs sh;
+    uint32_t* rgba;
+};
+// shade: shade sh's surface first; gen: write the next surface's rays and lists, their results prefilled;
+// final_image (without gen): shade the next surface too, unshadowed, and pack the image.
+cudaError_t launch_bounce(const BounceArgs& a, bool shade, bool gen, bool final_image, cudaStream_t s);
+
 // ---- object transforms and bounds (transform.cu)
 cudaError_t launch_transform(const float4* pos_rest, const float4* nrm_rest, const uint32_t* obj, uint32_t tri_count,
                              uint32_t n_objects, const float* model, const float* normal, float4* pos, float4* nrm,

@@ -9,18 +9,11 @@
 #include "common.cuh"
 #include "hash.cuh"
 #include "kernels.h"
+#include "pixel.cuh"
 
 namespace rsh {
 
 // ------------------------------------------------------------------ primary rays (tile order)
-// Tile row r of the ray order is image tile row tile_row(r): from the middle outwards (m, m - 1, m + 1,
-// m - 2, ... with m = rows / 2). Primary rays run longest in the view's centre band (on typical views the
-// horizon, where rays travel far), so a persistent traversal starts them first instead of ending on them.
-RSH_DEV uint32_t tile_row(uint32_t r, uint32_t rows) {
-    const uint32_t m = rows >> 1;
-    return (r & 1u) ? m - ((r + 1u) >> 1) : m + (r >> 1);
-}
-
 __global__ void k_raygen_primary(CameraP cam, uint32_t w, uint32_t h, uint32_t tiles_x, uint32_t tiles_y, uint32_t n,
                                  rsh_ray* rays, uint32_t* pixel_of_ray) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -57,31 +50,6 @@ cudaError_t launch_raygen_primary(const CameraP& cam, uint32_t w, uint32_t h, rs
 }
 
 // ------------------------------------------------------------------ shadow rays
-// Soft-shadow sample k (0..15) around light position lp for the shadow direction d: the reference's 4x4
-// grid without its centre row/column (RayTracer.cu:1550-1599): k = i + 4 j, a = i (+1 from i = 2),
-// b = j (+1 from j = 2), position lp + axis0 (a - 2) / 8 + axis1 (b - 2) / 8, axis0 = cross(e, d) for the
-// axis e the reference picks by min(|dx|, max(|dy|, |dz|)), axis1 = cross(d, axis0) (neither normalised).
-RSH_DEV v3 soft_sample_pos(v3 lp, v3 d, uint32_t k) {
-    const uint32_t i = k & 3u, j = k >> 2;
-    const float ca = (float)((int)(i + (i >= 2u ? 1u : 0u)) - 2), cb = (float)((int)(j + (j >= 2u ? 1u : 0u)) - 2);
-    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-    const float mn = fminf(ax, fmaxf(ay, az));
-    const v3 e = (ax == mn) ? v3{1.f, 0.f, 0.f} : (ay == mn) ? v3{0.f, 1.f, 0.f} : v3{0.f, 0.f, 1.f};
-    const v3 a0 = cross3(e, d);
-    const v3 a1 = cross3(d, a0);
-    return v3{(lp.x + (a0.x * ca) * 0.125f) + (a1.x * cb) * 0.125f, (lp.y + (a0.y * ca) * 0.125f) + (a1.y * cb) * 0.125f,
-              (lp.z + (a0.z * ca) * 0.125f) + (a1.z * cb) * 0.125f};
-}
-
-// A block's share of a segment's ray count and, in list mode, of its id list: reserves `rays` entries with one
-// atomic and returns the first to every thread. Every thread of the block calls it.
-RSH_DEV uint32_t reserve_rays(uint32_t* count, uint32_t rays) {
-    __shared__ uint32_t s_base;
-    if (threadIdx.x == 0) s_base = rays ? atomicAdd(count, rays) : 0u;
-    __syncthreads();
-    return s_base;
-}
-
 // One thread per pixel: the pixel's surface point and normal are read and the normal normalised once,
 // then its V = L x S slots are written (slot = x + W (v + V y), RayTracer.cu:700-702 with S samples per
 // light), each with the same arithmetic as a thread per slot would use. The block's rays are counted once and
@@ -117,31 +85,8 @@ k_raygen_shadow(const float4* __restrict__ spos, const float4* __restrict__ snrm
         uint32_t key = RSH_KEY_NONE;
         if (surface) {
             const v3 lp = mk3(s_lp[3u * l], s_lp[3u * l + 1u], s_lp[3u * l + 2u]);
-            const v3 vl = p - lp;
-            const float len = len3(vl);
-            const v3 d = v3{vl.x / len, vl.y / len, vl.z / len};
-            const float diffuse = dot3(d, -nn);
-            const float tmax = len - 2.0f * eps;
-            if (diffuse > 0.0f && tmax > eps) {
-                v3 src = lp, dir = d;
-                float tm = tmax;
-                bool ok = true;
-                if (S > 1) {  // a sample of the 4x4 grid: its own origin, direction and interval
-                    src = soft_sample_pos(lp, d, sm);
-                    const v3 vs = p - src;
-                    const float ls = len3(vs);
-                    dir = v3{vs.x / ls, vs.y / ls, vs.z / ls};
-                    tm = ls - 2.0f * eps;
-                    ok = tm > eps;
-                }
-                if (ok) {
-                    const v3 o = src + dir * eps;
-                    ro = make_float4(o.x, o.y, o.z, eps);
-                    rd = make_float4(dir.x, dir.y, dir.z, tm);
-                    key = keys ? ray_hash(o.x, o.y, o.z, dir.x, dir.y, dir.z, hp, v) : 0u;
-                    valid = true;
-                }
-            }
+            valid = shadow_ray(p, nn, lp, eps, S, sm, ro, rd);
+            if (valid && keys) key = ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, hp, v);
         }
         if (in_range) {
             // an empty slot holds an explicit no-ray (tmax < tmin) for consumers without keys
@@ -192,28 +137,6 @@ cudaError_t launch_raygen_shadow(const float4* spos, const float4* snrm, uint32_
 }
 
 // ------------------------------------------------------------------ reflection rays
-// Integer hash of (seed, slot, bounce) -> 32 random bits (PCG output permutation on an LCG step).
-RSH_DEV uint32_t rng_next(uint32_t& state) {
-    state = state * 747796405u + 2891336453u;
-    uint32_t w = ((state >> ((state >> 28) + 4u)) ^ state) * 277803737u;
-    return (w >> 22) ^ w;
-}
-// Uniform point on the unit sphere by Marsaglia's (1972) rejection method: sqrt only.
-RSH_DEV v3 sphere_sample(uint32_t seed, uint32_t slot, uint32_t bounce) {
-    uint32_t st = seed ^ (slot * 0x9E3779B9u) ^ (bounce * 0x85EBCA6Bu);
-    rng_next(st);
-    for (int it = 0; it < 32; ++it) {
-        const float x1 = (float)(rng_next(st) >> 9) * (1.0f / 4194304.0f) - 1.0f;
-        const float x2 = (float)(rng_next(st) >> 9) * (1.0f / 4194304.0f) - 1.0f;
-        const float q = x1 * x1 + x2 * x2;
-        if (q < 1.0f && q > 0.0f) {
-            const float t = 2.0f * sqrtf(1.0f - q);
-            return v3{x1 * t, x2 * t, 1.0f - 2.0f * q};
-        }
-    }
-    return v3{0.0f, 0.0f, 1.0f};
-}
-
 __global__ void k_raygen_reflect(const float4* __restrict__ spos, const float4* __restrict__ snrm,
                                  const rsh_ray* __restrict__ prev, v3 eye, uint32_t n, float eps,
                                  float jitter, uint32_t seed, uint32_t bounce, HashP hp,
@@ -238,26 +161,11 @@ __global__ void k_raygen_reflect(const float4* __restrict__ spos, const float4* 
             } else {
                 i = norm3(p - eye);
             }
-            const float k2 = 2.0f * dot3(nn, i);
-            v3 r = i - nn * k2;  // reflect(i, n)
-            if (jitter > 0.0f) {
-                const v3 u = sphere_sample(seed, slot, bounce);
-                r = r + u * jitter;
-                const float rn = dot3(r, nn);
-                if (rn < 0.0f) r = r - nn * (2.0f * rn);
-            }
-            r = norm3(r);
-            if (r.x == r.x && r.y == r.y && r.z == r.z) {  // drop degenerate (NaN) directions
-                const v3 o = p + r * eps;
-                ro = make_float4(o.x, o.y, o.z, eps);
-                rd = make_float4(r.x, r.y, r.z, __int_as_float(0x7f800000));
-                store_ray32(rays, slot, ro, rd, a32);
-                key = keys ? ray_hash(o.x, o.y, o.z, r.x, r.y, r.z, hp, 0u) : 0u;
-                valid = true;
-            }
+            valid = reflect_ray(p, nn, i, eps, jitter, seed, slot, bounce, ro, rd);
+            if (valid && keys) key = ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, hp, 0u);
         }
         // no ray: stored as such, also for the next bounce, which reads this array as its incident rays
-        if (!valid) store_ray32(rays, slot, ro, rd, a32);
+        store_ray32(rays, slot, ro, rd, a32);
         if (keys) keys[slot] = key;
     }
     if (out.count) {
