@@ -29,21 +29,40 @@ namespace {
 constexpr uint32_t FLAG_AGG = 1u << 30;
 constexpr uint32_t FLAG_PRE = 2u << 30;
 constexpr uint32_t VAL_MASK = (1u << 30) - 1u;
-// Tile shapes (threads, keys a thread, CTAs per SM): large tiles for long runs of one digit in the output and few
-// tiles to look back over; small ones where large ones would leave SMs without a tile (512 x 14 against 256 x 8:
-// 16 M random 31-bit pairs 440 / 590 us, 1 M 69 / 85, 320,000 64 / 56, 20,000 57 / 45).
-constexpr int L_T = 512, L_I = 14, L_MB = 2, S_T = 256, S_I = 8, S_MB = 6;
-constexpr uint32_t SMALL_PAIRS = 1u << 19;
-constexpr uint32_t L_TILE = L_T * L_I, S_TILE = S_T * S_I;
-inline bool small_tiles(uint32_t n_max) { return n_max <= SMALL_PAIRS; }
-inline uint32_t tile_of(uint32_t n_max) { return small_tiles(n_max) ? S_TILE : L_TILE; }
+constexpr uint32_t SW_T = 512, SW_I = 14, SW_MIN = 2;  // threads, most and fewest rows of T keys a tile
+constexpr int SW_MB = 2;                                // CTAs per SM
+// Rows of a tile, from the actual count, which a kernel knows and the host may not: as many as make one tile a CTA,
+// within the limits. Large tiles give long runs of one digit in the output and few tiles to look back over; small
+// ones leave no SM without a tile. us, against 2048-key tiles up to 512 K pairs of capacity and 7168-key tiles above:
+// 320,000 random pairs 53 -> 48, 600,000 of a capacity of 2.76 M 70 -> 60, 50,000 of it 63 -> 38; the same at 20,000
+// and 16 M. From SW_NEAR rows on all SW_I: nearly as few idle SMs, and nothing to check row by row.
+constexpr uint32_t SW_NEAR = 11;
+__host__ __device__ __forceinline__ uint32_t tile_rows(uint32_t n, uint32_t ctas) {
+    const uint32_t r = (uint32_t)(((uint64_t)n + (uint64_t)ctas * SW_T - 1u) / ((uint64_t)ctas * SW_T));
+    return r < SW_MIN ? SW_MIN : r >= SW_NEAR ? SW_I : r;
+}
+// The CTAs of a pass for up to n_max keys on `sms` SMs: one a tile and SM while the tiles that gives hold the keys
+// (a tile that shares its SM ends last), else as many as are resident at once.
+inline uint32_t sweep_ctas(uint32_t n_max, uint32_t sms) {
+    return n_max <= sms * SW_T * SW_I ? std::min(sms, (n_max + SW_T * SW_MIN - 1) / (SW_T * SW_MIN))
+                                      : sms * (uint32_t)SW_MB;
+}
+inline size_t most_tiles(uint32_t n_max, uint32_t ctas) {
+    return std::max<size_t>(ctas, (n_max + SW_T * SW_I - 1) / (SW_T * SW_I)) + 1;
+}
+inline uint32_t sm_count() {
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (uint32_t)sms;
+}
 inline uint32_t num_passes(uint32_t key_bits) { return key_bits == 0 ? 1u : (key_bits + 7u) / 8u; }
 }  // namespace
 
 // --- histograms of every pass in one read; also clears the look-back status rows of the tiles that
 // the passes will use (ceil(n / tile) rows of 256 words per pass, pass stride `stride` words)
 __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
-                            const uint32_t* __restrict__ d_count, uint32_t passes, uint32_t tile_keys,
+                            const uint32_t* __restrict__ d_count, uint32_t passes, uint32_t ctas,
                             uint32_t* __restrict__ hist, uint32_t* __restrict__ status, size_t stride,
                             uint32_t* __restrict__ done) {
     __shared__ uint32_t sh[4][256];
@@ -53,6 +72,7 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
     __syncthreads();
     const uint32_t n = dev_count(d_count, n_max);
     {
+        const uint32_t tile_keys = SW_T * tile_rows(n, ctas);
         const size_t words = (size_t)((n + tile_keys - 1) / tile_keys) * 256u;  // multiple of 4
         const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
         for (uint32_t p = 0; p < passes; ++p) {
@@ -146,7 +166,7 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
     }
 }
 
-// One digit pass. T threads, I keys a thread; MB CTAs per SM.
+// One digit pass. T threads, up to I keys a thread; MB CTAs per SM.
 template <int T, int I>
 struct SweepSmem {
     uint32_t keys[T * I];
@@ -159,13 +179,15 @@ struct SweepSmem {
     uint32_t tile, next;
 };
 
-template <int T, int I, int MB>
+// FULL: every tile has I rows (known before the launch: no count on the device).
+template <int T, int I, int MB, bool FULL>
 __global__ void __launch_bounds__(T, MB)
 k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
            uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n_max,
            const uint32_t* __restrict__ d_count, uint32_t shift, const uint32_t* __restrict__ hist,
-           uint32_t* __restrict__ status, uint32_t* __restrict__ ticket, uint32_t* err, uint32_t spin_limit) {
-    constexpr uint32_t TILE = T * I, W = T / 32;
+           uint32_t* __restrict__ status, uint32_t* __restrict__ ticket, uint32_t* err, uint32_t spin_limit,
+           uint32_t ctas) {
+    constexpr uint32_t W = T / 32;
     static_assert(T >= 256, "a thread per digit");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SweepSmem<T, I>& S = *reinterpret_cast<SweepSmem<T, I>*>(smem_raw);
@@ -175,15 +197,17 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t n = dev_count(d_count, n_max);
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const uint32_t rows = FULL ? I : tile_rows(n, ctas), TILE = T * rows;
     const uint32_t num_tiles = (n + TILE - 1) / TILE;
     uint2* rk = S.rk[warp];
     uint32_t key[I];
     auto load_keys = [&](uint32_t t) {
         if (t >= num_tiles) return;
-        const uint32_t b = t * TILE + warp * (I * 32u) + lane;
+        const uint32_t b = t * TILE + warp * (rows * 32u) + lane;
         const bool whole = t * TILE + TILE <= n;
 #pragma unroll
-        for (int j = 0; j < I; ++j) key[j] = whole || b + j * 32u < n ? __ldg(keys_in + b + j * 32u) : 0xFFFFFFFFu;
+        for (int j = 0; j < I; ++j)
+            if (FULL || (uint32_t)j < rows) key[j] = whole || b + j * 32u < n ? __ldg(keys_in + b + j * 32u) : 0xFFFFFFFFu;
     };
     if (tid == 0) S.tile = atomicAdd(ticket, 1u);
     __syncthreads();
@@ -198,13 +222,14 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
             for (uint32_t i = tid; i < W * 128u; i += T) z[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         __syncthreads();
-        const uint32_t base = tile * TILE, wbase = base + warp * (I * 32u);
+        const uint32_t base = tile * TILE, wbase = base + warp * (rows * 32u);
         const bool full = base + TILE <= n;  // the whole tile holds valid items
         // stable in-warp ranking: items in (j, lane) order = index order. The lanes of a digit find each other
         // through a lane mask in shared memory
         uint32_t rank[(I + 1) / 2];  // two 16-bit ranks a word
 #pragma unroll
         for (int j = 0; j < I; ++j) {
+            if (!FULL && (uint32_t)j >= rows) break;
             const bool valid = full || wbase + j * 32u + lane < n;
             const uint32_t d = (key[j] >> shift) & 255u;
             if (valid) atomicOr(&rk[d].y, 1u << lane);
@@ -253,12 +278,14 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
             uint32_t val[I];
 #pragma unroll
             for (int j = 0; j < I; ++j) {
+                if (!FULL && (uint32_t)j >= rows) break;
                 const uint32_t idx = wbase + j * 32u + lane;
                 val[j] = idx;
                 if (vals_in && (full || idx < n)) val[j] = __ldg(vals_in + idx);
             }
 #pragma unroll
             for (int j = 0; j < I; ++j) {
+                if (!FULL && (uint32_t)j >= rows) break;
                 if (full || wbase + j * 32u + lane < n) {
                     const uint32_t pos = rk[(key[j] >> shift) & 255u].x + ((rank[j / 2] >> (16 * (j & 1))) & 0xFFFFu);
                     S.keys[pos] = key[j];
@@ -330,30 +357,24 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
 
 namespace {
 
-template <int T, int I, int MB>
-cudaError_t sweep(uint32_t n_max, uint32_t sms, uint32_t grid_max, bool chained, const uint32_t* ki, const uint32_t* vi,
-                  uint32_t* ko, uint32_t* vo, const uint32_t* d_count, uint32_t shift, const uint32_t* hist,
-                  uint32_t* status, uint32_t* ticket, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
-    const auto kernel = k_onesweep<T, I, MB>;
-    constexpr size_t smem = sizeof(SweepSmem<T, I>), SM_BYTES = 228 * 1024, MOST = 227 * 1024;
+// One pass over up to n_max keys: `ctas` CTAs (at most those resident at once: every ticket below a CTA's tile is
+// held by a running CTA, which is the look-back's forward progress).
+cudaError_t sweep(uint32_t n_max, uint32_t sms, uint32_t ctas, uint32_t grid, bool chained, const uint32_t* ki,
+                  const uint32_t* vi, uint32_t* ko, uint32_t* vo, const uint32_t* d_count, uint32_t shift,
+                  const uint32_t* hist, uint32_t* status, uint32_t* ticket, uint32_t* err, uint32_t spin_limit,
+                  cudaStream_t s) {
+    const auto kernel = !d_count && tile_rows(n_max, ctas) == SW_I ? k_onesweep<(int)SW_T, (int)SW_I, SW_MB, true>
+                                                                   : k_onesweep<(int)SW_T, (int)SW_I, SW_MB, false>;
+    constexpr size_t smem = sizeof(SweepSmem<(int)SW_T, (int)SW_I>), MOST = 227 * 1024;
+    static_assert(SW_MB * (smem + 1024) <= 228 * 1024, "SW_MB CTAs fit an SM");
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST);
     if (e != cudaSuccess) return e;
-    // at most the CTAs resident at once: tiles beyond the device count cost nothing, and every ticket below a
-    // CTA's tile is held by a running CTA (forward progress of the look-back)
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, T, smem);
-    if (per_sm < 1) per_sm = 1;
-    const uint32_t tiles = (n_max + T * I - 1) / (T * I);
-    const uint32_t grid = std::min(std::min(tiles, sms * (uint32_t)per_sm), grid_max);
     // A chained launch's CTAs are placed while the pass before it still runs, on whichever SMs have room: with
-    // room for more CTAs than an SM's share, some SMs get several and others none. Asking for the shared memory
-    // of an SM's share leaves room for no more
-    const uint32_t share = (grid + sms - 1) / sms;
-    // (1 M random pairs: 61 us, 71 unchained, 75 chained without this; 16 M: 428 / 440).
-    const size_t padded = share < (uint32_t)per_sm
-                              ? std::max(smem, std::min(MOST, SM_BYTES / share - 1024) & ~size_t(127)) : smem;
-    e = launch_chained(chained, kernel, grid, T, padded, s, ki, vi, ko, vo, n_max, d_count, shift, hist, status, ticket,
-                       err, spin_limit);
+    // room for more CTAs than an SM's share, some SMs get several and others none. With no more CTAs than SMs,
+    // asking for an SM's shared memory leaves room for one (1 M random pairs: 61 us, 71 unchained, 75 chained
+    // without this; 16 M: 428 / 440).
+    e = launch_chained(chained, kernel, grid, SW_T, ctas <= sms ? MOST : smem, s, ki, vi, ko, vo, n_max, d_count, shift,
+                       hist, status, ticket, err, spin_limit, ctas);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -362,8 +383,7 @@ cudaError_t sweep(uint32_t n_max, uint32_t sms, uint32_t grid_max, bool chained,
 
 size_t sort_scratch_bytes(uint32_t n_max, uint32_t key_bits) {
     const size_t passes = num_passes(key_bits);
-    const size_t tiles = (n_max + tile_of(n_max) - 1) / tile_of(n_max) + 1;
-    const size_t words = 4 * 256 + 16 + passes * tiles * 256;
+    const size_t words = 4 * 256 + 16 + passes * most_tiles(n_max, sweep_ctas(n_max, sm_count())) * 256;
     return words * 4 + 2 * (size_t)n_max * 4 + 1024;
 }
 
@@ -372,8 +392,8 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
                               uint32_t key_bits, void* scratch, uint32_t* err, cudaStream_t s, bool keys_wanted) {
     if (n_max == 0) return cudaSuccess;
     const uint32_t passes = num_passes(key_bits);
-    const uint32_t tile = tile_of(n_max);
-    const size_t tiles = (n_max + tile - 1) / tile + 1;
+    const uint32_t sms = sm_count(), ctas = sweep_ctas(n_max, sms);
+    const size_t tiles = most_tiles(n_max, ctas);
     uint32_t* w = static_cast<uint32_t*>(scratch);
     uint32_t* hist = w;                       // passes * 256 (room for 4)
     uint32_t* tickets = w + 4 * 256;          // 16: one per pass, [8] = histogram CTAs done
@@ -383,13 +403,10 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
     uint32_t* alt_vals = alt_keys + n_max;
     cudaError_t e = cudaMemsetAsync(w, 0, (4 * 256 + 16) * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // four CTAs per SM count 16 M keys in half the time of two; fewer when there is not a run of 16 keys for each
     // thread
-    const uint32_t hgrid = std::min<uint32_t>((uint32_t)sms * 4u, (n_max + 4095u) / 4096u);
-    k_sort_hist<<<hgrid, 256, 0, s>>>(keys_in, n_max, d_count, passes, tile, hist, status, tiles * 256, tickets + 8);
+    const uint32_t hgrid = std::min<uint32_t>(sms * 4u, (n_max + 4095u) / 4096u);
+    k_sort_hist<<<hgrid, 256, 0, s>>>(keys_in, n_max, d_count, passes, ctas, hist, status, tiles * 256, tickets + 8);
     note_launch();
     // ping-pong so that the last pass lands in the output
     const uint32_t* ki = keys_in;
@@ -400,11 +417,8 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
         uint32_t* ko = to_out ? keys_out : alt_keys;
         uint32_t* vo = to_out ? vals_out : alt_vals;
         if (p + 1 == passes && !keys_wanted) ko = nullptr;
-        e = small_tiles(n_max)
-                ? sweep<S_T, S_I, S_MB>(n_max, (uint32_t)sms, ~0u, true, ki, vi, ko, vo, d_count, 8u * p, hist + 256u * p,
-                                        status + p * tiles * 256, tickets + p, err, RSH_SPIN_LIMIT, s)
-                : sweep<L_T, L_I, L_MB>(n_max, (uint32_t)sms, ~0u, true, ki, vi, ko, vo, d_count, 8u * p, hist + 256u * p,
-                                        status + p * tiles * 256, tickets + p, err, RSH_SPIN_LIMIT, s);
+        e = sweep(n_max, sms, ctas, ctas, true, ki, vi, ko, vo, d_count, 8u * p, hist + 256u * p,
+                  status + p * tiles * 256, tickets + p, err, RSH_SPIN_LIMIT, s);
         if (e != cudaSuccess) return e;
         ki = ko;
         vi = vo;
@@ -412,16 +426,18 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
     return cudaSuccess;
 }
 
+constexpr uint32_t SELF_TILE = SW_T * SW_MIN;  // two tiles for two CTAs: of the fewest rows
+
 // Self-test of the bounded look-back wait: one sort pass over two tiles whose first tile is never run
 // (its ticket is taken before the launch), so the second tile waits on a status word that nothing
 // publishes. The wait must give up after `spin_limit` polls and raise RSH_DEVERR_TIMEOUT in *err
 // instead of hanging; every write stays in bounds. Buffers (2 tiles of keys in/out, status, tickets)
 // come from the caller's scratch of sort_selftest_scratch_bytes().
-size_t sort_selftest_scratch_bytes() { return (size_t)(4 * 2 * S_TILE + 2 * 256 + 256 + 8) * 4 + 1024; }
+size_t sort_selftest_scratch_bytes() { return (size_t)(4 * 2 * SELF_TILE + 2 * 256 + 256 + 8) * 4 + 1024; }
 
 cudaError_t sort_selftest_timeout(void* scratch, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
     uint32_t* w = static_cast<uint32_t*>(scratch);
-    const uint32_t n = 2 * S_TILE;
+    const uint32_t n = 2 * SELF_TILE;
     uint32_t* keys_in = w;
     uint32_t* vals_in = keys_in + n;
     uint32_t* keys_out = vals_in + n;
@@ -433,8 +449,8 @@ cudaError_t sort_selftest_timeout(void* scratch, uint32_t* err, uint32_t spin_li
     if (e != cudaSuccess) return e;
     const uint32_t one = 1u;  // tile 0's ticket is already gone: the one CTA gets tile 1
     if ((e = cudaMemcpyAsync(ticket, &one, 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-    e = sweep<S_T, S_I, S_MB>(n, 1u, 1u, false, keys_in, vals_in, keys_out, vals_out, nullptr, 0u, hist, status, ticket,
-                              err, spin_limit, s);
+    e = sweep(n, sm_count(), 2u, 1u, false, keys_in, vals_in, keys_out, vals_out, nullptr, 0u, hist, status, ticket, err,
+              spin_limit, s);
     if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(s);
 }
