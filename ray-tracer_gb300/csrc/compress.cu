@@ -6,27 +6,27 @@
 // CreateChunkSizes :956-991). Semantics kept: trimmed order = slot order; a chunk is a maximal run of
 // equal keys in trimmed order; chunk c has key, base (trimmed index of its head) and size.
 //
-// GB300 form: reduce-then-scan in three launches, with no inter-CTA waiting at all:
-//   k_compress_reduce  one CTA per 4096-slot tile reduces the tile to the associative summary (valid
-//                      count, head count, first key, last key);
-//   k_compress_scan    one CTA scans the tile summaries into tile prefixes (and writes the counts and
-//                      the sentinel chunk_bases[C] = R);
-//   k_compress_write   one CTA per tile re-reads its keys (an L2 hit at frame sizes), combines tile,
-//                      warp and lane prefixes, and writes trimmed ids, chunk keys and chunk bases
-//                      through one shared-memory staging buffer, coalesced.
-// At frame sizes (2-10 M slots, one or a few waves of tiles) a single-pass decoupled look-back spends
-// most of its time in the first wave's look-back chain (every predecessor holds an aggregate only),
-// which this form does not have. Counts stay on the device.
+// GB300 form: reduce-then-scan in two launches, with no inter-CTA waiting at all:
+//   k_compress_reduce  a fixed number of CTAs share the slots; each warp reduces a contiguous range of whole rows of
+//                      32 to the associative summary (valid count, head count, first key, last key);
+//   k_compress_write   the same CTAs fold the summaries before theirs, re-read their keys (an L2 hit at frame sizes)
+//                      and write trimmed ids, chunk keys and chunk bases.
+// A lane takes a slot of each row, and ballots give the places: reads and writes are coalesced without staging
+// (16 consecutive slots a thread staged through shared memory, 16-way bank conflicts, and a third launch for the scan
+// of the tiles' summaries before: with 2.76 M slots 3 us more of 152 from raygen to the hierarchy). A few hundred
+// summaries are cheap for every CTA to fold; a single pass with decoupled look-back spends most of its time in the
+// first wave's chain at frame sizes. Bound by issue slots (65% busy), 9 + 13 us. Counts stay on the device.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
 namespace rsh {
 
 namespace {
-constexpr int CT_THREADS = 256;
-constexpr int CT_ITEMS = 16;
-constexpr int CT_TILE = CT_THREADS * CT_ITEMS;  // 4096
-constexpr int CS_THREADS = 1024;                // the summary scan
+constexpr uint32_t CT_THREADS = 256, CT_WARPS = CT_THREADS / 32;
+constexpr uint32_t CT_CTAS = 4 * 152;   // most CTAs: four per SM
+constexpr uint32_t CT_BATCH = 16;       // rows whose loads are in flight together
 
 struct Summ {  // summary of a key range: valid count, heads (first valid counted), first/last key
     uint32_t n, h, first, last;
@@ -50,203 +50,137 @@ RSH_DEV Summ shfl_up(const Summ& s, int d) {
 RSH_DEV uint4 to4(const Summ& s) { return make_uint4(s.n, s.h, s.first, s.last); }
 RSH_DEV Summ from4(const uint4& v) { return Summ{v.x, v.y, v.z, v.w}; }
 
-// The tile's keys, 16 consecutive slots per thread (vector loads when aligned and whole).
-RSH_DEV void load_tile(const uint32_t* __restrict__ keys, uint32_t n_slots, bool vec_ok, uint32_t t0,
-                       uint32_t (&k)[CT_ITEMS]) {
-    if (vec_ok && t0 + CT_ITEMS <= n_slots) {
-        const uint4* p = reinterpret_cast<const uint4*>(keys + t0);
+
+// The warp's slots [b, e), row by row: f(slot, key, valid lanes, heads) with the lanes that hold a ray and the ones
+// that start a chunk, given the last key before (if any). Returns the heads and rays added to n and h; first is set
+// at the first ray of the range (`any` false).
+struct Range {
+    uint32_t n, h, last;
+    bool any;
+};
+RSH_DEV void load_rows(const uint32_t* __restrict__ keys, uint32_t q, uint32_t e, uint32_t (&k)[CT_BATCH]) {
 #pragma unroll
-        for (int q = 0; q < CT_ITEMS / 4; ++q) {
-            const uint4 v = __ldg(p + q);
-            k[4 * q] = v.x;
-            k[4 * q + 1] = v.y;
-            k[4 * q + 2] = v.z;
-            k[4 * q + 3] = v.w;
+    for (uint32_t i = 0; i < CT_BATCH; ++i) {
+        const uint32_t s = 32u * i + lane_id();
+        k[i] = q < e && s < e - q ? __ldg(keys + q + s) : RSH_KEY_NONE;
+    }
+}
+template <class F>
+RSH_DEV void rows(const uint32_t* __restrict__ keys, uint32_t b, uint32_t e, uint32_t (&k)[CT_BATCH], Range& r, F f) {
+    const uint32_t lane = lane_id(), below = lanemask_lt();
+    for (uint32_t q = b; q < e;) {
+        const uint32_t next = e - q > 32u * CT_BATCH ? q + 32u * CT_BATCH : e;
+        uint32_t kn[CT_BATCH];
+        load_rows(keys, next, e, kn);
+#pragma unroll
+        for (uint32_t i = 0; i < CT_BATCH; ++i) {
+            const bool valid = k[i] != RSH_KEY_NONE;
+            const uint32_t v = __ballot_sync(0xffffffffu, valid);
+            if (v == 0u) continue;
+            const uint32_t vb = v & below;
+            const uint32_t before = __shfl_sync(0xffffffffu, k[i], vb ? 31 - __clz(vb) : 0);
+            const bool head = valid && (vb ? before != k[i] : !r.any || r.last != k[i]);
+            const uint32_t hm = __ballot_sync(0xffffffffu, head);
+            f(q + 32u * i + lane, k[i], v, hm, valid, head);
+            r.n += __popc(v);
+            r.h += __popc(hm);
+            r.last = __shfl_sync(0xffffffffu, k[i], 31 - __clz(v));
+            r.any = true;
         }
-    } else {
 #pragma unroll
-        for (int i = 0; i < CT_ITEMS; ++i) k[i] = (t0 + i < n_slots) ? __ldg(keys + t0 + i) : RSH_KEY_NONE;
+        for (uint32_t i = 0; i < CT_BATCH; ++i) k[i] = kn[i];
+        q = next;
     }
 }
 
-RSH_DEV Summ thread_summary(const uint32_t (&k)[CT_ITEMS]) {
-    Summ ts{0u, 0u, 0u, 0u};
-#pragma unroll
-    for (int i = 0; i < CT_ITEMS; ++i) {
-        if (k[i] != RSH_KEY_NONE) {
-            if (ts.n == 0u) {
-                ts.first = k[i];
-                ts.h = 1u;
-            } else if (k[i] != ts.last) {
-                ts.h += 1u;
-            }
-            ts.last = k[i];
-            ts.n += 1u;
-        }
-    }
-    return ts;
-}
-
-// Block-wide: warp-inclusive scan of the thread summaries; s_warp[w] becomes the exclusive prefix of
-// warp w inside the tile; returns the thread's warp-inclusive summary; *tile_total (thread 0) the tile's.
-RSH_DEV Summ block_scan(const Summ& ts, Summ* s_warp, Summ* tile_total) {
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    Summ inc = ts;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const Summ o = shfl_up(inc, d);
-        if (lane >= (uint32_t)d) inc = combine(o, inc);
-    }
-    if (lane == 31) s_warp[warp] = inc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        Summ run{0u, 0u, 0u, 0u};
-        for (int w = 0; w < CT_THREADS / 32; ++w) {
-            const Summ wv = s_warp[w];
-            s_warp[w] = run;
-            run = combine(run, wv);
-        }
-        *tile_total = run;
-    }
-    __syncthreads();
-    return inc;
+// The slots of a warp: whole rows, the same number for every warp but the last ones.
+RSH_DEV void warp_range(uint32_t n_slots, uint32_t ctas, uint32_t& b, uint32_t& e) {
+    const uint64_t per = 32ull * (((uint64_t)n_slots + 32ull * CT_WARPS * ctas - 1u) / (32ull * CT_WARPS * ctas));
+    const uint64_t x = per * (blockIdx.x * CT_WARPS + (threadIdx.x >> 5));
+    b = (uint32_t)min(x, (uint64_t)n_slots);
+    e = (uint32_t)min(x + per, (uint64_t)n_slots);
 }
 }  // namespace
 
+// csumm: a summary per CTA; wsumm: per warp
 __global__ void __launch_bounds__(CT_THREADS)
-k_compress_reduce(const uint32_t* __restrict__ keys, uint32_t n_slots, bool vec_ok, uint4* __restrict__ tsumm) {
-    __shared__ Summ s_warp[CT_THREADS / 32];
-    __shared__ Summ s_tot;
-    const uint32_t t0 = blockIdx.x * CT_TILE + threadIdx.x * CT_ITEMS;
-    uint32_t k[CT_ITEMS];
-    load_tile(keys, n_slots, vec_ok, t0, k);
-    block_scan(thread_summary(k), s_warp, &s_tot);
-    if (threadIdx.x == 0) tsumm[blockIdx.x] = to4(s_tot);
-}
-
-// One CTA: exclusive prefixes of the tile summaries (each thread folds a run of consecutive tiles).
-__global__ void __launch_bounds__(CS_THREADS)
-k_compress_scan(const uint4* __restrict__ tsumm, uint32_t tiles, uint32_t n_slots, uint4* __restrict__ tpre,
-                uint32_t* __restrict__ counts, uint32_t* __restrict__ chunk_bases) {
-    __shared__ Summ s_w[CS_THREADS / 32];
-    const uint32_t per = (tiles + CS_THREADS - 1) / CS_THREADS;
-    const uint32_t b = threadIdx.x * per, e = min(b + per, tiles);
-    Summ ts{0u, 0u, 0u, 0u};
-    for (uint32_t i = b; i < e; ++i) ts = combine(ts, from4(__ldg(tsumm + i)));
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    Summ inc = ts;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const Summ o = shfl_up(inc, d);
-        if (lane >= (uint32_t)d) inc = combine(o, inc);
+k_compress_reduce(const uint32_t* __restrict__ keys, uint32_t n_slots, uint4* __restrict__ csumm,
+                  uint4* __restrict__ wsumm) {
+    __shared__ Summ s_warp[CT_WARPS];
+    asm volatile("griddepcontrol.launch_dependents;");
+    uint32_t b, e;
+    warp_range(n_slots, gridDim.x, b, e);
+    uint32_t k[CT_BATCH];
+    load_rows(keys, b, e, k);
+    Range r{0u, 0u, 0u, false};
+    uint32_t first = 0u;
+    rows(keys, b, e, k, r, [&](uint32_t, uint32_t key, uint32_t v, uint32_t, bool, bool) {
+        if (!r.any) first = __shfl_sync(0xffffffffu, key, __ffs(v) - 1);
+    });
+    const uint32_t warp = threadIdx.x >> 5;
+    if (lane_id() == 0u) {
+        s_warp[warp] = Summ{r.n, r.h, first, r.last};
+        wsumm[blockIdx.x * CT_WARPS + warp] = to4(s_warp[warp]);
     }
-    if (lane == 31) s_w[warp] = inc;
     __syncthreads();
     if (threadIdx.x == 0) {
-        Summ run{0u, 0u, 0u, 0u};
-        for (int w = 0; w < CS_THREADS / 32; ++w) {
-            const Summ wv = s_w[w];
-            s_w[w] = run;
-            run = combine(run, wv);
-        }
-        const uint32_t R = run.n < n_slots ? run.n : n_slots;
-        const uint32_t C = run.h < n_slots ? run.h : n_slots;
-        counts[0] = R;
-        counts[1] = C;
-        chunk_bases[C] = R;
-    }
-    __syncthreads();
-    Summ lane_ex = shfl_up(inc, 1);
-    if (lane == 0) lane_ex = Summ{0u, 0u, 0u, 0u};
-    Summ run = combine(s_w[warp], lane_ex);
-    for (uint32_t i = b; i < e; ++i) {
-        tpre[i] = to4(run);
-        run = combine(run, from4(__ldg(tsumm + i)));
+        Summ t = s_warp[0];
+        for (uint32_t w = 1; w < CT_WARPS; ++w) t = combine(t, s_warp[w]);
+        csumm[blockIdx.x] = to4(t);
     }
 }
 
 __global__ void __launch_bounds__(CT_THREADS)
-k_compress_write(const uint32_t* __restrict__ keys, uint32_t n_slots, bool vec_ok, const uint4* __restrict__ tpre,
-                 uint32_t* __restrict__ trimmed_ids, uint32_t* __restrict__ chunk_keys,
-                 uint32_t* __restrict__ chunk_bases) {
-    __shared__ uint32_t s_buf[CT_TILE];
-    __shared__ Summ s_warp[CT_THREADS / 32];
-    __shared__ Summ s_tot;
-    __shared__ uint32_t s_tn, s_th;
+k_compress_write(const uint32_t* __restrict__ keys, uint32_t n_slots, const uint4* __restrict__ csumm,
+                 const uint4* __restrict__ wsumm, uint32_t* __restrict__ trimmed_ids,
+                 uint32_t* __restrict__ chunk_keys, uint32_t* __restrict__ chunk_bases,
+                 uint32_t* __restrict__ counts) {
+    constexpr uint32_t PER = (CT_CTAS + CT_THREADS - 1) / CT_THREADS;
+    __shared__ Summ s_fold[CT_WARPS], s_own[CT_WARPS];
+    uint32_t b, e, k[CT_BATCH];
+    warp_range(n_slots, gridDim.x, b, e);
+    load_rows(keys, b, e, k);  // (what the kernel before this one reads too)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint32_t t0 = blockIdx.x * CT_TILE + threadIdx.x * CT_ITEMS;
-    uint32_t k[CT_ITEMS];
-    load_tile(keys, n_slots, vec_ok, t0, k);
-    const Summ inc = block_scan(thread_summary(k), s_warp, &s_tot);
-    // exclusive prefix of this thread = tile prefix (x) warp prefix (x) lane-exclusive
-    Summ lane_ex = shfl_up(inc, 1);
-    if (lane == 0) lane_ex = Summ{0u, 0u, 0u, 0u};
-    const Summ tile_pre = from4(__ldg(tpre + blockIdx.x));
-    const Summ run0 = combine(combine(tile_pre, s_warp[warp]), lane_ex);
-    const uint32_t r_base = tile_pre.n;  // trimmed index of the tile's first valid slot
-    // chunk index of the tile's first head: a tile that starts inside a run from the previous tile
-    // has no head there, which combine() already accounted for in tile_pre.h
-    const uint32_t h_tile0 = tile_pre.h;
-    // pass 1: trimmed ids
-    Summ run = run0;
+    // the CTAs before this one: a few in a row per thread, then in order across the lanes and the warps
+    Summ t{0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int i = 0; i < CT_ITEMS; ++i) {
-        if (k[i] != RSH_KEY_NONE) {
-            const uint32_t r = run.n - r_base;
-            if (r < (uint32_t)CT_TILE) s_buf[r] = t0 + i;
-            run.n += 1u;
-        }
+    for (uint32_t i = 0; i < PER; ++i) {
+        const uint32_t c = threadIdx.x * PER + i;
+        if (c < blockIdx.x) t = combine(t, from4(__ldcg(csumm + c)));
     }
-    if (threadIdx.x == CT_THREADS - 1) s_tn = min(run.n - r_base, (uint32_t)CT_TILE);
-    __syncthreads();
-    const uint32_t tn = s_tn;
-    for (uint32_t i = threadIdx.x; i < tn; i += CT_THREADS)
-        if (r_base + i < n_slots) trimmed_ids[r_base + i] = s_buf[i];
-    __syncthreads();
-    // pass 2: chunk keys of the heads
-    run = run0;
 #pragma unroll
-    for (int i = 0; i < CT_ITEMS; ++i) {
-        const uint32_t key = k[i];
-        if (key != RSH_KEY_NONE) {
-            if ((run.n == 0u) || (key != run.last)) {
-                const uint32_t c = run.h - h_tile0;
-                if (c < (uint32_t)CT_TILE) s_buf[c] = key;
-                run.h += 1u;
-            }
-            run.n += 1u;
-            run.last = key;
-        }
+    for (int d = 1; d < 32; d <<= 1) {
+        const Summ o = shfl_up(t, d);
+        if (lane >= (uint32_t)d) t = combine(o, t);
     }
-    if (threadIdx.x == CT_THREADS - 1) s_th = min(run.h - h_tile0, (uint32_t)CT_TILE);
+    if (lane == 31u) s_fold[warp] = t;
+    if (threadIdx.x < CT_WARPS) s_own[threadIdx.x] = from4(__ldcg(wsumm + blockIdx.x * CT_WARPS + threadIdx.x));
     __syncthreads();
-    const uint32_t th = s_th;
-    for (uint32_t i = threadIdx.x; i < th; i += CT_THREADS)
-        if (h_tile0 + i < n_slots) chunk_keys[h_tile0 + i] = s_buf[i];
-    __syncthreads();
-    // pass 3: chunk bases (trimmed index of each head)
-    run = run0;
-#pragma unroll
-    for (int i = 0; i < CT_ITEMS; ++i) {
-        const uint32_t key = k[i];
-        if (key != RSH_KEY_NONE) {
-            if ((run.n == 0u) || (key != run.last)) {
-                const uint32_t c = run.h - h_tile0;
-                if (c < (uint32_t)CT_TILE) s_buf[c] = run.n;
-                run.h += 1u;
-            }
-            run.n += 1u;
-            run.last = key;
-        }
+    Summ pre{0u, 0u, 0u, 0u};
+    for (uint32_t w = 0; w < CT_WARPS; ++w) pre = combine(pre, s_fold[w]);
+    for (uint32_t w = 0; w < warp; ++w) pre = combine(pre, s_own[w]);
+    if (blockIdx.x == gridDim.x - 1u && threadIdx.x == CT_THREADS - 32u) {  // the last warp: the totals
+        const Summ all = combine(pre, s_own[warp]);
+        counts[0] = all.n;
+        counts[1] = all.h;
+        chunk_bases[all.h] = all.n;
     }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < th; i += CT_THREADS)
-        if (h_tile0 + i < n_slots) chunk_bases[h_tile0 + i] = s_buf[i];
+    Range r{pre.n, pre.h, pre.last, pre.n > 0u};
+    const uint32_t below = lanemask_lt();
+    rows(keys, b, e, k, r, [&](uint32_t slot, uint32_t key, uint32_t v, uint32_t hm, bool valid, bool head) {
+        const uint32_t at = r.n + __popc(v & below), c = r.h + __popc(hm & below);
+        if (valid && at < n_slots) trimmed_ids[at] = slot;
+        if (head && c < n_slots) {
+            chunk_keys[c] = key;
+            chunk_bases[c] = at;
+        }
+    });
 }
 
 size_t compress_scratch_bytes(uint32_t n_slots) {
-    const size_t tiles = (n_slots + CT_TILE - 1) / CT_TILE + 1;
-    return tiles * 2 * sizeof(uint4) + 256;
+    (void)n_slots;
+    return (size_t)CT_CTAS * (1 + CT_WARPS) * sizeof(uint4) + 256;
 }
 
 cudaError_t launch_compress(const uint32_t* keys, uint32_t n_slots, uint32_t* trimmed_ids,
@@ -258,17 +192,16 @@ cudaError_t launch_compress(const uint32_t* keys, uint32_t n_slots, uint32_t* tr
         cudaMemsetAsync(chunk_bases, 0, sizeof(uint32_t), s);
         return cudaGetLastError();
     }
-    const uint32_t tiles = (n_slots + CT_TILE - 1) / CT_TILE;
-    uint4* tsumm = static_cast<uint4*>(scratch);
-    uint4* tpre = tsumm + tiles;
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
-    k_compress_reduce<<<tiles, CT_THREADS, 0, s>>>(keys, n_slots, vec_ok, tsumm);
+    // two rows a warp at least
+    const uint32_t ctas = std::min(CT_CTAS, (n_slots - 1u) / (64u * CT_WARPS) + 1u);
+    uint4* csumm = static_cast<uint4*>(scratch);
+    uint4* wsumm = csumm + ctas;
+    k_compress_reduce<<<ctas, CT_THREADS, 0, s>>>(keys, n_slots, csumm, wsumm);
     note_launch();
-    k_compress_scan<<<1, CS_THREADS, 0, s>>>(tsumm, tiles, n_slots, tpre, counts, chunk_bases);
+    const cudaError_t e = launch_chained(true, k_compress_write, ctas, CT_THREADS, 0, s, keys, n_slots, csumm, wsumm,
+                                         trimmed_ids, chunk_keys, chunk_bases, counts);
     note_launch();
-    k_compress_write<<<tiles, CT_THREADS, 0, s>>>(keys, n_slots, vec_ok, tpre, trimmed_ids, chunk_keys, chunk_bases);
-    note_launch();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 __global__ void k_chunk_sizes(const uint32_t* __restrict__ bases, const uint32_t* __restrict__ counts,

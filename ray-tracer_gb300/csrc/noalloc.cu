@@ -15,8 +15,8 @@ namespace {
 
 // Largest slot count one call accepts (16,777,216 = e.g. 1920 x 1080 pixels x 8 lights).
 constexpr uint32_t kMaxSlots = 1u << 24;
-// Room for compress tiles of 3072 slots or more at 9 words per tile; the current kernels use 4096-slot
-// tiles at 8 words per tile (compress_scratch_bytes), checked against the array below on every call.
+// Room for compress tiles of 3072 slots or more at 9 words per tile; the current kernels need less, whatever
+// n_slots is (compress_scratch_bytes), checked against the array below on every call.
 constexpr uint32_t kTileSlots = 3072u;
 constexpr uint32_t kMaxTiles = (kMaxSlots + kTileSlots - 1) / kTileSlots + 1;
 constexpr uint32_t kScratchWords = 4u + 9u * kMaxTiles;   // 49,171 words = 196,684 bytes
