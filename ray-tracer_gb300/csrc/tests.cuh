@@ -80,32 +80,29 @@ RSH_DEV bool ray_hits_sphere(float ox, float oy, float oz, float dx, float dy, f
 // Woop, Benthin & Wald, "Watertight Ray/Triangle Intersection", JCGT 2(1), 2013: shear the triangle
 // into the ray's frame (largest |d| axis becomes z), evaluate the 2-D edge functions, fall back to
 // double precision when one is exactly zero. Hit iff tmin < t < tmax with t = T / det (IEEE divide).
+// The axes after kz keep their cyclic order for both signs of d[kz]: swapping them, as the paper does to keep the
+// winding, negates U, V, W, det and T, and every test of them and T / det stay the same. So the permutation is one of
+// three, chosen by two predicates instead of six.
 struct RayWT {
     float ox, oy, oz;
     float sx, sy, sz;
-    int kx, ky, kz;
+    int kz;
     float tmin, tmax;
 };
-RSH_DEV float comp(float x, float y, float z, int k) { return k == 0 ? x : (k == 1 ? y : z); }
+// x, y, z of a vector -> its components along kz + 1, kz + 2 and kz (mod 3)
+RSH_DEV v3 turn(float x, float y, float z, int kz) {
+    const bool p = kz == 0, q = kz == 1;
+    return v3{p ? y : (q ? z : x), p ? z : (q ? x : y), p ? x : (q ? y : z)};
+}
 
 RSH_DEV RayWT wt_setup(float4 o, float4 d) {
     RayWT r;
     const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-    int kz = (ax >= ay) ? ((ax >= az) ? 0 : 2) : ((ay >= az) ? 1 : 2);
-    int kx = kz + 1 == 3 ? 0 : kz + 1;
-    int ky = kx + 1 == 3 ? 0 : kx + 1;
-    const float dz = comp(d.x, d.y, d.z, kz);
-    if (dz < 0.0f) {
-        const int t = kx;
-        kx = ky;
-        ky = t;
-    }
-    r.kx = kx;
-    r.ky = ky;
-    r.kz = kz;
-    r.sx = comp(d.x, d.y, d.z, kx) / dz;
-    r.sy = comp(d.x, d.y, d.z, ky) / dz;
-    r.sz = 1.0f / dz;
+    r.kz = (ax >= ay) ? ((ax >= az) ? 0 : 2) : ((ay >= az) ? 1 : 2);
+    const v3 t = turn(d.x, d.y, d.z, r.kz);
+    r.sx = t.x / t.z;
+    r.sy = t.y / t.z;
+    r.sz = 1.0f / t.z;
     r.ox = o.x;
     r.oy = o.y;
     r.oz = o.z;
@@ -115,28 +112,25 @@ RSH_DEV RayWT wt_setup(float4 o, float4 d) {
 }
 
 RSH_DEV bool wt_hit(const RayWT& r, float4 p0, float4 p1, float4 p2, float& t_out) {
-    const float A0 = p0.x - r.ox, A1 = p0.y - r.oy, A2 = p0.z - r.oz;
-    const float B0 = p1.x - r.ox, B1 = p1.y - r.oy, B2 = p1.z - r.oz;
-    const float C0 = p2.x - r.ox, C1 = p2.y - r.oy, C2 = p2.z - r.oz;
-    const float Akz = comp(A0, A1, A2, r.kz), Bkz = comp(B0, B1, B2, r.kz), Ckz = comp(C0, C1, C2, r.kz);
-    const float Ax = comp(A0, A1, A2, r.kx) - r.sx * Akz;
-    const float Ay = comp(A0, A1, A2, r.ky) - r.sy * Akz;
-    const float Bx = comp(B0, B1, B2, r.kx) - r.sx * Bkz;
-    const float By = comp(B0, B1, B2, r.ky) - r.sy * Bkz;
-    const float Cx = comp(C0, C1, C2, r.kx) - r.sx * Ckz;
-    const float Cy = comp(C0, C1, C2, r.ky) - r.sy * Ckz;
+    const v3 A = turn(p0.x - r.ox, p0.y - r.oy, p0.z - r.oz, r.kz);
+    const v3 B = turn(p1.x - r.ox, p1.y - r.oy, p1.z - r.oz, r.kz);
+    const v3 C = turn(p2.x - r.ox, p2.y - r.oy, p2.z - r.oz, r.kz);
+    const float Ax = A.x - r.sx * A.z, Ay = A.y - r.sy * A.z;
+    const float Bx = B.x - r.sx * B.z, By = B.y - r.sy * B.z;
+    const float Cx = C.x - r.sx * C.z, Cy = C.y - r.sy * C.z;
     float U = Cx * By - Cy * Bx;
     float V = Ax * Cy - Ay * Cx;
     float W = Bx * Ay - By * Ax;
-    if (U == 0.0f || V == 0.0f || W == 0.0f) {
+    if (fminf(fminf(fabsf(U), fabsf(V)), fabsf(W)) == 0.0f) {
         U = (float)((double)Cx * (double)By - (double)Cy * (double)Bx);
         V = (float)((double)Ax * (double)Cy - (double)Ay * (double)Cx);
         W = (float)((double)Bx * (double)Ay - (double)By * (double)Ax);
     }
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
+    // (a NaN counts as neither sign)
+    if (fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f) return false;
     const float det = (U + V) + W;
     if (det == 0.0f) return false;
-    const float Az = r.sz * Akz, Bz = r.sz * Bkz, Cz = r.sz * Ckz;
+    const float Az = r.sz * A.z, Bz = r.sz * B.z, Cz = r.sz * C.z;
     const float T = (U * Az + V * Bz) + W * Cz;
     const float t = T / det;
     t_out = t;
