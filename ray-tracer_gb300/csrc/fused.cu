@@ -648,7 +648,7 @@ RSH_DEV void slab4(float4 px, float4 py, float4 pz, float ix, float iy, float iz
 }
 
 #ifndef RSH_RAYS_MIN_BLOCKS
-#define RSH_RAYS_MIN_BLOCKS 7
+#define RSH_RAYS_MIN_BLOCKS 8  // of the SHARE instance, whose triangle tests' operands are in shared memory
 #endif
 #ifndef RSH_SHARE_BUSY
 #define RSH_SHARE_BUSY 16  // busy lanes at or below which a drained warp shares its rays (SHARE)
@@ -678,12 +678,19 @@ __host__ __device__ __forceinline__ uint32_t tail_split(uint32_t units, uint32_t
 enum RaysOf { SEGS_CLOSEST = 0, SEGS_ANY = 1, ONE_CLOSEST = 2, ONE_ANY = 3 };
 
 template <int U, bool SHARE, int OF>
-__global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(const __grid_constant__ FusedArgs a) {
+__global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fused_rays(const __grid_constant__ FusedArgs a) {
     constexpr bool ONE = OF == ONE_CLOSEST || OF == ONE_ANY, any = OF == SEGS_ANY || OF == ONE_ANY;
     // SHARE: a drained warp's rays shared among its idle lanes; the records of the rays being shared, one per
     // lane: the owner's best hit key (closest hit), occluded (any hit), helpers still on a subtree of it
     __shared__ unsigned long long sh_best[SHARE ? FW : 1][32];
     __shared__ uint32_t sh_occ[SHARE ? FW : 1][32], sh_pend[SHARE ? FW : 1][32];
+    // SHARE: what a triangle test needs of a lane's ray; a cluster step's clusters in lane order (first triangle less
+    // the triangles before it, the ray's lane, dominant axis and the lane it is tested for; with segments, the
+    // triangles); the best hit of the cluster's lane
+    __shared__ float4 sh_w0[SHARE ? FW : 1][32], sh_w1[SHARE ? FW : 1][32];
+    __shared__ uint2 sh_job[SHARE ? FW : 1][32];
+    __shared__ const float4* sh_tris[SHARE && !ONE ? FW : 1][32];
+    __shared__ unsigned long long sh_hit[SHARE ? FW : 1][32];
     __shared__ uint32_t s_rays, s_ended;  // a.valid: the block's rays, its warps that have ended
     const uint32_t lane = lane_id();
     asm volatile("griddepcontrol.launch_dependents;");
@@ -715,7 +722,8 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
     float ox = 0.f, oy = 0.f, oz = 0.f, tmin = 0.f, tcur = 0.f;
     float ix = 0.f, iy = 0.f, iz = 0.f, oix = 0.f, oiy = 0.f, oiz = 0.f;
     uint32_t oct = 0;  // the direction's octant: bit a set when component a is negative
-    RayWT w;
+    RayWT w;            // !SHARE
+    uint32_t kz = 0u;   // SHARE
     unsigned long long best = RSH_HIT_NONE;
     bool sharing = false;  // warp-uniform (SHARE): the warp shares its last rays
     bool done = false;     // sharing: the lane's subtree is done, its result not yet merged
@@ -834,7 +842,15 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                         oix = ox * ix;
                         oiy = oy * iy;
                         oiz = oz * iz;
-                        w = wt_setup(o, d);
+                        if (SHARE) {
+                            const RayWT r = wt_setup(o, d);
+                            const uint32_t wp = threadIdx.x >> 5;
+                            sh_w0[wp][lane] = make_float4(r.ox, r.oy, r.oz, r.sx);
+                            sh_w1[wp][lane] = make_float4(r.sy, r.sz, r.tmin, r.tmax);
+                            kz = (uint32_t)r.kz;
+                        } else {
+                            w = wt_setup(o, d);
+                        }
                         best = RSH_HIT_NONE;
                         oct = (ix < 0.f ? 1u : 0u) | (iy < 0.f ? 2u : 0u) | (iz < 0.f ? 4u : 0u);
                         top = sg.wnroot;
@@ -923,15 +939,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
                 oiy = __shfl_sync(0xffffffffu, oiy, src);
                 oiz = __shfl_sync(0xffffffffu, oiz, src);
                 oct = __shfl_sync(0xffffffffu, oct, src);
-                w.ox = __shfl_sync(0xffffffffu, w.ox, src);
-                w.oy = __shfl_sync(0xffffffffu, w.oy, src);
-                w.oz = __shfl_sync(0xffffffffu, w.oz, src);
-                w.sx = __shfl_sync(0xffffffffu, w.sx, src);
-                w.sy = __shfl_sync(0xffffffffu, w.sy, src);
-                w.sz = __shfl_sync(0xffffffffu, w.sz, src);
-                w.kz = __shfl_sync(0xffffffffu, w.kz, src);
-                w.tmin = __shfl_sync(0xffffffffu, w.tmin, src);
-                w.tmax = __shfl_sync(0xffffffffu, w.tmax, src);
+                kz = __shfl_sync(0xffffffffu, kz, src);
                 if (recv) {
                     own = go;
                     top = ge;
@@ -951,9 +959,73 @@ __global__ void __launch_bounds__(FW * 32, RSH_RAYS_MIN_BLOCKS) k_fused_rays(con
             const uint32_t nc = __popc(__ballot_sync(0xffffffffu, has && !node));
             do_nodes = nn >= nc;
         }
-        if (has && ((top >> 31) != 0u) == do_nodes) {
+        if (SHARE && !do_nodes) {
+            // The triangles of all the clusters at hand, spread over the lanes: one after the other per lane, the step
+            // took as long as its largest cluster and left most lanes idle. What a test needs of a ray is in shared
+            // memory, which frees the registers for an eighth CTA per SM (8 CTAs, this way / before with 7: 1 M rays
+            // 683 / 708 us, soup frame 2.25 / 2.35 ms, 64 batches 4.72 / 4.87, 20,001 shadow rays 31 / 35 us).
+            const uint32_t wp = threadIdx.x >> 5;
+            const bool mine = has && !(top >> 31);
+            const uint32_t owners = __ballot_sync(0xffffffffu, mine);
+            const uint32_t cnt = mine ? ((top >> 23) & 63u) + 1u : 0u;
+            uint32_t before = cnt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, before, d);
+                if (lane >= (uint32_t)d) before += y;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, before, 31);
+            before -= cnt;
+            if (mine) {
+                const uint32_t r = __popc(owners & lanemask_lt());
+                sh_job[wp][r] = make_uint2((top & 0x7FFFFFu) - before, own | (kz << 8) | (lane << 16));
+                if (!ONE) sh_tris[wp][r] = tris_v;
+                sh_hit[wp][lane] = best;
+            }
+            __syncwarp();
+            uint32_t jobs = 0;  // that start in the rows before
+            for (uint32_t base = 0; base < total; base += 32u) {
+                const uint32_t at = before - base;
+                const uint32_t starts = __reduce_or_sync(0xffffffffu, mine && at < 32u ? 1u << at : 0u);
+                const uint32_t q = jobs + __popc(starts & (lanemask_lt() | (1u << lane))) - 1u;
+                jobs += __popc(starts);
+                if (base + lane < total) {
+                    const uint2 j = sh_job[wp][q];
+                    const float4 a0 = sh_w0[wp][j.y & 31u], a1 = sh_w1[wp][j.y & 31u];
+                    const float4* __restrict__ tris = ONE ? a.one.wtris : sh_tris[wp][q];
+                    const uint32_t tt = j.x + (base + lane);
+                    const float4 v0 = __ldg(tris + 3ull * tt), v1 = __ldg(tris + 3ull * tt + 1),
+                                 v2 = __ldg(tris + 3ull * tt + 2);
+                    const RayWT r{a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, (int)((j.y >> 8) & 3u), a1.z, a1.w};
+                    float th;
+                    if (wt_hit(r, v0, v1, v2, th)) {
+                        atomicMin(&sh_hit[wp][j.y >> 16],
+                                  any ? (unsigned long long)tt : hit_key(th, __float_as_uint(v0.w)));
+                    }
+                }
+            }
+            __syncwarp();
+            if (mine) {
+                ttests += cnt;
+                if (ONE) ++ncand;
+                const unsigned long long b = sh_hit[wp][lane];
+                if (any && b != RSH_HIT_NONE) {
+                    // the tests up to the first hit count, as in the other instance
+                    ttests -= (top & 0x7FFFFFu) + cnt - 1u - (uint32_t)b;
+                    best = 0ull;
+                    sp = 0;
+                    finish();
+                } else {
+                    if (!any && b < best) {
+                        best = b;
+                        tcur = fminf(tcur, __uint_as_float((uint32_t)(b >> 32)));
+                    }
+                    pop();
+                }
+            }
+        } else if (has && ((top >> 31) != 0u) == do_nodes) {
             const uint32_t e = top;
-            if (!(e >> 31)) {
+            if (!SHARE && !(e >> 31)) {
                 // a cluster: its triangles t0 .. t0 + count - 1 (its box was tested with the parent's
                 // children; a closest-hit ray re-checks only its entry distance, above)
                 const float4* __restrict__ tris = ONE ? a.one.wtris : tris_v;
