@@ -574,11 +574,11 @@ __global__ void __launch_bounds__(FW * 32, RSH_FUSED_MIN_BLOCKS) k_fused(FusedAr
 // record index, or a cluster's first triangle | (triangles - 1) << 23. A node step reads the
 // record's near planes and far planes for the ray's octant (12 float4 loads, no per-axis min / max) and
 // the entries of the children it pushes. The warp keeps no per-unit state: it takes work units
-// (RSH_RAYS_UNIT sorted rays, never straddling a segment) by atomic ticket, and every lane whose ray has
-// finished takes the next ray of the warp's current unit straight from global memory (its id from the
-// sorted order, the ray itself from the segment's array), fetching the next unit when the current one runs
-// out. So lanes are refilled continuously and no lane waits for the slowest ray of a unit; a lane writes its
-// ray's result (shadow flag or hit record) itself when the ray ends. The stack's top entry lives in a register:
+// (RSH_RAYS_UNIT sorted rays, never straddling a segment) by atomic ticket, and the lanes whose rays have
+// finished take the next rays of the warp's current unit straight from global memory (the id from the
+// sorted order, the ray itself from the segment's array), RSH_REFILL of them at a time, fetching the next unit
+// when the current one runs out. So no lane waits for the slowest ray of a unit; a lane writes its
+// ray's result (shadow flag or hit record) itself. The stack's top entry lives in a register:
 // most node steps hit one child, which is then the next step without a store to and a load from local memory
 // in between (frames 2.8-3.9% faster: the architecture frame 3.79 ms against 3.90, the soup frame 3.34 against
 // 3.47; loading a plane of eight children with one 32-byte load instead of two 16-byte ones took 4.17 ms at this
@@ -649,6 +649,12 @@ RSH_DEV void slab4(float4 px, float4 py, float4 pz, float ix, float iy, float iz
 
 #ifndef RSH_RAYS_MIN_BLOCKS
 #define RSH_RAYS_MIN_BLOCKS 8  // of the SHARE instance, whose triangle tests' operands are in shared memory
+#endif
+// Idle lanes at which a warp takes new rays. Setting a ray up costs as much as one or two steps, whether for one lane
+// or for all: at every ray's end (1) 64 batches took 4.80 ms, 1 M rays 684 us, the architecture frame 2.88 ms and the
+// soup frame 2.26; at 8 4.25, 644, 2.77 and 2.09; at 16 4.06, 637, 2.76 and 2.06; at 20 4.13, 658, 2.81 and 2.10.
+#ifndef RSH_REFILL
+#define RSH_REFILL 16
 #endif
 #ifndef RSH_SHARE_BUSY
 #define RSH_SHARE_BUSY 16  // busy lanes at or below which a drained warp shares its rays (SHARE)
@@ -726,16 +732,10 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
     uint32_t kz = 0u;   // SHARE
     unsigned long long best = RSH_HIT_NONE;
     bool sharing = false;  // warp-uniform (SHARE): the warp shares its last rays
-    bool done = false;     // sharing: the lane's subtree is done, its result not yet merged
+    bool done = false;     // the lane's ray (sharing: subtree) is done, its result not yet written (merged)
     uint32_t own = lane;   // sharing: the lane whose ray this lane works on
     auto seg_of = [&](uint32_t i) -> const FusedSeg& { return ONE ? a.one : a.segs[i]; };
-    // the ray is done: its result, written by its own lane (while sharing: merged at the loop's top)
-    auto finish = [&]() {
-        has = false;
-        if (SHARE && sharing) {
-            done = true;
-            return;
-        }
+    auto write = [&]() {  // by the ray's own lane
         const FusedSeg& sg = seg_of(seg);
         if (any) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
         else sg.hits[slot] = best;
@@ -746,6 +746,14 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
             if (ONE && a.cand_pairs) atomicAdd(a.cand_pairs, (unsigned long long)ncand);
             ntests = ttests = ncand = 0;
         }
+    };
+    // the ray (sharing: the lane's subtree) is done. With segments its result is written at the loop's top, by all
+    // lanes that have one: a store with its segment's look-up by the one or two lanes that end in a step costs every
+    // step its instructions (64 batches 3.89 ms instead of 4.07; single batches and frames are 1% faster writing at once)
+    auto finish = [&]() {
+        has = false;
+        if (ONE && !(SHARE && sharing)) write();
+        else done = true;
     };
     // the next entry of the lane's stack into `top`; closest hit: entries that the ray enters beyond its
     // current best are dropped unread (their subtrees cannot hold a nearer hit: a child's box lies inside its
@@ -772,7 +780,11 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
         // idle lanes take the next rays of the warp's unit, units are fetched as they run out
         for (;;) {
             const uint32_t need = __ballot_sync(0xffffffffu, !has);
-            if (!need) break;
+            if (__popc(need) < RSH_REFILL && (ONE || !drained || sharing)) break;
+            if (!ONE && done && !(SHARE && sharing)) {
+                write();
+                done = false;
+            }
             if (nk >= nend) {
                 if (drained) break;
                 uint32_t t = 0;
@@ -865,7 +877,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
             }
             nk = min(nend, nk + __popc(need));
         }
-        if (!__any_sync(0xffffffffu, has || (SHARE && done))) break;  // nothing in flight, nothing to fetch
+        if (!__any_sync(0xffffffffu, has || ((SHARE || !ONE) && done))) break;  // nothing in flight, nothing to fetch
         // SHARE: once no ray is left to take and at most RSH_SHARE_BUSY lanes still trace one, idle lanes take
         // stack entries (subtrees) of the warp's rays in flight, so that a long ray near the launch's end
         // runs on many lanes instead of one. A ray's lane (its owner) keeps its result; a helper merges its
@@ -896,9 +908,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
                 // the owner, with no helper left: the ray's merged result
                 if (any) best = (best == 0ull || sh_occ[wp][lane]) ? 0ull : best;
                 else best = min(best, sh_best[wp][lane]);
-                const FusedSeg& sg = seg_of(seg);
-                if (any) sg.flags[slot] = best == 0ull ? RSH_OCCLUDED : 0u;
-                else sg.hits[slot] = best;
+                write();
                 done = false;
             } else if (done && own != lane) {
                 // a helper's subtree is done: its result into the owner's record
@@ -957,7 +967,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
             const bool node = has && (top >> 31) != 0u;
             const uint32_t nn = __popc(__ballot_sync(0xffffffffu, node));
             const uint32_t nc = __popc(__ballot_sync(0xffffffffu, has && !node));
-            do_nodes = nn >= nc;
+                        do_nodes = nn >= nc;
         }
         if (SHARE && !do_nodes) {
             // The triangles of all the clusters at hand, spread over the lanes: one after the other per lane, the step
