@@ -799,12 +799,12 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
                 if (drained) break;
                 uint32_t t = 0;
                 // A warp's first ticket is its own number: 4,000 warps that start at once queue for 7 us at one counter
-                // (a Cornell frame 133 -> 131 us, 20,001 rays 36 -> 35). Not for a pair of launches, whose warps
-                // start as others end.
-                if (a.pair == 0u && nk == ~0u) {
+                // (a Cornell frame 133 -> 131 us, 20,001 rays 36 -> 35). Not for the second of a pair of launches,
+                // whose warps start as the first one's end.
+                if (a.pair != 2u && nk == ~0u) {
                     t = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
                 } else {
-                    if (lane == 0) t = atomicAdd(&a.work[0], 1u) + (a.pair ? 0u : gridDim.x * FW);
+                    if (lane == 0) t = atomicAdd(&a.work[0], 1u) + (a.pair == 2u ? 0u : gridDim.x * FW);
                     t = __shfl_sync(0xffffffffu, t, 0);
                 }
                 if (t >= tickets) {
