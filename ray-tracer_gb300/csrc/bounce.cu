@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(BT) k_bounce(const __grid_constant__ BounceArg
     // ---- the next surface
     resolve_hit(a.pos, a.nrm, a.mat, ro, rd, h, sp, sn);
     const bool surface = sp.w != 0.0f;
-    if (in_range) {
+    if (in_range && a.spos) {
         a.spos[pix] = sp;
         a.snrm[pix] = sn;
     }

@@ -316,7 +316,7 @@ struct BounceArgs {
     const rsh_ray* rays;              // the traced rays whose hits are the next surface: the primary rays (tile
     const unsigned long long* hits;   // order: tiles_x x tiles_y tiles) or reflection rays by pixel (tiles_x 0)
     uint32_t tiles_x, tiles_y;
-    float4 *spos, *snrm;              // that surface (written)
+    float4 *spos, *snrm;              // that surface (written; null: not)
     // its rays (ray generation)
     LightsP lights;
     float eps, jitter;

@@ -205,34 +205,62 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
             lists.push_back(SegList{nullptr, nullptr});
         } else {
             const uint32_t b = q->stage - 1;
-            RayOut so, ro;
-            if (alone) {
-                so.ids = ids;
-                so.count = counts + segs.size();
-                so.flags = q->flags + (size_t)b * npix * L;
-                ro.ids = ids + (size_t)npix * L;
-                ro.count = counts + segs.size() + 1;
-                ro.hits = q->hits + (size_t)b * npix;
-                ids += (size_t)npix * (L + 1u);
-            }
-            HashP hp_r;
-            RSH_TRY(make_hash_params(sc, s->ctx->cfg, 0, hp_r));
             LightsP lp{};
             lp.count = L;
             lp.samples = 1;
             for (uint32_t l = 0; l < L; ++l)
                 for (int i = 0; i < 3; ++i) lp.pos[l][i] = r.lights[l].position[i];
-            RSH_CUDA(launch_raygen_shadow(q->spos, q->snrm, W, H, lp, s->ctx->cfg.epsilon, hp_r, q->srays, nullptr,
-                                          st, so));
             const rsh_ray* prev = (b == 0) ? nullptr : q->rrays[(b - 1) & 1];
             rsh_ray* cur = q->rrays[b & 1];
-            RSH_CUDA(launch_raygen_reflect(q->spos, q->snrm, prev, r.camera.eye, W, H, s->ctx->cfg.epsilon,
-                                           s->ctx->cfg.reflect_jitter, s->ctx->cfg.seed, b, hp_r, cur, nullptr, st, ro));
+            uint32_t* flags = q->flags + (size_t)b * npix * L;
+            unsigned long long* hits = q->hits + (size_t)b * npix;
+            SegList shadow{nullptr, nullptr}, reflect{nullptr, nullptr};
+            if (alone) {
+                // one kernel from the stage before's hits to this stage's rays and lists, like a frame's (three of
+                // them a stage, with the surface written and read back in between: 1.5 ms of a burst of 16
+                // requests, now 0.9)
+                shadow = SegList{ids, counts + segs.size()};
+                reflect = SegList{ids + (size_t)npix * L, counts + segs.size() + 1};
+                ids += (size_t)npix * (L + 1u);
+                BounceArgs ba{};
+                ba.w = W;
+                ba.h = H;
+                ba.pos = sc->pos;
+                ba.nrm = sc->nrm;
+                ba.mat = sc->mat;
+                ba.rays = b == 0 ? q->prim_rays : prev;
+                ba.hits = b == 0 ? q->prim_hits : hits - npix;
+                ba.tiles_x = b == 0 ? (W + 7) / 8 : 0u;
+                ba.tiles_y = b == 0 ? (H + 7) / 8 : 0u;
+                ba.lights = lp;
+                ba.eps = s->ctx->cfg.epsilon;
+                ba.jitter = s->ctx->cfg.reflect_jitter;
+                ba.seed = s->ctx->cfg.seed;
+                ba.bounce = b;
+                for (int i = 0; i < 3; ++i) ba.eye[i] = r.camera.eye[i];
+                ba.srays = q->srays;
+                ba.rrays = cur;
+                ba.sflags = flags;
+                ba.sids = const_cast<uint32_t*>(shadow.ids);
+                ba.scount = const_cast<uint32_t*>(shadow.count);
+                ba.rids = const_cast<uint32_t*>(reflect.ids);
+                ba.rcount = const_cast<uint32_t*>(reflect.count);
+                ba.rhits = hits;
+                RSH_CUDA(launch_bounce(ba, false, true, false, st));
+            } else {
+                HashP hp_r;
+                RSH_TRY(make_hash_params(sc, s->ctx->cfg, 0, hp_r));
+                RSH_CUDA(launch_raygen_shadow(q->spos, q->snrm, W, H, lp, s->ctx->cfg.epsilon, hp_r, q->srays, nullptr,
+                                              st, RayOut{}));
+                RSH_CUDA(launch_raygen_reflect(q->spos, q->snrm, prev, r.camera.eye, W, H, s->ctx->cfg.epsilon,
+                                               s->ctx->cfg.reflect_jitter, s->ctx->cfg.seed, b, hp_r, cur, nullptr, st,
+                                               RayOut{}));
+            }
             segs.push_back(rsh_batch_segment{sc, q->srays, npix * L, 1, nullptr, q->flags + (size_t)b * npix * L});
             segs.push_back(rsh_batch_segment{sc, cur, npix, 0,
                                              reinterpret_cast<uint64_t*>(q->hits + (size_t)b * npix), nullptr});
-            lists.push_back(SegList{so.ids, so.count});
-            lists.push_back(SegList{ro.ids, ro.count});
+            lists.push_back(shadow);
+            lists.push_back(reflect);
         }
     }
     if (alone) RSH_TRY(batch_trace_listed(s->ctx, segs.data(), lists.data(), (uint32_t)segs.size(), st));
@@ -246,8 +274,9 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
     // rays traced per segment (after trimming): read when the step retires
     RSH_CUDA(cudaMemcpyAsync(rec.pinned, alone ? counts : s->ctx->bufs["b_seg_cnt"].ptr, 4 * segs.size(),
                              cudaMemcpyDeviceToHost, st));
-    // advance: resolve hits into the next surface
+    // advance: resolve hits into the next surface (rays alone: with the next stage's rays)
     for (Req* q : rec.act) {
+        if (alone) break;
         const rsh_request& r = q->r;
         const rsh_scene* sc = s->scenes[r.scene_index];
         const uint32_t W = r.width, H = r.height, npix = W * H;
