@@ -173,6 +173,13 @@ RSH_DEV unsigned long long look_back2(unsigned long long* status, uint32_t tile,
     return dead ? LB_FAILED : excl;
 }
 
+// First in every kernel that launch_chained launches: the next one's CTAs may be placed from here on, and what the one
+// before wrote may be read (all its CTAs are done; a kernel that skipped the wait could be done before it).
+RSH_DEV void chain() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // device count helper: n = *d_count when given (clamped to n_max), else n_max
 RSH_DEV uint32_t dev_count(const uint32_t* d_count, uint32_t n_max) {
     if (!d_count) return n_max;

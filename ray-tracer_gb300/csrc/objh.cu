@@ -43,6 +43,7 @@ constexpr float kRadSlack = 1.0f + 1.0f / 1048576.0f;
 }
 
 __global__ void k_morton(const float4* __restrict__ pos, uint32_t n, v3 lo, v3 sc, uint32_t* codes) {
+    chain();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 a = __ldg(pos + 3ull * i), b = __ldg(pos + 3ull * i + 1), c = __ldg(pos + 3ull * i + 2);
@@ -57,6 +58,7 @@ __global__ void k_morton(const float4* __restrict__ pos, uint32_t n, v3 lo, v3 s
 
 __global__ void k_gather_tris(const float4* __restrict__ pos, const uint32_t* __restrict__ perm,
                               uint32_t n, float4* __restrict__ tris, uint32_t* __restrict__ order) {
+    chain();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t t = __ldg(perm + k);
@@ -70,6 +72,7 @@ __global__ void k_gather_tris(const float4* __restrict__ pos, const uint32_t* __
 
 // boundary strength before sorted triangle k (k = 0 and k = T: 64, stronger than any)
 __global__ void k_delta_tri(const uint32_t* __restrict__ scode, uint32_t T, uint32_t* __restrict__ dtri) {
+    chain();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > T) return;
     uint32_t d = 64u;
@@ -223,6 +226,7 @@ RSH_DEV bool level_items(const LevelArrays& A, uint32_t l, uint32_t& items, uint
 __global__ void __launch_bounds__(LV_TILE)
 k_level_cuts(LevelArrays A, uint32_t l, uint32_t* __restrict__ firsts, unsigned long long* __restrict__ status,
              uint32_t* __restrict__ ticket) {
+    chain();
     __shared__ uint32_t s_tile, s_warp[LV_TILE / 32], s_delta[LV_TILE + 2 * MAX_G];
     __shared__ unsigned long long s_excl;
     uint32_t items, off;
@@ -266,6 +270,7 @@ k_level_cuts(LevelArrays A, uint32_t l, uint32_t* __restrict__ firsts, unsigned 
 // Node g of the new level: children [firsts[g], firsts[g+1]) of the items, triangles
 // [start(firsts[g]), start(firsts[g+1])).
 __global__ void __launch_bounds__(128) k_level_nodes(LevelArrays A, uint32_t l, const uint32_t* __restrict__ firsts) {
+    chain();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t items, off;
     const uint32_t* start;
@@ -285,6 +290,7 @@ __global__ void __launch_bounds__(128) k_level_nodes(LevelArrays A, uint32_t l, 
 
 // Every level from l0 on (over at most TAIL_ITEMS items) in one block: cuts, a block scan, nodes.
 __global__ void __launch_bounds__(TAIL_THREADS) k_level_tail(LevelArrays A, uint32_t l0, uint32_t* firsts) {
+    chain();
     __shared__ uint32_t s_warp[32], s_total, s_delta[TAIL_ITEMS + 2 * MAX_G];
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     constexpr uint32_t PER = TAIL_ITEMS / TAIL_THREADS;
@@ -350,6 +356,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_level_tail(LevelArrays A, uint
 // level). Where all 32 triangles lie in one node their largest distance from its centre is one atomic max (of a
 // non-negative float's bits), else every lane's own.
 __global__ void __launch_bounds__(256) k_level_radii(LevelArrays A) {
+    chain();
     const uint32_t lane = lane_id(), t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u, t = t0 + lane;
     if (t0 >= A.n) return;
     const uint32_t t1 = min(t0 + 31u, A.n - 1u);
@@ -393,6 +400,7 @@ __global__ void __launch_bounds__(256) k_level_radii(LevelArrays A) {
 }
 
 __global__ void k_level_radii_end(const Level* __restrict__ lv, float4* __restrict__ sph) {
+    chain();
     uint32_t total = 0;
     for (uint32_t l = 0; l < 16; ++l) total += lv[l].size;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x)
@@ -481,12 +489,13 @@ cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t n, uint
     if (hi[1] - lo[1] > ext) ext = hi[1] - lo[1];
     if (hi[2] - lo[2] > ext) ext = hi[2] - lo[2];
     const float sc1 = (ext > 0.0f) ? 1024.0f / ext : 0.0f;
-    k_morton<<<(n + 255) / 256, 256, 0, s>>>(positions_dev, n, v3{lo[0], lo[1], lo[2]}, v3{sc1, sc1, sc1}, w.codes);
+    launch_chained(true, k_morton, (n + 255) / 256, 256, 0, s, positions_dev, n, v3{lo[0], lo[1], lo[2]},
+                   v3{sc1, sc1, sc1}, w.codes);
     note_launch();
     e = launch_sort_pairs(w.codes, nullptr, w.sorted_codes, w.perm, n, nullptr, 30, w.sort, err, s);
     if (e != cudaSuccess) return e;
-    k_gather_tris<<<(n + 255) / 256, 256, 0, s>>>(positions_dev, w.perm, n, h.tris, h.order);
-    k_delta_tri<<<(n + 256) / 256, 256, 0, s>>>(w.sorted_codes, n, w.dtri);
+    launch_chained(true, k_gather_tris, (n + 255) / 256, 256, 0, s, positions_dev, w.perm, n, h.tris, h.order);
+    launch_chained(true, k_delta_tri, (n + 256) / 256, 256, 0, s, w.sorted_codes, n, w.dtri);
     note_launch(2);
     // cluster boxes are widened by 1e-5 of the scene's largest coordinate magnitude: far more than the
     // rounding of a float slab test over the scene, so the box cull never drops a hit of the watertight test
@@ -501,15 +510,16 @@ cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t n, uint
     for (; l < 16 && most > TAIL_ITEMS; ++l) {
         const uint32_t G = (l == 0) ? cluster : 8u;
         const uint64_t nodes = std::max<uint64_t>(l == 0 ? (most + 1) / 2 : (most + 3) / 4, (most + G - 1) / G);
-        k_level_cuts<<<(uint32_t)((most + LV_TILE - 1) / LV_TILE), LV_TILE, 0, s>>>(A, l, w.firsts, w.status,
-                                                                                   w.tickets + l);
-        k_level_nodes<<<(uint32_t)((nodes + 128) / 128), 128, 0, s>>>(A, l, w.firsts);
+        launch_chained(true, k_level_cuts, (uint32_t)((most + LV_TILE - 1) / LV_TILE), LV_TILE, 0, s, A, l, w.firsts,
+                       w.status, w.tickets + l);
+        launch_chained(true, k_level_nodes, (uint32_t)((nodes + 128) / 128), 128, 0, s, A, l, w.firsts);
         note_launch(2);
         most = nodes;
     }
-    k_level_tail<<<1, TAIL_THREADS, 0, s>>>(A, l, w.firsts);
-    k_level_radii<<<(n + 255) / 256, 256, 0, s>>>(A);
-    k_level_radii_end<<<(uint32_t)std::min<size_t>((node_capacity(n) + 255) / 256, 1216), 256, 0, s>>>(w.lv, h.spheres);
+    launch_chained(true, k_level_tail, 1, TAIL_THREADS, 0, s, A, l, w.firsts);
+    launch_chained(true, k_level_radii, (n + 255) / 256, 256, 0, s, A);
+    launch_chained(true, k_level_radii_end, (uint32_t)std::min<size_t>((node_capacity(n) + 255) / 256, 1216), 256, 0, s,
+                   w.lv, h.spheres);
     note_launch(3);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // the single-ray box tree over the same Morton-ordered triangles, with the same padding

@@ -32,6 +32,7 @@ __global__ void k_transform(const float4* __restrict__ pos_rest, const float4* _
                             const uint32_t* __restrict__ obj, uint32_t n_vertices, uint32_t n_objects,
                             const float* __restrict__ model, const float* __restrict__ normal,
                             float4* __restrict__ pos, float4* __restrict__ nrm) {
+    chain();
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n_vertices) return;
     uint32_t id = __ldg(obj + x / 3);
@@ -47,6 +48,7 @@ __global__ void k_transform(const float4* __restrict__ pos_rest, const float4* _
 
 // Exact min / max of the vertex coordinates: per-block partials, then one block over them.
 __global__ void k_bounds_partial(const float4* __restrict__ pos, uint32_t n_vertices, float* __restrict__ part) {
+    chain();
     __shared__ float s[6][256];
     const float inf = __int_as_float(0x7f800000);
     float mn[3] = {inf, inf, inf}, mx[3] = {-inf, -inf, -inf};
@@ -74,6 +76,7 @@ __global__ void k_bounds_partial(const float4* __restrict__ pos, uint32_t n_vert
 // One warp per bound folds the blocks' partials (a thread each, one after the other, took 23 us for 608 blocks).
 __global__ void __launch_bounds__(192) k_bounds_final(const float* __restrict__ part, uint32_t blocks,
                                                       float* __restrict__ out) {
+    chain();
     const uint32_t a = threadIdx.x >> 5;
     const bool is_min = a < 3;
     float v = is_min ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000);
@@ -94,7 +97,8 @@ cudaError_t launch_transform(const float4* pos_rest, const float4* nrm_rest, con
                              cudaStream_t s) {
     const uint32_t nv = 3 * tri_count;
     if (nv == 0) return cudaSuccess;
-    k_transform<<<(nv + 255) / 256, 256, 0, s>>>(pos_rest, nrm_rest, obj, nv, n_objects, model, normal, pos, nrm);
+    launch_chained(true, k_transform, (nv + 255) / 256, 256, 0, s, pos_rest, nrm_rest, obj, nv, n_objects, model, normal,
+                   pos, nrm);
     note_launch();
     return cudaGetLastError();
 }
@@ -105,9 +109,9 @@ cudaError_t launch_bounds(const float4* pos, uint32_t tri_count, void* scratch, 
     const uint32_t nv = 3 * tri_count;
     const uint32_t blocks = std::min<uint32_t>(608u, (nv + 255) / 256 > 0 ? (nv + 255) / 256 : 1u);
     float* part = static_cast<float*>(scratch);
-    k_bounds_partial<<<blocks, 256, 0, s>>>(pos, nv, part);
+    launch_chained(true, k_bounds_partial, blocks, 256, 0, s, pos, nv, part);
     note_launch();
-    k_bounds_final<<<1, 192, 0, s>>>(part, blocks, out6);
+    launch_chained(true, k_bounds_final, 1, 192, 0, s, part, blocks, out6);
     note_launch();
     return cudaGetLastError();
 }
