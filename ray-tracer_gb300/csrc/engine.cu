@@ -326,6 +326,11 @@ rsh_status rsh_create(const rsh_config* cfg, rsh_ctx** out) {
     cudaMemset(ctx->d_err, 0, 256);
     cudaMemset(ctx->d_stats, 0, 256);
     for (auto& ev : ctx->ev) cudaEventCreate(&ev);
+    if ((e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking)) != cudaSuccess) {
+        rsh_status st = cuda_status(e, "rsh_create");
+        rsh_destroy(ctx);
+        return st;
+    }
     *out = ctx;
     return RSH_OK;
 }
@@ -335,6 +340,7 @@ rsh_status rsh_destroy(rsh_ctx* ctx) {
     cudaDeviceSynchronize();
     batch_release_ctx(ctx);
     for (const cudaEvent_t ev : ctx->tev) cudaEventDestroy(ev);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     for (auto& kv : ctx->bufs) release_buf(ctx, kv.second);
     for (auto& b : ctx->bounce) {
         release_buf(ctx, b.shadow_rays);
@@ -608,7 +614,7 @@ rsh_status rsh_scene_upload(rsh_ctx* ctx, const rsh_scene_desc* d, rsh_scene** o
         rsh_scene_destroy(ctx, sc);
         return cuda_status(e, "rsh_scene_upload scratch");
     }
-    e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, lo, hi, sc->h, scr, ctx->d_err, s);
+    e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, lo, hi, sc->h, scr, ctx->d_err, s, ctx->side);
     cudaFree(scr);
     if (e != cudaSuccess) {
         rsh_scene_destroy(ctx, sc);
@@ -673,7 +679,7 @@ rsh_status rsh_build_object_hierarchy(rsh_ctx* ctx, rsh_scene* sc, rsh_stream_t 
     if (!scr) RSH_CUDA(cudaMalloc(&scr, objh_scratch_bytes(T)));
     if (keep) sc->build_scratch = scr;
     const cudaError_t e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, sc->lo, sc->hi, sc->h, scr,
-                                                 ctx->d_err, s);
+                                                 ctx->d_err, s, ctx->side);
     if (!keep) cudaFree(scr);
     if (e != cudaSuccess) return cuda_status(e, "rsh_build_object_hierarchy");
     return RSH_OK;

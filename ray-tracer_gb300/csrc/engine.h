@@ -79,6 +79,7 @@ struct rsh_ctx {
     rsh_frame_stats stats{};
     rsh_frame_stats batch_stats{};
     cudaEvent_t ev[16] = {};
+    cudaStream_t side = nullptr;             // the object-sphere levels' build, beside the box tree's
     cudaStream_t last_stream = nullptr;
     std::vector<uint32_t> batch_counts_host;
     uint32_t overflow_passes = 0;
