@@ -659,8 +659,10 @@ RSH_DEV void slab4(float4 px, float4 py, float4 pz, float ix, float iy, float iz
 #ifndef RSH_SHARE_BUSY
 #define RSH_SHARE_BUSY 16  // busy lanes at or below which a drained warp shares its rays (SHARE)
 #endif
+// units per warp that go out in pieces: a single batch's last 8 (16: the architecture frame 0.3% slower, 4: 1.2%); of
+// many segments, whose units cost a warp a search each, the last 2 (64 batches 3.79 ms, with 4 3.80, 16 3.86)
 #ifndef RSH_TAIL_PER_WARP
-#define RSH_TAIL_PER_WARP 16
+#define RSH_TAIL_PER_WARP (ONE ? 8 : 2)
 #endif
 
 // log2 of the pieces that a launch's last units are cut into, for `units` of RSH_RAYS_UNIT rays over `warps` warps:
@@ -706,7 +708,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
     }
     const uint32_t units = ONE ? (dev_count(a.one.count, a.one.n) + U - 1u) / U : dev_count(a.d_units, a.units_max);
     // the last units go out in pieces of U >> split rays
-    const uint32_t tail = min(units, (uint32_t)RSH_TAIL_PER_WARP * gridDim.x * FW), 
+    const uint32_t tail = min(units, (uint32_t)RSH_TAIL_PER_WARP * gridDim.x * FW),
                    split = tail_split(units, a.warps, a.pixel_order);
     const uint32_t head = units - tail, tickets = head + (tail << split);
     uint32_t ntests = 0, ttests = 0;  // the lane's counts, flushed to the launch's counters before 2^31
