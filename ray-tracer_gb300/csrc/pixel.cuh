@@ -165,11 +165,17 @@ RSH_DEV void shade_surface(const ShadeArgs& a, const rsh_light* s_light, const u
     const rsh_material m = a.materials[mid];
     float cr = 0.f, cg = 0.f, cb = 0.f;
     const uint32_t S = a.samples ? a.samples : 1u;
+    // one sample a light: the flags of all lights (at most 8) before any of them is used, so that their loads overlap
+    uint32_t occluded = 0;
+    if (S == 1 && shadow) {
+        const uint32_t* f = shadow + (x + (size_t)a.w * a.lights * y);
+#pragma unroll 4
+        for (uint32_t l = 0; l < a.lights; ++l) occluded |= (__ldg(f + a.w * l) == RSH_OCCLUDED ? 1u : 0u) << l;
+    }
     for (uint32_t l = 0; l < a.lights; ++l) {
         float factor = 1.0f;
         if (S == 1) {
-            const uint32_t slot = x + a.w * (l + a.lights * y);
-            if (shadow && shadow[slot] == RSH_OCCLUDED) continue;
+            if ((occluded >> l) & 1u) continue;
         } else if (shadow) {
             // soft shadows (RayTracer.cu:1680-1696): weighted unoccluded samples, log2(1 + 2 sum)
             float sf = 0.0f;
