@@ -699,6 +699,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
     __shared__ uint2 sh_job[SHARE ? FW : 1][32];
     __shared__ const float4* sh_tris[SHARE && !ONE ? FW : 1][32];
     __shared__ unsigned long long sh_hit[SHARE ? FW : 1][32];
+    __shared__ uint32_t sh_don[SHARE ? FW : 1][32];  // SHARE: the donors of a hand-out, by rank
     __shared__ uint32_t s_rays, s_ended;  // a.valid: the block's rays, its warps that have ended
     const uint32_t lane = lane_id();
     asm volatile("griddepcontrol.launch_dependents;");
@@ -938,7 +939,11 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
             if (idle && donors) {
                 const uint32_t r = __popc(idle & lanemask_lt());
                 const bool recv = !has && !done && r < (uint32_t)__popc(donors);
-                const uint32_t src = recv ? __fns(donors, 0u, (int)r + 1) : lane;
+                // the r-th donor, by its rank in shared memory (__fns is a loop: 20,001 rays 31.3 us with it, 29.6 without,
+                // 1000 rays 23.1 / 21.3, Cornell frame 125 / 124, architecture frame 2.70 / 2.69 ms)
+                if (has && sp >= 1) sh_don[wp][__popc(donors & lanemask_lt())] = lane;
+                __syncwarp();
+                const uint32_t src = recv ? sh_don[wp][r] : lane;
                 const bool give = has && sp >= 1 && (uint32_t)__popc(donors & lanemask_lt()) < (uint32_t)__popc(idle);
                 uint32_t ge = 0u;  // the donor's second entry; it goes on with its top
                 if (give) ge = any ? take_last() : stk[--sp];
