@@ -137,32 +137,28 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // exclusive digit offsets of every pass: one block-wide scan of the 256 bins per pass
-    for (uint32_t p = 0; p < passes; ++p) {
-        uint32_t* h = hist + 256u * p;
-        const uint32_t t = threadIdx.x;  // blockDim.x == 256
-        const uint32_t v = __ldcg(h + t);
-        uint32_t x = v;
+    // exclusive digit offsets: a block-wide scan of the 256 bins, of all passes at once
+    {
+        const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;  // blockDim.x == 256
+        uint32_t v[4], x[4];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((t & 31u) >= (uint32_t)o) x += y;
-        }
-        if ((t & 31u) == 31u) sh[0][t >> 5] = x;  // the shared counters are free now
-        __syncthreads();
-        if (t < 32) {
-            uint32_t ws = t < 8u ? sh[0][t] : 0u;
+        for (uint32_t p = 0; p < 4; ++p) v[p] = x[p] = p < passes ? __ldcg(hist + 256u * p + t) : 0u;
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, ws, o);
-                if (t >= (uint32_t)o) ws += y;
+        for (uint32_t p = 0; p < 4; ++p) {
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x[p], o);
+                if (lane >= (uint32_t)o) x[p] += y;
             }
-            if (t < 8u) sh[1][t] = ws;
+            if (lane == 31u) sh[p][warp] = x[p];  // the shared counters are free now
         }
         __syncthreads();
-        const uint32_t warp_off = (t >= 32u) ? sh[1][(t >> 5) - 1] : 0u;
-        h[t] = warp_off + x - v;
-        __syncthreads();
+#pragma unroll
+        for (uint32_t p = 0; p < 4; ++p) {
+            uint32_t before = 0;
+            for (uint32_t w = 0; w < warp; ++w) before += sh[p][w];
+            if (p < passes) hist[256u * p + t] = before + x[p] - v[p];
+        }
     }
 }
 
