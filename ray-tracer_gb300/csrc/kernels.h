@@ -66,13 +66,10 @@ struct CameraP {
 // ---- raygen + hash (raygen.cu)
 cudaError_t launch_raygen_primary(const CameraP& cam, uint32_t w, uint32_t h, rsh_ray* rays,
                                   uint32_t* pixel_of_ray, cudaStream_t s);
-// What ray generation writes for a traversal beside the rays, with the segment's results prefilled (flags 0 for
-// an any-hit segment, hits RSH_HIT_NONE otherwise) and its ray count added to *count (one atomic per block):
-//   ids   the slots that hold a ray, appended block by block: a trimmed list for rays traced alone, in the order
-//         of the pixels, with no key, compression or sort;
-//   keys  the keys of a batched call whose rays use packets: tag | (ray hash >> drop) or RSH_KEY_NONE.
+// What ray generation writes beside the rays for a batched call whose rays use packets: its keys (tag | (ray hash >>
+// drop) or RSH_KEY_NONE), with the segment's results prefilled (flags 0 for an any-hit segment, hits RSH_HIT_NONE
+// otherwise) and its ray count added to *count (one atomic per block).
 struct RayOut {
-    uint32_t* ids = nullptr;
     uint32_t* keys = nullptr;      // the batch's key array at the segment's first slot
     uint32_t tag = 0;
     uint32_t drop = 0;
@@ -96,9 +93,6 @@ cudaError_t launch_hash(const rsh_ray* rays, uint32_t n, const HashP& hp, uint32
                         uint32_t* keys, cudaStream_t s);
 // Segmented hash for the batched form: segment s covers rays [seg_start[s], seg_start[s+1]) of the
 // concatenated ray array; tag = segment index; hash params per segment (scene bounds).
-cudaError_t launch_hash_segments(const rsh_ray* rays, uint32_t n, const uint32_t* seg_start,
-                                 uint32_t nseg, const HashP* hps_dev, uint32_t tag_shift,
-                                 uint32_t* keys, cudaStream_t s);
 
 // ---- trim + compress (compress.cu)
 size_t compress_scratch_bytes(uint32_t n_slots);
@@ -342,8 +336,6 @@ size_t bounds_scratch_bytes();
 cudaError_t launch_bounds(const float4* pos, uint32_t tri_count, void* scratch, float* out6, cudaStream_t s);
 
 // ---- misc (util kernels in raygen.cu)
-cudaError_t launch_fill_u32(uint32_t* p, uint32_t v, size_t n, cudaStream_t s);
 cudaError_t launch_fill_u64(unsigned long long* p, unsigned long long v, size_t n, cudaStream_t s);
-cudaError_t launch_mark_hit_counts(const uint32_t* counts, unsigned long long* acc, cudaStream_t s);
 
 }  // namespace rsh

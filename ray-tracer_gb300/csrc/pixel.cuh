@@ -67,15 +67,6 @@ RSH_DEV bool shadow_ray(v3 p, v3 nn, v3 lp, float eps, uint32_t S, uint32_t sm, 
     return true;
 }
 
-// A block's share of a segment's ray count and, in list mode, of its id list: reserves `rays` entries with one
-// atomic and returns the first to every thread. Every thread of the block calls it.
-RSH_DEV uint32_t reserve_rays(uint32_t* count, uint32_t rays) {
-    __shared__ uint32_t s_base;
-    if (threadIdx.x == 0) s_base = rays ? atomicAdd(count, rays) : 0u;
-    __syncthreads();
-    return s_base;
-}
-
 // ------------------------------------------------------------------ reflection rays
 // Integer hash of (seed, slot, bounce) -> 32 random bits (PCG output permutation on an LCG step).
 RSH_DEV uint32_t rng_next(uint32_t& state) {

@@ -52,18 +52,20 @@ cudaError_t launch_raygen_primary(const CameraP& cam, uint32_t w, uint32_t h, rs
 // ------------------------------------------------------------------ shadow rays
 // One thread per pixel: the pixel's surface point and normal are read and the normal normalised once,
 // then its V = L x S slots are written (slot = x + W (v + V y), RayTracer.cu:700-702 with S samples per
-// light), each with the same arithmetic as a thread per slot would use. The block's rays are counted once and
-// listed warp by warp, a light's 32 pixels together (RayOut). The light positions are copied to shared memory
+// light), each with the same arithmetic as a thread per slot would use. The block's rays are counted once
+// (RayOut). The light positions are copied to shared memory
 // first: indexing the parameter bank with the light number is a constant load with a register index, which the
 // SM issues through its narrow address-divergence pipe, and three of those per slot made that pipe the kernel's
 // bound. 12 blocks per SM (at most 40 registers, no spills) keep enough warps in flight to cover the surface
 // reads.
 constexpr uint32_t RS_THREADS = 128;
+// BATCH: for a batched call (out), else keys of its own or none. One hash in the loop instead of two, and no tests for
+// the other form: 2.76 M slots 32.6 -> 28.2 us, bound by issue slots (exact divides and roots, the hash).
+template <bool BATCH>
 __global__ void __launch_bounds__(RS_THREADS, 12)
 k_raygen_shadow(const float4* __restrict__ spos, const float4* __restrict__ snrm, uint32_t w, uint32_t h,
                 LightsP lights, float eps, HashP hp, rsh_ray* rays, uint32_t* keys, RayOut out) {
     __shared__ float s_lp[8 * 3];
-    __shared__ uint32_t s_bal[RS_THREADS / 32][8 * 16];  // per warp and light sample: the lanes with a ray
     __shared__ uint32_t s_cnt[RS_THREADS / 32];
     const uint32_t L = lights.count, S = lights.samples ? lights.samples : 1u, V = L * S;
     const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x, lane = lane_id(), warp = threadIdx.x >> 5;
@@ -86,42 +88,33 @@ k_raygen_shadow(const float4* __restrict__ spos, const float4* __restrict__ snrm
         if (surface) {
             const v3 lp = mk3(s_lp[3u * l], s_lp[3u * l + 1u], s_lp[3u * l + 2u]);
             valid = shadow_ray(p, nn, lp, eps, S, sm, ro, rd);
-            if (valid && keys) key = ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, hp, v);
+            if (!BATCH && valid && keys) key = ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, hp, v);
         }
         if (in_range) {
             // an empty slot holds an explicit no-ray (tmax < tmin) for consumers without keys
             store_ray32(rays, slot, ro, rd, a32);
-            if (keys) keys[slot] = key;
-            if (out.count) {
-                if (out.keys)
-                    out.keys[slot] = valid ? out.tag | (ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, out.hp, 0u) >> out.drop)
-                                           : RSH_KEY_NONE;
+            if (!BATCH && keys) keys[slot] = key;
+            if (BATCH) {
+                out.keys[slot] = valid ? out.tag | (ray_hash(ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, out.hp, 0u) >> out.drop)
+                                       : RSH_KEY_NONE;
                 if (out.flags) out.flags[slot] = 0u;
                 else out.hits[slot] = RSH_HIT_NONE;
             }
         }
-        if (out.count) {
+        if (BATCH) {
             const uint32_t b = __ballot_sync(0xffffffffu, valid);
             nvalid += __popc(b);
-            if (out.ids && lane == 0) s_bal[warp][v] = b;
         }
     }
-    if (out.count) {
+    if (BATCH) {
         if (lane == 0) s_cnt[warp] = nvalid;
         __syncthreads();
-        uint32_t before = 0, all = 0;
+        if (threadIdx.x == 0) {
+            uint32_t all = 0;
 #pragma unroll
-        for (uint32_t q = 0; q < RS_THREADS / 32; ++q) {
-            if (q < warp) before += s_cnt[q];
-            all += s_cnt[q];
+            for (uint32_t q = 0; q < RS_THREADS / 32; ++q) all += s_cnt[q];
+            if (all) atomicAdd(out.count, all);
         }
-        uint32_t at = reserve_rays(out.count, all) + before;
-        if (out.ids)
-            for (uint32_t v = 0; v < V; ++v) {
-                const uint32_t b = s_bal[warp][v];
-                if ((b >> lane) & 1u) out.ids[at + __popc(b & lanemask_lt())] = x + w * (v + V * y);
-                at += __popc(b);
-            }
     }
 }
 
@@ -130,8 +123,8 @@ cudaError_t launch_raygen_shadow(const float4* spos, const float4* snrm, uint32_
                                  uint32_t* keys, cudaStream_t s, const RayOut& out) {
     const uint32_t n = w * h;
     if (n == 0 || lights.count == 0) return cudaSuccess;
-    k_raygen_shadow<<<(n + RS_THREADS - 1u) / RS_THREADS, RS_THREADS, 0, s>>>(spos, snrm, w, h, lights, eps, hp, rays,
-                                                                              keys, out);
+    const auto kernel = out.count ? k_raygen_shadow<true> : k_raygen_shadow<false>;
+    kernel<<<(n + RS_THREADS - 1u) / RS_THREADS, RS_THREADS, 0, s>>>(spos, snrm, w, h, lights, eps, hp, rays, keys, out);
     note_launch();
     return cudaGetLastError();
 }
@@ -179,14 +172,12 @@ __global__ void k_raygen_reflect(const float4* __restrict__ spos, const float4* 
         const uint32_t warp = threadIdx.x >> 5, b = __ballot_sync(0xffffffffu, valid);
         if (lane_id() == 0) s_cnt[warp] = __popc(b);
         __syncthreads();
-        uint32_t before = 0, all = 0;
+        if (threadIdx.x == 0) {
+            uint32_t all = 0;
 #pragma unroll
-        for (uint32_t q = 0; q < 8; ++q) {  // 256 threads
-            if (q < warp) before += s_cnt[q];
-            all += s_cnt[q];
+            for (uint32_t q = 0; q < 8; ++q) all += s_cnt[q];  // 256 threads
+            if (all) atomicAdd(out.count, all);
         }
-        const uint32_t at = reserve_rays(out.count, all) + before;
-        if (out.ids && valid) out.ids[at + __popc(b & lanemask_lt())] = slot;
     }
 }
 
@@ -271,56 +262,11 @@ cudaError_t launch_hash(const rsh_ray* rays, uint32_t n, const HashP& hp, uint32
     return cudaGetLastError();
 }
 
-// Segmented: binary search of the segment of ray i; the key's tag is the segment index placed at
-// bit tag_shift (above every segment's hash bits).
-__global__ void k_hash_segments(const rsh_ray* __restrict__ rays, uint32_t n,
-                                const uint32_t* __restrict__ seg_start, uint32_t nseg,
-                                const HashP* __restrict__ hps, uint32_t tag_shift, uint32_t* keys) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t lo = 0, hi = nseg;  // find last s with seg_start[s] <= i
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(seg_start + mid) <= i) lo = mid; else hi = mid;
-    }
-    float4 o, d;
-    load_ray(rays, i, o, d);
-    uint32_t key = RSH_KEY_NONE;
-    if (d.w > o.w) {
-        const HashP hp = hps[lo];
-        key = (lo << tag_shift) | ray_hash(o.x, o.y, o.z, d.x, d.y, d.z, hp, 0u);
-    }
-    keys[i] = key;
-}
-
-cudaError_t launch_hash_segments(const rsh_ray* rays, uint32_t n, const uint32_t* seg_start,
-                                 uint32_t nseg, const HashP* hps_dev, uint32_t tag_shift,
-                                 uint32_t* keys, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_hash_segments<<<(n + 255u) / 256u, 256, 0, s>>>(rays, n, seg_start, nseg, hps_dev, tag_shift,
-                                                    keys);
-    note_launch();
-    return cudaGetLastError();
-}
-
 // ------------------------------------------------------------------ fills
-__global__ void k_fill_u32(uint32_t* p, uint32_t v, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x)
-        p[i] = v;
-}
 __global__ void k_fill_u64(unsigned long long* p, unsigned long long v, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x)
         p[i] = v;
-}
-cudaError_t launch_fill_u32(uint32_t* p, uint32_t v, size_t n, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    size_t blocks = (n + 255) / 256;
-    if (blocks > 152 * 16) blocks = 152 * 16;
-    k_fill_u32<<<(unsigned)blocks, 256, 0, s>>>(p, v, n);
-    note_launch();
-    return cudaGetLastError();
 }
 cudaError_t launch_fill_u64(unsigned long long* p, unsigned long long v, size_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
