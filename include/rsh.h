@@ -165,13 +165,12 @@ typedef struct rsh_config {
  * compression or decompression), for incoherent batches whose keys hardly repeat; rsh_autotune_scenes tries
  * both. Rays alone from the root (the default switch level) are never cut into runs. */
 #define RSH_FLAG_NO_COMPRESS 16u
-/* Batched form: every ray is traced by one lane from its first step to its last. By default, once a warp
- * of the rays-only kernel has no ray left to take and at most 16 of its lanes still trace one, its idle
- * lanes take subtrees (stack entries) of those rays, which shortens launches that would end on a few long
- * rays (scenes with long sight lines); results are the same either way. The default costs the steps about
- * 4% (the kernel runs at its register limit) and changes the node and triangle test counts through the
- * order the hits are met in; with this flag the counts equal a sequential traversal's, ray by ray, and
- * scenes whose launches end evenly run faster. */
+/* Every ray is traced by one lane from its first step to its last. By default the rays-only kernel spreads the
+ * triangles of a warp's clusters over its lanes, and once a warp has no ray left to take and at most 16 of its
+ * lanes still trace one, its idle lanes take subtrees (stack entries) of those rays; results are the same either
+ * way. The default changes the node and triangle test counts through the order the hits are met in; with this flag
+ * the counts equal a sequential traversal's, ray by ray. Scenes of a few triangles run a little faster with it,
+ * others 4-15% slower. */
 #define RSH_FLAG_SEQUENTIAL_RAYS 32u
 #define RSH_FLAG_RAH 4u            /* plain path: ray-hierarchy ablation without hashing/sorting: packets
                                       of consecutive trimmed rays (the reference's algorithm 1 "RAH",
@@ -189,7 +188,8 @@ typedef struct rsh_frame_stats {
     uint64_t node_tests;         /* node tests executed (packet-node x sphere; a single ray x node box);
                                     rsh_render_frame: secondary rays only */
     uint64_t tri_tests;          /* ray x triangle tests executed (rsh_render_frame: secondary rays only) */
-    float secondary_ms;          /* first secondary raygen .. last secondary intersection */
+    float secondary_ms;          /* first secondary raygen .. last secondary intersection; rays alone: from the
+                                    kernel that resolves the primary hits to the packed image */
     float frame_ms;
     float stage_ms[12];          /* see RSH_STAGE_* */
     uint32_t overflow_passes;    /* traversal restarts after a full candidate buffer */
