@@ -250,7 +250,8 @@ struct BatchPlan {
 
 // Rays at or below this count are traced in their own order. Sorting incoherent rays makes their traversal 11-13%
 // shorter (their nodes are in the L1 more often), whatever their number; the hash and the sort cost 0.10 ms for
-// 1.3 M rays in 8 segments (traversal 0.526 against 0.587 ms), 0.6 ms for 13.8 M in 64 (4.95 against 5.77 ms).
+// 1.3 M rays in 8 segments (traversal 0.526 against 0.587 ms then), 0.5 ms for 13.8 M in 64 (all of it 3.86 ms
+// sorted, 4.19 unsorted).
 constexpr uint32_t SORT_RAYS = 2000000;
 
 // The context's configuration with a scene's own tuning (rsh_scene_set_tuning) applied.
