@@ -681,6 +681,7 @@ rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, u
                        uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair, bool count_tests) {
     FusedArgs fa = alone_args(ctx, ticket);
     fa.pair = pair;
+    fa.wait = pair != 2u ? 1u : 0u;  // behind the kernel that generated its rays
     fa.pixel_order = true;
     if (!count_tests) fa.node_tests = fa.tri_tests = nullptr;
     fa.one.wtris = sc->h.wtris;

@@ -703,6 +703,8 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
     __shared__ uint32_t sh_don[SHARE ? FW : 1][32];  // SHARE: the donors of a hand-out, by rank
     __shared__ uint32_t s_rays, s_ended;  // a.valid: the block's rays, its warps that have ended
     const uint32_t lane = lane_id();
+    // (a.wait: what the kernel before wrote is there; the second of a pair starts only then, too)
+    if (a.wait) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     if (a.valid) {
         if (threadIdx.x == 0) s_rays = s_ended = 0u;
@@ -1194,7 +1196,7 @@ static cudaError_t launch_fused_rays_s(FusedArgs a, cudaStream_t s) {
     // a piece a warp: with more warps some SMs' would take them all
     const uint64_t need = (((uint64_t)most << tail_split(most, a.warps, a.pixel_order)) + FW - 1) / FW;
     if (need < grid) grid = need > 0 ? (uint32_t)need : 1;
-    const cudaError_t e = launch_chained(a.pair == 2u, k_fused_rays<U, SHARE, OF>, grid, FW * 32, 0, s, a);
+    const cudaError_t e = launch_chained(a.pair == 2u || a.wait, k_fused_rays<U, SHARE, OF>, grid, FW * 32, 0, s, a);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }

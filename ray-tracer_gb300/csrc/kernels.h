@@ -267,6 +267,7 @@ struct FusedArgs {
     bool pixel_order;                  // rays of neighbouring pixels lie together
     uint32_t pair;                     // rays-only: 1, 2: the first / second of two launches that neither read
                                        // nor write what the other writes; the second may start while the first runs
+    uint32_t wait;                     // rays-only: the launch is chained behind a kernel whose results it reads
     FusedSeg one;                      // launch_rays_one: the one segment (slot_base 0)
     uint32_t* valid;                   // rays-only: the rays traced are added to valid[0] and valid[1] (null: not)
     unsigned long long* cand_pairs;    // launch_rays_one: counts (ray, cluster) pairs tested (null: not counted)

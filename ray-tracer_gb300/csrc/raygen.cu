@@ -16,6 +16,7 @@ namespace rsh {
 // ------------------------------------------------------------------ primary rays (tile order)
 __global__ void k_raygen_primary(CameraP cam, uint32_t w, uint32_t h, uint32_t tiles_x, uint32_t tiles_y, uint32_t n,
                                  rsh_ray* rays, uint32_t* pixel_of_ray) {
+    asm volatile("griddepcontrol.launch_dependents;");  // the traversal waits for the rays itself
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t tile = k >> 6, within = k & 63u;
