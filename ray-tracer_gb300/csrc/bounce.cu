@@ -32,6 +32,11 @@ __global__ void __launch_bounds__(BT, 10) k_bounce(const __grid_constant__ Bounc
     if (GEN && threadIdx.x < 3u * a.lights.count) s_lp[threadIdx.x] = (&a.lights.pos[0][0])[threadIdx.x];
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!GEN && blockIdx.x == 0)
+        for (int q = 0; q < 2; ++q) {
+            for (uint32_t i = threadIdx.x; i < a.counters.n[q]; i += BT) a.counters.to[q][i] = __ldcg(a.counters.p[q] + i);
+            __syncthreads();  // one after the other, like copies in a stream
+        }
     const uint32_t pix = blockIdx.x * BT + threadIdx.x, w = a.w;
     const bool in_range = pix < w * a.h;
     const uint32_t y = pix / w, x = pix - y * w;

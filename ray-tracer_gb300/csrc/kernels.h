@@ -64,8 +64,14 @@ struct CameraP {
 };
 
 // ---- raygen + hash (raygen.cu)
+// Two ranges of words: zeroed, or copied from the first to the second.
+struct Words2 {
+    uint32_t *p[2], *to[2];
+    uint32_t n[2];
+};
+// zero: words set to 0 beside it (a frame's counters: no memset of their own)
 cudaError_t launch_raygen_primary(const CameraP& cam, uint32_t w, uint32_t h, rsh_ray* rays,
-                                  uint32_t* pixel_of_ray, cudaStream_t s);
+                                  uint32_t* pixel_of_ray, cudaStream_t s, const Words2& zero = Words2());
 // What ray generation writes beside the rays for a batched call whose rays use packets: its keys (tag | (ray hash >>
 // drop) or RSH_KEY_NONE), with the segment's results prefilled (flags 0 for an any-hit segment, hits RSH_HIT_NONE
 // otherwise) and its ray count added to *count (one atomic per block).
@@ -324,6 +330,7 @@ struct BounceArgs {
     // shading of the surface before it (ShadeArgs: its surface, flags, bounce and incident rays), the image
     ShadeArgs sh;
     uint32_t* rgba;
+    Words2 counters;                  // without gen: words copied to (pinned host) memory, the frame's counters
 };
 // shade: shade sh's surface first; gen: write the next surface's rays and lists, their results prefilled;
 // final_image (without gen): shade the next surface too, unshadowed, and pack the image.

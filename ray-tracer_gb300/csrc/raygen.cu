@@ -15,8 +15,11 @@ namespace rsh {
 
 // ------------------------------------------------------------------ primary rays (tile order)
 __global__ void k_raygen_primary(CameraP cam, uint32_t w, uint32_t h, uint32_t tiles_x, uint32_t tiles_y, uint32_t n,
-                                 rsh_ray* rays, uint32_t* pixel_of_ray) {
+                                 rsh_ray* rays, uint32_t* pixel_of_ray, const Words2 zero) {
     asm volatile("griddepcontrol.launch_dependents;");  // the traversal waits for the rays itself
+    if (blockIdx.x == 0)
+        for (int q = 0; q < 2; ++q)
+            for (uint32_t i = threadIdx.x; i < zero.n[q]; i += blockDim.x) zero.p[q][i] = 0u;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t tile = k >> 6, within = k & 63u;
@@ -41,11 +44,11 @@ __global__ void k_raygen_primary(CameraP cam, uint32_t w, uint32_t h, uint32_t t
 }
 
 cudaError_t launch_raygen_primary(const CameraP& cam, uint32_t w, uint32_t h, rsh_ray* rays,
-                                  uint32_t* pixel_of_ray, cudaStream_t s) {
+                                  uint32_t* pixel_of_ray, cudaStream_t s, const Words2& zero) {
     const uint32_t tx = (w + 7u) / 8u, ty = (h + 7u) / 8u;
     const uint32_t n = tx * ty * 64u;
     if (n == 0) return cudaSuccess;
-    k_raygen_primary<<<(n + 255u) / 256u, 256, 0, s>>>(cam, w, h, tx, ty, n, rays, pixel_of_ray);
+    k_raygen_primary<<<(n + 255u) / 256u, 256, 0, s>>>(cam, w, h, tx, ty, n, rays, pixel_of_ray, zero);
     note_launch();
     return cudaGetLastError();
 }
