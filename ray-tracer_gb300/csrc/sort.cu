@@ -59,6 +59,11 @@ inline uint32_t sm_count() {
 inline uint32_t num_passes(uint32_t key_bits) { return key_bits == 0 ? 1u : (key_bits + 7u) / 8u; }
 }  // namespace
 
+__global__ void k_sort_zero(uint32_t* __restrict__ w) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    w[blockIdx.x * blockDim.x + threadIdx.x] = 0u;
+}
+
 // --- histograms of every pass in one read; also clears the look-back status rows of the tiles that
 // the passes will use (ceil(n / tile) rows of 256 words per pass, pass stride `stride` words)
 __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
@@ -70,6 +75,7 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n_max,
     asm volatile("griddepcontrol.launch_dependents;");
     for (uint32_t i = threadIdx.x; i < 4u * 256u; i += blockDim.x) (&sh[0][0])[i] = 0u;
     __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the zeroed counters (k_sort_zero)
     const uint32_t n = dev_count(d_count, n_max);
     {
         const uint32_t tile_keys = SW_T * tile_rows(n, ctas);
@@ -397,13 +403,19 @@ cudaError_t launch_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
     uint32_t* alt_keys = status + passes * tiles * 256;
     alt_keys = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(alt_keys) + 255) & ~uintptr_t(255));
     uint32_t* alt_vals = alt_keys + n_max;
-    cudaError_t e = cudaMemsetAsync(w, 0, (4 * 256 + 16) * sizeof(uint32_t), s);
+    // a kernel, not a memset: the next launch can be chained behind it (20,000 pairs 34.9 -> 33.5 us, 1 M 58.6 ->
+    // 56.9)
+    k_sort_zero<<<5, 208, 0, s>>>(w);
+    note_launch();
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     // four CTAs per SM count 16 M keys in half the time of two; fewer when there is not a run of 16 keys for each
     // thread
     const uint32_t hgrid = std::min<uint32_t>(sms * 4u, (n_max + 4095u) / 4096u);
-    k_sort_hist<<<hgrid, 256, 0, s>>>(keys_in, n_max, d_count, passes, ctas, hist, status, tiles * 256, tickets + 8);
+    e = launch_chained(true, k_sort_hist, hgrid, 256, 0, s, keys_in, n_max, d_count, passes, ctas, hist, status, tiles * 256,
+                       tickets + 8);
     note_launch();
+    if (e != cudaSuccess) return e;
     // ping-pong so that the last pass lands in the output
     const uint32_t* ki = keys_in;
     const uint32_t* vi = vals_in;
