@@ -174,10 +174,16 @@ RSH_DEV unsigned long long look_back2(unsigned long long* status, uint32_t tile,
 }
 
 // First in every kernel that launch_chained launches: the next one's CTAs may be placed from here on, and what the one
-// before wrote may be read (all its CTAs are done; a kernel that skipped the wait could be done before it).
+// before wrote may be read (all its CTAs are done; a kernel that skipped the wait could be done before it). What the
+// chain writes is read with plain or .cg loads: a read-only load (__ldg, or through a const __restrict__ pointer) is
+// taken to read memory that nothing writes while the kernel lives, and may be moved above the wait.
 RSH_DEV void chain() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class T>
+RSH_DEV T ld_chain(const T* p) {
+    return *p;
 }
 
 // device count helper: n = *d_count when given (clamped to n_max), else n_max

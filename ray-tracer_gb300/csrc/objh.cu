@@ -42,11 +42,11 @@ namespace {
 constexpr float kRadSlack = 1.0f + 1.0f / 1048576.0f;
 }
 
-__global__ void k_morton(const float4* __restrict__ pos, uint32_t n, v3 lo, v3 sc, uint32_t* codes) {
+__global__ void k_morton(const float4* pos, uint32_t n, v3 lo, v3 sc, uint32_t* codes) {
     chain();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 a = __ldg(pos + 3ull * i), b = __ldg(pos + 3ull * i + 1), c = __ldg(pos + 3ull * i + 2);
+    const float4 a = ld_chain(pos + 3ull * i), b = ld_chain(pos + 3ull * i + 1), c = ld_chain(pos + 3ull * i + 2);
     const float cx = ((a.x + b.x) + c.x) / 3.0f;
     const float cy = ((a.y + b.y) + c.y) / 3.0f;
     const float cz = ((a.z + b.z) + c.z) / 3.0f;
@@ -56,28 +56,28 @@ __global__ void k_morton(const float4* __restrict__ pos, uint32_t n, v3 lo, v3 s
     codes[i] = (spread3((uint32_t)fx) << 2) | (spread3((uint32_t)fy) << 1) | spread3((uint32_t)fz);
 }
 
-__global__ void k_gather_tris(const float4* __restrict__ pos, const uint32_t* __restrict__ perm,
-                              uint32_t n, float4* __restrict__ tris, uint32_t* __restrict__ order) {
+__global__ void k_gather_tris(const float4* pos, const uint32_t* perm,
+                              uint32_t n, float4* tris, uint32_t* order) {
     chain();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const uint32_t t = __ldg(perm + k);
-    float4 a = __ldg(pos + 3ull * t);
+    const uint32_t t = ld_chain(perm + k);
+    float4 a = ld_chain(pos + 3ull * t);
     a.w = __uint_as_float(t);
     tris[3ull * k] = a;
-    tris[3ull * k + 1] = __ldg(pos + 3ull * t + 1);
-    tris[3ull * k + 2] = __ldg(pos + 3ull * t + 2);
+    tris[3ull * k + 1] = ld_chain(pos + 3ull * t + 1);
+    tris[3ull * k + 2] = ld_chain(pos + 3ull * t + 2);
     order[k] = t;
 }
 
 // boundary strength before sorted triangle k (k = 0 and k = T: 64, stronger than any)
-__global__ void k_delta_tri(const uint32_t* __restrict__ scode, uint32_t T, uint32_t* __restrict__ dtri) {
+__global__ void k_delta_tri(const uint32_t* scode, uint32_t T, uint32_t* dtri) {
     chain();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > T) return;
     uint32_t d = 64u;
     if (k > 0 && k < T) {
-        const uint32_t a = __ldg(scode + k - 1), b = __ldg(scode + k);
+        const uint32_t a = ld_chain(scode + k - 1), b = ld_chain(scode + k);
         d = (a != b) ? 32u + (31u - (uint32_t)__clz(a ^ b)) : 31u - (uint32_t)__clz((k - 1) ^ k);
     }
     dtri[k] = d;
@@ -150,7 +150,7 @@ RSH_DEV void write_node(const float4* tris, const RawBox* child_raw, uint32_t l,
     float mn[3] = {inf, inf, inf}, mx[3] = {-inf, -inf, -inf};
     if (l == 0) {
         for (uint64_t v = 3ull * f; v < 3ull * f1; ++v) {
-            const float4 p = __ldg(tris + v);
+            const float4 p = ld_chain(tris + v);
             mn[0] = fminf(mn[0], p.x), mn[1] = fminf(mn[1], p.y), mn[2] = fminf(mn[2], p.z);
             mx[0] = fmaxf(mx[0], p.x), mx[1] = fmaxf(mx[1], p.y), mx[2] = fmaxf(mx[2], p.z);
         }
@@ -181,7 +181,7 @@ RSH_DEV void write_node(const float4* tris, const RawBox* child_raw, uint32_t l,
     float r2 = 0.f;
     if (l == 0)
         for (uint64_t v = 3ull * f; v < 3ull * f1; ++v) {
-            const float4 p = __ldg(tris + v);
+            const float4 p = ld_chain(tris + v);
             const v3 d = v3{p.x - c.x, p.y - c.y, p.z - c.z};
             r2 = fmaxf(r2, dot3(d, d));
         }
@@ -224,8 +224,8 @@ RSH_DEV bool level_items(const LevelArrays& A, uint32_t l, uint32_t& items, uint
 // One level's cuts, compacted: firsts[k] = the first item of Morton group k. The last tile writes the level's
 // record (size 0: the level does not exist).
 __global__ void __launch_bounds__(LV_TILE)
-k_level_cuts(LevelArrays A, uint32_t l, uint32_t* __restrict__ firsts, unsigned long long* __restrict__ status,
-             uint32_t* __restrict__ ticket) {
+k_level_cuts(LevelArrays A, uint32_t l, uint32_t* firsts, unsigned long long* status,
+             uint32_t* ticket) {
     chain();
     __shared__ uint32_t s_tile, s_warp[LV_TILE / 32], s_delta[LV_TILE + 2 * MAX_G];
     __shared__ unsigned long long s_excl;
@@ -269,7 +269,7 @@ k_level_cuts(LevelArrays A, uint32_t l, uint32_t* __restrict__ firsts, unsigned 
 
 // Node g of the new level: children [firsts[g], firsts[g+1]) of the items, triangles
 // [start(firsts[g]), start(firsts[g+1])).
-__global__ void __launch_bounds__(128) k_level_nodes(LevelArrays A, uint32_t l, const uint32_t* __restrict__ firsts) {
+__global__ void __launch_bounds__(128) k_level_nodes(LevelArrays A, uint32_t l, const uint32_t* firsts) {
     chain();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t items, off;
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(256) k_level_radii(LevelArrays A) {
     const uint32_t t1 = min(t0 + 31u, A.n - 1u);
     float4 p[3];
     const bool in = t < A.n;
-    for (int v = 0; v < 3; ++v) p[v] = in ? __ldg(A.tris + 3ull * t + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int v = 0; v < 3; ++v) p[v] = in ? ld_chain(A.tris + 3ull * t + v) : make_float4(0.f, 0.f, 0.f, 0.f);
     const uint32_t size_l = lane < 16u ? A.lv[lane].size : 0u;
     const uint32_t some = __ballot_sync(0xffffffffu, size_l > 0u);
     if (some == 0u) return;  // a look-back gave up: no levels
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(256) k_level_radii(LevelArrays A) {
     }
 }
 
-__global__ void k_level_radii_end(const Level* __restrict__ lv, float4* __restrict__ sph) {
+__global__ void k_level_radii_end(const Level* lv, float4* sph) {
     chain();
     uint32_t total = 0;
     for (uint32_t l = 0; l < 16; ++l) total += lv[l].size;

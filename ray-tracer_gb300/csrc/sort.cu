@@ -299,7 +299,7 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
         load_keys(next);
         if (tid < 256u) {
             // global digit offset of this pass (exclusive, from the histogram kernel)
-            const uint32_t gex = __ldg(hist + tid);
+            const uint32_t gex = __ldcg(hist + tid);
             // decoupled look-back for this digit, LB predecessors per step: their status words are loaded
             // together (flag and count share one word, so relaxed loads suffice) and folded newest first up to
             // the first one holding an inclusive prefix; a not-yet-published word restarts the step there

@@ -13,47 +13,47 @@
 
 namespace rsh {
 
-RSH_DEV float4 mat4_apply(const float* __restrict__ m, float4 v) {
+RSH_DEV float4 mat4_apply(const float* m, float4 v) {
     float o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         float s = 0.0f;
-        s += __ldg(m + 4 * i + 0) * v.x;
-        s += __ldg(m + 4 * i + 1) * v.y;
-        s += __ldg(m + 4 * i + 2) * v.z;
-        s += __ldg(m + 4 * i + 3) * v.w;
+        s += ld_chain(m + 4 * i + 0) * v.x;
+        s += ld_chain(m + 4 * i + 1) * v.y;
+        s += ld_chain(m + 4 * i + 2) * v.z;
+        s += ld_chain(m + 4 * i + 3) * v.w;
         o[i] = s;
     }
     return make_float4(o[0], o[1], o[2], o[3]);
 }
 
 // One thread per vertex (3 per triangle). w of a position keeps its rest value; normals get w = 0.
-__global__ void k_transform(const float4* __restrict__ pos_rest, const float4* __restrict__ nrm_rest,
-                            const uint32_t* __restrict__ obj, uint32_t n_vertices, uint32_t n_objects,
-                            const float* __restrict__ model, const float* __restrict__ normal,
-                            float4* __restrict__ pos, float4* __restrict__ nrm) {
+__global__ void k_transform(const float4* pos_rest, const float4* nrm_rest,
+                            const uint32_t* obj, uint32_t n_vertices, uint32_t n_objects,
+                            const float* model, const float* normal,
+                            float4* pos, float4* nrm) {
     chain();
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n_vertices) return;
-    uint32_t id = __ldg(obj + x / 3);
+    uint32_t id = ld_chain(obj + x / 3);
     if (id >= n_objects) id = 0;
-    const float4 p = __ldg(pos_rest + x);
+    const float4 p = ld_chain(pos_rest + x);
     const float4 q = mat4_apply(model + 16ull * id, p);
     pos[x] = make_float4(q.x, q.y, q.z, p.w);
-    const float4 nr = __ldg(nrm_rest + x);
+    const float4 nr = ld_chain(nrm_rest + x);
     const float4 m = mat4_apply((normal ? normal : model) + 16ull * id, make_float4(nr.x, nr.y, nr.z, nr.w));
     const v3 u = norm3(v3{m.x, m.y, m.z});
     nrm[x] = make_float4(u.x, u.y, u.z, 0.0f);
 }
 
 // Exact min / max of the vertex coordinates: per-block partials, then one block over them.
-__global__ void k_bounds_partial(const float4* __restrict__ pos, uint32_t n_vertices, float* __restrict__ part) {
+__global__ void k_bounds_partial(const float4* pos, uint32_t n_vertices, float* part) {
     chain();
     __shared__ float s[6][256];
     const float inf = __int_as_float(0x7f800000);
     float mn[3] = {inf, inf, inf}, mx[3] = {-inf, -inf, -inf};
     for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < n_vertices; x += gridDim.x * blockDim.x) {
-        const float4 p = __ldg(pos + x);
+        const float4 p = ld_chain(pos + x);
         mn[0] = fminf(mn[0], p.x), mn[1] = fminf(mn[1], p.y), mn[2] = fminf(mn[2], p.z);
         mx[0] = fmaxf(mx[0], p.x), mx[1] = fmaxf(mx[1], p.y), mx[2] = fmaxf(mx[2], p.z);
     }
@@ -74,8 +74,8 @@ __global__ void k_bounds_partial(const float4* __restrict__ pos, uint32_t n_vert
 }
 
 // One warp per bound folds the blocks' partials (a thread each, one after the other, took 23 us for 608 blocks).
-__global__ void __launch_bounds__(192) k_bounds_final(const float* __restrict__ part, uint32_t blocks,
-                                                      float* __restrict__ out) {
+__global__ void __launch_bounds__(192) k_bounds_final(const float* part, uint32_t blocks,
+                                                      float* out) {
     chain();
     const uint32_t a = threadIdx.x >> 5;
     const bool is_min = a < 3;

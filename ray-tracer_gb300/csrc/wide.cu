@@ -153,13 +153,13 @@ struct Ploc {
     uint32_t m, next_id, src, pad;
 };
 
-__global__ void k_wide_leaves(const float4* __restrict__ tris, Tree T, int32_t* __restrict__ list,
-                              Ploc* __restrict__ st) {
+__global__ void k_wide_leaves(const float4* tris, Tree T, int32_t* list,
+                              Ploc* st) {
     chain();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k == 0) st[0] = Ploc{T.n, T.n, 0u, 0u};
     if (k >= T.n) return;
-    const float4 a = __ldg(tris + 3ull * k), b = __ldg(tris + 3ull * k + 1), c = __ldg(tris + 3ull * k + 2);
+    const float4 a = ld_chain(tris + 3ull * k), b = ld_chain(tris + 3ull * k + 1), c = ld_chain(tris + 3ull * k + 2);
     WNode w;
     w.lo = make_float4(fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z),
                        __uint_as_float(1u));
@@ -396,18 +396,18 @@ k_ploc_tail(Tree T, const Ploc* st, const int32_t* list0, const int32_t* list1, 
 }
 
 // Every triangle's depth-first position: the sum of what lies left of it on the way up.
-__global__ void k_wide_tris(const float4* __restrict__ tris, uint32_t n, const int2* __restrict__ up,
-                            const int32_t* __restrict__ root, uint32_t* __restrict__ first, float4* __restrict__ out) {
+__global__ void k_wide_tris(const float4* tris, uint32_t n, const int2* up,
+                            const int32_t* root, uint32_t* first, float4* out) {
     chain();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || *root < 0) return;
     uint32_t f = 0;
-    for (int2 u = __ldg(up + k); u.x >= 0; u = __ldg(up + u.x)) f += (uint32_t)u.y;
+    for (int2 u = ld_chain(up + k); u.x >= 0; u = ld_chain(up + u.x)) f += (uint32_t)u.y;
     first[k] = f;
     const uint64_t d = 3ull * f;
-    out[d] = __ldg(tris + 3ull * k);
-    out[d + 1] = __ldg(tris + 3ull * k + 1);
-    out[d + 2] = __ldg(tris + 3ull * k + 2);
+    out[d] = ld_chain(tris + 3ull * k);
+    out[d + 1] = ld_chain(tris + 3ull * k + 1);
+    out[d + 2] = ld_chain(tris + 3ull * k + 2);
 }
 
 // One breadth-first level of the collapse: the slots [base, base + count); `recs`: nodes (records) before it.
@@ -415,8 +415,8 @@ struct Bfs {
     uint32_t base, count, recs, pad;
 };
 
-__global__ void k_bfs_init(const int32_t* __restrict__ root, int32_t* __restrict__ item, Bfs* __restrict__ lv,
-                           float4* __restrict__ boxes) {
+__global__ void k_bfs_init(const int32_t* root, int32_t* item, Bfs* lv,
+                           float4* boxes) {
     chain();
     item[0] = *root;
     lv[0] = Bfs{0u, *root >= 0 ? 1u : 0u, 0u, 0u};
@@ -429,7 +429,7 @@ __global__ void k_bfs_init(const int32_t* __restrict__ root, int32_t* __restrict
 // and words (cluster: triangle range; node: its stack entry), rec_of[slot] for nodes, and rec_kids[record] =
 // the stack entry of the record's children.
 __global__ void __launch_bounds__(PT)
-k_bfs_level(Tree T, const uint32_t* __restrict__ first, Bfs* lv, uint32_t l, int32_t* item, uint32_t* rec_of, uint32_t* rec_kids, float pad,
+k_bfs_level(Tree T, const uint32_t* first, Bfs* lv, uint32_t l, int32_t* item, uint32_t* rec_of, uint32_t* rec_kids, float pad,
             float4* boxes, unsigned long long* status, uint32_t* ticket, uint32_t epoch, uint32_t* err) {
     chain();
     __shared__ uint32_t s_tile, s_kids[PT / 32], s_recs[PT / 32];
@@ -519,7 +519,7 @@ k_bfs_level(Tree T, const uint32_t* __restrict__ first, Bfs* lv, uint32_t l, int
     const WNode w = T.box[x];
     uint32_t lw, hw;
     if (m == 0u) {  // a cluster
-        lw = __ldg(first + ((uint32_t)x < T.n ? x : T.left[x - T.n]));
+        lw = ld_chain(first + ((uint32_t)x < T.n ? x : T.left[x - T.n]));
         hw = CLUSTER_BIT | __float_as_uint(w.lo.w);
     } else {
         lw = (1u << 27) | ((m - 1u) << 24) | (f & 0xFFFFFFu);
@@ -541,8 +541,8 @@ k_bfs_level(Tree T, const uint32_t* __restrict__ first, Bfs* lv, uint32_t l, int
 // ray misses) and entry 0. A child's entry: a cluster's first triangle | (triangles - 1) << 23 (bit 31 clear;
 // fewer than 2^23 triangles, at most 64 per cluster), or a node's REC_NODE | (children - 1) << 28 | record
 // index (kernels.h). Eight lanes a record, one per child.
-__global__ void k_rec_write(const float4* __restrict__ boxes, uint32_t recs, const uint32_t* __restrict__ rec_kids,
-                            const uint32_t* __restrict__ rec_of, float4* __restrict__ out) {
+__global__ void k_rec_write(const float4* boxes, uint32_t recs, const uint32_t* rec_kids,
+                            const uint32_t* rec_of, float4* out) {
     chain();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t rec = g >> 3, c = g & 7u;
