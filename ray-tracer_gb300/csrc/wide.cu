@@ -31,7 +31,7 @@
 // most TAIL_CLUSTERS are left one block runs all remaining passes from shared memory. A merge computes its
 // collapse costs at once (its children's are known) and tells its children how far right of it they start, so
 // neither needs a pass of its own: a triangle's place in the depth-first order is the sum on its way up. A
-// breadth-first level is one launch. 0.58 ms of kernels and 3 synchronisations for the same scene (a frame of 1001
+// breadth-first level is one launch. 0.58 ms of kernels and 2 synchronisations for the same scene (a frame of 1001
 // moving objects: 8.6 ms, then 1.8). The build's launches are chained: a pass's CTAs are placed while the one before
 // it ends (the same frame 1.40 ms unchained, 1.31 chained).
 // Slot layout (2 float4 per slot, padded box lo and hi): a cluster keeps its first triangle in lo.w and
@@ -565,7 +565,15 @@ __global__ void k_rec_write(const float4* boxes, uint32_t recs, const uint32_t* 
     reinterpret_cast<uint32_t*>(r)[48] = entry;
 }
 
+// What the host reads of a build.
+struct State {
+    int32_t root, pad[3];
+    Ploc ploc[PLOC_BUNCH + 1];
+    Bfs bfs[BFS_BUNCH + 1];
+};
+
 struct Scratch {
+    State* state = nullptr;  // root, ploc and bfs point into it
     Tree T;
     int32_t *list0, *list1, *root, *item;
     uint32_t *first, *rec_of, *rec_kids, *tickets;
@@ -595,10 +603,9 @@ size_t layout(uint32_t n, char* base, Scratch* out) {
     s.item = reinterpret_cast<int32_t*>(take(4ull * (2ull * n + 8)));
     s.rec_of = reinterpret_cast<uint32_t*>(take(4ull * (2ull * n + 8)));
     s.rec_kids = reinterpret_cast<uint32_t*>(take(4ull * (n + 8)));
-    s.root = reinterpret_cast<int32_t*>(take(4));
-    s.ploc = reinterpret_cast<Ploc*>(take(sizeof(Ploc) * (PLOC_BUNCH + 1)));
-    s.bfs = reinterpret_cast<Bfs*>(take(sizeof(Bfs) * (BFS_BUNCH + 1)));
-    s.tickets = reinterpret_cast<uint32_t*>(take(4ull * std::max(PLOC_BUNCH, BFS_BUNCH)));
+    s.state = reinterpret_cast<State*>(take(sizeof(State)));
+    if (s.state) s.root = &s.state->root, s.ploc = s.state->ploc, s.bfs = s.state->bfs;
+    s.tickets = reinterpret_cast<uint32_t*>(take(4ull * (PLOC_BUNCH + BFS_BUNCH)));
     s.status_words = (2ull * n + 8 + PT - 1) / PT + 1;
     s.status = reinterpret_cast<unsigned long long*>(take(8 * s.status_words));
     if (out) *out = s;
@@ -631,17 +638,33 @@ cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* 
             epoch = 0;
             RSH_BT(cudaMemsetAsync(w.status, 0, 8 * w.status_words, s));
         }
-        return cudaMemsetAsync(w.tickets, 0, 4ull * std::max(PLOC_BUNCH, BFS_BUNCH), s);
+        return cudaMemsetAsync(w.tickets, 0, 4ull * (PLOC_BUNCH + BFS_BUNCH), s);
     };
     RSH_BT(clear(true));
     RSH_BT(cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TailSmem)));
+    // breadth-first levels; each has at most 8 times the slots of the one before it
+    uint64_t most = 1;
+    auto levels = [&]() {
+        for (uint32_t l = 0; l < BFS_BUNCH; ++l) {
+            launch_chained(true, k_bfs_level, blocks(most), PT, 0, s, w.T, w.first, w.bfs, l, w.item, w.rec_of,
+                           w.rec_kids, pad, h.wboxes, w.status, w.tickets + PLOC_BUNCH + l, ++epoch, err);
+            most = std::min<uint64_t>(most * 8, 2ull * n + 8);
+        }
+        note_launch(BFS_BUNCH);
+        return cudaGetLastError();
+    };
+    State st;
+    auto read = [&]() -> cudaError_t {
+        RSH_BT(cudaMemcpyAsync(&st, w.state, sizeof(st), cudaMemcpyDeviceToHost, s));
+        return cudaStreamSynchronize(s);
+    };
     // 1. PLOC passes, then the last ones in one block
     launch_chained(true, k_wide_leaves, blocks(n), PT, 0, s, h.tris, w.T, w.list0, w.ploc);
     note_launch();
     uint32_t m = n;
     for (;;) {
         // enough passes to get from m to the tail when each keeps 4/5 of its clusters (0.76 on a soup of spheres);
-        // a pass too many costs its launch alone, one too few a read-back
+        // a pass too many costs its launch alone, one too few another round
         uint32_t passes = 0;
         for (uint64_t k = m; k > TAIL_CLUSTERS && passes < PLOC_BUNCH; k = k * 4 / 5) ++passes;
         for (uint32_t p = 0; p < passes; ++p)
@@ -650,45 +673,33 @@ cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* 
         launch_chained(true, k_ploc_tail, 1, TAIL_T, sizeof(TailSmem), s, w.T, w.ploc + passes, w.list0, w.list1,
                        w.root);
         note_launch(passes + 1);
-        RSH_BT(cudaGetLastError());
-        int32_t root = -1;
-        Ploc st{};
-        RSH_BT(cudaMemcpyAsync(&st, w.ploc + passes, sizeof(st), cudaMemcpyDeviceToHost, s));
-        RSH_BT(cudaMemcpyAsync(&root, w.root, 4, cudaMemcpyDeviceToHost, s));
-        RSH_BT(cudaStreamSynchronize(s));
-        if (root >= 0) break;
+        // 2. triangles in depth-first order, 3. the collapse, level by level: enqueued before the root is known to be
+        // there (without one these kernels do nothing), for one read-back of all the build's state (a frame of 1001
+        // moving objects 1.19 -> 1.16 ms)
+        launch_chained(true, k_wide_tris, blocks(n), PT, 0, s, h.tris, n, w.T.up, w.root, w.first, h.wtris);
+        launch_chained(true, k_bfs_init, 1, 1, 0, s, w.root, w.item, w.bfs, h.wboxes);
+        note_launch(2);
+        most = 1;
+        RSH_BT(levels());
+        RSH_BT(read());
+        if (st.root >= 0) break;
         // a pass that merged nothing cannot happen (the closest pair is mutual); never loop forever
-        if (st.m <= TAIL_CLUSTERS || st.m >= m) return cudaErrorUnknown;
-        m = st.m;
+        const Ploc& end = st.ploc[passes];
+        if (end.m <= TAIL_CLUSTERS || end.m >= m) return cudaErrorUnknown;
+        m = end.m;
         RSH_BT(cudaMemcpyAsync(w.ploc, w.ploc + passes, sizeof(Ploc), cudaMemcpyDeviceToDevice, s));
-        RSH_BT(clear(epoch + PLOC_BUNCH >= LB_EPOCHS));
+        RSH_BT(clear(epoch + PLOC_BUNCH + BFS_BUNCH >= LB_EPOCHS));
     }
-    // 2. triangles in depth-first order
-    launch_chained(true, k_wide_tris, blocks(n), PT, 0, s, h.tris, n, w.T.up, w.root, w.first, h.wtris);
-    // 3. the collapse, level by level; each level has at most 8 times the slots of the one before it
-    launch_chained(true, k_bfs_init, 1, 1, 0, s, w.root, w.item, w.bfs, h.wboxes);
-    note_launch(2);
-    Bfs lv[BFS_BUNCH + 1];
-    uint64_t most = 1;
-    for (bool first = true;; first = false) {
-        RSH_BT(clear(epoch + BFS_BUNCH >= LB_EPOCHS));
-        for (uint32_t l = 0; l < BFS_BUNCH; ++l) {
-            launch_chained(true, k_bfs_level, blocks(most), PT, 0, s, w.T, w.first, w.bfs, l, w.item, w.rec_of,
-                           w.rec_kids, pad, h.wboxes, w.status, w.tickets + l, ++epoch, err);
-            most = std::min<uint64_t>(most * 8, 2ull * n + 8);
-        }
-        note_launch(BFS_BUNCH);
-        RSH_BT(cudaGetLastError());
-        RSH_BT(cudaMemcpyAsync(lv, w.bfs, sizeof(lv), cudaMemcpyDeviceToHost, s));
-        RSH_BT(cudaStreamSynchronize(s));
-        if (first) {
-            if (lv[1].count == 0 || lv[1].count > 8) return cudaErrorUnknown;  // the root always has children
-            h.wroot = (1u << 27) | ((lv[1].count - 1u) << 24) | 1u;
-            h.wnroot = REC_NODE | ((lv[1].count - 1u) << 28);
-        }
-        if (lv[BFS_BUNCH].count == 0) break;
+    const Bfs* lv = st.bfs;
+    if (lv[1].count == 0 || lv[1].count > 8) return cudaErrorUnknown;  // the root always has children
+    h.wroot = (1u << 27) | ((lv[1].count - 1u) << 24) | 1u;
+    h.wnroot = REC_NODE | ((lv[1].count - 1u) << 28);
+    while (lv[BFS_BUNCH].count != 0) {
         most = lv[BFS_BUNCH].count;
         RSH_BT(cudaMemcpyAsync(w.bfs, w.bfs + BFS_BUNCH, sizeof(Bfs), cudaMemcpyDeviceToDevice, s));
+        RSH_BT(clear(epoch + BFS_BUNCH >= LB_EPOCHS));
+        RSH_BT(levels());
+        RSH_BT(read());
     }
     if (lv[BFS_BUNCH].base == 0) return cudaErrorUnknown;  // a look-back gave up
     h.wslots = lv[BFS_BUNCH].base;
