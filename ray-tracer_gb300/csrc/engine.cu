@@ -1337,7 +1337,9 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
         snrm = static_cast<const float4*>(bb.surf_nrm.ptr);
         incident = rrays;
     }
-    RSH_CUDA(cudaEventRecord(ctx->ev[2], s));  // secondary window ends
+    // secondary window ends (rays alone: with the frame, at ev[3]; each event is an operation of its own, 2.5 us in a
+    // small frame's chain)
+    if (!alone) RSH_CUDA(cudaEventRecord(ctx->ev[2], s));
     if (rgba_out && !alone) {
         th = stage_begin(ctx, RSH_STAGE_SHADE, s);
         sa.spos = spos;
@@ -1388,7 +1390,7 @@ rsh_status rsh_frame_stats_get(rsh_ctx* ctx, rsh_frame_stats* out) {
     st.node_tests = d[0];
     st.tri_tests = d[1];
     st.candidates += d[STAT_CAND];
-    cudaEventElapsedTime(&st.secondary_ms, ctx->ev[1], ctx->ev[2]);
+    cudaEventElapsedTime(&st.secondary_ms, ctx->ev[1], ctx->ev[ctx->falone ? 3 : 2]);
     cudaEventElapsedTime(&st.frame_ms, ctx->ev[0], ctx->ev[3]);
     for (float& v : st.stage_ms) v = 0.0f;
     for (const auto& m : ctx->tmarks) {
