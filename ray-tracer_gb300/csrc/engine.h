@@ -67,6 +67,7 @@ struct rsh_ctx {
     uint32_t* d_err = nullptr;
     unsigned long long* d_stats = nullptr;   // [0] node tests [1] tri tests [STAT_CAND] (ray, cluster) pairs
     uint32_t* h_pinned = nullptr;            // small pinned readback area
+    float* h_build = nullptr;                // pinned: what the host reads of a hierarchy build (BUILD_HOST_BYTES)
     rsh_light lights[8]{};
     uint32_t light_count = 0;
     rsh_camera cam{};

@@ -171,13 +171,14 @@ constexpr uint32_t REC_NODE = 0x80000000u;
 // Builds the single-ray box tree from h.tris (Morton order) and h.cluster; boxes widened by `pad`. The scratch
 // is the caller's (box_tree_scratch_bytes). Synchronises the stream.
 size_t box_tree_scratch_bytes(uint32_t tri_count);
-cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* err, cudaStream_t s);
+constexpr size_t BUILD_HOST_BYTES = 2048;
+cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* err, cudaStream_t s, void* host);
 // Builds (or, for the same triangle count, rebuilds in place) the object hierarchy and the box tree; scratch of
-// objh_scratch_bytes. The levels are built on `side`, a stream of the caller's that nothing else waits for.
+// objh_scratch_bytes; host: BUILD_HOST_BYTES of pinned memory. The levels are built on `side`, a stream of the caller's that nothing else waits for.
 // Synchronises both streams.
 cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t tri_count, uint32_t cluster,
                                    const float lo[3], const float hi[3], ObjHierarchy& h,
-                                   void* scratch, uint32_t* err, cudaStream_t s, cudaStream_t side);
+                                   void* scratch, uint32_t* err, cudaStream_t s, cudaStream_t side, void* host);
 size_t objh_scratch_bytes(uint32_t tri_count);
 void free_object_hierarchy(ObjHierarchy& h);
 

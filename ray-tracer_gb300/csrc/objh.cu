@@ -462,7 +462,7 @@ void free_object_hierarchy(ObjHierarchy& h) {
 
 cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t n, uint32_t cluster,
                                    const float lo[3], const float hi[3], ObjHierarchy& h,
-                                   void* scratch, uint32_t* err, cudaStream_t s, cudaStream_t side) {
+                                   void* scratch, uint32_t* err, cudaStream_t s, cudaStream_t side, void* host) {
     h.levels = 0;
     h.wslots = 0;
     h.wroot = 0;
@@ -530,10 +530,11 @@ cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t n, uint
     note_launch(3);
     e = cudaGetLastError();
     // the single-ray box tree over the same Morton-ordered triangles, with the same padding
-    if (e == cudaSuccess) e = build_box_tree(h, box_pad, w.box_tree, err, s);
+    if (e == cudaSuccess) e = build_box_tree(h, box_pad, w.box_tree, err, s, host);
     // whatever failed, nothing is left in flight on either stream
-    Level lv[16];
-    cudaError_t e2 = cudaMemcpyAsync(lv, w.lv, sizeof(lv), cudaMemcpyDeviceToHost, side);
+    static_assert(16 * sizeof(Level) <= BUILD_HOST_BYTES, "the levels fit");
+    Level* lv = static_cast<Level*>(host);  // (the box tree's build is done with it)
+    cudaError_t e2 = cudaMemcpyAsync(lv, w.lv, 16 * sizeof(Level), cudaMemcpyDeviceToHost, side);
     for (const cudaStream_t q : {side, s}) {
         const cudaError_t e3 = cudaStreamSynchronize(q);
         if (e2 == cudaSuccess) e2 = e3;

@@ -622,7 +622,7 @@ size_t box_tree_scratch_bytes(uint32_t tri_count) { return layout(tri_count ? tr
         if (e_ != cudaSuccess) return e_;          \
     } while (0)
 
-cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* err, cudaStream_t s) {
+cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* err, cudaStream_t s, void* host) {
     const uint32_t n = h.tri_count;
     h.wslots = 0;
     h.wroot = 0;
@@ -653,7 +653,8 @@ cudaError_t build_box_tree(ObjHierarchy& h, float pad, void* scratch, uint32_t* 
         note_launch(BFS_BUNCH);
         return cudaGetLastError();
     };
-    State st;
+    static_assert(sizeof(State) <= BUILD_HOST_BYTES, "the state fits");
+    State& st = *static_cast<State*>(host);
     auto read = [&]() -> cudaError_t {
         RSH_BT(cudaMemcpyAsync(&st, w.state, sizeof(st), cudaMemcpyDeviceToHost, s));
         return cudaStreamSynchronize(s);
