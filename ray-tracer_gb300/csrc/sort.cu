@@ -17,7 +17,7 @@
 // What bounds a pass: at 16 M random pairs 102 us (2.5 TB/s of its 16 B a pair), with the shared-memory pipe at
 // 70%: a row of 32 keys costs about 44 of its cycles (random banks: ranking, counters, scatter). Eight ballots a
 // key instead of the lane mask were bound by issue slots (139 us a pass at 24 warps an SM; alternating the two
-// row by row 103 us). 16 M random 31-bit pairs: 625 us before, now 428; 20,000: 54 -> 36.
+// row by row 103 us). 16 M random 31-bit pairs: 625 us before, now 423; 20,000: 54 -> 33.5.
 #include <algorithm>
 
 #include "common.cuh"
