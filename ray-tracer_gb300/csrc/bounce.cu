@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(BT, 10) k_bounce(const __grid_constant__ Bounc
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!GEN && blockIdx.x == 0)
         for (int q = 0; q < 2; ++q) {
-            for (uint32_t i = threadIdx.x; i < a.counters.n[q]; i += BT) a.counters.to[q][i] = __ldcg(a.counters.p[q] + i);
+            for (uint32_t i = threadIdx.x; i < a.counters.n[q]; i += BT) a.counters.to[q][i] = ld_chain(a.counters.p[q] + i);
             __syncthreads();  // one after the other, like copies in a stream
         }
     const uint32_t pix = blockIdx.x * BT + threadIdx.x, w = a.w;
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(BT, 10) k_bounce(const __grid_constant__ Bounc
     const uint32_t k = a.tiles_x ? primary_of_pixel(x, y, a.tiles_x, a.tiles_y) : pix;
     const unsigned long long h = in_range ? a.hits[k] : RSH_HIT_NONE;
     float4 ro = make_float4(0.f, 0.f, 0.f, 0.f), rd = ro, sp, sn;
-    if (h != RSH_HIT_NONE) load_ray(a.rays, k, ro, rd);
+    if (h != RSH_HIT_NONE) load_ray_chain(a.rays, k, ro, rd);
     // ---- shading of the surface the ray left
     float4 acc = make_float4(0.f, 0.f, 0.f, 1.f);
     if (SHADE && in_range) {
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(BT, 10) k_bounce(const __grid_constant__ Bounc
             v3 inc;
             if (a.sh.incident) {
                 float4 io, id;
-                load_ray(a.sh.incident, pix, io, id);
+                load_ray_chain(a.sh.incident, pix, io, id);
                 inc = mk3(id);
             } else {
                 inc = norm3(mk3(p4) - v3{a.sh.eye[0], a.sh.eye[1], a.sh.eye[2]});

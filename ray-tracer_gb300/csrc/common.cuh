@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "../../include/rsh.h"
 
@@ -174,16 +175,41 @@ RSH_DEV unsigned long long look_back2(unsigned long long* status, uint32_t tile,
 }
 
 // First in every kernel that launch_chained launches: the next one's CTAs may be placed from here on, and what the one
-// before wrote may be read (all its CTAs are done; a kernel that skipped the wait could be done before it). What the
-// chain writes is read with plain or .cg loads: a read-only load (__ldg, or through a const __restrict__ pointer) is
-// taken to read memory that nothing writes while the kernel lives, and may be moved above the wait.
+// before wrote may be read (all its CTAs are done; a kernel that skipped the wait could be done before it).
+// The rule of a chained kernel's loads: what another kernel of the chain writes -- while this one's CTAs may already be
+// resident -- is read with ld_chain, or plainly through a pointer that is not const __restrict__. A read-only load
+// (__ldg, or a plain one through a const __restrict__ pointer) is taken to read memory that nothing writes while the
+// kernel lives: it may be moved above the wait and may be served from an L1 line older than the write. Data complete
+// before the chain's first kernel starts (scenes, the sort's and the compression's input keys) may be read either way.
 RSH_DEV void chain() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// A load of what an earlier kernel of the chain wrote: coherent whatever the pointer's qualifiers, and, being volatile
+// like the wait, never above it. (Not for what this kernel itself writes.)
 template <class T>
 RSH_DEV T ld_chain(const T* p) {
-    return *p;
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "one load");
+    T r;
+    if constexpr (sizeof(T) == 4) {
+        uint32_t v;
+        asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+        memcpy(&r, &v, 4);
+    } else if constexpr (sizeof(T) == 8) {
+        unsigned long long v;
+        asm volatile("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+        memcpy(&r, &v, 8);
+    } else {
+        uint4 v;
+        asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+        memcpy(&r, &v, 16);
+    }
+    return r;
+}
+RSH_DEV void load_ray_chain(const rsh_ray* rays, uint32_t i, float4& o, float4& d) {
+    const float4* p = reinterpret_cast<const float4*>(rays) + 2ull * i;
+    o = ld_chain(p);
+    d = ld_chain(p + 1);
 }
 
 // device count helper: n = *d_count when given (clamped to n_max), else n_max

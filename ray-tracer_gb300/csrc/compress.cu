@@ -147,7 +147,7 @@ k_compress_write(const uint32_t* __restrict__ keys, uint32_t n_slots, const uint
 #pragma unroll
     for (uint32_t i = 0; i < PER; ++i) {
         const uint32_t c = threadIdx.x * PER + i;
-        if (c < blockIdx.x) t = combine(t, from4(__ldcg(csumm + c)));
+        if (c < blockIdx.x) t = combine(t, from4(ld_chain(csumm + c)));
     }
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -155,7 +155,7 @@ k_compress_write(const uint32_t* __restrict__ keys, uint32_t n_slots, const uint
         if (lane >= (uint32_t)d) t = combine(o, t);
     }
     if (lane == 31u) s_fold[warp] = t;
-    if (threadIdx.x < CT_WARPS) s_own[threadIdx.x] = from4(__ldcg(wsumm + blockIdx.x * CT_WARPS + threadIdx.x));
+    if (threadIdx.x < CT_WARPS) s_own[threadIdx.x] = from4(ld_chain(wsumm + blockIdx.x * CT_WARPS + threadIdx.x));
     __syncthreads();
     Summ pre{0u, 0u, 0u, 0u};
     for (uint32_t w = 0; w < CT_WARPS; ++w) pre = combine(pre, s_fold[w]);

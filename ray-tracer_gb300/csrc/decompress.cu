@@ -102,12 +102,12 @@ k_dc_write(const uint32_t* __restrict__ ssize, const uint32_t* __restrict__ coun
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     // what comes before the warp: the CTAs before this one, and the warps before it
     uint32_t run = 0;
-    for (uint32_t c = threadIdx.x; c < blockIdx.x; c += DS_THREADS) run += __ldcg(csum + c);
+    for (uint32_t c = threadIdx.x; c < blockIdx.x; c += DS_THREADS) run += ld_chain(csum + c);
     run = warp_sum(run);
     if (lane == 0u) s_warp[warp] = run;
     __syncthreads();
     run = lane < DS_WARPS ? s_warp[lane] : 0u;
-    if (lane < warp) run += __ldcg(wsum + blockIdx.x * DS_WARPS + lane);  // (warp < DS_WARPS)
+    if (lane < warp) run += ld_chain(wsum + blockIdx.x * DS_WARPS + lane);  // (warp < DS_WARPS)
     run = warp_sum(run);
     uint32_t b, e;
     warp_range(C, b, e);
@@ -116,7 +116,7 @@ k_dc_write(const uint32_t* __restrict__ ssize, const uint32_t* __restrict__ coun
 #pragma unroll
         for (uint32_t i = 0; i < DS_BATCH; ++i) {
             const uint32_t x = q + 32u * i + lane;
-            sz[i] = x < e ? __ldcg(ssize + x) : 0u;
+            sz[i] = x < e ? ld_chain(ssize + x) : 0u;
         }
 #pragma unroll
         for (uint32_t i = 0; i < DS_BATCH; ++i) {
@@ -161,15 +161,15 @@ k_dc_expand(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sba
     // chunks x0..x1 cover the tile's outputs: x0 holds the first, and the chunk holding the next tile's first
     // output is at or after the one holding this one's last (one extra chunk may be staged)
     const uint32_t ntiles = (R + DE_TILE - 1) / DE_TILE;
-    const uint32_t x0 = min(__ldcg(tile_chunk + blockIdx.x), C - 1u);
-    uint32_t x1 = (blockIdx.x + 1 < ntiles) ? __ldcg(tile_chunk + blockIdx.x + 1) : C - 1;
+    const uint32_t x0 = min(ld_chain(tile_chunk + blockIdx.x), C - 1u);
+    uint32_t x1 = (blockIdx.x + 1 < ntiles) ? ld_chain(tile_chunk + blockIdx.x + 1) : C - 1;
     if (x1 >= C) x1 = C - 1;
     if (x1 < x0) x1 = x0;
     const uint32_t m = (x1 - x0 + 1 < DE_TILE + 1) ? x1 - x0 + 1 : DE_TILE + 1;
     __syncthreads();
     for (uint32_t i = tid; i < m; i += DE_THREADS) {
-        const uint32_t x = x0 + i, o = __ldcg(off + x);
-        s_add[i] = __ldcg(sbase + x) - o;
+        const uint32_t x = x0 + i, o = ld_chain(off + x);
+        s_add[i] = ld_chain(sbase + x) - o;
         s_key[i] = skeys ? __ldg(skeys + x) : 0u;
         const uint32_t at = o > k0 ? o - k0 : 0u;  // only the first one may start before the tile
         if (at < DE_TILE) atomicOr(&s_mark[at >> 5], 1u << (at & 31u));

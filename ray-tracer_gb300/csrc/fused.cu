@@ -840,11 +840,11 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
             bool ray = false;
             if (!has && k < nend) {
                 const FusedSeg& sg = seg_of(cs);
-                uint32_t id = sg.ids ? __ldg(sg.ids + k) : k;
+                uint32_t id = sg.ids ? ld_chain(sg.ids + k) : k;
                 if (!ONE) id -= sg.slot_base;
                 if (id < sg.slots) {
                     float4 o, d;
-                    load_ray(sg.rays, id, o, d);
+                    load_ray_chain(sg.rays, id, o, d);
                     ray = d.w > o.w;
                     if (!ray || sg.levels == 0u) {
                         // no ray, or a scene without triangles (no tree): a miss

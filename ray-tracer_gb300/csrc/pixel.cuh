@@ -147,7 +147,7 @@ RSH_DEV float soft_weight(uint32_t k) {
 
 // One bounce's shading of pixel pix = (x, y) whose surface is (p4, n4) and incident direction inc, added to acc
 // (rgb, weight in w); shadow == nullptr: unshadowed. Blinn-Phong per unoccluded light (RayTracer.cu:1616-1709).
-RSH_DEV void shade_surface(const ShadeArgs& a, const rsh_light* s_light, const uint32_t* __restrict__ shadow,
+RSH_DEV void shade_surface(const ShadeArgs& a, const rsh_light* s_light, const uint32_t* shadow,
                            uint32_t x, uint32_t y, float4 p4, float4 n4, v3 inc, float4& acc) {
     const v3 p = mk3(p4);
     const v3 n = norm3(mk3(n4));
@@ -161,7 +161,7 @@ RSH_DEV void shade_surface(const ShadeArgs& a, const rsh_light* s_light, const u
     if (S == 1 && shadow) {
         const uint32_t* f = shadow + (x + (size_t)a.w * a.lights * y);
 #pragma unroll 4
-        for (uint32_t l = 0; l < a.lights; ++l) occluded |= (__ldg(f + a.w * l) == RSH_OCCLUDED ? 1u : 0u) << l;
+        for (uint32_t l = 0; l < a.lights; ++l) occluded |= (ld_chain(f + a.w * l) == RSH_OCCLUDED ? 1u : 0u) << l;
     }
     for (uint32_t l = 0; l < a.lights; ++l) {
         float factor = 1.0f;
@@ -171,7 +171,7 @@ RSH_DEV void shade_surface(const ShadeArgs& a, const rsh_light* s_light, const u
             // soft shadows (RayTracer.cu:1680-1696): weighted unoccluded samples, log2(1 + 2 sum)
             float sf = 0.0f;
             for (uint32_t k = 0; k < S; ++k)
-                if (shadow[x + a.w * ((l * S + k) + a.lights * S * y)] != RSH_OCCLUDED) sf += soft_weight(k);
+                if (ld_chain(shadow + (x + a.w * ((l * S + k) + a.lights * S * y))) != RSH_OCCLUDED) sf += soft_weight(k);
             factor = log2f(1.0f + sf * 2.0f);
         }
         const rsh_light& L = s_light[l];

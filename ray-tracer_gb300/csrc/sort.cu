@@ -209,7 +209,7 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
         const bool whole = t * TILE + TILE <= n;
 #pragma unroll
         for (int j = 0; j < I; ++j)
-            if (FULL || (uint32_t)j < rows) key[j] = whole || b + j * 32u < n ? __ldg(keys_in + b + j * 32u) : 0xFFFFFFFFu;
+            if (FULL || (uint32_t)j < rows) key[j] = whole || b + j * 32u < n ? ld_chain(keys_in + b + j * 32u) : 0xFFFFFFFFu;
     };
     if (tid == 0) S.tile = atomicAdd(ticket, 1u);
     __syncthreads();
@@ -283,7 +283,7 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
                 if (!FULL && (uint32_t)j >= rows) break;
                 const uint32_t idx = wbase + j * 32u + lane;
                 val[j] = idx;
-                if (vals_in && (full || idx < n)) val[j] = __ldg(vals_in + idx);
+                if (vals_in && (full || idx < n)) val[j] = ld_chain(vals_in + idx);
             }
 #pragma unroll
             for (int j = 0; j < I; ++j) {
@@ -299,7 +299,7 @@ k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ va
         load_keys(next);
         if (tid < 256u) {
             // global digit offset of this pass (exclusive, from the histogram kernel)
-            const uint32_t gex = __ldcg(hist + tid);
+            const uint32_t gex = ld_chain(hist + tid);
             // decoupled look-back for this digit, LB predecessors per step: their status words are loaded
             // together (flag and count share one word, so relaxed loads suffice) and folded newest first up to
             // the first one holding an inclusive prefix; a not-yet-published word restarts the step there
