@@ -678,9 +678,13 @@ struct GraphExec {
 namespace rsh {
 rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
-                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair, bool count_tests) {
+                       uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair, bool count_tests,
+                       uint32_t* ready) {
     FusedArgs fa = alone_args(ctx, ticket);
     fa.pair = pair;
+    if (pair == 1u) ++ctx->pairs;
+    fa.ready = ready;
+    fa.ready_is = ctx->pairs;
     fa.wait = pair != 2u ? 1u : 0u;  // behind the kernel that generated its rays
     fa.pixel_order = true;
     if (!count_tests) fa.node_tests = fa.tri_tests = nullptr;

@@ -1140,16 +1140,16 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     }
     void* cnt_acc;
     // per bounce (rays, chunks) of the shadow and of the reflection batch, then a work ticket per launch of rays
-    // alone (the primary rays' and two a bounce)
+    // alone (the primary rays' and two a bounce) and a word per pair of them
     const size_t fc_bytes = 16ull * (depth + 1);
-    RSH_TRY(ensure(ctx, "frame_counts", fc_bytes + 4ull * (2 * depth + 1), &cnt_acc));
+    RSH_TRY(ensure(ctx, "frame_counts", fc_bytes + 4ull * (3 * depth + 1), &cnt_acc));
     uint32_t* fc = static_cast<uint32_t*>(cnt_acc);
     uint32_t* tickets = fc + 4 * (depth + 1);
     unsigned long long* pairs = fused ? nullptr : ctx->d_stats + STAT_CAND;
     // the frame's counters and tickets: zeroed by its first kernel, copied out by its last one (memsets and copies of
     // their own: 4 more operations in the chain, a Cornell frame 120 us, now 108; 64x64 73, now 63)
     uint32_t* stats = reinterpret_cast<uint32_t*>(ctx->d_stats);
-    const Words2 zero{{fc, stats}, {}, {(uint32_t)(fc_bytes / 4) + 2 * depth + 1, 2 * (STAT_CAND + 1)}};
+    const Words2 zero{{fc, stats}, {}, {(uint32_t)(fc_bytes / 4) + 3 * depth + 1, 2 * (STAT_CAND + 1)}};
     const Words2 counters{{fc, stats},
                           {ctx->h_pinned + 16, ctx->h_pinned + 256},
                           {(uint32_t)(fc_bytes / 4), 2 * (STAT_CAND + 1)}};
@@ -1254,10 +1254,11 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
             th = stage_begin(ctx, RSH_STAGE_TRAVERSE, s);
             // side by side: the shadow rays' warps start as the reflection rays' end (Cornell frame 200 -> 171 us,
             // architecture frame 3.37 -> 3.27 ms)
+            uint32_t* ready = tickets + 1 + 2 * depth + b;
             RSH_TRY(trace_alone(ctx, sc, ba.rrays, npix, ba.rids, ba.rcount, false, nullptr, ba.rhits,
-                                tickets + 1 + 2 * b, pairs, s, 1));
+                                tickets + 1 + 2 * b, pairs, s, 1, true, ready));
             RSH_TRY(trace_alone(ctx, sc, ba.srays, npix * LS, ba.sids, ba.scount, true, ba.sflags, nullptr,
-                                tickets + 2 + 2 * b, pairs, s, 2));
+                                tickets + 2 + 2 * b, pairs, s, 2, true, ready));
             stage_end(ctx, th, s);
             spos = ba.spos;
             snrm = ba.snrm;

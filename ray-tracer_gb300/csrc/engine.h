@@ -84,6 +84,7 @@ struct rsh_ctx {
     cudaStream_t last_stream = nullptr;
     std::vector<uint32_t> batch_counts_host;
     uint32_t overflow_passes = 0;
+    uint32_t pairs = 0;  // pairs of traversal launches so far (FusedArgs::ready_is)
     // per-stage CUDA events (RSH_FLAG_STAGE_TIMERS): pool and the (stage, start event) pairs of a frame
     std::vector<cudaEvent_t> tev;
     std::vector<std::pair<int, uint32_t>> tmarks;
@@ -139,11 +140,11 @@ constexpr uint32_t STAT_CAND = 8;
 // The rays of one segment alone from the root of the scene's box tree (batch.cu), in one launch: the slots
 // ids[0 .. *d_count), whose results are prefilled, or (ids null) every slot, the results of empty ones written
 // too. ticket: a zeroed device word. pair: 1, 2 for the first and the second of two independent launches, of which
-// the second may start while the first still runs (FusedArgs::pair).
+// the second may start while the first still runs (FusedArgs::pair, FusedArgs::ready).
 rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, uint32_t slots, const uint32_t* ids,
                        const uint32_t* d_count, bool any_hit, uint32_t* flags, unsigned long long* hits,
                        uint32_t* ticket, unsigned long long* cand_pairs, cudaStream_t s, uint32_t pair = 0,
-                       bool count_tests = true);
+                       bool count_tests = true, uint32_t* ready = nullptr);
 
 // One secondary batch through compress -> sort -> decompress -> build -> traverse -> intersect.
 // keys: per slot (RSH_KEY_NONE = no ray); rays indexed by slot. Output flags/hits indexed by slot

@@ -703,8 +703,32 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
     __shared__ uint32_t sh_don[SHARE ? FW : 1][32];  // SHARE: the donors of a hand-out, by rank
     __shared__ uint32_t s_rays, s_ended;  // a.valid: the block's rays, its warps that have ended
     const uint32_t lane = lane_id();
-    // (a.wait: what the kernel before wrote is there; the second of a pair starts only then, too)
     if (a.wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The second of a pair reads what the kernel before the first wrote, and does not wait for the first itself. That
+    // its CTAs start only after the first's wait does not make those writes visible to them (a trigger orders
+    // nothing): the first releases a word after its wait, before its trigger, and the second acquires it -- at the
+    // first look, as a rule.
+    if (ONE && a.ready) {
+        bool late = false;
+        if (threadIdx.x == 0) {
+            if (a.pair == 1u) {
+                if (blockIdx.x == 0) st_release_u32(a.ready, a.ready_is);
+            } else {
+                for (uint32_t spins = 0; ld_acquire_u32(a.ready) != a.ready_is; ++spins) {
+                    if (spins > RSH_SPIN_LIMIT) {
+                        raise_device_error(a.err, RSH_DEVERR_TIMEOUT);
+                        late = true;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+            }
+        }
+        if (__syncthreads_or(late)) {  // traces nothing, ends after the first like every second launch
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            return;
+        }
+    }
     asm volatile("griddepcontrol.launch_dependents;");
     if (a.valid) {
         if (threadIdx.x == 0) s_rays = s_ended = 0u;

@@ -18,7 +18,8 @@ namespace rsh {
 void note_launch(unsigned n = 1);
 
 // A kernel that may start while the one before it in the stream still runs; it waits itself
-// (griddepcontrol.wait) before it touches what that one wrote.
+// (griddepcontrol.wait) before it touches what that one wrote. (The second of a pair of traversals reads nothing of
+// the first's and waits at its end; what the first waited for, too, it gets through FusedArgs::ready.)
 template <class... P, class... A>
 inline cudaError_t launch_chained(bool chained, void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem,
                            cudaStream_t s, A... args) {
@@ -275,6 +276,10 @@ struct FusedArgs {
     uint32_t pair;                     // rays-only: 1, 2: the first / second of two launches that neither read
                                        // nor write what the other writes; the second may start while the first runs
     uint32_t wait;                     // rays-only: the launch is chained behind a kernel whose results it reads
+    // a pair whose first launch waits for results that the second reads, too: the word by which the first passes them
+    // on, and the value that says so (null: what both read was complete before the first started)
+    uint32_t* ready;
+    uint32_t ready_is;
     FusedSeg one;                      // launch_rays_one: the one segment (slot_base 0)
     uint32_t* valid;                   // rays-only: the rays traced are added to valid[0] and valid[1] (null: not)
     unsigned long long* cand_pairs;    // launch_rays_one: counts (ray, cluster) pairs tested (null: not counted)

@@ -72,3 +72,16 @@ def test_shading_reads_shadow_flags_by_the_rule():
     fns = {n: (p, b) for n, p, b in _functions((CSRC / "pixel.cuh").read_text(), r"RSH_DEV void ")}
     params, body = fns["shade_surface"]
     assert not re.search(r"__restrict__\s+shadow", params) and "__ldg" not in body
+
+
+def test_the_second_of_a_pair_acquires_before_it_reads():
+    """k_fused_rays as the second launch of a frame's pair does not wait for the first, so what the kernel before both
+    wrote (lists, counts, rays) is visible to it only through the word that the first releases after its own wait."""
+    body = KERNELS["k_fused_rays"][1]
+    wait, release = body.index("griddepcontrol.wait"), body.index("st_release_u32(a.ready")
+    acquire, trigger = body.index("ld_acquire_u32(a.ready)"), body.index("griddepcontrol.launch_dependents")
+    assert wait < release < trigger and acquire < trigger < body.index("dev_count(")
+    spin = body[body.rindex("for (", 0, acquire):trigger]
+    assert "RSH_SPIN_LIMIT" in spin and "raise_device_error" in spin  # the wait ends, with an error
+    frame = (CSRC / "engine.cu").read_text()
+    assert len(re.findall(r"trace_alone\([^;]*\btrue, ready\)", frame)) == 2  # both launches of a frame's pair
