@@ -106,6 +106,22 @@ rsh_status make_hash_params(const rsh_scene* sc, const rsh_config& cfg, uint32_t
     return RSH_OK;
 }
 
+// The context's pinned words for a frame's counters: at least `words`. A larger block replaces the one before it once
+// nothing writes that any more.
+static rsh_status ensure_frame_words(rsh_ctx* ctx, size_t words) {
+    if (ctx->h_frame_words >= words) return RSH_OK;
+    if (ctx->h_frame) {
+        RSH_CUDA(cudaDeviceSynchronize());
+        cudaFreeHost(ctx->h_frame);
+        ctx->h_frame = nullptr;
+        ctx->h_frame_words = 0;
+    }
+    RSH_CUDA(cudaMallocHost(&ctx->h_frame, 4 * words));
+    std::memset(ctx->h_frame, 0, 4 * words);
+    ctx->h_frame_words = words;
+    return RSH_OK;
+}
+
 static uint64_t cand_capacity(const rsh_ctx* ctx) {
     return ctx->cfg.candidate_capacity ? ctx->cfg.candidate_capacity : (1ull << 28);  // 2 GiB of candidates
 }
@@ -327,6 +343,10 @@ rsh_status rsh_create(const rsh_config* cfg, rsh_ctx** out) {
     cudaMemset(ctx->d_err, 0, 256);
     cudaMemset(ctx->d_stats, 0, 256);
     for (auto& ev : ctx->ev) cudaEventCreate(&ev);
+    if (const rsh_status st = ensure_frame_words(ctx, 1024); st != RSH_OK) {
+        rsh_destroy(ctx);
+        return st;
+    }
     if ((e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking)) != cudaSuccess) {
         rsh_status st = cuda_status(e, "rsh_create");
         rsh_destroy(ctx);
@@ -358,6 +378,7 @@ rsh_status rsh_destroy(rsh_ctx* ctx) {
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->d_stats) cudaFree(ctx->d_stats);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+    if (ctx->h_frame) cudaFreeHost(ctx->h_frame);
     if (ctx->h_build) cudaFreeHost(ctx->h_build);
     for (auto& ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
@@ -1143,6 +1164,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     // alone (the primary rays' and two a bounce) and a word per pair of them
     const size_t fc_bytes = 16ull * (depth + 1);
     RSH_TRY(ensure(ctx, "frame_counts", fc_bytes + 4ull * (3 * depth + 1), &cnt_acc));
+    RSH_TRY(ensure_frame_words(ctx, FRAME_COUNTS + fc_bytes / 4));
     uint32_t* fc = static_cast<uint32_t*>(cnt_acc);
     uint32_t* tickets = fc + 4 * (depth + 1);
     unsigned long long* pairs = fused ? nullptr : ctx->d_stats + STAT_CAND;
@@ -1151,7 +1173,7 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     uint32_t* stats = reinterpret_cast<uint32_t*>(ctx->d_stats);
     const Words2 zero{{fc, stats}, {}, {(uint32_t)(fc_bytes / 4) + 3 * depth + 1, 2 * (STAT_CAND + 1)}};
     const Words2 counters{{fc, stats},
-                          {ctx->h_pinned + 16, ctx->h_pinned + 256},
+                          {ctx->h_frame + FRAME_COUNTS, ctx->h_frame},
                           {(uint32_t)(fc_bytes / 4), 2 * (STAT_CAND + 1)}};
     RSH_CUDA(cudaEventRecord(ctx->ev[0], s));
     int th = stage_begin(ctx, RSH_STAGE_PRIMARY, s);
@@ -1357,8 +1379,8 @@ rsh_status rsh_render_frame(rsh_ctx* ctx, const rsh_scene* sc, uint32_t W, uint3
     RSH_CUDA(cudaEventRecord(ctx->ev[3], s));
     // counters (async; read by rsh_frame_stats_get)
     if (!alone) {
-        RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 16, fc, fc_bytes, cudaMemcpyDeviceToHost, s));
-        RSH_CUDA(cudaMemcpyAsync(ctx->h_pinned + 256, ctx->d_stats, 8 * (STAT_CAND + 1), cudaMemcpyDeviceToHost, s));
+        RSH_CUDA(cudaMemcpyAsync(ctx->h_frame + FRAME_COUNTS, fc, fc_bytes, cudaMemcpyDeviceToHost, s));
+        RSH_CUDA(cudaMemcpyAsync(ctx->h_frame, ctx->d_stats, 8 * (STAT_CAND + 1), cudaMemcpyDeviceToHost, s));
     }
     ctx->stats.primary_rays = (uint64_t)W * H;
     return RSH_OK;
@@ -1381,7 +1403,7 @@ rsh_status rsh_frame_stats_get(rsh_ctx* ctx, rsh_frame_stats* out) {
     RSH_CUDA(cudaStreamSynchronize(ctx->last_stream));
     rsh_frame_stats st = ctx->stats;
     st.shadow_rays = st.reflection_rays = st.chunks = 0;
-    const uint32_t* fc = ctx->h_pinned + 16;
+    const uint32_t* fc = ctx->h_frame + FRAME_COUNTS;
     for (uint32_t b = 0; b < ctx->fdepth; ++b) {
         st.shadow_rays += fc[4 * b];
         // rays alone are not cut into runs: a run each
@@ -1389,7 +1411,7 @@ rsh_status rsh_frame_stats_get(rsh_ctx* ctx, rsh_frame_stats* out) {
         st.reflection_rays += fc[4 * b + 2];
     }
     unsigned long long d[STAT_CAND + 1];
-    std::memcpy(d, ctx->h_pinned + 256, sizeof(d));
+    std::memcpy(d, ctx->h_frame, sizeof(d));
     st.node_tests = d[0];
     st.tri_tests = d[1];
     st.candidates += d[STAT_CAND];

@@ -67,6 +67,10 @@ struct rsh_ctx {
     uint32_t* d_err = nullptr;
     unsigned long long* d_stats = nullptr;   // [0] node tests [1] tri tests [STAT_CAND] (ray, cluster) pairs
     uint32_t* h_pinned = nullptr;            // small pinned readback area
+    // pinned: what the last frame's counters are copied to, the statistics, then from FRAME_COUNTS on 4 words a bounce
+    // and 4 more; written by the frame's last kernel, so it has to hold a frame of any depth (h_frame_words)
+    uint32_t* h_frame = nullptr;
+    size_t h_frame_words = 0;
     float* h_build = nullptr;                // pinned: what the host reads of a hierarchy build (BUILD_HOST_BYTES)
     rsh_light lights[8]{};
     uint32_t light_count = 0;
@@ -137,6 +141,8 @@ rsh_status trace_plain(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t 
 // ctx->d_stats word of a frame's (ray, cluster) pairs: past the words a frame zeroes again after its primary
 // rays (the pairs cover them, the test counts do not)
 constexpr uint32_t STAT_CAND = 8;
+constexpr uint32_t FRAME_COUNTS = 32;
+static_assert(2 * (STAT_CAND + 1) <= FRAME_COUNTS, "the statistics lie before the counts");
 // The rays of one segment alone from the root of the scene's box tree (batch.cu), in one launch: the slots
 // ids[0 .. *d_count), whose results are prefilled, or (ids null) every slot, the results of empty ones written
 // too. ticket: a zeroed device word. pair: 1, 2 for the first and the second of two independent launches, of which
