@@ -259,6 +259,11 @@ size_t table_bytes(uint32_t nseg) { return (sizeof(PrepSeg) + sizeof(FusedSeg) +
 // 1.3 M rays in 8 segments (traversal 0.526 against 0.587 ms then), 0.5 ms for 13.8 M in 64 (all of it 3.86 ms
 // sorted, 4.19 unsorted).
 constexpr uint32_t SORT_RAYS = 2000000;
+// From this many slots on they are traced in their own order, too: a digit's count in the sort has 30 bits, and without
+// run compression one digit may have them all.
+constexpr uint32_t SORT_MOST = 1u << 30;
+// The plain path takes as many rays as a 32-bit count holds, in parts of at most this many.
+constexpr uint32_t PLAIN_PART = 1u << 29;
 
 // The context's configuration with a scene's own tuning (rsh_scene_set_tuning) applied.
 rsh_config tuned_config(const rsh_config& base, const rsh_scene* sc) {
@@ -318,7 +323,8 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         if (tuned_config(ctx->cfg, segs[s].scene).ray_level < segs[s].scene->h.levels) pl.rays_only = 0;
     pl.listed = lists != nullptr;
     if (pl.listed && !pl.rays_only) return RSH_ERR_INVALID;
-    pl.sorted = !pl.listed && (!pl.rays_only || (pl.total > SORT_RAYS && !(plain && (ctx->cfg.flags & RSH_FLAG_RAH))));
+    pl.sorted = !pl.listed && (!pl.rays_only || (pl.total > SORT_RAYS && pl.total < SORT_MOST &&
+                                                 !(plain && (ctx->cfg.flags & RSH_FLAG_RAH))));
     const bool packets = !pl.rays_only;
     {
         // slots sorted as they are: an empty slot's key has every bit set, so it goes last by the tag alone
@@ -724,9 +730,17 @@ rsh_status batch_trace_listed(rsh_ctx* ctx, const rsh_batch_segment* segments, c
 }
 
 rsh_status trace_plain(rsh_ctx* ctx, const rsh_batch_segment& seg, cudaStream_t s) {
-    BatchPlan pl;
-    RSH_TRY(batch_prepare(ctx, &seg, 1, pl, nullptr, true));
-    return batch_enqueue(ctx, pl, s, nullptr, false);  // the test counters run on
+    for (uint64_t at = 0; at < seg.n; at += PLAIN_PART) {
+        rsh_batch_segment part = seg;
+        part.rays += at;
+        part.n = (uint32_t)std::min<uint64_t>(seg.n - at, PLAIN_PART);
+        if (part.hits) part.hits += at;
+        if (part.flags) part.flags += at;
+        BatchPlan pl;
+        RSH_TRY(batch_prepare(ctx, &part, 1, pl, nullptr, true));
+        RSH_TRY(batch_enqueue(ctx, pl, s, nullptr, false));  // the test counters run on
+    }
+    return RSH_OK;
 }
 
 // rsh_batch_trace without resetting the stage timers (a fused frame keeps its own).
