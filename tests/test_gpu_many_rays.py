@@ -14,6 +14,7 @@ from rsh import scenes
 pytestmark = pytest.mark.gpu
 
 N = (1 << 31) + 1000
+M = (1 << 30) + 1010
 NEED = 32 * N + 4 * N + (24 << 30)
 
 
@@ -26,7 +27,8 @@ def test_more_rays_than_a_sort_or_31_bits_hold():
     c = rsh.Context(rsh.default_config())
     sc = c.scene(s.positions, s.normals, s.material_ids, s.materials)
     rays = rsh.DeviceArray(N, rsh.RAY_DTYPE, zero=True)  # tmax = tmin: no ray
-    out = rsh.DeviceArray(N + 1000, np.uint32)
+    out = rsh.DeviceArray(M, np.uint64)  # flags of N rays, then hits of M
+    assert out.nbytes >= max(4 * N, 8 * M)
     rng = np.random.default_rng(5)
     marks = {}
     for at in (0, (1 << 29) - 1000, (1 << 30) - 1000, (1 << 30) + 10, 3 * (1 << 29) - 7, N - 1000):
@@ -50,9 +52,8 @@ def test_more_rays_than_a_sort_or_31_bits_hold():
     out.fill_bytes(0x5A)
     rsh.check(rsh.lib().rsh_trace_rays(c.handle, sc.handle, rays.ptr, N, 1, None, out.ptr, None), "plain")
     check(N, True, np.uint32, 0)
-    n = (1 << 30) + 1010
     out.fill_bytes(0x5A)
-    rsh.check(rsh.lib().rsh_trace_rays_fused(c.handle, sc.handle, rays.ptr, n, 0, out.ptr, None, None), "batched")
-    check(n, False, np.uint64, rsh.HIT_NONE)
+    rsh.check(rsh.lib().rsh_trace_rays_fused(c.handle, sc.handle, rays.ptr, M, 0, out.ptr, None, None), "batched")
+    check(M, False, np.uint64, rsh.HIT_NONE)
     sc.destroy()
     c.destroy()
