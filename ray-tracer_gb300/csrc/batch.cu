@@ -285,8 +285,8 @@ rsh_status check_batched_scene(const rsh_scene* sc) {
     return RSH_OK;
 }
 
-// lists: every segment's ids and their device counts, from ray generation (rays alone only). plain: the plain
-// path's rays alone, whatever the scenes' tuning and switch levels.
+// lists: every segment's ids and their device counts, from ray generation: rays alone, whatever the scenes' switch
+// levels. plain: the plain path's rays alone, whatever the scenes' tuning and switch levels.
 rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t count, BatchPlan& pl,
                          const SegList* lists = nullptr, bool plain = false) {
     if (!ctx || (!segs && count)) return RSH_ERR_INVALID;
@@ -319,10 +319,9 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
         return RSH_ERR_INVALID;
     }
     pl.P = ctx->cfg.packet_size;
-    for (uint32_t s = 0; s < count && !plain; ++s)
-        if (tuned_config(ctx->cfg, segs[s].scene).ray_level < segs[s].scene->h.levels) pl.rays_only = 0;
     pl.listed = lists != nullptr;
-    if (pl.listed && !pl.rays_only) return RSH_ERR_INVALID;
+    for (uint32_t s = 0; s < count && !plain && !pl.listed; ++s)
+        if (tuned_config(ctx->cfg, segs[s].scene).ray_level < segs[s].scene->h.levels) pl.rays_only = 0;
     pl.sorted = !pl.listed && (!pl.rays_only || (pl.total > SORT_RAYS && pl.total < SORT_MOST &&
                                                  !(plain && (ctx->cfg.flags & RSH_FLAG_RAH))));
     const bool packets = !pl.rays_only;

@@ -128,7 +128,7 @@ rsh_status batch_key_layout(rsh_ctx* ctx, const rsh_batch_segment* segments, uin
 bool batch_alone(const rsh_ctx* ctx, const rsh_scene* sc);
 rsh_status check_alone(rsh_ctx* ctx, const rsh_scene* sc);
 // A batched call whose segments' rays ray generation has listed (trimmed ids and their device counts) and whose
-// results it has prefilled: no hash, no sort. Every segment's rays must go alone.
+// results it has prefilled: no hash, no sort. The rays go alone.
 struct SegList {
     const uint32_t* ids;
     const uint32_t* count;  // null: every slot, ids unused

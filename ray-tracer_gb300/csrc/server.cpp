@@ -3,14 +3,14 @@
 // The reference renders one scene per GLUT frame callback (display(), main.cpp:1077-1368) with no
 // request queue. Here a host thread runs steps: every step (1) admits queued requests while their
 // device memory fits the server's HBM budget, (2) generates the current stage's rays of every in-flight
-// request (primary rays, or one bounce's shadow + reflection rays), (3) traces all of them in ONE
-// batched call (segmented hash/compress/sort/decompress, one persistent fused traversal + intersection
-// launch), (4) resolves hits and advances each request; finished requests leave and new ones join
-// between steps. Steps are enqueued without waiting for the GPU (at most two outstanding): the host
-// admits and prepares the next step while the current one runs, and retires steps in order as their
-// events complete. Ray state and results stay on the device until rsh_server_wait
-// copies them out. A request's results do not depend on what else is in the batch: its rays form their
-// own key segment, sort stably within it, and pack into work units of their own.
+// request (primary rays, or one bounce's shadow + reflection rays, from the stage before's hits), (3) traces
+// all of them in one batched call (rays alone, in the pixels' order; the requests whose scene uses packets
+// below the root in a second call, hashed and sorted); finished requests leave and new ones join between
+// steps. Steps are enqueued without waiting for the GPU (at most two outstanding): the host admits and
+// prepares the next step while the current one runs, and retires steps in order as their events complete.
+// Ray state and results stay on the device until rsh_server_wait copies them out. A request's results do not
+// depend on what else is in the batch: its rays form their own segment, listed or sorted within it, and pack
+// into work units of their own.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -155,41 +155,45 @@ void free_request(rsh_server* s, Req* q) {
 }
 
 // One step, enqueued without waiting (server thread, no lock held): generate the current stage's rays of
-// every request in `act`, trace them all in one batched call, resolve the hits into the next surfaces,
-// copy the segment counts and the device error word to the step's pinned slot and record its event.
+// every request in `act` from the stage before's hits, trace them all in one batched call (two when some scenes' rays
+// go alone and others' use packets), copy the segment counts and the device error word to the step's pinned slot and
+// record its event.
 // The host goes on admitting and enqueueing the next step while this one runs (at most kDepth steps are
 // outstanding); steps retire in order when their events complete.
 constexpr size_t kDepth = 2;
 
 rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
     cudaStream_t st = s->stream;
-    std::vector<rsh_batch_segment> segs;
-    std::vector<SegList> lists;
-    segs.reserve(rec.act.size() * 2);
-    rec.seg_at.clear();
-    // Rays alone (no scene of the step uses packets below the root): ray generation lists each segment's rays,
-    // counts them and prefills their results, so the batch neither reads the rays back to hash them nor sorts
-    // them (k_batch_prep alone was 0.9 of the 13.9 ms of kernels of a burst of 16 requests).
-    bool alone = true;
+    // How a request's rays are traced goes by its scene, not by what else is in the step (a scene's switch level may
+    // also change while its requests are in flight), so nothing a stage leaves behind depends on it: hits are resolved
+    // by the stage that needs the surface, from the stage before's hits.
+    // Rays alone: ray generation lists each segment's rays, counts them and prefills their results, so the batch
+    // neither reads the rays back to hash them nor sorts them (k_batch_prep alone was 0.9 of the 13.9 ms of kernels of
+    // a burst of 16 requests). Packets below the root: a batched call of their own, with hash, sort and hierarchy.
+    std::vector<rsh_batch_segment> segs[2];  // 0: rays alone, 1: packets
+    std::vector<SegList> lists;              // of segs[0]
+    std::vector<uint8_t> form;               // of each request: its segs
     uint64_t ids_total = 0;
+    rec.seg_at.clear();
     for (Req* q : rec.act) {
-        alone = alone && batch_alone(s->ctx, s->scenes[q->r.scene_index]);
-        if (q->stage > 0) ids_total += (uint64_t)q->r.width * q->r.height * (q->r.light_count + 1u);
+        form.push_back(batch_alone(s->ctx, s->scenes[q->r.scene_index]) ? 0 : 1);
+        if (q->stage > 0 && form.back() == 0) ids_total += (uint64_t)q->r.width * q->r.height * (q->r.light_count + 1u);
     }
     void *ids_buf = nullptr, *cnt_buf = nullptr;
     RSH_TRY(ensure(s->ctx, "step_counts", 4ull * 2 * (rec.act.size() + 1), &cnt_buf));
-    uint32_t* counts = static_cast<uint32_t*>(cnt_buf);  // per segment
-    uint32_t* ids = nullptr;
-    if (alone) {
-        RSH_TRY(ensure(s->ctx, "step_ids", 4ull * (ids_total + 1), &ids_buf));
-        ids = static_cast<uint32_t*>(ids_buf);
-        RSH_CUDA(cudaMemsetAsync(counts, 0, 4ull * 2 * rec.act.size(), st));
-    }
-    for (Req* q : rec.act) {
+    RSH_TRY(ensure(s->ctx, "step_ids", 4ull * (ids_total + 1), &ids_buf));
+    uint32_t* counts = static_cast<uint32_t*>(cnt_buf);  // per segment of segs[0]
+    uint32_t* ids = static_cast<uint32_t*>(ids_buf);
+    RSH_CUDA(cudaMemsetAsync(counts, 0, 4ull * 2 * rec.act.size(), st));
+    for (size_t k = 0; k < rec.act.size(); ++k) {
+        Req* q = rec.act[k];
         const rsh_request& r = q->r;
         const rsh_scene* sc = s->scenes[r.scene_index];
         const uint32_t W = r.width, H = r.height, npix = W * H, L = r.light_count;
-        rec.seg_at.push_back(segs.size());
+        const bool alone = form[k] == 0;
+        std::vector<rsh_batch_segment>& out = segs[form[k]];
+        rec.seg_at.push_back(out.size());
+        const uint32_t np = ((W + 7) / 8) * ((H + 7) / 8) * 64;
         if (q->stage == 0) {
             CameraP cp;
             for (int i = 0; i < 3; ++i) {
@@ -199,10 +203,9 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
                 cp.up[i] = r.camera.up[i];
             }
             RSH_CUDA(launch_raygen_primary(cp, W, H, q->prim_rays, q->prim_pix, st));
-            const uint32_t np = ((W + 7) / 8) * ((H + 7) / 8) * 64;
-            segs.push_back(rsh_batch_segment{sc, q->prim_rays, np, 0, reinterpret_cast<uint64_t*>(q->prim_hits),
-                                             nullptr});
-            lists.push_back(SegList{nullptr, nullptr});
+            out.push_back(rsh_batch_segment{sc, q->prim_rays, np, 0, reinterpret_cast<uint64_t*>(q->prim_hits),
+                                            nullptr});
+            if (alone) lists.push_back(SegList{nullptr, nullptr});
         } else {
             const uint32_t b = q->stage - 1;
             LightsP lp{};
@@ -210,17 +213,19 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
             lp.samples = 1;
             for (uint32_t l = 0; l < L; ++l)
                 for (int i = 0; i < 3; ++i) lp.pos[l][i] = r.lights[l].position[i];
+            // the stage before's rays and hits, this stage's
             const rsh_ray* prev = (b == 0) ? nullptr : q->rrays[(b - 1) & 1];
             rsh_ray* cur = q->rrays[b & 1];
             uint32_t* flags = q->flags + (size_t)b * npix * L;
             unsigned long long* hits = q->hits + (size_t)b * npix;
-            SegList shadow{nullptr, nullptr}, reflect{nullptr, nullptr};
+            const rsh_ray* before = b == 0 ? q->prim_rays : prev;
+            const unsigned long long* met = b == 0 ? q->prim_hits : hits - npix;
             if (alone) {
                 // one kernel from the stage before's hits to this stage's rays and lists, like a frame's (three of
                 // them a stage, with the surface written and read back in between: 1.5 ms of a burst of 16
                 // requests, now 0.9)
-                shadow = SegList{ids, counts + segs.size()};
-                reflect = SegList{ids + (size_t)npix * L, counts + segs.size() + 1};
+                const SegList shadow{ids, counts + out.size()};
+                const SegList reflect{ids + (size_t)npix * L, counts + out.size() + 1};
                 ids += (size_t)npix * (L + 1u);
                 BounceArgs ba{};
                 ba.w = W;
@@ -228,8 +233,8 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
                 ba.pos = sc->pos;
                 ba.nrm = sc->nrm;
                 ba.mat = sc->mat;
-                ba.rays = b == 0 ? q->prim_rays : prev;
-                ba.hits = b == 0 ? q->prim_hits : hits - npix;
+                ba.rays = before;
+                ba.hits = met;
                 ba.tiles_x = b == 0 ? (W + 7) / 8 : 0u;
                 ba.tiles_y = b == 0 ? (H + 7) / 8 : 0u;
                 ba.lights = lp;
@@ -247,7 +252,11 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
                 ba.rcount = const_cast<uint32_t*>(reflect.count);
                 ba.rhits = hits;
                 RSH_CUDA(launch_bounce(ba, false, true, false, st));
+                lists.push_back(shadow);
+                lists.push_back(reflect);
             } else {
+                RSH_CUDA(launch_resolve(sc->pos, sc->nrm, sc->mat, before, met, b == 0 ? q->prim_pix : nullptr,
+                                        b == 0 ? np : npix, q->spos, q->snrm, st));
                 HashP hp_r;
                 RSH_TRY(make_hash_params(sc, s->ctx->cfg, 0, hp_r));
                 RSH_CUDA(launch_raygen_shadow(q->spos, q->snrm, W, H, lp, s->ctx->cfg.epsilon, hp_r, q->srays, nullptr,
@@ -256,42 +265,31 @@ rsh_status enqueue_step(rsh_server* s, rsh_server::Step& rec) {
                                                s->ctx->cfg.reflect_jitter, s->ctx->cfg.seed, b, hp_r, cur, nullptr, st,
                                                RayOut{}));
             }
-            segs.push_back(rsh_batch_segment{sc, q->srays, npix * L, 1, nullptr, q->flags + (size_t)b * npix * L});
-            segs.push_back(rsh_batch_segment{sc, cur, npix, 0,
-                                             reinterpret_cast<uint64_t*>(q->hits + (size_t)b * npix), nullptr});
-            lists.push_back(shadow);
-            lists.push_back(reflect);
+            out.push_back(rsh_batch_segment{sc, q->srays, npix * L, 1, nullptr, flags});
+            out.push_back(rsh_batch_segment{sc, cur, npix, 0, reinterpret_cast<uint64_t*>(hits), nullptr});
         }
     }
-    if (alone) RSH_TRY(batch_trace_listed(s->ctx, segs.data(), lists.data(), (uint32_t)segs.size(), st));
-    else RSH_TRY(rsh_batch_trace(s->ctx, segs.data(), (uint32_t)segs.size(), st));
-    if (rec.cap < segs.size() + 1) {
+    const size_t na = segs[0].size(), total = na + segs[1].size();
+    for (size_t k = 0; k < rec.act.size(); ++k)
+        if (form[k]) rec.seg_at[k] += na;
+    if (na) RSH_TRY(batch_trace_listed(s->ctx, segs[0].data(), lists.data(), (uint32_t)na, st));
+    if (total > na) {  // (the test counters and stage timers run on over both calls)
+        if (na) RSH_TRY(batch_trace(s->ctx, segs[1].data(), (uint32_t)(total - na), st, false));
+        else RSH_TRY(rsh_batch_trace(s->ctx, segs[1].data(), (uint32_t)total, st));
+    }
+    if (rec.cap < total + 1) {
         if (rec.pinned) cudaFreeHost(rec.pinned);
         rec.pinned = nullptr;
-        rec.cap = std::max<size_t>(segs.size() + 1, 256);
+        rec.cap = std::max<size_t>(total + 1, 256);
         RSH_CUDA(cudaMallocHost(&rec.pinned, 4 * rec.cap));
     }
     // rays traced per segment (after trimming): read when the step retires
-    RSH_CUDA(cudaMemcpyAsync(rec.pinned, alone ? counts : s->ctx->bufs["b_seg_cnt"].ptr, 4 * segs.size(),
-                             cudaMemcpyDeviceToHost, st));
-    // advance: resolve hits into the next surface (rays alone: with the next stage's rays)
-    for (Req* q : rec.act) {
-        if (alone) break;
-        const rsh_request& r = q->r;
-        const rsh_scene* sc = s->scenes[r.scene_index];
-        const uint32_t W = r.width, H = r.height, npix = W * H;
-        if (q->stage == 0) {
-            const uint32_t np = ((W + 7) / 8) * ((H + 7) / 8) * 64;
-            RSH_CUDA(launch_resolve(sc->pos, sc->nrm, sc->mat, q->prim_rays, q->prim_hits, q->prim_pix, np, q->spos,
-                                    q->snrm, st));
-        } else {
-            const uint32_t b = q->stage - 1;
-            RSH_CUDA(launch_resolve(sc->pos, sc->nrm, sc->mat, q->rrays[b & 1], q->hits + (size_t)b * npix, nullptr,
-                                    npix, q->spos, q->snrm, st));
-        }
-    }
+    if (na) RSH_CUDA(cudaMemcpyAsync(rec.pinned, counts, 4 * na, cudaMemcpyDeviceToHost, st));
+    if (total > na)
+        RSH_CUDA(cudaMemcpyAsync(rec.pinned + na, s->ctx->bufs["b_seg_cnt"].ptr, 4 * (total - na), cudaMemcpyDeviceToHost,
+                                 st));
     // the device error word after this step (read, then cleared, in stream order)
-    RSH_CUDA(cudaMemcpyAsync(rec.pinned + segs.size(), s->ctx->d_err, 4, cudaMemcpyDeviceToHost, st));
+    RSH_CUDA(cudaMemcpyAsync(rec.pinned + total, s->ctx->d_err, 4, cudaMemcpyDeviceToHost, st));
     RSH_CUDA(cudaMemsetAsync(s->ctx->d_err, 0, 4, st));
     if (!rec.done) RSH_CUDA(cudaEventCreateWithFlags(&rec.done, cudaEventDisableTiming));
     RSH_CUDA(cudaEventRecord(rec.done, st));
@@ -315,7 +313,8 @@ bool retire_oldest(rsh_server* s, std::unique_lock<std::mutex>& lk, bool block) 
     // the step's segments: each request's primary stage has one, a bounce two (steps retire in order, so a
     // request's stage in this step is its count of retired stages)
     size_t total_segs = 0;
-    for (size_t k = 0; k < rec.act.size(); ++k) total_segs = rec.seg_at[k] + (rec.act[k]->stage_done == 0 ? 1 : 2);
+    for (size_t k = 0; k < rec.act.size(); ++k)
+        total_segs = std::max<size_t>(total_segs, rec.seg_at[k] + (rec.act[k]->stage_done == 0 ? 1 : 2));
     const uint32_t derr = rec.act.empty() ? 0u : rec.pinned[total_segs];
     for (size_t k = 0; k < rec.act.size(); ++k) {
         Req* q = rec.act[k];
