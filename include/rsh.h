@@ -279,7 +279,9 @@ rsh_status rsh_scene_destroy(rsh_ctx* ctx, rsh_scene* scene);
  * (NULL: the model matrix; normals renormalised), row-major, out[i] = sum_j M[4i + j] v[j] -- UpdateVertex
  * (RayTracer.cu:448-511) as main.cpp:1131-1196 drives it. Transforms apply to the pose uploaded first
  * (the rest pose), not to the previous frame's; the scene bounds and the object-sphere hierarchy are then
- * rebuilt on the GPU (replacing UpdateBoundingSphere, :513-570). */
+ * rebuilt on the GPU (replacing UpdateBoundingSphere, :513-570). The context keeps the rebuild's scratch for the
+ * next pose (about 230 bytes a triangle of the largest such scene, in rsh_bytes_allocated) as long as the HBM
+ * budget has room for it. */
 rsh_status rsh_scene_set_transforms(rsh_ctx* ctx, rsh_scene* scene, const float* model_matrices,
                                     const float* normal_matrices, uint32_t object_count, rsh_stream_t stream);
 

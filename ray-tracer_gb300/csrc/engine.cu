@@ -59,10 +59,16 @@ rsh_status cuda_status(cudaError_t e, const char* where) {
     return e == cudaErrorMemoryAllocation ? RSH_ERR_OOM : RSH_ERR_CUDA;
 }
 
+// Gives the kept build scratch back if `bytes` more would not fit the budget beside it.
+static void make_room(rsh_ctx* ctx, size_t bytes) {
+    if (ctx->allocated + bytes > ctx->budget) release_buf(ctx, ctx->build_scratch);
+}
+
 rsh_status ensure_buf(rsh_ctx* ctx, DevBuf& b, size_t bytes) {
     if (bytes == 0) bytes = 256;
     if (b.bytes >= bytes) return RSH_OK;
     const size_t want = ((bytes + (bytes >> 3)) + 255) & ~size_t(255);  // grow with 12.5% headroom
+    if (&b != &ctx->build_scratch) make_room(ctx, want - b.bytes);
     if (ctx->allocated - b.bytes + want > ctx->budget) {
         set_error("HBM budget exceeded");
         return RSH_ERR_OOM;
@@ -362,6 +368,7 @@ rsh_status rsh_destroy(rsh_ctx* ctx) {
     batch_release_ctx(ctx);
     for (const cudaEvent_t ev : ctx->tev) cudaEventDestroy(ev);
     if (ctx->side) cudaStreamDestroy(ctx->side);
+    release_buf(ctx, ctx->build_scratch);
     for (auto& kv : ctx->bufs) release_buf(ctx, kv.second);
     for (auto& b : ctx->bounce) {
         release_buf(ctx, b.shadow_rays);
@@ -584,6 +591,7 @@ rsh_status rsh_scene_upload(rsh_ctx* ctx, const rsh_scene_desc* d, rsh_scene** o
                 return RSH_ERR_INVALID;
             }
     const size_t need = T * (48ull * 2 + 48 + 4 + 4) + 64ull * d->material_count + 4096;
+    make_room(ctx, need);
     if (ctx->allocated + need > ctx->budget) {
         delete sc;
         set_error("HBM budget exceeded by the scene");
@@ -644,12 +652,8 @@ rsh_status rsh_scene_upload(rsh_ctx* ctx, const rsh_scene_desc* d, rsh_scene** o
         rsh_scene_destroy(ctx, sc);
         return cuda_status(e, "build_object_hierarchy");
     }
-    uint32_t total = 0;
-    for (uint32_t l = 0; l < sc->h.levels; ++l) total += sc->h.level_size[l];
-    // + the single-ray box tree: 2 float4 per slot (at most 2T + 8), its traversal records (224 B per node,
-    // at most T + 4 nodes) and its own copy of the triangles
-    sc->bytes = tri_bytes * 3 + 8ull * T + 48ull * total + 32ull * (2ull * T + 8) + 224ull * (T + 4) + 48ull * T +
-                sizeof(rsh_material) * sc->material_count;
+    sc->bytes = 2 * tri_bytes + 8ull * (T ? T : 1) + sizeof(rsh_material) * sc->material_count +
+                object_hierarchy_bytes(sc->h);
     ctx->allocated += sc->bytes;
     *out = sc;
     return RSH_OK;
@@ -665,7 +669,7 @@ rsh_status rsh_scene_destroy(rsh_ctx* ctx, rsh_scene* sc) {
     if (sc->pos_rest) cudaFree(sc->pos_rest);
     if (sc->nrm_rest) cudaFree(sc->nrm_rest);
     if (sc->materials) cudaFree(sc->materials);
-    if (sc->build_scratch) cudaFree(sc->build_scratch);
+    if (ctx && sc->pos_rest) release_buf(ctx, ctx->build_scratch);  // another scene that moves takes its own size
     free_object_hierarchy(sc->h);
     if (ctx && ctx->allocated >= sc->bytes) ctx->allocated -= sc->bytes;
     delete sc;
@@ -695,14 +699,17 @@ rsh_status rsh_build_object_hierarchy(rsh_ctx* ctx, rsh_scene* sc, rsh_stream_t 
         }
     }
     if (!T) RSH_CUDA(cudaDeviceSynchronize());
-    // a scene whose objects move (it has a rest pose) keeps the build's scratch for its next pose; it goes with
-    // the scene
-    const bool keep = sc->pos_rest != nullptr;
-    void* scr = sc->build_scratch;
-    if (!scr) RSH_CUDA(cudaMalloc(&scr, objh_scratch_bytes(T)));
-    if (keep) sc->build_scratch = scr;
+    // for a scene whose objects move (it has a rest pose) the context keeps the build's scratch for the next pose, if
+    // the budget has room for it
+    const bool keep = sc->pos_rest && ensure_buf(ctx, ctx->build_scratch, objh_scratch_bytes(T)) == RSH_OK;
+    void* scr = ctx->build_scratch.ptr;
+    if (!keep) RSH_CUDA(cudaMalloc(&scr, objh_scratch_bytes(T)));
+    const size_t before = object_hierarchy_bytes(sc->h);
     const cudaError_t e = build_object_hierarchy(sc->pos, T, ctx->cfg.cluster_size, sc->lo, sc->hi, sc->h, scr,
                                                  ctx->d_err, s, ctx->side, ctx->h_build);
+    const size_t after = object_hierarchy_bytes(sc->h);
+    sc->bytes += after - before;
+    ctx->allocated += after - before;
     if (!keep) cudaFree(scr);
     if (e != cudaSuccess) return cuda_status(e, "rsh_build_object_hierarchy");
     return RSH_OK;

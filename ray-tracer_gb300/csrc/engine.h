@@ -45,7 +45,6 @@ struct rsh_scene {
     uint32_t object_count = 1;
     float4* pos_rest = nullptr;  // rest pose for rsh_scene_set_transforms (kept from the first call on)
     float4* nrm_rest = nullptr;
-    void* build_scratch = nullptr;  // of a scene with a rest pose: the hierarchy build's scratch
     rsh_material* materials = nullptr;
     uint32_t material_count = 0;
     rsh::ObjHierarchy h;
@@ -64,6 +63,10 @@ struct rsh_ctx {
     uint64_t budget = 0;
     uint64_t allocated = 0;
     std::map<std::string, rsh::DevBuf> bufs;
+    // The hierarchy build's scratch, kept between the poses of scenes whose objects move (a rebuild waits for its
+    // kernels, so one serves all scenes). Counted in `allocated`; given back when the budget is short of room, and with
+    // a scene that moved.
+    rsh::DevBuf build_scratch;
     uint32_t* d_err = nullptr;
     unsigned long long* d_stats = nullptr;   // [0] node tests [1] tri tests [STAT_CAND] (ray, cluster) pairs
     uint32_t* h_pinned = nullptr;            // small pinned readback area

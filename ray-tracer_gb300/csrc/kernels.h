@@ -182,6 +182,7 @@ cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t tri_cou
                                    void* scratch, uint32_t* err, cudaStream_t s, cudaStream_t side, void* host);
 size_t objh_scratch_bytes(uint32_t tri_count);
 void free_object_hierarchy(ObjHierarchy& h);
+size_t object_hierarchy_bytes(const ObjHierarchy& h);  // what its arrays take
 
 // ---- traversal (traverse.cu)
 struct TravArgs {

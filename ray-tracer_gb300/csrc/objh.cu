@@ -460,6 +460,12 @@ void free_object_hierarchy(ObjHierarchy& h) {
     h = ObjHierarchy();
 }
 
+size_t object_hierarchy_bytes(const ObjHierarchy& h) {
+    if (!h.wtris) return 0;
+    const size_t n = h.tri_count, cap = node_capacity(h.tri_count);
+    return (16 + 4 + 32) * cap + 4 * 16 + (48 + 4) * n + 32 * (2 * n + 8) + 48 * n + 16 * REC_F4 * (size_t)h.wnode_cap;
+}
+
 cudaError_t build_object_hierarchy(const float4* positions_dev, uint32_t n, uint32_t cluster,
                                    const float lo[3], const float hi[3], ObjHierarchy& h,
                                    void* scratch, uint32_t* err, cudaStream_t s, cudaStream_t side, void* host) {
