@@ -350,7 +350,8 @@ rsh_status batch_prepare(rsh_ctx* ctx, const rsh_batch_segment* segs, uint32_t c
     if (pl.contiguous) pl.rays_all = const_cast<rsh_ray*>(segs[0].rays);
     else if (pl.gather) RSH_TRY(ensure(ctx, "b_rays", sizeof(rsh_ray) * (size_t)n, &pl.rays_all));
     else pl.rays_all = nullptr;
-    RSH_TRY(ensure(ctx, "b_counts", 64, &pl.counts));
+    // (rsh_batch_stats_get reads the last batched call's)
+    RSH_TRY(ensure(ctx, plain ? "p_counts" : "b_counts", 64, &pl.counts));
     RSH_TRY(ensure(ctx, "b_totals", 64, &pl.totals));
     pl.work = static_cast<char*>(pl.counts) + WORK_AT;
     // the segment tables, back to back as in the host's staging: one copy (6 small batches 36.4 us with three, now 35.2)
