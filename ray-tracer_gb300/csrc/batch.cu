@@ -769,7 +769,6 @@ rsh_status batch_trace(rsh_ctx* ctx, const rsh_batch_segment* segments, uint32_t
     RSH_TRY(batch_prepare(ctx, segments, count, pl));
     ctx->last_stream = stream;
     RSH_TRY(batch_enqueue(ctx, pl, stream, nullptr, reset_stats, prekeyed));
-    ctx->batch_counts_host.assign(1, pl.total);
     return RSH_OK;
 }
 

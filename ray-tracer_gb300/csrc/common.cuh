@@ -83,14 +83,6 @@ RSH_DEV uint32_t ld_acquire_u32(const uint32_t* p) {
 RSH_DEV void st_release_u32(uint32_t* p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-RSH_DEV unsigned long long ld_acquire_u64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-RSH_DEV void st_release_u64(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 RSH_DEV void st_relaxed_u32(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -236,9 +228,3 @@ RSH_DEV uint32_t spread2(uint32_t v) {  // 16 bits -> every second bit
     v = (v | (v << 1)) & 0x55555555u;
     return v;
 }
-
-// ------------------------------------------------------------------ geometry access
-// Scene triangles in cluster order: 3 float4 per triangle; w of vertex 0 carries the original id.
-struct TriSoA {
-    const float4* v;   // 3 per triangle
-};

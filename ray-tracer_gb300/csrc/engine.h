@@ -89,7 +89,6 @@ struct rsh_ctx {
     cudaEvent_t ev[16] = {};
     cudaStream_t side = nullptr;             // the object-sphere levels' build, beside the box tree's
     cudaStream_t last_stream = nullptr;
-    std::vector<uint32_t> batch_counts_host;
     uint32_t overflow_passes = 0;
     uint32_t pairs = 0;  // pairs of traversal launches so far (FusedArgs::ready_is)
     // per-stage CUDA events (RSH_FLAG_STAGE_TIMERS): pool and the (stage, start event) pairs of a frame

@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(FW * 32, RSH_FUSED_MIN_BLOCKS) k_fused(FusedAr
 // the instance without it (RSH_FLAG_SEQUENTIAL_RAYS) keeps a ray on its lane, with exact counters (1 M incoherent
 // rays 729 us, with SHARE 632; architecture frame 2.81 / 2.69 ms; Cornell frame 121 / 129 us).
 //
-// Box test (box_hit_fma): t = b * (1 / d) - o * (1 / d) as one fused multiply-add per plane, with direction
+// Box test (slab4): t = b * (1 / d) - o * (1 / d) as one fused multiply-add per plane, with direction
 // components below 1e-20 in magnitude replaced by +-1e-20 (finite reciprocals, no inf - inf), and the
 // entry / exit distances reduced with three-input min / max. The change of rounding against (b - o) / d is
 // about one ulp of the coordinates, far below the boxes' padding (1e-5 of the scene's largest coordinate),
@@ -608,15 +608,6 @@ RSH_DEV float safe_rcp(float d) {
     const float m = 1e-20f;
     return __frcp_rn(fabsf(d) < m ? copysignf(m, d) : d);
 }
-RSH_DEV bool box_hit_fma(float4 b0, float4 b1, float ix, float iy, float iz, float oix, float oiy, float oiz,
-                         float tmin, float tmax, float& tn) {
-    const float ax = __fmaf_rn(b0.x, ix, -oix), bx = __fmaf_rn(b1.x, ix, -oix);
-    const float ay = __fmaf_rn(b0.y, iy, -oiy), by = __fmaf_rn(b1.y, iy, -oiy);
-    const float az = __fmaf_rn(b0.z, iz, -oiz), bz = __fmaf_rn(b1.z, iz, -oiz);
-    tn = fmaxf(fmax3f(tmin, fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
-    const float tf = fminf(fmin3f(tmax, fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
-    return tn <= tf;
-}
 
 // Two plane distances at once: the packed FP32 fused multiply-add (fma.rn.f32x2, sm_100 and later), each
 // half rounded exactly like a scalar fma.rn.
@@ -631,9 +622,8 @@ RSH_DEV void fma2(float a0, float a1, float b, float c, float& r0, float& r1) {
 
 // Entry (near) or exit (far) distances of four children of a traversal record from one plane of each axis:
 // near: max(tmin, tx, ty, tz); far: min(tmax, tx, ty, tz), each t = plane * (1 / d) - o * (1 / d). With the
-// plane chosen by the direction's sign (the lower plane is the near one for a positive component), tx equals
-// the min (near) or the max (far) of the two planes' distances that box_hit_fma takes, so both tests decide
-// every box alike.
+// plane chosen by the direction's sign (the lower plane is the near one for a positive component), tx is the
+// smaller (near) or the larger (far) of the axis' two distances, without computing both.
 RSH_DEV void slab4(float4 px, float4 py, float4 pz, float ix, float iy, float iz, float oix, float oiy, float oiz,
                    float lim, float* t, bool near) {
     float tx[4], ty[4], tz[4];
@@ -1011,7 +1001,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
             const bool node = has && (top >> 31) != 0u;
             const uint32_t nn = __popc(__ballot_sync(0xffffffffu, node));
             const uint32_t nc = __popc(__ballot_sync(0xffffffffu, has && !node));
-                        do_nodes = nn >= nc;
+            do_nodes = nn >= nc;
         }
         if (SHARE && !do_nodes) {
             // The triangles of all the clusters at hand, spread over the lanes: one after the other per lane, the step

@@ -98,8 +98,6 @@ cudaError_t launch_raygen_refract(const float4* spos, const float4* snrm, const 
                                   uint32_t* keys, cudaStream_t s);
 cudaError_t launch_hash(const rsh_ray* rays, uint32_t n, const HashP& hp, uint32_t tag,
                         uint32_t* keys, cudaStream_t s);
-// Segmented hash for the batched form: segment s covers rays [seg_start[s], seg_start[s+1]) of the
-// concatenated ray array; tag = segment index; hash params per segment (scene bounds).
 
 // ---- trim + compress (compress.cu)
 size_t compress_scratch_bytes(uint32_t n_slots);
