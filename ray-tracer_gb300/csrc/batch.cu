@@ -655,6 +655,7 @@ rsh_status batch_enqueue(rsh_ctx* ctx, BatchPlan& pl, cudaStream_t s, char* pre_
     fa.nodes = static_cast<rsh_node*>(pl.nodes);
     hierarchy_capacity(pl.max_padded, pl.P, fa.node_off);
     fa.packet = pl.P;
+    for (const FusedSeg& f : pl.h_fsegs) fa.ray_level = std::max(fa.ray_level, f.ray_level);
     fa.rays = static_cast<rsh_ray*>(pl.rays_all);
     fa.sorted_ids = static_cast<uint32_t*>(pl.padded);
     fa.segs = static_cast<FusedSeg*>(pl.fsegs);

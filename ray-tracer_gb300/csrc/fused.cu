@@ -314,11 +314,14 @@ RSH_DEV void refresh_packets(FusedSmem<P>& S, bool any, uint32_t q, uint32_t ch,
     }
 }
 
-#ifndef RSH_FUSED_MIN_BLOCKS
-#define RSH_FUSED_MIN_BLOCKS 5
-#endif
-template <int P>
-__global__ void __launch_bounds__(FW * 32, RSH_FUSED_MIN_BLOCKS) k_fused(FusedArgs a) {
+// MB: CTAs per SM that the registers must allow. Packets that stay together to the clusters or nearly (a switch level of
+// PACKETS_DEEP or lower in every segment) are a few long chains of node steps: 4 CTAs, 124 registers, no spills. Above
+// that the jobs of single rays want the fifth (96 registers, spills). 5 / 4: level 0, 2000 incoherent rays 63.7 / 59.4
+// ms, 60,000 67.9 / 62.4, soup frame 640x360 128.7 / 118.9; level 2, the frame 8.0 / 7.2; level 3, the 1080p soup frame
+// 9.2 / 8.7, 1 M incoherent rays 5.33 / 5.45; level 6, 4.41 / 4.42 and 1.90 / 2.07.
+constexpr uint32_t PACKETS_DEEP = 2;
+template <int P, int MB>
+__global__ void __launch_bounds__(FW * 32, MB) k_fused(FusedArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FusedSmem<P>& S = reinterpret_cast<FusedSmem<P>*>(smem_raw)[threadIdx.x >> 5];
     const uint32_t lane = lane_id();
@@ -1222,18 +1225,19 @@ static cudaError_t launch_fused_rays_u(const FusedArgs& a, cudaStream_t s) {
 template <int P>
 static cudaError_t launch_fused_p(const FusedArgs& a, cudaStream_t s) {
     const size_t smem = sizeof(FusedSmem<P>) * FW;
-    cudaError_t e = cudaFuncSetAttribute(k_fused<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = a.ray_level <= PACKETS_DEEP ? k_fused<P, 4> : k_fused<P, 5>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 152, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<P>, FW * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FW * 32, smem);
     if (per_sm < 1) per_sm = 1;
     if (a.blocks_per_sm && (int)a.blocks_per_sm < per_sm) per_sm = (int)a.blocks_per_sm;
     uint32_t grid = (uint32_t)(sms * per_sm);
     const uint32_t need = (a.units_max + FW - 1) / FW;
     if (need < grid) grid = need > 0 ? need : 1;
-    k_fused<P><<<grid, FW * 32, smem, s>>>(a);
+    kernel<<<grid, FW * 32, smem, s>>>(a);
     note_launch();
     return cudaGetLastError();
 }

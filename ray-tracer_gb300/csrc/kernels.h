@@ -258,6 +258,7 @@ struct FusedArgs {
     const rsh_node* nodes;
     uint32_t node_off[4];
     uint32_t packet;
+    uint32_t ray_level;            // packet kernel: the segments' highest switch level
     const rsh_ray* rays;
     const uint32_t* sorted_ids;    // packet kernel
     const FusedSeg* segs;          // device; rays-only: count already folded into n
