@@ -5,12 +5,13 @@ Workload (default): the procedural-architecture scene (40x40 tessellated pillars
 1,010,240 triangles), 1920x1080, 4 point lights, depth 2 (shadow + cosine-lobe-perturbed reflection per
 bounce), FP32, seeded synthetic input. One step = one frame through rsh_render_frame.
 
-  value       secondary rays traced (after trimming) / GPU time from the first secondary ray generation to
-              the last secondary intersection of each frame (CUDA events on the frame's stream), through
-              rsh_render_frame in its batched form (RSH_FLAG_FUSED: per bounce one segmented hash/sort and
-              one persistent fused traversal + intersection launch)
-  plain       the same frames through the plain per-frame path (separate traversal -> candidates ->
-              intersection kernels, as the reference's wrappers); identical results
+  value       secondary rays traced (after trimming) / GPU time from the kernel that resolves the primary hits
+              and generates the first secondary rays to the packed image of each frame (CUDA events on the
+              frame's stream), through rsh_render_frame in its batched form (RSH_FLAG_FUSED: per bounce one
+              kernel of shading, hit resolve and ray generation, and a pair of persistent traversal +
+              intersection launches)
+  plain       the same frames through the plain per-frame path (the same kernels; it counts (ray, cluster)
+              pairs, too); identical results
   e2e         the same metric through the C ABI with host buffers: camera + lights from host structs in,
               the RGBA8 frame copied to pinned host memory, both inside the timed region
   roofline    the dominant kernel's achieved rate against its roofline (per-stage CUDA events)

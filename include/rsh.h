@@ -397,7 +397,7 @@ rsh_status rsh_raygen_refract(const float* surface_pos, const float* surface_nrm
 rsh_status rsh_hash(const rsh_ray* rays, uint32_t n, const rsh_hash_params* hp, uint32_t tag,
                     uint32_t* keys, rsh_stream_t stream);
 
-/* Trim + compress (reduce-then-scan over 4096-slot tiles): keeps slots whose key != RSH_KEY_NONE in slot
+/* Trim + compress (reduce-then-scan): keeps slots whose key != RSH_KEY_NONE in slot
  * order (trimmed_ids = their slot indices), and cuts the trimmed keys into runs of equal keys.
  * Outputs chunk_keys[c], chunk_bases[c] (trimmed index of the run head; chunk_bases[C] = R) and, if
  * non-NULL, chunk_sizes[c]; counts[0] = R (rays), counts[1] = C (chunks), device memory.
@@ -410,7 +410,7 @@ rsh_status rsh_compress(rsh_ctx* ctx, const uint32_t* keys, uint32_t n_slots, ui
 /* rsh_compress without allocating: same outputs and semantics, no context, no cudaMalloc/cudaFree.
  * For callers that may not allocate device memory themselves or let a library do it: hosts that own and
  * pre-partition all device memory, and loops that allocate once at start-up and must not allocate while
- * they run. No counterpart in the reference. The scratch (per-tile summaries and prefixes) is a static
+ * they run. No counterpart in the reference. The scratch (summaries of slot ranges) is a static
  * device array of 196,684 bytes that every GPU loading the library keeps until the process exits;
  * n_slots above 16,777,216 is rejected with RSH_ERR_INVALID. The
  * first call on a device looks up the array's device address (call it once before any stream capture);
@@ -499,10 +499,11 @@ typedef struct rsh_batch_segment {
     uint32_t* flags;    /* shadow output (any_hit != 0) */
 } rsh_batch_segment;
 
-/* Traces many ray batches of uneven size over several resident scenes in ONE persistent fused traversal +
- * intersection launch. Up to two million rays are traced in their own order; more are hashed and sorted first
- * (the segment index is the key's tag). With packets below the root (ray_level below a scene's tree depth): one
- * hash, one compress, one sort and one decompress over all segments, one hierarchy build, then the launch.
+/* Traces many ray batches of uneven size over several resident scenes in one persistent traversal +
+ * intersection launch, or two side by side when closest-hit and any-hit segments are mixed. Up to two million
+ * rays are traced in their own order; more are hashed and sorted first (the segment index is the key's tag; from
+ * 2^30 slots on they keep their order, too). With packets below the root (ray_level below a scene's tree depth):
+ * one hash, one compress, one sort and one decompress over all segments, one hierarchy build, then one launch.
  * Without host synchronisation, so the whole call can be captured in a CUDA graph (rsh_batch_graph_*). */
 rsh_status rsh_batch_trace(rsh_ctx* ctx, const rsh_batch_segment* segments, uint32_t count,
                            rsh_stream_t stream);
@@ -517,7 +518,9 @@ rsh_status rsh_batch_graph_destroy(void* graph_exec);
 rsh_status rsh_batch_stats_get(rsh_ctx* ctx, rsh_frame_stats* out);
 
 /* Autotuner: times rsh_batch_trace on `segments` for each (grid_bits, dir_log2, packet_size) in the
- * given lists and stores the fastest in the context's configuration (and in *best). */
+ * given lists and stores the fastest in the context's configuration (and in *best). Rays alone from the root (the
+ * default ray_level) read the packet size never and the hash widths only above two million rays: below, the
+ * combinations time alike, and one of them is stored. */
 rsh_status rsh_autotune(rsh_ctx* ctx, const rsh_batch_segment* segments, uint32_t count,
                         const uint32_t* grid_bits, uint32_t n_grid, const uint32_t* dir_log2,
                         uint32_t n_dir, const uint32_t* packet_sizes, uint32_t n_packet,

@@ -3,10 +3,12 @@
 // The reference has no batched path: every batch is a host loop of wrappers with a blocking count
 // readback after each stage (main.cpp:951-1054, RayTracer.cu:2316-2832). Here, for S segments:
 // Rays alone (switch level at or above every segment's tree depth, the default):
-//   up to SORT_RAYS rays, they are traced as they come, in ONE launch that also writes the misses of empty
+//   up to SORT_RAYS rays, they are traced as they come, by a launch that also writes the misses of empty
 //   slots; above that they are hashed (k_batch_prep), sorted by key -- the slots themselves, the last pass
 //   leaving each segment's trimmed ids -- and k_batch_units gives each segment its range and its work units.
-//   No run compression: the traversal reads ids, and runs of incoherent rays hardly repeat.
+//   No run compression: the traversal reads ids, and runs of incoherent rays hardly repeat. Closest-hit and
+//   any-hit segments are a launch each, side by side. Rays that ray generation has listed (frames, the server)
+//   are traced by their lists, without hash or sort.
 // Packets below the root (k_fused):
 //   k_batch_prep     one pass over all rays: key = segment << shift | hash (per-segment scene box),
 //                    pre-fill each segment's output, count each segment's rays (shared-memory counters,
@@ -254,10 +256,13 @@ constexpr size_t WORK_AT = 32;
 static_assert(sizeof(PrepSeg) % 8 == 0 && sizeof(FusedSeg) % 8 == 0, "the tables lie back to back");
 size_t table_bytes(uint32_t nseg) { return (sizeof(PrepSeg) + sizeof(FusedSeg) + 4ull) * nseg + 256; }
 
-// Rays at or below this count are traced in their own order. Sorting incoherent rays makes their traversal 11-13%
-// shorter (their nodes are in the L1 more often), whatever their number; the hash and the sort cost 0.10 ms for
-// 1.3 M rays in 8 segments (traversal 0.526 against 0.587 ms then), 0.5 ms for 13.8 M in 64 (all of it 3.86 ms
-// sorted, 4.19 unsorted).
+// Rays at or below this count are traced in their own order. Sorting incoherent rays makes their traversal 15-23%
+// shorter (their nodes are in the L1 more often), whatever their number; the hash, the sort and the tables cost a
+// small batch more than that. Whole calls of closest-hit surface rays, own order / sorted, us, over 320,000 and 12,000
+// triangles (the line lies between where one segment and where sixteen break even):
+//   one segment       1 M 638 / 631  294 / 295   1.5 M  916 /  884   425 / 413   2 M 1195 / 1134   552 / 518
+//   sixteen segments  1 M 658 / 692  309 / 340   2 M   1233 / 1238   573 / 586   3 M 1805 / 1792   839 / 834
+//   one segment, 13.8 M 7759 / 6508 and 3573 / 2961; sixteen, 7967 / 7392 and 3678 / 3262
 constexpr uint32_t SORT_RAYS = 2000000;
 // From this many slots on they are traced in their own order, too: a digit's count in the sort has 30 bits, and without
 // run compression one digit may have them all.
