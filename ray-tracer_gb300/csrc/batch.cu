@@ -694,7 +694,7 @@ rsh_status trace_alone(rsh_ctx* ctx, const rsh_scene* sc, const rsh_ray* rays, u
                        uint32_t* ready) {
     FusedArgs fa = alone_args(ctx, ticket);
     fa.pair = pair;
-    if (pair == 1u) ++ctx->pairs;
+    if (pair == 1u && ++ctx->pairs == 0u) ctx->pairs = 1u;  // (0: no pair has started)
     fa.ready = ready;
     fa.ready_is = ctx->pairs;
     fa.wait = pair != 2u ? 1u : 0u;  // behind the kernel that generated its rays
