@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(FW * 32, SHARE ? RSH_RAYS_MIN_BLOCKS : 7) k_fu
     // The second of a pair reads what the kernel before the first wrote, and does not wait for the first itself. That
     // its CTAs start only after the first's wait does not make those writes visible to them (a trigger orders
     // nothing): the first releases a word after its wait, before its trigger, and the second acquires it -- at the
-    // first look, as a rule.
+    // first look, as a rule (a Cornell frame of 512x512 pixels 105.5 us without the word, 106-107 with it).
     if (ONE && a.ready) {
         bool late = false;
         if (threadIdx.x == 0) {
